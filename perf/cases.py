@@ -260,6 +260,133 @@ def run(state):
     return packed, mld.pack_scales(scale, True), sums
 
 
+# ------------------------------------------------------------------------ the same in 64 bits, by plain torch
+def _over(a, b):
+    """a / b, rounded once (with a plain number on either side torch multiplies by a reciprocal instead)"""
+    return torch.div(*(t if torch.is_tensor(t) else torch.tensor(t, device="cuda") for t in (a, b)))
+
+
+def _quantised(w, bits, block):
+    """(integers, scales [n][groups]): the largest magnitude of a row or block maps to 127 (7), halves round to even."""
+    n, k = w.shape
+    blocks = w.reshape(n, -1, block if bits == 4 and block else k)
+    top = 127.0 if bits == 8 else 7.0
+    scale = _over(blocks.abs().amax(-1), top)
+    scale = torch.where(scale == 0, torch.ones_like(scale), scale)
+    return torch.round(blocks / scale[..., None]).clamp_(-top - 1, top).to(torch.int8), scale
+
+
+def _weights64(gen, n, k, bits, block, dtype, zero_point=False):
+    """The [n][k] weights that the packed tensors stand for, drawn as _symmetric and _asymmetric draw them."""
+    w = _randn(gen, n, k).mul_(0.02)
+    if not zero_point:
+        q, scale = _quantised(w, bits, block)
+        return (q.double() * scale.to(dtype).double()[..., None]).reshape(n, k)
+    w = w.reshape(n, -1, block or k)
+    low, high = w.amin(-1, keepdim=True), w.amax(-1, keepdim=True)
+    top, offset = 2 ** bits - 1, 2 ** (bits - 1)
+    scale = (high - low) / top
+    zero = torch.round(-low / scale) - offset
+    q = torch.clamp(torch.round(w / scale) + zero, -offset, offset - 1)
+    return ((q.double() - zero.to(dtype).double()) * scale.to(dtype).double()).reshape(n, k)
+
+
+def _rows(x, channels):
+    """[slices][tokens][4] -> [tokens][channels]"""
+    return x.permute(1, 0, 2).reshape(x.shape[1], -1)[:, :channels]
+
+
+def _sliced(y):
+    """[tokens][channels] -> [slices][tokens][4], zeros in the padded channels"""
+    y = torch.nn.functional.pad(y, (0, -y.shape[1] % 4))
+    return y.reshape(y.shape[0], -1, 4).permute(1, 0, 2).contiguous()
+
+
+def _act_quantised(x, symmetric):
+    """The value that each activation stands for after its quantisation to 8 bits per token (a 32-bit rule)."""
+    x = x.float()
+    if symmetric:
+        inv = torch.clamp(_over(x.abs().amax(1, keepdim=True), 127.0), min=2.0 ** -14)
+        q = torch.floor(x * _over(1.0, inv) + 128.5).clamp(0, 255) - 128
+        return q.double() * inv.double()
+    low, high = x.amin(1, keepdim=True), x.amax(1, keepdim=True)
+    span = high - low
+    q = ((x - low) * _over(255.0, span) + 0.5).to(torch.int32).clamp(0, 255) - 128
+    return q.double() * _over(span, 255.0).double() + (low + span * (128.0 / 255.0)).double()
+
+
+def _exact_fc(c, gen):
+    dtype = torch.float32 if c["precision"] == "f32" else torch.float16
+    w = _weights64(gen, c["n"], c["k"], c["bits"], c["block"], dtype, c["zero_point"])
+    bias = _randn(gen, c["n"]).mul_(0.01).to(dtype).double() if c["bias"] else 0.0
+    x = _rows(_activations(gen, c["k"], c["tokens"], dtype), c["k"])
+    x = _act_quantised(x, c["act_quant"] == 1) if c["act_quant"] and c["tokens"] > 8 else x.double()
+    return _sliced(x @ w.T + bias)
+
+
+def _rope64(v, pos):
+    half = v.shape[-1] // 2
+    angle = pos / 1.0e6 ** (torch.arange(half, dtype=torch.float64, device=v.device) / half)
+    c, s, a, b = torch.cos(angle), torch.sin(angle), v[..., :half], v[..., half:]
+    return torch.cat((a * c - b * s, b * c + a * s), -1)
+
+
+def _attend64(q, k, v):
+    """q [heads][128], k and v [tokens][heads][128]"""
+    return torch.einsum("ht,thd->hd", torch.softmax(torch.einsum("hd,thd->ht", q, k), 1), v)
+
+
+def _exact_decoder(c, gen):
+    heads, ffn, layers, pos = c["heads"], c["ffn"], c["layers"], c["pos"]
+    d = heads * 128
+    k_cache = _randn(gen, layers, c["max_seq"], d).half().double()
+    v_cache = _randn(gen, layers, c["max_seq"], d).half().double()
+    stack = []
+    for _ in range(layers):
+        weights = [_quantised(_randn(gen, n, k).mul_(0.02), 4, c["block"])
+                   for n, k in ((3 * d, d), (d, d), (2 * ffn, d), (d, ffn))]
+        stack.append((weights, [(1.0 + 0.1 * _randn(gen, d)).half().double() for _ in range(2)]))
+    x = _randn(gen, d).half().double()
+
+    def project(weight, v):
+        q, scale = weight
+        return (q.double() * scale.half().double()[..., None]).reshape(q.shape[0], -1) @ v
+
+    def norm(v, gamma):
+        return v * torch.rsqrt(v.square().mean() + 1e-6) * gamma
+
+    for layer, ((qkv, o, gate_up, down), (gamma1, gamma2)) in enumerate(stack):
+        q, k, v = project(qkv, norm(x, gamma1)).reshape(3, heads, 128)
+        k_cache[layer, pos], v_cache[layer, pos] = _rope64(k, pos).reshape(-1), v.reshape(-1)
+        keys, values = (t[layer, :pos + 1].reshape(pos + 1, heads, 128) for t in (k_cache, v_cache))
+        x = x + project(o, _attend64(_rope64(q, pos) / math.sqrt(128), keys, values).reshape(-1))
+        gate, up = project(gate_up, norm(x, gamma2)).reshape(ffn, 2).T  # rows alternate gate, up
+        x = x + project(down, torch.nn.functional.silu(gate) * up)
+    return (x.cpu() if c["host"] else x), k_cache, v_cache
+
+
+def exact(case, seed):
+    gen = _generator(seed)
+    c, kind = case, case["kind"]
+    if kind == "fc":
+        return _exact_fc(c, gen)
+    if kind == "vocabulary":
+        w = _weights64(gen, c["vocab"], c["dim"], c["bits"], c["block"], torch.float16)
+        ids = torch.randint(0, c["vocab"], (c["tokens"],), generator=gen, device="cuda", dtype=torch.int32)
+        hidden = _rows(_activations(gen, c["dim"], 1, torch.float16), c["dim"]).double()
+        return w[ids.long()], _sliced(hidden @ w.T)
+    if kind == "decoder":
+        return _exact_decoder(c, gen)
+    if kind == "attention":
+        q = (_randn(gen, c["heads"], 128) / math.sqrt(128)).half().double()
+        k, v = (_randn(gen, c["tokens"], c["heads"], 128).half().double() for _ in range(2))
+        return _attend64(q, k, v)
+    w = _randn(gen, c["n"], c["k"]).mul_(0.02).double()
+    bound = w.reshape(c["n"], -1, c["block"] if c["bits"] == 4 and c["block"] else c["k"]).abs().amax(-1)
+    scale = torch.nn.functional.pad(bound / (127.0 if c["bits"] == 8 else 7.0), (0, 0, 0, -c["n"] % 4))
+    return None, scale.T.contiguous(), None  # (the other two are whole numbers)
+
+
 # --------------------------------------------------------------------------- what a pass cannot do without
 def _weights_bytes(n, k, bits, block, element, zero_point=False):
     n4, k4 = -(-n // 4) * 4, -(-k // 4) * 4
