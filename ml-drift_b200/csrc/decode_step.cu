@@ -15,7 +15,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -77,109 +76,184 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_kernel(const __half* __restr
   }
 }
 
-// Decode attention for one query token, split over the cached tokens.
-// grid (heads, splits), 128 threads.  Eight lanes share a token (16 dims each);
-// every 8-lane group keeps its own running max / sum / output and the groups
-// are merged at the end.  head_dim is fixed at 128.  Partial results:
-// part_o [heads][splits][128] fp32, part_ml [heads][splits][2] (max, sum).
 constexpr int kHeadDim = 128;
-__global__ void __launch_bounds__(128) attn_decode_kernel(const __half* __restrict__ q, const __half* __restrict__ kcache,
-                                                          const __half* __restrict__ vcache, float* __restrict__ part_o,
-                                                          float* __restrict__ part_ml, int heads, int n_tokens,
-                                                          int splits) {
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Stores one float at `local` (a shared-memory address of this CTA) in the cluster's CTA 0.
+__device__ __forceinline__ void st_cta0_f32(const float* local, float v) {
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, 0;\n\tst.shared::cluster.f32 [r], %1;\n\t}"
+      ::"r"(smem_u32(local)), "f"(v)
+      : "memory");
+}
+
+// Decode attention for one query token over a KV cache of n_tokens rows, head_dim 128.  Bound by the K and V bytes
+// (32 heads x 8191 tokens: 134 MB, 20.5 us at the measured copy rate), so the kernel keeps them in flight: eight
+// lanes share a token (two 16-byte pieces of its row each, dims 8 sub + {0..7} and 64 + 8 sub + {0..7}, so that a
+// warp's load covers whole 128-byte lines), a lane asks for the K and V pieces of kAttnAhead tokens at once
+// (256 bytes) and folds them into its running max / sum / output with one rescale.
+// A cluster of up to 16 CTAs shares a head and cuts its tokens into even parts; the parts' results meet in the shared
+// memory of the cluster's first CTA, so no scratch in global memory and no second kernel are needed, and calls on
+// several streams share nothing.  32 heads x 8191 tokens, launch after launch: 32.0 us (48.0 with K, then V a token at a
+// time and a launch of its own for the merge).
+constexpr int kAttnAhead = 4;
+constexpr int kMaxAttnParts = 16;
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+    attn_decode_kernel(const __half* __restrict__ q, const __half* __restrict__ kcache, const __half* __restrict__ vcache,
+                       __half* __restrict__ out, int heads, int n_tokens, int parts) {
+  __shared__ float warp_ml[WARPS][2], warp_o[WARPS][kHeadDim];
+  __shared__ float part_ml[kMaxAttnParts][2], part_o[kMaxAttnParts][kHeadDim];  // used in the cluster's CTA 0
   pdl_wait();
   pdl_launch_dependents();
-  const int head = blockIdx.x, split = blockIdx.y;
-  const int per = (n_tokens + splits - 1) / splits;
-  const int t0 = split * per, t1 = min(n_tokens, t0 + per);
-  const int grp = threadIdx.x >> 3, sub = threadIdx.x & 7;  // 16 groups of 8 lanes
-  const int width = heads * kHeadDim;
+  if (parts > 1) cluster_arrive();  // (waited for before the first store into CTA 0)
+  const int head = blockIdx.x / parts, part = blockIdx.x - head * parts;
+  const int t0 = static_cast<int>((int64_t)n_tokens * part / parts), t1 = static_cast<int>((int64_t)n_tokens * (part + 1) / parts);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
+  const size_t width = (size_t)heads * kHeadDim;
   float qv[16];
   {
-    const __half* qp = q + (size_t)head * kHeadDim + sub * 16;
+    const __half* qp = q + (size_t)head * kHeadDim + sub * 8;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) qv[j] = __half2float(qp[j]);
+    for (int j = 0; j < 8; ++j) {
+      qv[j] = __half2float(qp[j]);
+      qv[8 + j] = __half2float(qp[64 + j]);
+    }
   }
+  const __half* kbase = kcache + (size_t)head * kHeadDim + sub * 8;
+  const __half* vbase = vcache + (size_t)head * kHeadDim + sub * 8;
   float m = -INFINITY, l = 0.0f, acc[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) acc[j] = 0.0f;
-  const unsigned gmask = 0xFFu << (threadIdx.x & 24);
-  for (int t = t0 + grp; t < t1; t += 16) {
-    const uint4* kp = reinterpret_cast<const uint4*>(kcache + (size_t)t * width + head * kHeadDim + sub * 16);
-    const uint4 k0 = kp[0], k1 = kp[1];
-    const __half2* kh = reinterpret_cast<const __half2*>(&k0);
-    const __half2* kh2 = reinterpret_cast<const __half2*>(&k1);
-    float s = 0.0f;
+  constexpr int kStep = WARPS * 4;  // tokens between two of a lane's
+  // (whole warps stay in the loop together: the lanes of tokens past the end repeat the part's last token, unweighted)
+  for (int tw = t0 + warp * 4; tw < t1; tw += kStep * kAttnAhead) {
+    uint4 kr[kAttnAhead][2], vr[kAttnAhead][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 a = __half22float2(kh[j]), b = __half22float2(kh2[j]);
-      s += qv[2 * j] * a.x + qv[2 * j + 1] * a.y + qv[8 + 2 * j] * b.x + qv[8 + 2 * j + 1] * b.y;
+    for (int u = 0; u < kAttnAhead; ++u) {
+      const size_t row = (size_t)min(tw + u * kStep + grp, t1 - 1) * width;
+      kr[u][0] = __ldcs(reinterpret_cast<const uint4*>(kbase + row));
+      kr[u][1] = __ldcs(reinterpret_cast<const uint4*>(kbase + row + 64));
     }
-    // the eight lanes of a token group run this loop together; other groups of
-    // the warp may have a different trip count, so the shuffle names only them
-    s += __shfl_xor_sync(gmask, s, 1);
-    s += __shfl_xor_sync(gmask, s, 2);
-    s += __shfl_xor_sync(gmask, s, 4);
-    const float m_new = fmaxf(m, s);
-    const float corr = __expf(m - m_new), p = __expf(s - m_new);
-    const uint4* vp = reinterpret_cast<const uint4*>(vcache + (size_t)t * width + head * kHeadDim + sub * 16);
-    const uint4 v0 = vp[0], v1 = vp[1];
-    const __half2* vh = reinterpret_cast<const __half2*>(&v0);
-    const __half2* vh2 = reinterpret_cast<const __half2*>(&v1);
-    l = l * corr + p;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 a = __half22float2(vh[j]), b = __half22float2(vh2[j]);
-      acc[2 * j] = acc[2 * j] * corr + p * a.x;
-      acc[2 * j + 1] = acc[2 * j + 1] * corr + p * a.y;
-      acc[8 + 2 * j] = acc[8 + 2 * j] * corr + p * b.x;
-      acc[8 + 2 * j + 1] = acc[8 + 2 * j + 1] * corr + p * b.y;
+    for (int u = 0; u < kAttnAhead; ++u) {
+      const size_t row = (size_t)min(tw + u * kStep + grp, t1 - 1) * width;
+      vr[u][0] = __ldcs(reinterpret_cast<const uint4*>(vbase + row));
+      vr[u][1] = __ldcs(reinterpret_cast<const uint4*>(vbase + row + 64));
     }
-    m = m_new;
-  }
-  // merge the 16 groups
-  __shared__ float sm_m[16], sm_l[16], sm_o[16][kHeadDim];
-  if (sub == 0) {
-    sm_m[grp] = m;
-    sm_l[grp] = l;
-  }
+    if (tw + (kAttnAhead - 1) * kStep + 4 > t1) {  // the last round: what stands in for missing tokens must weigh nothing
 #pragma unroll
-  for (int j = 0; j < 16; ++j) sm_o[grp][sub * 16 + j] = acc[j];
+      for (int u = 0; u < kAttnAhead; ++u)
+        if (tw + u * kStep + grp >= t1) vr[u][0] = vr[u][1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    float s[kAttnAhead];
+#pragma unroll
+    for (int u = 0; u < kAttnAhead; ++u) {
+      float d[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const __half2* kh = reinterpret_cast<const __half2*>(&kr[u][h]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __half22float2(kh[j]);
+          d[0] = fmaf(qv[8 * h + 2 * j], f.x, d[0]);
+          d[1] = fmaf(qv[8 * h + 2 * j + 1], f.y, d[1]);
+        }
+      }
+      s[u] = d[0] + d[1];
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1)
+#pragma unroll
+      for (int u = 0; u < kAttnAhead; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], off);
+    float m_new = m;
+#pragma unroll
+    for (int u = 0; u < kAttnAhead; ++u) {
+      if (tw + u * kStep + grp >= t1) s[u] = -INFINITY;
+      m_new = fmaxf(m_new, s[u]);
+    }
+    if (tw + grp < t1) {  // (a lane group without a token keeps its empty state)
+      const float corr = __expf(m - m_new);
+      l *= corr;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) acc[j] *= corr;
+      m = m_new;
+#pragma unroll
+      for (int u = 0; u < kAttnAhead; ++u) {
+        const float p = __expf(s[u] - m_new);
+        l += p;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const __half2* vh = reinterpret_cast<const __half2*>(&vr[u][h]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(vh[j]);
+            acc[8 * h + 2 * j] = fmaf(p, f.x, acc[8 * h + 2 * j]);
+            acc[8 * h + 2 * j + 1] = fmaf(p, f.y, acc[8 * h + 2 * j + 1]);
+          }
+        }
+      }
+    }
+  }
+  // the warp's four lane groups
+  {
+    float gm = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+    gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, 16));
+    const float w = m == -INFINITY ? 0.0f : __expf(m - gm);
+    l *= w;
+    l += __shfl_xor_sync(0xffffffffu, l, 8);
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      acc[j] *= w;
+      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 8);
+      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
+    }
+    if (grp == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        warp_o[warp][sub * 8 + j] = acc[j];
+        warp_o[warp][64 + sub * 8 + j] = acc[8 + j];
+      }
+    }
+    if (lane == 0) {
+      warp_ml[warp][0] = gm;
+      warp_ml[warp][1] = l;
+    }
+  }
   __syncthreads();
-  float gm = -INFINITY;
+  const int dim = threadIdx.x;  // the first 128 threads own an output dim each
+  float gm = -INFINITY, o = 0.0f, ls = 0.0f;
+  if (dim < kHeadDim) {
 #pragma unroll
-  for (int g = 0; g < 16; ++g) gm = fmaxf(gm, sm_m[g]);
-  const int dim = threadIdx.x;  // 128 threads, one output dim each
-  float o = 0.0f, lsum = 0.0f;
+    for (int w = 0; w < WARPS; ++w) gm = fmaxf(gm, warp_ml[w][0]);
 #pragma unroll
-  for (int g = 0; g < 16; ++g) {
-    const float w = sm_m[g] == -INFINITY ? 0.0f : __expf(sm_m[g] - gm);
-    o += w * sm_o[g][dim];
-    lsum += w * sm_l[g];
+    for (int w = 0; w < WARPS; ++w) {
+      const float f = warp_ml[w][0] == -INFINITY ? 0.0f : __expf(warp_ml[w][0] - gm);
+      o = fmaf(f, warp_o[w][dim], o);
+      ls = fmaf(f, warp_ml[w][1], ls);
+    }
   }
-  part_o[((size_t)head * splits + split) * kHeadDim + dim] = o;
-  if (dim == 0) {
-    part_ml[((size_t)head * splits + split) * 2 + 0] = gm;
-    part_ml[((size_t)head * splits + split) * 2 + 1] = lsum;
+  if (parts > 1) {
+    cluster_wait();  // every CTA of the cluster has started
+    if (dim < kHeadDim) {
+      st_cta0_f32(&part_o[part][dim], o);
+      if (dim < 2) st_cta0_f32(&part_ml[part][dim], dim == 0 ? gm : ls);
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (part != 0 || dim >= kHeadDim) return;
+    gm = -INFINITY;
+    for (int c = 0; c < parts; ++c) gm = fmaxf(gm, part_ml[c][0]);
+    o = ls = 0.0f;
+    for (int c = 0; c < parts; ++c) {
+      const float f = part_ml[c][0] == -INFINITY ? 0.0f : __expf(part_ml[c][0] - gm);
+      o = fmaf(f, part_o[c][dim], o);
+      ls = fmaf(f, part_ml[c][1], ls);
+    }
   }
-}
-
-__global__ void __launch_bounds__(128) attn_combine_kernel(const float* __restrict__ part_o,
-                                                           const float* __restrict__ part_ml, __half* __restrict__ out,
-                                                           int splits) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int head = blockIdx.x, dim = threadIdx.x;
-  float gm = -INFINITY;
-  for (int s = 0; s < splits; ++s) gm = fmaxf(gm, part_ml[((size_t)head * splits + s) * 2]);
-  float o = 0.0f, l = 0.0f;
-  for (int s = 0; s < splits; ++s) {
-    const float ms = part_ml[((size_t)head * splits + s) * 2];
-    const float w = ms == -INFINITY ? 0.0f : __expf(ms - gm);
-    o += w * part_o[((size_t)head * splits + s) * kHeadDim + dim];
-    l += w * part_ml[((size_t)head * splits + s) * 2 + 1];
-  }
-  out[(size_t)head * kHeadDim + dim] = __float2half_rn(o / l);
+  if (dim < kHeadDim) out[(size_t)head * kHeadDim + dim] = __float2half_rn(o / ls);
 }
 
 // The decoder's attention node in one launch: rotary embedding of q and of the
@@ -390,21 +464,48 @@ int attn_splits(int heads, int sms) {
   return splits;
 }
 
-int launch_attn_decode(const __half* q, const __half* kcache, const __half* vcache, float* part_o, float* part_ml,
-                       __half* out, int heads, int n_tokens, int splits, cudaStream_t stream) {
-  int rc = launch_glue(attn_decode_kernel, dim3(heads, splits), dim3(128), stream, q, kcache, vcache, part_o, part_ml,
-                       heads, n_tokens, splits);
-  if (rc != MLD_OK) return rc;
-  return launch_glue(attn_combine_kernel, dim3(heads), dim3(128), stream, part_o, part_ml, out, splits);
+template <int WARPS>
+int launch_attn_decode_t(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
+                         int parts, cudaStream_t stream) {
+  auto kern = attn_decode_kernel<WARPS>;
+  static bool configured[kMaxDevices];
+  int dev;
+  if (needs_configure(configured, &dev)) {
+    MLD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (dev >= 0) configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(heads) * parts);
+  cfg.blockDim = dim3(WARPS * 32);
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = parts;
+  attrs[1].val.clusterDim.y = 1;
+  attrs[1].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = parts > 1 ? 2 : 1;
+  MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, q, kcache, vcache, out, heads, n_tokens, parts));
+  count_launch();
+  return MLD_OK;
 }
 
-// Grow-only per-device scratch of mld_attn_decode.
-struct AttnScratch {
-  void* ptr = nullptr;
-  size_t bytes = 0;
-};
-AttnScratch g_attn_scratch[64];
-std::mutex g_attn_mu;
+// CTAs that share a head: all of the launch resident at once with room for whole clusters in every GPC (3.5 CTAs of
+// four warps per SM of the four that fit; 16 heads and fewer take CTAs of eight warps, since 16 parts of four would
+// leave SMs short of loads in flight), and no more parts than each has tokens for one round of its warps.
+int launch_attn_decode(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
+                       int sms, cudaStream_t stream) {
+  const int warps = heads <= 16 ? 8 : 4;
+  int parts = 7 * sms * 2 / warps / heads;
+  const int rounds = div_up(n_tokens, warps * 4 * kAttnAhead);
+  if (parts > rounds) parts = rounds;
+  if (parts > kMaxAttnParts) parts = kMaxAttnParts;
+  if (parts < 1) parts = 1;
+  if (warps == 8) return launch_attn_decode_t<8>(q, kcache, vcache, out, heads, n_tokens, parts, stream);
+  return launch_attn_decode_t<4>(q, kcache, vcache, out, heads, n_tokens, parts, stream);
+}
 
 }  // namespace
 
@@ -495,84 +596,33 @@ int mld_comm_unique_id(void* id128) {
   return MLD_OK;
 }
 
-int mld_attn_decode(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads,
-                    int32_t head_dim, int32_t n_tokens, void* stream) {
+static int attn_decode(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads, int32_t head_dim,
+                       int32_t n_tokens, int32_t max_heads, void* stream) {
   MLD_REQUIRE(q != nullptr && kcache != nullptr && vcache != nullptr && out != nullptr, "null tensor");
   MLD_REQUIRE(head_dim == kHeadDim, "head_dim must be 128");
   MLD_REQUIRE(heads > 0 && n_tokens > 0, "bad shape");
-  int device = 0;
-  MLD_CUDA_CHECK(cudaGetDevice(&device));
-  MLD_REQUIRE(device < 64, "device ordinal too large");
-  const int splits = attn_splits(heads, sm_count(device));
-  const size_t need = (size_t)heads * splits * (kHeadDim + 2) * sizeof(float);
-  float* base;
-  {
-    std::lock_guard<std::mutex> lock(g_attn_mu);
-    AttnScratch& sc = g_attn_scratch[device];
-    if (sc.bytes < need) {
-      if (sc.ptr != nullptr) MLD_CUDA_CHECK(cudaFree(sc.ptr));
-      sc.ptr = nullptr;
-      sc.bytes = 0;
-      MLD_CUDA_CHECK(cudaMalloc(&sc.ptr, need));
-      sc.bytes = need;
-    }
-    base = static_cast<float*>(sc.ptr);
-  }
-  return launch_attn_decode(static_cast<const __half*>(q), static_cast<const __half*>(kcache),
-                            static_cast<const __half*>(vcache), base, base + (size_t)heads * splits * kHeadDim,
-                            static_cast<__half*>(out), heads, n_tokens, splits, static_cast<cudaStream_t>(stream));
-}
-
-// ------------------------------------------------------------------------
-// Allocation-free decode attention.
-//
-// Some hosts cannot let a library allocate device memory on their behalf: a
-// serving process whose own pool already owns the whole GPU (a late cudaMalloc
-// then fails, and it stalls every stream while the driver looks), or an
-// embedded runtime that fixes its memory plan before the first dispatch, the
-// way ML Drift's InferenceContext does.  For them the split-KV partial results
-// live in this fixed array, which every GPU that loads the library carries
-// until the process exits (2.03 MB).
-constexpr int kStaticPairs = 4096;  // (head, split) pairs the array can hold
-static __device__ __align__(256) float g_attn_static_scratch[kStaticPairs * (kHeadDim + 2)];
-
-namespace {
-// Device address of the array, looked up once per device.  In host code the
-// symbol's name is only a handle, never a pointer a kernel could use.
-float* g_attn_static_ptr[64] = {nullptr};
-std::mutex g_attn_static_mu;
-}  // namespace
-
-int mld_attn_decode_static(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads,
-                           int32_t head_dim, int32_t n_tokens, void* stream) {
-  MLD_REQUIRE(q != nullptr && kcache != nullptr && vcache != nullptr && out != nullptr, "null tensor");
-  MLD_REQUIRE(head_dim == kHeadDim, "head_dim must be 128");
-  MLD_REQUIRE(heads > 0 && n_tokens > 0, "bad shape");
-  if (heads > kStaticPairs) {
-    set_last_error_text("mld_attn_decode_static: more than 4096 heads do not fit the fixed scratch array");
+  if (heads > max_heads) {
+    set_last_error_text("mld_attn_decode_static: more than 4096 heads");
     return MLD_OUT_OF_RANGE;
   }
   int device = 0;
   MLD_CUDA_CHECK(cudaGetDevice(&device));
   MLD_REQUIRE(device < 64, "device ordinal too large");
-  float* base;
-  {
-    std::lock_guard<std::mutex> lock(g_attn_static_mu);
-    if (g_attn_static_ptr[device] == nullptr) {
-      // first call on this device (which is current): resolve the symbol
-      void* p = nullptr;
-      MLD_CUDA_CHECK(cudaGetSymbolAddress(&p, g_attn_static_scratch));
-      g_attn_static_ptr[device] = static_cast<float*>(p);
-    }
-    base = g_attn_static_ptr[device];
-  }
-  int splits = attn_splits(heads, sm_count(device));
-  if (heads * splits > kStaticPairs) splits = kStaticPairs / heads;
-  // every (head, split) slot used below is rewritten by this call, so nothing
-  // left from an earlier call can leak into the result
   return launch_attn_decode(static_cast<const __half*>(q), static_cast<const __half*>(kcache),
-                            static_cast<const __half*>(vcache), base, base + (size_t)heads * splits * kHeadDim,
-                            static_cast<__half*>(out), heads, n_tokens, splits, static_cast<cudaStream_t>(stream));
+                            static_cast<const __half*>(vcache), static_cast<__half*>(out), heads, n_tokens,
+                            sm_count(device), static_cast<cudaStream_t>(stream));
+}
+
+int mld_attn_decode(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads, int32_t head_dim,
+                    int32_t n_tokens, void* stream) {
+  return attn_decode(q, kcache, vcache, out, heads, head_dim, n_tokens, INT32_MAX, stream);
+}
+
+// The entry point of hosts that cannot let a library allocate device memory on their behalf.  Neither entry point
+// allocates any; this one keeps its bound on the head count.
+int mld_attn_decode_static(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads,
+                           int32_t head_dim, int32_t n_tokens, void* stream) {
+  return attn_decode(q, kcache, vcache, out, heads, head_dim, n_tokens, 4096, stream);
 }
 
 int mld_decoder_create(const mld_decoder_desc* d, const void* nccl_id128, mld_decoder** out) {

@@ -410,3 +410,38 @@ def test_attention_decode_matches_softmax(mld, heads, n_tokens):
     ref = np.einsum("ht,thd->hd", p, v.astype(np.float64))
     got = out.float().cpu().numpy()
     assert np.max(np.abs(got - ref)) <= 2e-3 * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("heads,n_tokens", [
+    (1, 1), (1, 129), (8, 128), (8, 16000), (12, 1000), (16, 2049),  # CTAs of eight warps, 1 .. 16 parts per head
+    (17, 65), (24, 4097), (32, 8191), (40, 511),                     # CTAs of four warps
+    (300, 700), (600, 40)])                                         # one part per head
+def test_attention_decode_parts(mld, heads, n_tokens):
+    # fp32 sums of fp16 inputs, rounded to fp16 once: half an ulp (2^-11) of the largest output, and as much again for
+    # the fp32 sums and exponentials
+    g = torch.Generator(device="cuda").manual_seed(heads * 100003 + n_tokens)
+    q = (torch.randn((heads, 128), generator=g, device="cuda") / np.sqrt(128)).half()
+    k, v = (torch.randn((n_tokens, heads, 128), generator=g, device="cuda").half() for _ in range(2))
+    out = torch.full((heads, 128), float("nan"), dtype=torch.float16, device="cuda")
+    mld.attn_decode(q, k, v, out, heads, n_tokens)
+    p = torch.softmax(torch.einsum("hd,thd->ht", q.double(), k.double()), 1)
+    ref = torch.einsum("ht,thd->hd", p, v.double())
+    assert (out.double() - ref).abs().max() <= 2.0 ** -10 * ref.abs().max()
+
+
+def test_attention_decode_on_two_streams(mld):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    cases = []
+    for heads, n_tokens in ((32, 4096), (8, 3000)):
+        q = (torch.randn((heads, 128), generator=g, device="cuda") / np.sqrt(128)).half()
+        k, v = (torch.randn((n_tokens, heads, 128), generator=g, device="cuda").half() for _ in range(2))
+        want = torch.empty((heads, 128), dtype=torch.float16, device="cuda")
+        mld.attn_decode(q, k, v, want, heads, n_tokens)
+        cases.append((q, k, v, want, heads, n_tokens, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    outs = [[torch.empty_like(c[3]) for _ in range(20)] for c in cases]
+    for i in range(20):
+        for c, o in zip(cases, outs):
+            mld.attn_decode(c[0], c[1], c[2], o[i], c[4], c[5], stream=c[6])
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, c[3]) for c, o in zip(cases, outs) for x in o)
