@@ -134,3 +134,42 @@ def test_full_size_packing_roundtrip(mld):
     rec = blocks.permute(1, 3, 0, 2).reshape(O, I)
     assert torch.equal(rec.to(torch.int8), q)
     assert torch.equal(sums, q.to(torch.int32).sum(dim=1).to(torch.int32))
+
+
+@pytest.mark.parametrize("bits,block", [(8, 0), (4, 32), (4, 0), (4, 128)])
+def test_quantiser_next_to_ties_and_extremes(mld, oracle, bits, block):
+    # values a few ulps around every halfway point, rows whose scale is tiny, huge or subnormal
+    rng = np.random.default_rng(bits * 1000 + block)
+    O, I, top = 64, 256, 127 if bits == 8 else 7
+    bound = np.float32(10.0) ** rng.uniform(-6, 6, (O, 1)).astype(np.float32)
+    bound[0], bound[1], bound[2], bound[3] = 1e-42, 3e-38, 3e38, 0.0
+    sc = (bound / np.float32(top)).astype(np.float32)
+    k = rng.integers(-top, top, (O, I)) + 0.5
+    w = (k * sc).astype(np.float32)
+    w = (w.view(np.int32) + rng.integers(-3, 4, (O, I)) * (w != 0)).view(np.float32)
+    w = np.clip(w, -bound, bound).astype(np.float32)
+    w[:, ::32] = bound
+    q, s = mld.quantize_weights(_dev(w), bits, block)
+    qr, sr = oracle.quantize_int8_sym(w) if bits == 8 else oracle.quantize_int4_sym(w, block)
+    assert np.array_equal(q.cpu().numpy(), qr)
+    assert np.array_equal(s.cpu().numpy().reshape(-1), sr.reshape(-1))
+
+
+@pytest.mark.parametrize("O,I", [(16, 16), (128, 272), (144, 1024), (132, 128), (126, 144)])
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("offset", [0, 16])
+def test_pack_wide_stores(mld, oracle, O, I, bits, offset):
+    # whole and partial groups of 16 outputs; a destination that is 32-byte aligned and one that is not
+    import ctypes as C
+    rng = np.random.default_rng(O + I)
+    q = rng.integers(-8, 8, size=(O, 1, 1, I), dtype=np.int8)
+    ref = oracle.rearrange_int8_as_uint8(q) if bits == 8 else oracle.rearrange_int8_as_uint4(q)
+    buf = torch.full((ref.size + 64,), 0x5A, dtype=torch.uint8, device="cuda")
+    d = mld.binding.PackDesc(O, 1, 1, I, bits, 0, mld.binding.SRC_INT8, 0, 128 if bits == 8 else 8)
+    src = _dev(q)
+    rc = mld.binding.lib().mld_pack_weights(C.byref(d), C.c_void_p(src.data_ptr()), C.c_void_p(buf.data_ptr() + offset),
+                                            None, 0, None)
+    torch.cuda.synchronize()
+    got = buf.cpu().numpy()
+    assert rc == 0 and np.array_equal(got[offset:offset + ref.size], ref.reshape(-1))
+    assert (got[:offset] == 0x5A).all() and (got[offset + ref.size:] == 0x5A).all()
