@@ -67,14 +67,51 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
-// D[tmem_d] (+)= A[tmem_a] B[desc_b]^T over the pair; A: 16 halves per lane in 8 columns of both CTAs' tensor memory.
-__device__ __forceinline__ void umma_pair_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
+// D[tmem_d] (+)= A[tmem_a] B[desc_b]^T over the pair (or by this CTA alone); A: 16 halves per lane in 8 columns of
+// tensor memory (of both CTAs').
+template <bool PAIR>
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                        uint32_t accumulate) {
+  if constexpr (PAIR) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+  }
+}
+// Arrives on the barrier (in both CTAs of a pair) once every MMA issued so far has completed.
+template <bool PAIR>
+__device__ __forceinline__ void commit(uint64_t* bar) {
+  if constexpr (PAIR) {
+    commit_pair(bar);
+  } else {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+  }
+}
+template <bool PAIR>
+__device__ __forceinline__ void tmem_alloc_all(uint32_t* smem_dst) {
+  if constexpr (PAIR) {
+    tmem_alloc_pair(smem_dst, 512);
+    tmem_relinquish_pair();
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(smem_dst)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+}
+template <bool PAIR>
+__device__ __forceinline__ void tmem_dealloc_all(uint32_t taddr) {
+  if constexpr (PAIR) {
+    tmem_dealloc_pair(taddr, 512);
+  } else {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(taddr) : "memory");
+  }
 }
 
 struct WtArgs {
@@ -85,7 +122,12 @@ struct WtArgs {
   int trace_flags;  // tuning builds only: 1 = no output stores, 2 = no lane exchange either
 };
 
-template <int MODE>
+// PAIR: the two-CTA form described above.  Otherwise a CTA works alone on tiles of 128 output channels x up to 128
+// tokens: no transformed stage has to be announced to another SM (a remote arrival takes about 800 cycles, which bounds a
+// pair's rate of stages), at the price of every CTA fetching all of the tile's tokens.  Bound by the MMAs: a stage's four
+// take about 740 cycles whatever the number of tokens, on one accumulator or several, from one issuing thread or two.
+// 77 tokens, 4096 x 11008 INT4: 41.1 us a call with pairs and whole tiles, 31.3 with lone CTAs and tiles cut along K.
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kPairThreads, 1)
     gemm_wtmem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, WtArgs wa) {
   const PairArgs& a = wa.p;
@@ -93,7 +135,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   constexpr int SLICES = 16;                            // packed rows per stage (64 input channels)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int half_tok = wa.tile_tok / 2;
+  constexpr int CTAS = PAIR ? 2 : 1;                    // CTAs per tile
+  const int cta_tok = wa.tile_tok / CTAS;               // token rows this CTA fetches
   constexpr int w_pitch = (kWtRows / 4) * BLK;          // bytes of one packed row of the box
   constexpr int w_stage = SLICES * w_pitch;             // 4 KB / 8 KB
   uint8_t* sX = smem;
@@ -108,8 +151,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xf_done + kWtStages);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank();
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  const int pair = blockIdx.x / CTAS, n_pairs = gridDim.x / CTAS;  // ("pair": whoever works on a tile)
   WorkList work0;
   {
     const int shared_units = a.shared_tiles * a.k_blocks;
@@ -128,45 +171,53 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       mbar_init(&w_empty[s], kTransformWarps);
     }
     for (int s = 0; s < kWtStages; ++s) {
-      mbar_init(&full_ab[s], 1 + 2);  // the producer's expect_tx, + one arrival per CTA for its weights
+      // the producer's expect_tx, + one arrival per CTA for its weights (a lone CTA's transform warps arrive themselves)
+      mbar_init(&full_ab[s], PAIR ? 1 + 2 : 1 + kTransformWarps);
       mbar_init(&empty[s], 1);
       mbar_init(&xf_done[s], kTransformWarps);
     }
     mbar_init(tmem_full, 1);
-    mbar_init(tmem_empty, 2 * 4 * kDrainParts);
+    mbar_init(tmem_empty, CTAS * 4 * kDrainParts);
     fence_barrier_init();
   }
-  if (warp == 1) {
-    tmem_alloc_pair(tmem_slot, 512);
-    tmem_relinquish_pair();
-  }
+  if (warp == 1) tmem_alloc_all<PAIR>(tmem_slot);
   tc_before();
   __syncthreads();
-  cluster_sync_all();  // the partner's barriers are initialised before anything arrives on them
+  if constexpr (PAIR) cluster_sync_all();  // the partner's barriers are initialised before anything arrives on them
   tc_after();
   pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t full_ab_lead = map_shared(smem_u32(full_ab), 0);
-  const uint32_t tmem_empty_lead = map_shared(smem_u32(tmem_empty), 0);
+  const uint32_t full_ab_lead = PAIR ? map_shared(smem_u32(full_ab), 0) : 0u;
+  const uint32_t tmem_empty_lead = PAIR ? map_shared(smem_u32(tmem_empty), 0) : 0u;
+  auto release_tmem = [&]() {
+    if constexpr (PAIR)
+      arrive_remote(tmem_empty_lead);
+    else
+      mbar_arrive(tmem_empty);
+  };
   // tile -> (token tile, channel tile): the token tiles of one channel tile follow each other
   auto tile_tok0 = [&](int tile) { return (tile % a.m_tiles) * wa.tile_tok; };
-  auto tile_n0 = [&](int tile) { return (tile / a.m_tiles) * 2 * kWtRows; };
+  auto tile_n0 = [&](int tile) { return (tile / a.m_tiles) * CTAS * kWtRows; };
 
   // Accumulators -> outputs, the share `part` of kDrainParts of the warps that can address this lane quarter
   // (one epilogue warp and the quarter's four transform warps, which have nothing to transform while the only
-  // accumulator buffer is being read): pieces of 16 token columns, part, part + kDrainParts, ...  A tile shared
-  // with a neighbouring pair (see gemm_pair_kernel): the pair that holds the tile's last k-blocks leaves its raw
-  // accumulators in the workspace slot of the pair before it, which adds them to its own and writes the outputs.
+  // accumulator buffer is being read): pieces of 16 token columns, part, part + kDrainParts, ...  A tile cut
+  // along K: a pair whose share does not begin with the tile's first k-block (always the first of its segments, so that
+  // nothing it waits for comes before) leaves its raw accumulators in its own workspace slot; the pair that has the
+  // first k-block adds the following pairs' slots to its own accumulators, in order, and writes the outputs.
   auto drain = [&](const Segment& sg, int part) -> bool {
     const int quad = warp & 3;  // TMEM lanes 32*quad .. 32*quad+31 belong to this warp
-    const bool hands_over = sg.kb0 > 0, takes_over = sg.kb1 < a.k_blocks;
-    const int slot = hands_over ? pair - 1 : pair;
-    uint4* const slot_rows =
-        reinterpret_cast<uint4*>(a.split_ws) + ((size_t)(slot * 2 + static_cast<int>(rank)) * 4 + quad) * (8 * 8 * 32) + lane;
-    uint32_t* const slot_flag = a.split_flags + ((slot * 2 + static_cast<int>(rank)) * 4 + quad) * 8 + part;
+    const bool hands_over = sg.kb0 > 0, takes_over = !hands_over && sg.kb1 < a.k_blocks;
+    const auto rows_of = [&](int slot) {
+      return reinterpret_cast<uint4*>(a.split_ws) + ((size_t)(slot * CTAS + static_cast<int>(rank)) * 4 + quad) * (8 * 8 * 32) + lane;
+    };
+    const auto flag_of = [&](int slot) { return a.split_flags + ((slot * CTAS + static_cast<int>(rank)) * 4 + quad) * 8 + part; };
+    // the pairs that hold the rest of a tile this pair completes
+    const int others = takes_over ? ((sg.tile + 1) * a.k_blocks - 1) / a.units_per_pair - pair : 0;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     const int n_pieces = wa.tile_tok >> 4;
     if (hands_over) {
+      uint4* const slot_rows = rows_of(pair);
       for (int pc = part; pc < n_pieces; pc += kDrainParts) {
         uint32_t r[16];
         tmem_ld16(lane_base + static_cast<uint32_t>(16 * pc), r);
@@ -178,24 +229,26 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       tc_before();
       __syncwarp();
       if (lane == 0) {
-        st_release_gpu(slot_flag, a.epoch);
-        arrive_remote(tmem_empty_lead);
+        st_release_gpu(flag_of(pair), a.epoch);
+        release_tmem();
       }
       return true;
     }
     if (takes_over) {
-      uint32_t seen = 0;
-      if (lane == 0) {
+      bool seen = true;
+      for (int o = lane; o < others; o += 32) {  // a lane per slot
+        const uint32_t* flag = flag_of(pair + 1 + o);
         const unsigned long long t0 = globaltimer_ns();
-        while ((seen = ld_acquire_gpu(slot_flag)) != a.epoch && globaltimer_ns() - t0 <= kWaitLimitNs) __nanosleep(64);
+        uint32_t v;
+        while ((v = ld_acquire_gpu(flag)) != a.epoch && globaltimer_ns() - t0 <= kWaitLimitNs) __nanosleep(32);
+        seen = seen && v == a.epoch;
       }
-      seen = __shfl_sync(0xffffffffu, seen, 0);
-      if (seen != a.epoch) {
+      if (!__all_sync(0xffffffffu, seen)) {
         atomicExch(a.error, kErrWtBase + 8);
         return false;
       }
     }
-    const int n = (sg.tile / a.m_tiles) * 2 * kWtRows + static_cast<int>(rank) * kWtRows + quad * 32 + lane;  // output channel
+    const int n = tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows + quad * 32 + lane;  // output channel
     const int m_first = (sg.tile % a.m_tiles) * wa.tile_tok;
     const bool has_n = n < a.N4;
     __half bias_h = __float2half_rn(0.0f);
@@ -206,14 +259,16 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       uint32_t r[16];
       tmem_ld16(lane_base + static_cast<uint32_t>(c0), r);
       tmem_ld_wait();
-      if (takes_over) {
+#pragma unroll 2
+      for (int o = 0; o < others; ++o) {
+        const uint4* const slot_rows = rows_of(pair + 1 + o);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const uint4 o = __ldcg(&slot_rows[(pc * 4 + j) * 32]);
-          r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + __uint_as_float(o.x));
-          r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + __uint_as_float(o.y));
-          r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + __uint_as_float(o.z));
-          r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + __uint_as_float(o.w));
+          const uint4 v = __ldcg(&slot_rows[(pc * 4 + j) * 32]);
+          r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + __uint_as_float(v.x));
+          r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + __uint_as_float(v.y));
+          r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + __uint_as_float(v.z));
+          r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + __uint_as_float(v.w));
         }
       }
       // token pairs as packed halves: h2[i] = tokens c0 + 2i, c0 + 2i + 1 of channel n
@@ -289,7 +344,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
     tc_before();
     __syncwarp();
-    if (lane == 0) arrive_remote(tmem_empty_lead);
+    if (lane == 0) release_tmem();
     return true;
   };
 
@@ -303,15 +358,18 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       WorkList work = work0;
       Segment sg;
       while (ok && work.next(sg)) {
-        const int m0 = tile_tok0(sg.tile) + static_cast<int>(rank) * half_tok;
+        const int m0 = tile_tok0(sg.tile) + static_cast<int>(rank) * cta_tok;
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1)) {
             atomicExch(a.error, kErrWtBase + 1);
             ok = false;
             break;
           }
-          if (rank == 0) mbar_arrive_expect_tx(&full_ab[stage], 2u * static_cast<uint32_t>(half_tok) * kKBytes);
-          tma_load_2d_pair(sX + (size_t)stage * kWtTokBytes, &tmap_x, full_ab_lead + stage * 8, kb * 64, m0);
+          if (rank == 0) mbar_arrive_expect_tx(&full_ab[stage], static_cast<uint32_t>(wa.tile_tok) * kKBytes);
+          if constexpr (PAIR)
+            tma_load_2d_pair(sX + (size_t)stage * kWtTokBytes, &tmap_x, full_ab_lead + stage * 8, kb * 64, m0);
+          else
+            tma_load_2d(sX + (size_t)stage * kWtTokBytes, &tmap_x, &full_ab[stage], kb * 64, m0);
           if (++stage == kWtStages) {
             stage = 0;
             phase ^= 1;
@@ -322,7 +380,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   } else if (warp == 1) {
     // ------------------------------------------------------------------- MMA issuer
     if (rank == 0 && lane == 0) {
-      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(wa.tile_tok >> 3) << 17) | (16u << 24);
+      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(wa.tile_tok >> 3) << 17) | ((PAIR ? 16u : 8u) << 24);
       int stage = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
@@ -352,15 +410,15 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           const uint32_t ta = tmem_base + kWtACol + static_cast<uint32_t>(stage * 32);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_pair_ts(tmem_base, ta + 8u * k, db + static_cast<uint64_t>((k * 32) >> 4), idesc,
-                         (kb > sg.kb0 || k > 0) ? 1u : 0u);
-          commit_pair(&empty[stage]);
+            umma_ts<PAIR>(tmem_base, ta + 8u * k, db + static_cast<uint64_t>((k * 32) >> 4), idesc,
+                          (kb > sg.kb0 || k > 0) ? 1u : 0u);
+          commit<PAIR>(&empty[stage]);
           if (++stage == kWtStages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) commit_pair(tmem_full);
+        if (ok) commit<PAIR>(tmem_full);
       }
 #ifdef MLD_TRACE
       if (wa.trace != nullptr) {
@@ -412,6 +470,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
     }
   } else if (warp >= 22) {
+    if constexpr (!PAIR) {
+      // (a lone CTA has nobody to tell)
+    } else {
     // ------------------------------------------------------------------- forwarders
     if (lane == 0) {
       const int parity_of_mine = warp - 22;  // stages of even / odd iterations
@@ -431,6 +492,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           phase ^= 1;
         }
       }
+    }
     }
   } else {
     // -------------------------------------------------------------------- transform
@@ -536,7 +598,10 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&w_empty[ws]);     // the box may be overwritten
-          mbar_arrive(&xf_done[stage]);  // local; a forwarder passes it on to the pair's first CTA
+          if constexpr (PAIR)
+            mbar_arrive(&xf_done[stage]);  // local; a forwarder passes it on to the pair's first CTA
+          else
+            mbar_arrive(&full_ab[stage]);
         }
         advance(kb + 1 < sg.kb1 ? 2 : 1);
       }
@@ -566,7 +631,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   // may still write this CTA's tensor memory.
   tc_before();
   __syncthreads();
-  cluster_sync_all();
+  if constexpr (PAIR) cluster_sync_all();
   if (*reinterpret_cast<volatile int*>(a.error) != 0) {
     // a wait ran out somewhere: copies may still be in flight towards this CTA's shared memory
     const unsigned long long t0 = globaltimer_ns();
@@ -574,7 +639,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   }
   if (warp == 1) {
     tc_after();
-    tmem_dealloc_pair(tmem_base, 512);
+    tmem_dealloc_all<PAIR>(tmem_base);
   }
 }
 
@@ -593,23 +658,36 @@ WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share
   const int N4 = align_n(N, 4);
   g.kp = align_n(K, 8);
   g.k_blocks = div_up(g.kp, 64);
-  g.n_tiles = div_up(N4, 2 * kWtRows);
-  g.tile_tok = M >= 256 ? 256 : align_n(M, 16);
+  // Up to 128 tokens a CTA works alone; with more, pairs share the fetching of the tokens.
+  g.ctas = M <= 128 || sms < 2 ? 1 : 2;
+  g.n_tiles = div_up(N4, g.ctas * kWtRows);
+  const int most = 128 * g.ctas;
+  g.tile_tok = M >= most ? most : align_n(M, 16);
 #ifdef MLD_TRACE
   if (const char* e = getenv("MLD_WT_TOK")) g.tile_tok = atoi(e);
 #endif
   g.tok_tiles = div_up(M, g.tile_tok);
-  const int pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const int pairs = sms < 2 ? 1 : sms / 2 * 2 / g.ctas;  // (the split workspace has a slot per CTA of sms / 2 pairs)
   const long tiles = (long)g.n_tiles * g.tok_tiles;
-  g.shares_tiles = may_share && tiles > pairs && tiles % pairs != 0;
+  // The last whole wave of tiles and the remainder are cut along K and dealt out evenly; so are the tiles of a launch
+  // that has fewer of them than pairs (43 tiles of 4096 x 11008 left 31 of 74 pairs without work), into parts of eight
+  // stages or more and no more than eight of them: the pair that completes a tile reads the other parts' accumulators
+  // one after another, which costs about as much as a few stages.
+  const bool few = tiles < pairs;
+  g.shares_tiles = may_share && tiles % pairs != 0;
   if (g.shares_tiles) {
-    g.shared_tiles = static_cast<int>(pairs + tiles % pairs);
-    g.units_per_pair = static_cast<int>(((long)g.shared_tiles * g.k_blocks + pairs - 1) / pairs);
-    g.grid = 2 * pairs;
+    g.shared_tiles = static_cast<int>(few ? tiles : pairs + tiles % pairs);
+    const long units = (long)g.shared_tiles * g.k_blocks;
+    g.units_per_pair = static_cast<int>((units + pairs - 1) / pairs);
+    int least = div_up(g.k_blocks, 8);
+    if (least < 8) least = 8;
+    if (least > g.k_blocks) least = g.k_blocks;
+    if (g.units_per_pair < least) g.units_per_pair = least;
+    g.grid = g.ctas * static_cast<int>(few ? (units + g.units_per_pair - 1) / g.units_per_pair : pairs);
   } else {
     g.shared_tiles = 0;
     g.units_per_pair = 0;
-    g.grid = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
+    g.grid = g.ctas * static_cast<int>(few ? tiles : pairs);
   }
   const int blk = mode == kModeInt4F16 ? 8 : 16;
   const int w_stage = 16 * (kWtRows / 4) * blk;
@@ -638,7 +716,7 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   const int SS = div_up(K, 4), DS = N4 / 4;
   CUtensorMap tx, tw;
   // activations: K-major rows [M][kp]; box = one swizzle atom of K x this CTA's half of the tile's tokens
-  int rc = make_tmap_2d(&tx, x_kmajor, (uint64_t)g.kp * 2, M, (uint64_t)g.kp * 2, kKBytes, g.tile_tok / 2, 2,
+  int rc = make_tmap_2d(&tx, x_kmajor, (uint64_t)g.kp * 2, M, (uint64_t)g.kp * 2, kKBytes, g.tile_tok / g.ctas, 2,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, true);
   if (rc != MLD_OK) return rc;
   // packed weights: [K/4] rows of N4/4 blocks; box = one stage's 16 rows x the CTA's 32 blocks, in 32-bit elements
@@ -682,12 +760,14 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   wa.trace_flags = getenv("MLD_WT_FLAGS") != nullptr ? atoi(getenv("MLD_WT_FLAGS")) : 0;
 #endif
   void (*kern)(CUtensorMap, CUtensorMap, WtArgs) =
-      mode == kModeInt4F16 ? gemm_wtmem_kernel<kModeInt4F16> : gemm_wtmem_kernel<kModeInt8F16>;
-  static bool configured[2][kMaxDevices];
+      g.ctas == 2 ? (mode == kModeInt4F16 ? gemm_wtmem_kernel<kModeInt4F16, true> : gemm_wtmem_kernel<kModeInt8F16, true>)
+                  : (mode == kModeInt4F16 ? gemm_wtmem_kernel<kModeInt4F16, false> : gemm_wtmem_kernel<kModeInt8F16, false>);
+  static bool configured[2][2][kMaxDevices];
+  bool(&done)[kMaxDevices] = configured[g.ctas - 1][mode];
   int dev;
-  if (needs_configure(configured[mode], &dev)) {
+  if (needs_configure(done, &dev)) {
     MLD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    if (dev >= 0) configured[mode][dev] = true;
+    if (dev >= 0) done[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.grid, 1, 1);
@@ -695,14 +775,14 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   cfg.dynamicSmemBytes = g.smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = g.ctas == 2 ? 2 : 1;
   MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tx, tw, wa));
   count_launch();
   return MLD_OK;

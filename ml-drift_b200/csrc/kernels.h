@@ -206,6 +206,7 @@ int launch_gemm_pair(int mode, const void* a_mat, const void* packed, const Pair
 
 // ------------------------------------------- prefill GEMM, dequantised weights in tensor memory (SM pairs)
 struct WtGeometry {
+  int ctas;  // 2: pairs of SMs share a tile; 1: every CTA its own
   int kp, tile_tok, tok_tiles, n_tiles, k_blocks, w_stages, grid;
   int shared_tiles, units_per_pair;
   bool shares_tiles;

@@ -253,3 +253,27 @@ def test_config3_full_size_sampled(mld, oracle, route):
     torch.cuda.synchronize()
     assert torch.equal(y2, y3)
     plan.close()
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,K,N", [
+    (33, 64, 128), (77, 4096, 1104), (128, 2048, 520), (40, 14336, 512), (100, 520, 16),   # lone CTAs, 1 .. 8 parts of a tile
+    (128, 640, 20000),                                                                     # more tiles than CTAs
+    (129, 4096, 520), (200, 1024, 2560), (500, 4096, 264)])                                # pairs, fewer tiles than pairs
+def test_tiles_cut_along_k(mld, oracle, bits, M, K, N):
+    # fp32 sums of half products in parts: as in test_int4_prefill_gemm_vs_oracle; twice, so that workspace slots and
+    # their flags are used again
+    rng = np.random.default_rng(M + K + N + bits)
+    w = (rng.standard_normal((N, K)) * 0.02).astype(np.float32)
+    q, s = oracle.quantize_int4_sym(w, 0 if K % 32 else 32) if bits == 4 else oracle.quantize_int8_sym(w)
+    packed = oracle.rearrange_int8_as_uint4(q) if bits == 4 else oracle.rearrange_int8_as_uint8(q)
+    G = s.shape[1] if s.ndim == 2 else 1
+    sgn = oracle.scale_layout(s, True)
+    x16 = rng.standard_normal((M, K)).astype(np.float16)
+    y = _run_gemm(mld, oracle, x16, packed, _dev(sgn.view(np.float16)), N, K, bits,
+                  mld.SCALE_BLOCK if G > 1 else mld.SCALE_PER_CHANNEL, G, reps=2, route="inline")
+    ref = oracle.f16_bits_to_f32(oracle.prefill_gemm_int4(x16.view(np.uint16), packed, sgn, N, bits=bits))
+    # 8 bits: half(u * s) with u around 128 is rounded by 0.05 s rms, against weights of 35 s rms, where the compiler does
+    # not fuse it into the addition of the offset (the restatement never does): up to 0.05 / 35 of the largest output,
+    # and the output's own rounding
+    assert _rel(y, ref) <= (1e-3 if bits == 4 else 0.05 / 35 + 2.0 ** -11)
