@@ -86,19 +86,19 @@ static int gm_stage_rows() { return strip_geometry(4, 64, 64, 1, 8, MLD_SCALE_BL
 struct TmapEntry {
   const void* w;
   const void* s;
-  int geom;
-  CUtensorMap tw, ts;
+  const void* z;
+  int boxes;  // width of the scale box, in weight boxes
+  CUtensorMap tw, ts, tz;
 };
 
 struct mld_fc_plan {
   mld_fc_desc d;
   int device;
   int sms;
-  bool stream_ok;        // the streaming GEMV can serve this operator
+  bool stream_ok;        // the streaming GEMV can serve this operator (strip_geometry_of says for how many tokens)
   bool subnormal;        // operand encoding of the streaming GEMV
   bool pdl;              // launch GEMVs with programmatic stream serialization
   int group_slices;
-  StripGeometry gm;
   int* error;            // device error word written by kernels whose bounded waits ran out
   int* error_shared;     // when set (a decoder's word), the kernels report there instead
   size_t ws_bytes;
@@ -288,7 +288,9 @@ int mld_fc_plan_create(const mld_fc_desc* d, mld_fc_plan** out) {
   p->pdl = d->no_overlap == 0;
 
   const int N4 = align_n(d->n, 4);
-  bool ok = d->precision != MLD_PRECISION_F32 && !d->has_zero_point && (N4 % 8 == 0) && (d->k % 8 == 0) &&
+  // (zero points: one per scale, for the operand form and the strip widths that the kernel has an instantiation of)
+  bool ok = d->precision != MLD_PRECISION_F32 && (N4 % 8 == 0) && (d->k % 8 == 0) &&
+            (!d->has_zero_point || (d->scale_mode != MLD_SCALE_SCALAR && p->subnormal && p->pdl)) &&
             p->sms > 0 && get_encode_tiled() != nullptr;
   if (d->scale_mode == MLD_SCALE_BLOCK) {
     const bool small = group_slices == 8 || group_slices == 16 || group_slices == 32;
@@ -296,12 +298,6 @@ int mld_fc_plan_create(const mld_fc_desc* d, mld_fc_plan** out) {
     ok = ok && (small || large) && (group_slices * d->groups == src_slices);
   }
   p->stream_ok = ok;
-  if (ok) {
-    const int max_m = d->max_tokens < 16 ? d->max_tokens : 16;
-    p->gm = strip_geometry(d->weight_bits, d->n, d->k, max_m, group_slices, d->scale_mode, p->sms, p->pdl,
-                           d->smem_limit_kb);
-    if (p->gm.stages < 2) p->stream_ok = false;
-  }
   {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaMalloc(&p->error, sizeof(int));
@@ -416,22 +412,30 @@ static int run_generic(mld_fc_plan* p, const void* src, const void* weights, con
   return launch_fc_generic(a, d.weight_bits, d.precision == MLD_PRECISION_F32, stream);
 }
 
-static int run_stream(mld_fc_plan* p, const void* src, const void* weights, const void* scale, const void* bias,
-                      void* dst, int tokens, cudaStream_t stream, const PeerScatter* scatter, const PeerWait* wait) {
+static StripGeometry strip_geometry_of(const mld_fc_plan* p, int tokens) {
   const mld_fc_desc& d = p->d;
-  const StripGeometry& gm = p->gm;
+  return strip_geometry(d.weight_bits, d.n, d.k, tokens, p->group_slices, d.scale_mode, p->sms, p->pdl, d.smem_limit_kb,
+                        d.has_zero_point != 0, p->subnormal);
+}
+
+static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, const void* weights, const void* scale,
+                      const void* zp, const void* bias, void* dst, int tokens, cudaStream_t stream,
+                      const PeerScatter* scatter, const PeerWait* wait) {
+  const mld_fc_desc& d = p->d;
   const int N4 = align_n(d.n, 4), SS = div_up(d.k, 4), DS = N4 / 4;
-  CUtensorMap tw, ts;
+  CUtensorMap tw, ts, tz;
   {
     std::lock_guard<std::mutex> lock(p->mu);
     const TmapEntry* te = nullptr;
     for (const TmapEntry& e : p->tmaps)
-      if (e.w == weights && e.s == scale) te = &e;
+      if (e.w == weights && e.s == scale && e.z == zp && e.boxes == gm.w) te = &e;
     if (te == nullptr) {
       TmapEntry e;
       e.w = weights;
       e.s = scale;
-      e.geom = 0;
+      e.z = zp;
+      e.boxes = gm.w;
+      memset(&e.tz, 0, sizeof e.tz);
       const uint64_t blk = d.weight_bits == 4 ? 8 : 16;
       int rc = make_tmap_2d(&e.tw, weights, (uint64_t)DS * blk, SS, (uint64_t)DS * blk, 128, gm.stage_rows, 1,
                             CU_TENSOR_MAP_SWIZZLE_128B);
@@ -441,6 +445,9 @@ static int run_stream(mld_fc_plan* p, const void* src, const void* weights, cons
         const int wt = gm.w * (d.weight_bits == 4 ? 64 : 32);
         rc = make_tmap_2d(&e.ts, scale, (uint64_t)N4 * 2, G, (uint64_t)N4 * 2, wt * 2, gm.scale_rows, 2,
                           CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc == MLD_OK && zp != nullptr)
+          rc = make_tmap_2d(&e.tz, zp, (uint64_t)N4 * 2, G, (uint64_t)N4 * 2, wt * 2, gm.scale_rows, 2,
+                            CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc != MLD_OK) return rc;
       } else {
         memset(&e.ts, 0, sizeof e.ts);
@@ -451,6 +458,7 @@ static int run_stream(mld_fc_plan* p, const void* src, const void* weights, cons
     }
     tw = te->tw;
     ts = te->ts;
+    tz = te->tz;
   }
   StripArgs a;
   a.x = src;
@@ -472,7 +480,11 @@ static int run_stream(mld_fc_plan* p, const void* src, const void* weights, cons
   a.scale_rows = gm.scale_rows;
   a.group_slices = gm.group_slices;
   a.gs_shift = gm.gs_shift;
+  a.zp_off = gm.zp_off;
   a.red_m = gm.red_m;
+  a.peer_m = gm.peer_m;
+  a.ts_shift = gm.ts_shift;
+  a.interleave = gm.interleave;
   a.dst_layout = d.dst_layout;
   a.epilogue = d.epilogue;
   a.scalar_scale = d.scalar_scale;
@@ -489,10 +501,10 @@ static int run_stream(mld_fc_plan* p, const void* src, const void* weights, cons
   a.next_w = p->next_w;
   a.next_w_bytes = p->next_w_bytes;
   p->next_w = nullptr;  // the hint is consumed by this call
-  for (int tok0 = 0; tok0 < tokens; tok0 += 8) {
+  for (int tok0 = 0; tok0 < tokens; tok0 += gm.launch_tokens) {
     a.tok0 = tok0;
-    a.M = tokens - tok0 < 8 ? tokens - tok0 : 8;
-    const int rc = launch_fc_strip(d.weight_bits, p->subnormal, tw, ts, a, gm, stream);
+    a.M = tokens - tok0 < gm.launch_tokens ? tokens - tok0 : gm.launch_tokens;
+    const int rc = launch_fc_strip(d.weight_bits, p->subnormal, tw, ts, zp != nullptr ? &tz : nullptr, a, gm, stream);
     if (rc != MLD_OK) return rc;
   }
   return MLD_OK;
@@ -625,6 +637,25 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
 
   int path = d.force_path;
   if (path == 0) path = mld_fc_is_gemv_recommended(d.precision, tokens) ? 1 : 2;
+  const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(scale) & 15) == 0 &&
+                       (reinterpret_cast<uintptr_t>(zp) & 15) == 0;
+  const bool layout_ok = d.src_layout == MLD_LAYOUT_SLICED || tokens == 1;
+  const bool streams = plan->stream_ok && aligned && layout_ok && (!d.has_zero_point || zp != nullptr);
+  // The streaming kernel beyond the decode rule's tokens.  Up to 16 its MMAs take no longer than the GEMM does (us a
+  // call, INT4, streaming / GEMM: 4096 x 4096, 9 tokens 12.4 / 17.0, 16 tokens 14.0 / 17.1; 4096 x 11008 27.2 / 27.9
+  // and 28.4 / 28.1; 8192 x 28672 80 / 104 and 82 / 104; at 24 tokens it loses, 47 / 29 on 4096 x 11008).  With zero
+  // points the alternative is the general kernel (2048 x 4096, 12 tokens: 48 against 9.5 us), so there it takes as many
+  // tokens as two launches hold.
+  const bool few = d.force_path == 0 && d.prefill_act_quant == 0 && d.prefill_route == MLD_PREFILL_ROUTE_AUTO &&
+                   d.cache_prepared_weights == 0 && outs == nullptr && tokens <= 16;
+  if (streams && path == 2 && (d.has_zero_point ? tokens <= 2 * kStripTokens : few && plan->pdl && plan->subnormal) &&
+      d.epilogue == MLD_EPILOGUE_NONE) {
+    const StripGeometry gm = strip_geometry_of(plan, tokens);
+    if (gm.stages >= 2) {
+      plan->last_route = MLD_ROUTE_DECODE_STREAMING;
+      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, stream, nullptr, nullptr);
+    }
+  }
   if (path == 2) {
     // the tensor-core route takes fp16 tensors without zero points; anything
     // else is served, correctly but slowly, by the general kernel below
@@ -645,12 +676,12 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
     set_last_error_text("the fused SiLU*mul write is available on the streaming decode kernel only");
     return MLD_UNIMPLEMENTED;
   }
-  const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
-                       (scale == nullptr || (reinterpret_cast<uintptr_t>(scale) & 15) == 0);
-  const bool layout_ok = d.src_layout == MLD_LAYOUT_SLICED || tokens == 1;
-  if (plan->stream_ok && tokens <= 16 && aligned && layout_ok) {
-    plan->last_route = MLD_ROUTE_DECODE_STREAMING;
-    return run_stream(plan, src, weights, scale, b, dst, tokens, stream, scatter, wait);
+  if (streams && tokens <= (plan->pdl && plan->subnormal ? 2 * kStripTokens : 16)) {
+    const StripGeometry gm = strip_geometry_of(plan, tokens);
+    if (gm.stages >= 2) {
+      plan->last_route = MLD_ROUTE_DECODE_STREAMING;
+      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, stream, scatter, wait);
+    }
   }
   if (d.epilogue != MLD_EPILOGUE_NONE) {
     set_last_error_text("the fused SiLU*mul write needs 16-byte aligned fp16 tensors in the sliced layout");

@@ -1,12 +1,12 @@
-// Decode-stage dequant-GEMV, streaming form (1..8 tokens per launch) over the
+// Decode-stage dequant-GEMV, streaming form (1..32 tokens per launch) over the
 // reference's packed weight layout [K/4][N/4][4 k][4 n].
 //
 // The kernel is HBM-bound, so it is organised around keeping the memory system
 // busy and the exit path short:
-//  * the grid is one CTA per SM; each CTA owns a contiguous strip of output
-//    columns (16-byte granularity, so the strips balance to within one chunk)
-//    and streams every K row of that strip - no split-K traffic through global
-//    memory.  When the matrix is too narrow for 148 useful strips, two CTAs of
+//  * the grid is one CTA per SM (two for matrices of several passes); each CTA
+//    owns a strip of output columns (16-byte granularity, so the strips balance
+//    to within one chunk) and streams every K row of that strip - no split-K
+//    traffic through global memory.  When the matrix is too narrow for 148 useful strips, two CTAs of
 //    a thread-block cluster share a strip, take half of K each and combine
 //    through distributed shared memory;
 //  * packed weights (128-byte-swizzled boxes), block scales and activations are
@@ -14,8 +14,8 @@
 //    completing on one mbarrier per stage;
 //  * eight consumer warps dequantise in registers and feed m16n8k16 tensor-core
 //    MMAs (weights as the 16-row operand, tokens as columns), fp32 accumulate;
-//    4-bit weights with a single token go through integer MMAs on 16-bit
-//    fixed-point activations instead (the DIGITS form below);
+//    a single token goes through integer MMAs on 16-bit fixed-point activations
+//    instead (the DIGITS form below);
 //  * with programmatic dependent launch the next GEMV starts streaming its
 //    weights while this one drains; only the activation loads wait for the
 //    predecessor.
@@ -46,7 +46,7 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
@@ -85,64 +85,54 @@ struct Frag {
 // SUBNORMAL operands: the raw masked bits, i.e. fp16 subnormals u * 2^-24 (x16
 // for high nibbles); the "- shift * sum(x)" term comes from one extra MMA per
 // step against a constant operand, and results carry a 2^-24 factor.
+// The A operand of MMA f from a lane's 16 bytes (f is a constant wherever this is inlined).
 template <int BITS, bool SUBNORMAL>
-__device__ __forceinline__ void unpack(const uint4& q, uint32_t (&a)[Frag<BITS>::NF][4]) {
+__device__ __forceinline__ void unpack(const uint4& q, int f, uint32_t (&a)[4]) {
   if constexpr (BITS == 4) {
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};  // blockA.lo(k0k1) blockA.hi(k2k3) blockB.lo blockB.hi
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const uint32_t lo = w[2 * b], hi = w[2 * b + 1];
-      const uint32_t lo8 = lo >> 8, hi8 = hi >> 8;
-      if constexpr (SUBNORMAL) {
-        a[2 * b][0] = lo & 0x000F000Fu;
-        a[2 * b][1] = lo & 0x00F000F0u;
-        a[2 * b][2] = hi & 0x000F000Fu;
-        a[2 * b][3] = hi & 0x00F000F0u;
-        a[2 * b + 1][0] = lo8 & 0x000F000Fu;
-        a[2 * b + 1][1] = lo8 & 0x00F000F0u;
-        a[2 * b + 1][2] = hi8 & 0x000F000Fu;
-        a[2 * b + 1][3] = hi8 & 0x00F000F0u;
-      } else {
-        const uint32_t kLo = 0x64086408u;  // half2(1032): 1024 + 8
-        const uint32_t kHi = 0x64806480u;  // half2(1152): 1024 + 16*8
-        a[2 * b][0] = hsub2_u32(lop3_and_or(lo, 0x000F000Fu, 0x64006400u), kLo);
-        a[2 * b][1] = hsub2_u32(lop3_and_or(lo, 0x00F000F0u, 0x64006400u), kHi);
-        a[2 * b][2] = hsub2_u32(lop3_and_or(hi, 0x000F000Fu, 0x64006400u), kLo);
-        a[2 * b][3] = hsub2_u32(lop3_and_or(hi, 0x00F000F0u, 0x64006400u), kHi);
-        a[2 * b + 1][0] = hsub2_u32(lop3_and_or(lo8, 0x000F000Fu, 0x64006400u), kLo);
-        a[2 * b + 1][1] = hsub2_u32(lop3_and_or(lo8, 0x00F000F0u, 0x64006400u), kHi);
-        a[2 * b + 1][2] = hsub2_u32(lop3_and_or(hi8, 0x000F000Fu, 0x64006400u), kLo);
-        a[2 * b + 1][3] = hsub2_u32(lop3_and_or(hi8, 0x00F000F0u, 0x64006400u), kHi);
-      }
+    // blockA.lo(k0k1) blockA.hi(k2k3) blockB.lo blockB.hi
+    const uint32_t lo = f < 2 ? q.x : q.z, hi = f < 2 ? q.y : q.w;
+    const uint32_t l = (f & 1) ? lo >> 8 : lo, h = (f & 1) ? hi >> 8 : hi;
+    if constexpr (SUBNORMAL) {
+      a[0] = l & 0x000F000Fu;
+      a[1] = l & 0x00F000F0u;
+      a[2] = h & 0x000F000Fu;
+      a[3] = h & 0x00F000F0u;
+    } else {
+      const uint32_t kLo = 0x64086408u;  // half2(1032): 1024 + 8
+      const uint32_t kHi = 0x64806480u;  // half2(1152): 1024 + 16*8
+      a[0] = hsub2_u32(lop3_and_or(l, 0x000F000Fu, 0x64006400u), kLo);
+      a[1] = hsub2_u32(lop3_and_or(l, 0x00F000F0u, 0x64006400u), kHi);
+      a[2] = hsub2_u32(lop3_and_or(h, 0x000F000Fu, 0x64006400u), kLo);
+      a[3] = hsub2_u32(lop3_and_or(h, 0x00F000F0u, 0x64006400u), kHi);
     }
   } else {
     // bytes: q.x = k0:(n0..n3), q.y = k1, q.z = k2, q.w = k3
-    const uint32_t p01 = prmt(q.x, q.y, 0x5140u);  // [k0n0 k1n0 k0n1 k1n1]
-    const uint32_t p23 = prmt(q.z, q.w, 0x5140u);
-    const uint32_t r01 = prmt(q.x, q.y, 0x7362u);  // [k0n2 k1n2 k0n3 k1n3]
-    const uint32_t r23 = prmt(q.z, q.w, 0x7362u);
+    const uint32_t sel = f == 0 ? 0x5140u : 0x7362u;   // outputs 0, 1 or 2, 3
+    const uint32_t k01 = prmt(q.x, q.y, sel), k23 = prmt(q.z, q.w, sel);  // [k0 n, k1 n, k0 n+1, k1 n+1], ...
     if constexpr (SUBNORMAL) {
-      a[0][0] = prmt(p01, 0u, 0x4140u);
-      a[0][1] = prmt(p01, 0u, 0x4342u);
-      a[0][2] = prmt(p23, 0u, 0x4140u);
-      a[0][3] = prmt(p23, 0u, 0x4342u);
-      a[1][0] = prmt(r01, 0u, 0x4140u);
-      a[1][1] = prmt(r01, 0u, 0x4342u);
-      a[1][2] = prmt(r23, 0u, 0x4140u);
-      a[1][3] = prmt(r23, 0u, 0x4342u);
+      a[0] = prmt(k01, 0u, 0x4140u);
+      a[1] = prmt(k01, 0u, 0x4342u);
+      a[2] = prmt(k23, 0u, 0x4140u);
+      a[3] = prmt(k23, 0u, 0x4342u);
     } else {
       const uint32_t kM = 0x64646464u;
       const uint32_t kOff = 0x64806480u;  // half2(1152) = 1024 + 128
-      a[0][0] = hsub2_u32(prmt(p01, kM, 0x4140u), kOff);
-      a[0][1] = hsub2_u32(prmt(p01, kM, 0x4342u), kOff);
-      a[0][2] = hsub2_u32(prmt(p23, kM, 0x4140u), kOff);
-      a[0][3] = hsub2_u32(prmt(p23, kM, 0x4342u), kOff);
-      a[1][0] = hsub2_u32(prmt(r01, kM, 0x4140u), kOff);
-      a[1][1] = hsub2_u32(prmt(r01, kM, 0x4342u), kOff);
-      a[1][2] = hsub2_u32(prmt(r23, kM, 0x4140u), kOff);
-      a[1][3] = hsub2_u32(prmt(r23, kM, 0x4342u), kOff);
+      a[0] = hsub2_u32(prmt(k01, kM, 0x4140u), kOff);
+      a[1] = hsub2_u32(prmt(k01, kM, 0x4342u), kOff);
+      a[2] = hsub2_u32(prmt(k23, kM, 0x4140u), kOff);
+      a[3] = hsub2_u32(prmt(k23, kM, 0x4342u), kOff);
     }
   }
+}
+
+// The bytes of a 4x4 block turned round: word i of `out` is byte i of the four words.
+__device__ __forceinline__ void transpose_bytes(const uint4& q, uint32_t (&out)[4]) {
+  const uint32_t a = prmt(q.x, q.y, 0x5140u), b = prmt(q.x, q.y, 0x7362u);
+  const uint32_t c = prmt(q.z, q.w, 0x5140u), d = prmt(q.z, q.w, 0x7362u);
+  out[0] = prmt(a, c, 0x5410u);
+  out[1] = prmt(a, c, 0x7632u);
+  out[2] = prmt(b, d, 0x5410u);
+  out[3] = prmt(b, d, 0x7632u);
 }
 
 // --------------------------------------------------------- cluster primitives
@@ -188,26 +178,34 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 
 // W: weight boxes per stage (strip width up to W * 128 bytes per pass).
 // MONE: single-token launch (only token column 0 is kept).
-// DIGITS (4-bit weights, one token, a one-token activation vector): integer MMAs instead.  The whole
+// DIGITS (one token, a one-token activation vector): integer MMAs instead.  The whole
 // activation vector is fetched once, and before the first stage is consumed the warps turn every unit
 // of 32 inputs into 16-bit fixed point with a power-of-two scale of its own, x ~ s (256 hi + lo).  One
-// m16n8k32 u8 x s8 MMA per 16 outputs and unit then multiplies the nibbles, as the bytes of the reference
-// layout that hold two outputs each, by the unit's two digits; four units share accumulators (their
-// digits sit in different B columns), so a stage costs 64 MMAs where the fp16 form needs 144, with two
-// byte permutes per MMA instead of shifts and masks.  Everything is exact in int32; the error is that
-// of the fixed point, at most 2^-16 of the unit's largest input per input.
-template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false>
+// m16n8k32 u8 x s8 MMA per 16 outputs and unit then multiplies the stored weights (4 bits: as the bytes of the
+// reference layout, which hold two outputs each; 8 bits: bytes of a block turned round) by the unit's two digits; four
+// units share accumulators (their digits sit in different B columns).  A 4-bit stage costs 64 MMAs where the fp16 form
+// needs 144, an 8-bit stage 32 against 96, and an fp16 MMA occupies the pipe twice as long: the 8-bit form was bound by
+// it (151936 x 2048: 64.0 us before).  Everything is exact in int32; the error is that of the fixed point, at most
+// 2^-16 of the unit's largest input per input.
+// SPLIT: more than eight tokens (an MMA's columns) are split over the warps: 2^ts_shift warps share 8 << ts_shift k-slice rows
+// of a stage and take eight tokens each.  They unpack the same weights, which costs less than the MMAs, and a lane's
+// accumulators stay eight tokens wide, so that two CTAs still fit an SM.
+// ZP: a zero point per scale; a second box of the scales' shape follows them in the stage.  (u - 8 - z) s x summed
+// over a group is s (sum(u x) - (1 + z / 8) 8 sum(x)), so the zero point only scales the offset term, in fp32
+// (2048 x 4096 INT4, 12 tokens: 9.2 us; the general kernel, which took such weights before, 45.8).
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT>
 __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     fc_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
-                    StripArgs a) {
+                    const __grid_constant__ CUtensorMap tmap_z, StripArgs a) {
   using F = Frag<BITS>;
+  static_assert(!ZP || SUBNORMAL, "the offset term comes from the constant operand of the subnormal form");
   constexpr int WT = W * F::BOX_N;       // outputs per pass
   constexpr int NJ = MONE ? 2 : 4;       // accumulator values kept per fragment
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* red = reinterpret_cast<float*>(smem + (size_t)a.stages * a.stage_bytes);  // [warps][WT][red_m]
-  float* peer = red + kConsumerWarps * WT * a.red_m;                                // [WT][red_m]
-  uint64_t* full = reinterpret_cast<uint64_t*>(peer + ((WT * a.red_m + 1) & ~1));
+  float* peer = red + kConsumerWarps * WT * a.red_m;                                // [WT][peer_m]
+  uint64_t* full = reinterpret_cast<uint64_t*>(peer + ((WT * a.peer_m + 1) & ~1));
   uint64_t* empty = full + a.stages;
   uint64_t* peer_bar = empty + a.stages;
   // DIGITS: the activation vector of this CTA's K range, digitised in place ([unit][hi: 8 words][lo: 8 words],
@@ -222,8 +220,12 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
 
   // strip -> chunk range (16-byte chunks of a weight row), balanced to one unit
   const int64_t u_lo = (int64_t)strip * a.units / a.strips, u_hi = (int64_t)(strip + 1) * a.units / a.strips;
-  const int cs = static_cast<int>(u_lo) * a.gran, ce = static_cast<int>(u_hi) * a.gran;
-  const int passes = (ce - cs + W * 8 - 1) / (W * 8);
+  // (interleaved: the passes of all strips side by side, pass p of strip s being the grid's (p strips + s)-th box or
+  // pair of boxes, so that what the SMs read at a time is one contiguous piece of every weight row)
+  const int cs = a.interleave ? strip * W * 8 : static_cast<int>(u_lo) * a.gran;
+  const int ce = a.interleave ? a.units * a.gran : static_cast<int>(u_hi) * a.gran;
+  const int pass_step = a.interleave ? a.strips * W * 8 : W * 8;
+  const int passes = (ce - cs + pass_step - 1) / pass_step;
   const int r_lo = kr * a.rows_per_split;
   const int r_hi = min(a.src_slices, r_lo + a.rows_per_split);
   const int n_st = (r_hi - r_lo + kStageRows - 1) / kStageRows;
@@ -261,20 +263,26 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     if (n_st > 0) {
       const uint64_t pol = policy_evict_first();
       const int total = passes * n_st;
-      const uint32_t s_bytes = a.scale_rows > 0 ? static_cast<uint32_t>(a.scale_rows) * WT * 2u : 0u;
+      const uint32_t s_bytes = a.scale_rows > 0 ? static_cast<uint32_t>(a.scale_rows) * WT * (ZP ? 4u : 2u) : 0u;
       auto issue_weights = [&](int item, int stage) {
         const int pass = item / n_st, si = item % n_st;
         uint8_t* st = smem + (size_t)stage * a.stage_bytes;
         const int row0 = r_lo + si * kStageRows;
         const int rows = min(kStageRows, r_hi - row0);
-        const int chunk0 = cs + pass * W * 8;
-        mbar_arrive_expect_tx(&full[stage],
-                              W * kBoxBytes + s_bytes + (DIGITS ? 0u : static_cast<uint32_t>(rows) * a.M_total * 8u));
+        const int chunk0 = cs + pass * pass_step;
+        // (boxes past the end of the strip, in its last pass, are not fetched: their sums, of whatever the stage held, are
+        // not stored)
+        const int boxes = min(W, (ce - chunk0 + 7) / 8);
+        mbar_arrive_expect_tx(&full[stage], boxes * kBoxBytes + s_bytes +
+                                                (DIGITS ? 0u : static_cast<uint32_t>(rows) * a.M_total * 8u));
 #pragma unroll
         for (int b = 0; b < W; ++b)
-          tma_load_2d_hint(st + b * kBoxBytes, &tmap_w, &full[stage], (chunk0 + b * 8) * 16, row0, pol);
-        if (a.scale_rows > 0)
+          if (b < boxes) tma_load_2d_hint(st + b * kBoxBytes, &tmap_w, &full[stage], (chunk0 + b * 8) * 16, row0, pol);
+        if (a.scale_rows > 0) {
           tma_load_2d(st + W * kBoxBytes, &tmap_s, &full[stage], chunk0 * F::NPL, row0 / a.group_slices);
+          if constexpr (ZP)
+            tma_load_2d(st + W * kBoxBytes + a.zp_off, &tmap_z, &full[stage], chunk0 * F::NPL, row0 / a.group_slices);
+        }
       };
       auto issue_x = [&](int item, int stage) {
         if constexpr (DIGITS) return;  // the whole vector is fetched once, below
@@ -350,7 +358,6 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   constexpr uint32_t kOnesA = BITS == 4 ? 0x00080008u : 0x00800080u;  // subnormal 8 / 128
   constexpr float kOdd = BITS == 4 ? 0.0625f : 1.0f;                  // high nibbles are carried x16
   constexpr float kOutScale = (SUBNORMAL && !DIGITS) ? 16777216.0f : 1.0f;
-  const int rbase = warp * 8;
   int stage = 0;
   uint32_t phase = 0;
   bool failed = false;
@@ -423,7 +430,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
           uint32_t* ud = reinterpret_cast<uint32_t*>(xdig + (size_t)u * 64);
           *reinterpret_cast<uint2*>(ud + 2 * q) = make_uint2(hiw[0], hiw[1]);
           *reinterpret_cast<uint2*>(ud + 8 + 2 * q) = make_uint2(low[0], low[1]);
-          if (q == 0) xmeta[u] = make_uint2(bad ? 0x7FC00000u : sbits, static_cast<uint32_t>(8 * isum));  // (nibbles = weights + 8)
+          if (q == 0) xmeta[u] = make_uint2(bad ? 0x7FC00000u : sbits, static_cast<uint32_t>((BITS == 4 ? 8 : 128) * isum));  // (stored weights = weights + 8, + 128)
         }
       }
     }
@@ -438,6 +445,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       for (int f = 0; f < F::NF; ++f)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) tot[b][f][j] = 0.0f;
+    [[maybe_unused]] const int boxes = min(W, (ce - cs - pass * pass_step + 7) / 8);  // of this pass
 
     for (int si = 0; si < n_st; ++si) {
 #ifdef MLD_TRACE
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       const uint8_t* xs = st + W * kBoxBytes + a.scale_stage_bytes;
       const int row0 = r_lo + si * kStageRows;
       if constexpr (DIGITS) {
-        static_assert(!DIGITS || (BITS == 4 && MONE), "the digit form is for 4-bit weights and one token");
+        static_assert(!DIGITS || MONE, "the digit form is for one token");
         // A stage is 2 W tasks: (half of its 64 k-slice rows = four units) x (box of 64 outputs).  The four
         // units of a task share accumulators: B column 2 j holds the high and 2 j + 1 the low digits of unit j
         // (lanes g supply column g, zero for the other units), so after the units' MMAs lane t holds both
@@ -475,13 +483,13 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         constexpr int T = W == 3 ? 8 : 2 * W;
         constexpr int GC = kConsumerWarps / T;
         const int task = warp % T, tb = task >> 1, hq = task & 1;
-        if (tb < W && si % GC == warp / T) {
+        if (tb < boxes && si % GC == warp / T) {
           const int ubase = si * 8 + hq * 4;  // the task's first unit within the CTA's K range
           const uint32_t* ud = reinterpret_cast<const uint32_t*>(xdig + (size_t)(ubase + (g >> 1)) * 64) + 8 * (g & 1);
           const uint32_t bm0 = ud[t], bm1 = ud[4 + t];
-          int acc[4][4];
+          int acc[F::NF][4];
 #pragma unroll
-          for (int f = 0; f < 4; ++f) acc[f][0] = acc[f][1] = acc[f][2] = acc[f][3] = 0;
+          for (int f = 0; f < F::NF; ++f) acc[f][0] = acc[f][1] = acc[f][2] = acc[f][3] = 0;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             // k-slice rows ra and ra + 4 of unit j are what lane t feeds the MMA's K with
@@ -490,55 +498,90 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
             const uint4 qb = *reinterpret_cast<const uint4*>(st + tb * kBoxBytes + rb * 128 + ((g ^ (rb & 7)) << 4));
             const bool mine = (g >> 1) == j;
             const uint32_t b0 = mine ? bm0 : 0u, b1 = mine ? bm1 : 0u;
+            if constexpr (BITS == 4) {
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-              // outputs 2f (low nibbles) and 2f + 1 (high nibbles) of this lane's eight: byte i of a block word is
-              // input i / 2, output pair i % 2, so the four inputs of a pair are bytes 0, 2 (or 1, 3) of the two words
-              const uint32_t sel = (f & 1) ? 0x7531u : 0x6420u;
-              const uint32_t wa = f < 2 ? prmt(qa.x, qa.y, sel) : prmt(qa.z, qa.w, sel);
-              const uint32_t wb = f < 2 ? prmt(qb.x, qb.y, sel) : prmt(qb.z, qb.w, sel);
-              // rows g take the whole byte (even output + 16 x odd output), rows g + 8 the odd output x 16
-              const uint32_t af[4] = {wa, wa & 0xF0F0F0F0u, wb, wb & 0xF0F0F0F0u};
-              mma_u8s8(acc[f], af, b0, b1);
+              for (int f = 0; f < 4; ++f) {
+                // outputs 2f (low nibbles) and 2f + 1 (high nibbles) of this lane's eight: byte i of a block word is
+                // input i / 2, output pair i % 2, so the four inputs of a pair are bytes 0, 2 (or 1, 3) of the two words
+                const uint32_t sel = (f & 1) ? 0x7531u : 0x6420u;
+                const uint32_t wa = f < 2 ? prmt(qa.x, qa.y, sel) : prmt(qa.z, qa.w, sel);
+                const uint32_t wb = f < 2 ? prmt(qb.x, qb.y, sel) : prmt(qb.z, qb.w, sel);
+                // rows g take the whole byte (even output + 16 x odd output), rows g + 8 the odd output x 16
+                const uint32_t af[4] = {wa, wa & 0xF0F0F0F0u, wb, wb & 0xF0F0F0F0u};
+                mma_u8s8(acc[f], af, b0, b1);
+              }
+            } else {
+              // a block is four inputs (words) x four outputs (bytes): turned round, a word is an output's four inputs
+              uint32_t wa[4], wb[4];
+              transpose_bytes(qa, wa);
+              transpose_bytes(qb, wb);
+#pragma unroll
+              for (int f = 0; f < 2; ++f) {
+                const uint32_t af[4] = {wa[2 * f], wa[2 * f + 1], wb[2 * f], wb[2 * f + 1]};  // rows g, g + 8: outputs 2f, 2f + 1
+                mma_u8s8(acc[f], af, b0, b1);
+              }
             }
           }
           // lane t finishes unit t: its digit scale and offset, the weight scales of its group
           const uint2 meta = xmeta[ubase + t];
           const float sx = __uint_as_float(meta.x);
           const int off = static_cast<int>(meta.y);
-          float sc[8];
+          float sc[F::NPL], zo[F::NPL];
+          const int gidx = a.gs_shift >= 0 ? ((32 * hq + 8 * t) >> a.gs_shift) : 0;
+          const auto load_params = [&](const uint8_t* box, float (&v)[F::NPL]) {
+            const __half* p = reinterpret_cast<const __half*>(box) + gidx * WT + tb * F::BOX_N + F::NPL * g;
+#pragma unroll
+            for (int i = 0; i < F::NPL / 4; ++i) {
+              const uint2 w = reinterpret_cast<const uint2*>(p)[i];
+              const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
+              const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+              v[4 * i] = f0.x; v[4 * i + 1] = f0.y; v[4 * i + 2] = f1.x; v[4 * i + 3] = f1.y;
+            }
+          };
           if (a.scale_rows > 0) {
-            const int gidx = a.gs_shift >= 0 ? ((32 * hq + 8 * t) >> a.gs_shift) : 0;
-            const __half* sp = reinterpret_cast<const __half*>(st + W * kBoxBytes) + gidx * WT + tb * F::BOX_N + F::NPL * g;
-            const uint4 sv = *reinterpret_cast<const uint4*>(sp);
-            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
-            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
-            const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&sv.z));
-            const float2 f3 = __half22float2(*reinterpret_cast<const __half2*>(&sv.w));
-            sc[0] = f0.x; sc[1] = f0.y; sc[2] = f1.x; sc[3] = f1.y;
-            sc[4] = f2.x; sc[5] = f2.y; sc[6] = f3.x; sc[7] = f3.y;
+            load_params(st + W * kBoxBytes, sc);
           } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) sc[i] = a.scalar_scale;
+            for (int i = 0; i < F::NPL; ++i) sc[i] = a.scalar_scale;
+          }
+          if constexpr (ZP) {  // the zero point's share of the unit, z sum(x), in units of the digit scale
+            load_params(st + W * kBoxBytes + a.zp_off, zo);
+            const float isum = static_cast<float>(off) * (BITS == 4 ? 0.125f : 0.0078125f);
+#pragma unroll
+            for (int i = 0; i < F::NPL; ++i) zo[i] *= isum;
           }
           // acc: {row g high digit, row g low, row g + 8 high, row g + 8 low} of unit t
 #pragma unroll
-          for (int f = 0; f < 4; ++f) {
-            const int even = (acc[f][0] - acc[f][2]) * 256 + (acc[f][1] - acc[f][3]) - off;
-            const int odd = ((acc[f][2] * 256 + acc[f][3]) >> 4) - off;
-            tot[0][f][0] = fmaf(sc[2 * f] * sx, static_cast<float>(even), tot[0][f][0]);
-            tot[0][f][1] = fmaf(sc[2 * f + 1] * sx, static_cast<float>(odd), tot[0][f][1]);
+          for (int f = 0; f < F::NF; ++f) {
+            int even, odd;
+            if constexpr (BITS == 4) {
+              even = (acc[f][0] - acc[f][2]) * 256 + (acc[f][1] - acc[f][3]) - off;
+              odd = ((acc[f][2] * 256 + acc[f][3]) >> 4) - off;
+            } else {  // (|sum| <= 32 * 255 * 32640 < 2^28)
+              even = acc[f][0] * 256 + acc[f][1] - off;
+              odd = acc[f][2] * 256 + acc[f][3] - off;
+            }
+            float ev = static_cast<float>(even), od = static_cast<float>(odd);
+            if constexpr (ZP) {
+              ev -= zo[2 * f];
+              od -= zo[2 * f + 1];
+            }
+            tot[0][f][0] = fmaf(sc[2 * f] * sx, ev, tot[0][f][0]);
+            tot[0][f][1] = fmaf(sc[2 * f + 1] * sx, od, tot[0][f][1]);
           }
         }
       } else {
-        // activation fragments of this warp's eight rows (two steps)
+        // eight rows (two steps) of the stage at a time: one per stage, or the 2^ts_shift of this warp's group
+        const int n_rr = SPLIT ? 1 << a.ts_shift : 1, token = (warp & (n_rr - 1)) * 8 + g;
+        for (int rr = 0; rr < n_rr; ++rr) {
+        const int rbase = ((warp & ~(n_rr - 1)) + rr) * 8;
         uint32_t bx[2][2];
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
           const int r = rbase + 2 * t + p;
           bx[p][0] = bx[p][1] = 0u;
-          if (row0 + r < r_hi && g < a.M) {
-            const uint2 xv = *reinterpret_cast<const uint2*>(xs + ((size_t)r * a.M_total + a.tok0 + g) * 8);
+          if (row0 + r < r_hi && token < a.M) {
+            const uint2 xv = *reinterpret_cast<const uint2*>(xs + ((size_t)r * a.M_total + a.tok0 + token) * 8);
             bx[p][0] = xv.x;
             bx[p][1] = xv.y;
           }
@@ -559,48 +602,62 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
           for (int p = 0; p < 2; ++p) {
             const int r = rbase + 2 * t + p;
             const uint4 q = *reinterpret_cast<const uint4*>(st + b * kBoxBytes + r * 128 + ((g ^ (r & 7)) << 4));
-            uint32_t av[F::NF][4];
-            unpack<BITS, SUBNORMAL>(q, av);
 #pragma unroll
-            for (int f = 0; f < F::NF; ++f) mma_f16(grp[f], av[f], bx[p][0], bx[p][1]);
+            for (int f = 0; f < F::NF; ++f) {
+              uint32_t av[4];
+              unpack<BITS, SUBNORMAL>(q, f, av);
+              mma_f16(grp[f], av, bx[p][0], bx[p][1]);
+            }
           }
-          // scales of this lane's outputs for the group these eight rows are in
-          float sc[F::NPL];
-          if (a.scale_rows > 0) {
-            const __half* sp = reinterpret_cast<const __half*>(st + W * kBoxBytes) + gidx * WT + b * F::BOX_N + F::NPL * g;
+          // scales (and zero points) of this lane's outputs for the group these eight rows are in
+          float sc[F::NPL], zf[F::NPL];
+          const auto load_params = [&](const uint8_t* box, float (&v)[F::NPL]) {
+            const __half* sp = reinterpret_cast<const __half*>(box) + gidx * WT + b * F::BOX_N + F::NPL * g;
+            uint32_t w[F::NPL / 2];
             if constexpr (BITS == 4) {
               const uint4 sv = *reinterpret_cast<const uint4*>(sp);
-              const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
-              const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
-              const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&sv.z));
-              const float2 f3 = __half22float2(*reinterpret_cast<const __half2*>(&sv.w));
-              sc[0] = f0.x; sc[1] = f0.y; sc[2] = f1.x; sc[3] = f1.y;
-              sc[4] = f2.x; sc[5] = f2.y; sc[6] = f3.x; sc[7] = f3.y;
+              w[0] = sv.x; w[1] = sv.y; w[2] = sv.z; w[3] = sv.w;
             } else {
               const uint2 sv = *reinterpret_cast<const uint2*>(sp);
-              const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&sv.x));
-              const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&sv.y));
-              sc[0] = f0.x; sc[1] = f0.y; sc[2] = f1.x; sc[3] = f1.y;
+              w[0] = sv.x; w[1] = sv.y;
             }
+#pragma unroll
+            for (int i = 0; i < F::NPL / 2; ++i) {
+              const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+              v[2 * i] = f2.x;
+              v[2 * i + 1] = f2.y;
+            }
+          };
+          if (a.scale_rows > 0) {
+            load_params(st + W * kBoxBytes, sc);
           } else {
 #pragma unroll
             for (int i = 0; i < F::NPL; ++i) sc[i] = a.scalar_scale;
           }
+          if constexpr (ZP) {
+            load_params(st + W * kBoxBytes + a.zp_off, zf);
+#pragma unroll
+            for (int i = 0; i < F::NPL; ++i) zf[i] = fmaf(zf[i], BITS == 4 ? 0.125f : 0.0078125f, 1.0f);
+          }
           // row g of MMA f is output 2f, row g+8 is output 2f+1
 #pragma unroll
-          for (int f = 0; f < F::NF; ++f)
+          for (int f = 0; f < F::NF; ++f) {
 #pragma unroll
             for (int jj = 0; jj < NJ; ++jj) {
               const int j = MONE ? 2 * jj : jj;  // MONE keeps (row g, token 2t) and (row g+8, token 2t)
               const bool odd = (j & 2) != 0;
               float v = grp[f][j];
               if constexpr (SUBNORMAL) {
-                v = odd ? fmaf(v, kOdd, -ones[j & 1]) : (v - ones[j & 1]);
+                float offset = ones[j & 1];
+                if constexpr (ZP) offset *= zf[2 * f + (odd ? 1 : 0)];
+                v = odd ? fmaf(v, kOdd, -offset) : (v - offset);
               } else {
                 if (odd) v *= kOdd;
               }
               tot[b][f][jj] = fmaf(sc[2 * f + (odd ? 1 : 0)], v, tot[b][f][jj]);
             }
+          }
+        }
         }
       }
       __syncwarp();
@@ -623,13 +680,18 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
 
     // ------------------------------------------------ pass epilogue
     if (tr && threadIdx.x == 0) tr[4] = globaltimer_ns();
+    const int chunk0 = cs + pass * pass_step;
+    const int n0 = chunk0 * F::NPL;               // first output of this pass
+    const int n_end = min(ce * F::NPL, a.N4);      // one past the last output this CTA owns
+    const int n_rr = SPLIT ? 1 << a.ts_shift : 1;
+    uint32_t peer_remote = 0, bar_remote = 0;
     if constexpr (DIGITS) {
       // tot[0] is this warp's box (tb) summed over the units the lane finished: add the four lanes t up; the
       // warp contributes nothing to the other boxes
       constexpr int T = W == 3 ? 8 : 2 * W;
       const int tb = (warp % T) >> 1;
 #pragma unroll
-      for (int f = 0; f < 4; ++f)
+      for (int f = 0; f < F::NF; ++f)
 #pragma unroll
         for (int jj = 0; jj < 2; ++jj) {
           float v = tot[0][f][jj];
@@ -651,15 +713,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
             const int j = MONE ? 2 * jj : jj;
             const int n_local = b * F::BOX_N + F::NPL * g + 2 * f + ((j >> 1) & 1);
             const int tok = 2 * t + (j & 1);
-            if (tok < a.M) red[(warp * WT + n_local) * a.red_m + tok] = tot[b][f][jj];
+            if (SPLIT || tok < a.M) red[(warp * WT + n_local) * a.red_m + tok] = tot[b][f][jj];
           }
     }
     MLD_CONSUMER_BARRIER();
-    const int chunk0 = cs + pass * W * 8;
-    const int n0 = chunk0 * F::NPL;               // first output of this pass
-    const int n_end = min(ce * F::NPL, a.N4);      // one past the last output this CTA owns
-    const int nvals = WT * a.M;
-    uint32_t peer_remote = 0, bar_remote = 0;
     if (a.ksplit > 1 && pass == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (a.ksplit > 1 && kr == 1) {
       peer_remote = map_to_rank(smem_u32(peer), 0);
@@ -671,39 +728,41 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         failed = true;
       }
     }
+    // the sum of output n_local for a token over the warps that hold a share of it: all of them, or every n_rr-th
+    const auto warp_sum = [&](int n_local, int tok) {
+      float v = 0.0f;
+      if (SPLIT) {
+        for (int w = tok >> 3; w < kConsumerWarps; w += n_rr) v += red[(w * WT + n_local) * a.red_m + (tok & 7)];
+      } else {
+#pragma unroll
+        for (int w = 0; w < kConsumerWarps; ++w) v += red[(w * WT + n_local) * a.red_m + tok];
+      }
+      return v;
+    };
     if (a.ksplit > 1 && kr == 1) {
       // upper half of K: hand the sums to the partner
-      for (int idx = threadIdx.x; idx < nvals && !failed; idx += kConsumerWarps * 32) {
+      for (int idx = threadIdx.x; idx < WT * a.M && !failed; idx += kConsumerWarps * 32) {
         const int n_local = idx / a.M, tok = idx - n_local * a.M;
-        float s = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kConsumerWarps; ++w) s += red[(w * WT + n_local) * a.red_m + tok];
-        st_cluster_f32(peer_remote + (n_local * a.red_m + tok) * 4, s);
+        st_cluster_f32(peer_remote + (n_local * a.peer_m + tok) * 4, warp_sum(n_local, tok));
       }
     } else if (a.epilogue == MLD_EPILOGUE_SWIGLU_PAIRS) {
       // rows alternate gate_i, up_i: out[i] = silu(gate_i) * up_i, each rounded to
       // fp16 where the unfused graph would store it
-      const int npairs = (WT / 2) * a.M;
-      for (int idx = threadIdx.x; idx < npairs && !failed; idx += kConsumerWarps * 32) {
+      for (int idx = threadIdx.x; idx < (WT / 2) * a.M && !failed; idx += kConsumerWarps * 32) {
         const int p_local = idx / a.M, tok = idx - p_local * a.M;
-        float sg = 0.0f, su = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kConsumerWarps; ++w) {
-          sg += red[(w * WT + 2 * p_local) * a.red_m + tok];
-          su += red[(w * WT + 2 * p_local + 1) * a.red_m + tok];
-        }
+        float sg = warp_sum(2 * p_local, tok), su = warp_sum(2 * p_local + 1, tok);
         if (a.ksplit > 1) {
-          sg += peer[(2 * p_local) * a.red_m + tok];
-          su += peer[(2 * p_local + 1) * a.red_m + tok];
+          sg += peer[(2 * p_local) * a.peer_m + tok];
+          su += peer[(2 * p_local + 1) * a.peer_m + tok];
         }
         const int n = n0 + 2 * p_local;
         if (n + 1 < n_end) {
           const float g = __half2float(__float2half_rn(sg * kOutScale));
           const float u = __half2float(__float2half_rn(su * kOutScale));
           const __half r = __float2half_rn(g / (1.0f + __expf(-g)) * u);
-          const int i = n >> 1, tk = a.tok0 + tok;
-          const int64_t yi = a.dst_layout == MLD_LAYOUT_SLICED ? (((int64_t)(i >> 2) * a.M_total + tk) * 4 + (i & 3))
-                                                               : ((int64_t)tk * (a.N / 2) + i);
+          const int i = n >> 1, tk_out = a.tok0 + tok;
+          const int64_t yi = a.dst_layout == MLD_LAYOUT_SLICED ? (((int64_t)(i >> 2) * a.M_total + tk_out) * 4 + (i & 3))
+                                                               : ((int64_t)tk_out * (a.N / 2) + i);
           if (a.scatter.world > 1) {
             for (int pr = 0; pr < a.scatter.world; ++pr) static_cast<__half*>(a.scatter.y_peers[pr])[yi] = r;
           } else {
@@ -712,25 +771,22 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         }
       }
     } else {
-      for (int idx = threadIdx.x; idx < nvals && !failed; idx += kConsumerWarps * 32) {
+      for (int idx = threadIdx.x; idx < WT * a.M && !failed; idx += kConsumerWarps * 32) {
         const int n_local = idx / a.M, tok = idx - n_local * a.M;
-        float s = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kConsumerWarps; ++w) s += red[(w * WT + n_local) * a.red_m + tok];
-        if (a.ksplit > 1) s += peer[n_local * a.red_m + tok];  // fixed order: lower half of K first
         const int n = n0 + n_local;
-        if (n < n_end) {
-          __half r = __float2half_rn(s * kOutScale);
-          if (a.bias != nullptr) r = __hadd(r, static_cast<const __half*>(a.bias)[n]);
-          const int tk = a.tok0 + tok;
-          const int64_t yi = a.dst_layout == MLD_LAYOUT_SLICED ? (((int64_t)(n >> 2) * a.M_total + tk) * 4 + (n & 3))
-                                                               : ((int64_t)tk * a.N + n);
-          if (a.dst_layout == MLD_LAYOUT_SLICED || n < a.N) {
-            if (a.scatter.world > 1) {
-              for (int pr = 0; pr < a.scatter.world; ++pr) static_cast<__half*>(a.scatter.y_peers[pr])[yi] = r;
-            } else {
-              static_cast<__half*>(a.y)[yi] = r;
-            }
+        if (n >= n_end) continue;
+        float s = warp_sum(n_local, tok);
+        if (a.ksplit > 1) s += peer[n_local * a.peer_m + tok];  // fixed order: lower half of K first
+        __half r = __float2half_rn(s * kOutScale);
+        if (a.bias != nullptr) r = __hadd(r, static_cast<const __half*>(a.bias)[n]);
+        const int tk_out = a.tok0 + tok;
+        const int64_t yi = a.dst_layout == MLD_LAYOUT_SLICED ? (((int64_t)(n >> 2) * a.M_total + tk_out) * 4 + (n & 3))
+                                                             : ((int64_t)tk_out * a.N + n);
+        if (a.dst_layout == MLD_LAYOUT_SLICED || n < a.N) {
+          if (a.scatter.world > 1) {
+            for (int pr = 0; pr < a.scatter.world; ++pr) static_cast<__half*>(a.scatter.y_peers[pr])[yi] = r;
+          } else {
+            static_cast<__half*>(a.y)[yi] = r;
           }
         }
       }
@@ -756,10 +812,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   }
 }
 
-template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false>
-int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const StripArgs& a, const StripGeometry& gm,
-                   cudaStream_t stream) {
-  auto kern = fc_strip_kernel<BITS, W, SUBNORMAL, MONE, DIGITS>;
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false, bool ZP = false, bool SPLIT = false>
+int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
+                   const StripGeometry& gm, cudaStream_t stream) {
+  auto kern = fc_strip_kernel<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT>;
   static bool configured[kMaxDevices];  // per instantiation and device
   int dev;
   if (needs_configure(configured, &dev)) {
@@ -787,50 +843,66 @@ int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const StripArgs
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
-  MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tw, ts, a));
+  MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tw, ts, tz, a));
   count_launch();
   return MLD_OK;
 }
 
-template <int BITS, int W>
-int launch_strip_w(bool subnormal, bool mone, const CUtensorMap& tw, const CUtensorMap& ts, const StripArgs& a,
-                   const StripGeometry& gm, cudaStream_t stream) {
-  if (subnormal) {
-    if constexpr (BITS == 4) {
-      if (mone && a.M_total == 1 && gm.xdig_bytes > 0) return launch_strip_t<BITS, W, true, true, true>(tw, ts, a, gm, stream);
-    }
-    if (mone) return launch_strip_t<BITS, W, true, true>(tw, ts, a, gm, stream);
-    return launch_strip_t<BITS, W, true, false>(tw, ts, a, gm, stream);
+template <int BITS, int W, bool ZP>
+int launch_strip_w(bool subnormal, bool mone, const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz,
+                   const StripArgs& a, const StripGeometry& gm, cudaStream_t stream) {
+  if constexpr (W <= 2) {
+    if (gm.ts_shift > 0) return launch_strip_t<BITS, W, true, false, false, ZP, true>(tw, ts, tz, a, gm, stream);
   }
-  if (mone) return launch_strip_t<BITS, W, false, true>(tw, ts, a, gm, stream);
-  return launch_strip_t<BITS, W, false, false>(tw, ts, a, gm, stream);
+  if (ZP || subnormal) {
+    if (mone && a.M_total == 1 && gm.xdig_bytes > 0)
+      return launch_strip_t<BITS, W, true, true, true, ZP>(tw, ts, tz, a, gm, stream);
+    if (mone) return launch_strip_t<BITS, W, true, true, false, ZP>(tw, ts, tz, a, gm, stream);
+    return launch_strip_t<BITS, W, true, false, false, ZP>(tw, ts, tz, a, gm, stream);
+  }
+  if constexpr (!ZP) {
+    if (mone) return launch_strip_t<BITS, W, false, true>(tw, ts, tz, a, gm, stream);
+    return launch_strip_t<BITS, W, false, false>(tw, ts, tz, a, gm, stream);
+  }
+  set_last_error_text("zero points take the subnormal operand form");
+  return MLD_INVALID_ARGUMENT;
 }
 
 }  // namespace
 
 StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slices, int scale_mode, int sms,
-                             bool pdl, int smem_limit_kb) {
+                             bool pdl, int smem_limit_kb, bool zero_point, bool split) {
   StripGeometry gm;
   memset(&gm, 0, sizeof gm);
+  // tokens per launch: an MMA's eight, or up to four times that where the warps can split them
+  gm.launch_tokens = split && pdl ? kStripTokens : 8;
+  gm.ts_shift = gm.launch_tokens == 8 ? 0 : m_total > 16 ? 2 : m_total > 8 ? 1 : 0;
   const int N4 = align_n(N, 4), SS = div_up(K, 4);
   const int box_n = bits == 4 ? 64 : 32;
   const int row_bytes = (N4 / 4) * (bits == 4 ? 8 : 16);
   gm.gran = bits == 4 ? 1 : 2;
   const int C = row_bytes / 16;
   gm.units = C / gm.gran;
+  // Overlapping launches need two CTAs per SM, which the register file grants to the instantiations of up
+  // to two boxes per stage: wider strips take more column passes instead.
+  const int w_max = pdl ? 2 : 4;
   // Two CTAs per strip (a cluster splitting K) when single strips would be
   // narrower than 128 bytes and K is long enough to halve.
   gm.ksplit = (C < 8 * sms && SS >= 4 * kStageRows && sms >= 2) ? 2 : 1;
   int strips = sms / gm.ksplit;
+  if (gm.ksplit == 1 && w_max <= 2 && C > 8 * w_max * sms) {
+    // More columns than one pass of one CTA per SM: two CTAs share each SM, so that one streams while the other is in a
+    // pass's epilogue (151936 x 2048 INT8, one token: 17 passes of a lone CTA 85.8 us, 9 of two 69.7; with the passes of
+    // all strips side by side 64.0, and with the integer digits 54.7, against 47.6 for the bytes at the copy rate).
+    strips = 2 * sms;
+    gm.interleave = C > 8 * w_max * strips ? 1 : 0;
+  }
   if (strips > gm.units) strips = gm.units;
   if (strips < 1) strips = 1;
   gm.strips = strips;
   gm.grid = strips * gm.ksplit;
   const int max_width = div_up(gm.units, strips) * gm.gran;  // chunks
   int w = div_up(max_width, 8);
-  // Overlapping launches need two CTAs per SM, which the register file grants to the instantiations of up
-  // to two boxes per stage: wider strips take more column passes instead.
-  const int w_max = pdl ? 2 : 4;
   if (gm.ksplit > 1 && w > w_max) {  // a cluster pair runs a single pass
     gm.ksplit = 1;
     strips = sms < gm.units ? sms : gm.units;
@@ -853,14 +925,16 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
         if ((1 << sh) == gm.group_slices) gm.gs_shift = sh;
   }
   const int wt = gm.w * box_n;
-  gm.scale_stage_bytes = align_n(gm.scale_rows * wt * 2, 128);
+  gm.zp_off = align_n(gm.scale_rows * wt * 2, 128);
+  gm.scale_stage_bytes = zero_point ? 2 * gm.zp_off : gm.zp_off;
   const int x_bytes = align_n(kStageRows * m_total * 8, 128);
   gm.stage_bytes = align_n(gm.w * kBoxBytes + gm.scale_stage_bytes + x_bytes, 1024);
   gm.red_m = m_total < 8 ? m_total : 8;
+  gm.peer_m = gm.ksplit == 1 ? 0 : m_total < gm.launch_tokens ? m_total : gm.launch_tokens;
   // 4-bit weights: room for a one-token activation vector of this CTA's K range as digits (8 bytes per k-slice,
   // 8 per unit of eight k-slices, a barrier)
-  gm.xdig_bytes = bits == 4 ? gm.rows_per_split * 9 + 48 : 0;
-  const int fixed = (kConsumerWarps + 1) * wt * gm.red_m * 4 + 8 + (2 * 16 + 1) * 8 + gm.xdig_bytes + 1024 + 64;
+  gm.xdig_bytes = m_total == 1 ? gm.rows_per_split * 9 + 48 : 0;
+  const int fixed = (kConsumerWarps * gm.red_m + gm.peer_m) * wt * 4 + 8 + (2 * 16 + 1) * 8 + gm.xdig_bytes + 1024 + 64;
   gm.stage_rows = kStageRows;
   // With programmatic dependent launch two consecutive GEMVs share an SM while
   // one drains and the next prefetches, so each takes at most half of it.
@@ -874,14 +948,29 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
   return gm;
 }
 
-int launch_fc_strip(int bits, bool subnormal, const CUtensorMap& tw, const CUtensorMap& ts, const StripArgs& a,
-                    const StripGeometry& gm, cudaStream_t stream) {
+int launch_fc_strip(int bits, bool subnormal, const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap* tz,
+                    const StripArgs& a, const StripGeometry& gm, cudaStream_t stream) {
   if (a.M == 0 || gm.grid == 0) return MLD_OK;
   const bool mone = a.M == 1;
 #define MLD_W(B, WV) \
   case WV:           \
-    return launch_strip_w<B, WV>(subnormal, mone, tw, ts, a, gm, stream)
-  if (bits == 4) {
+    return launch_strip_w<B, WV, false>(subnormal, mone, tw, ts, tw, a, gm, stream)
+#define MLD_WZ(B, WV) \
+  case WV:            \
+    return launch_strip_w<B, WV, true>(subnormal, mone, tw, ts, *tz, a, gm, stream)
+  if (tz != nullptr) {  // (zero points: strips of up to two boxes, see strip_serves)
+    if (bits == 4) {
+      switch (gm.w) {
+        MLD_WZ(4, 1);
+        MLD_WZ(4, 2);
+      }
+    } else {
+      switch (gm.w) {
+        MLD_WZ(8, 1);
+        MLD_WZ(8, 2);
+      }
+    }
+  } else if (bits == 4) {
     switch (gm.w) {
       MLD_W(4, 1);
       MLD_W(4, 2);
@@ -897,6 +986,7 @@ int launch_fc_strip(int bits, bool subnormal, const CUtensorMap& tw, const CUten
     }
   }
 #undef MLD_W
+#undef MLD_WZ
   set_last_error_text("bad strip geometry");
   return MLD_INVALID_ARGUMENT;
 }

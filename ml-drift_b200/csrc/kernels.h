@@ -65,12 +65,13 @@ struct PeerOutputs {
   void* y[8];
 };
 
+constexpr int kStripTokens = 32;  // tokens of one launch of the streaming kernel at most
 struct StripArgs {
   const void* x;      // fp16, sliced [K/4][M_total][4] (for one token a plain vector)
   const void* bias;   // fp16 [N4] or null
   void* y;            // fp16
   int* error;         // device error word (0 = ok)
-  int M;              // tokens handled by this launch (1..8)
+  int M;              // tokens handled by this launch (1..kStripTokens)
   int M_total;        // tokens in the x / y tensors
   int tok0;           // first token handled by this launch
   int N, N4;
@@ -82,7 +83,11 @@ struct StripArgs {
   int scale_rows;     // rows of the per-stage scale box (0 = scalar scale)
   int group_slices;   // k-slices per scale group
   int gs_shift;       // log2(group_slices) when it is a power of two below a stage, else -1
-  int red_m;          // token stride of the reduction buffers
+  int zp_off;         // where the zero-point box starts behind the scale box's start
+  int red_m;          // token stride of the reduction buffer (one token tile)
+  int peer_m;         // token stride of the cluster partner's sums
+  int ts_shift;       // 2^ts_shift warps split a launch's tokens
+  int interleave;     // a strip's passes lie a grid's width apart instead of side by side
   int dst_layout;
   int epilogue;       // mld_epilogue
   float scalar_scale;
@@ -99,12 +104,13 @@ struct StripGeometry {
   int gran, units, strips, ksplit, grid, w;
   int rows_per_split;
   int scale_rows, group_slices, gs_shift;
-  int scale_stage_bytes, stage_bytes, stages, red_m, stage_rows;
+  int scale_stage_bytes, zp_off, stage_bytes, stages, red_m, peer_m, stage_rows;
+  int ts_shift, launch_tokens, interleave;
   int xdig_bytes;  // shared memory kept for the digitised activation vector (4-bit weights), else 0
   size_t smem_bytes;
 };
 StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slices, int scale_mode, int sms,
-                             bool pdl, int smem_limit_kb = 0);
+                             bool pdl, int smem_limit_kb = 0, bool zero_point = false, bool split = true);
 // Makes the plan's kernels report their bounded waits that ran out in `word` (a device int the caller
 // owns and reads) instead of the plan's own word.
 void fc_plan_share_error(mld_fc_plan* plan, int* word);
@@ -114,8 +120,9 @@ int fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights, con
                     const PeerWait* wait, const PeerOutputs* outs = nullptr, bool* outs_used = nullptr);
 // Shape facts of a plan the sharded entry points need.
 void fc_plan_shape(const mld_fc_plan* plan, int* n, int* dst_layout, int* max_tokens, int* device);
-int launch_fc_strip(int bits, bool subnormal, const CUtensorMap& tw, const CUtensorMap& ts, const StripArgs& a,
-                    const StripGeometry& gm, cudaStream_t stream);
+// tz: the zero points' tensor map, or null
+int launch_fc_strip(int bits, bool subnormal, const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap* tz,
+                    const StripArgs& a, const StripGeometry& gm, cudaStream_t stream);
 
 // ------------------------------------------------- persistent decode-step kernel
 struct MegaConfig {

@@ -336,3 +336,57 @@ def test_errors(mld):
         plan.run(x, x, x, x, 3)          # more tokens than planned
     with pytest.raises(mld.MldError):
         plan.run(x, x, None, x, 1)       # per-channel scale tensor missing
+
+
+# ------------------------------------------------- the streaming kernel over its token and scale-layout range
+def _exact_fc(x, q, scale, zp=None):
+    """[M][N] in 64 bits from fp16 activations, integers [N][K], fp16 scales and zero points [N][G]"""
+    N, K = q.shape
+    z = 0.0 if zp is None else zp.astype(np.float16).astype(np.float64)[..., None]
+    w = (q.reshape(N, scale.shape[1], -1).astype(np.float64) - z) * scale.astype(np.float16).astype(np.float64)[..., None]
+    return x.astype(np.float64) @ w.reshape(N, K).T
+
+
+@pytest.mark.parametrize("M", [1, 2, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("bits,K,N,block", [(4, 520, 136, 0), (4, 1024, 4096, 32), (4, 2048, 1000, 128),
+                                            (8, 1032, 520, 0), (8, 512, 9600, 0), (4, 256, 19008, 64)])
+@pytest.mark.parametrize("use_zp", [False, True])
+def test_streaming_token_ranges(mld, oracle, M, bits, K, N, block, use_zp):
+    # the dispatch's own choice; rounding to fp16 once (2^-11) and the digits' 2^-16: 1e-3 of the largest output
+    if M > 16 and not use_zp:
+        pytest.skip("served by the GEMM: test_gpu_gemm.py")
+    rng = np.random.default_rng(M * 7 + K + N)
+    G = K // block if block else 1
+    lo, hi = (-128, 128) if bits == 8 else (-8, 8)
+    q = rng.integers(lo, hi, size=(N, K), dtype=np.int8)
+    scale = (rng.uniform(0.5, 1.5, (N, G)) / hi / 16).astype(np.float32)
+    zp = rng.integers(lo, hi, size=(N, G)).astype(np.float32) if use_zp else None
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    packed = oracle.rearrange_int8_as_uint8(q) if bits == 8 else oracle.rearrange_int8_as_uint4(q)
+    params = [_dev(oracle.scale_layout(t, True).view(np.float16)) if t is not None else None for t in (scale, zp)]
+    plan = mld.FullyConnectedPlan(N, K, bits, scale_mode=mld.SCALE_BLOCK if block else mld.SCALE_PER_CHANNEL, groups=G,
+                                  has_zero_point=use_zp, precision=mld.F32F16, max_tokens=M)
+    y = torch.full(((N + 3) // 4, M, 4), float("nan"), dtype=torch.float16, device="cuda")
+    plan.run(_dev(oracle.to_sliced(x.astype(np.float32)).astype(np.float16)), _dev(packed), params[0], y, M,
+             zero_point=params[1])
+    torch.cuda.synchronize()
+    assert plan.last_route() == mld.ROUTE_DECODE_STREAMING and plan.device_status() == 0
+    got = oracle.from_sliced(y.float().cpu().numpy(), N)
+    assert _rel(got, _exact_fc(x, q, scale, zp)) <= 1e-3
+
+
+def test_streaming_many_passes(mld, oracle):
+    # strips of several passes, the last of them with fewer boxes than the others; one and three tokens
+    rng = np.random.default_rng(5)
+    for bits, K, N in ((8, 256, 40968), (4, 256, 100008)):
+        q = rng.integers(-8, 8, size=(N, K), dtype=np.int8)
+        scale = rng.uniform(0.5, 1.5, (N, 1)).astype(np.float32) / 128
+        packed = _dev(oracle.rearrange_int8_as_uint8(q) if bits == 8 else oracle.rearrange_int8_as_uint4(q))
+        sc = _dev(oracle.scale_layout(scale, True).view(np.float16))
+        for M in (1, 3):
+            x = rng.standard_normal((M, K)).astype(np.float16)
+            plan = mld.FullyConnectedPlan(N, K, bits, max_tokens=M)
+            y = torch.full((N // 4, M, 4), float("nan"), dtype=torch.float16, device="cuda")
+            plan.run(_dev(oracle.to_sliced(x.astype(np.float32)).astype(np.float16)), packed, sc, y, M)
+            torch.cuda.synchronize()
+            assert _rel(oracle.from_sliced(y.float().cpu().numpy(), N), _exact_fc(x, q, scale)) <= 1e-3
