@@ -148,6 +148,7 @@ struct Waiter {
     if (mbar_try_wait(bar, parity)) return true;
     if (*s_fail) return false;
     const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
     for (;;) {
 #pragma unroll 1
       for (int i = 0; i < 64; ++i)
@@ -164,6 +165,7 @@ struct Waiter {
   __device__ __forceinline__ void wait_count(volatile int* counter, int want, int code) const {
     if (*counter - want >= 0 || *s_fail) return;
     const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
     while (*counter - want < 0) {
       if (*s_fail) return;
       if (globaltimer_ns() - t0 > limit) {
@@ -206,6 +208,7 @@ __device__ __forceinline__ __half ld_tagged(const Waiter& w, const uint32_t* p, 
   uint32_t v = ld_word(p, w.sys);
   if ((v >> 16) != tag && !*w.s_fail) {
     const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
     for (;;) {
       v = ld_word(p, w.sys);
       if ((v >> 16) == tag || *w.s_fail) break;
@@ -234,6 +237,7 @@ __device__ __forceinline__ uint4 ld_tagged8(const Waiter& w, const uint32_t* p, 
   };
   if (!ok(a, b) && !*w.s_fail) {
     const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
     for (;;) {
       a = ld_word4(p, w.sys);
       b = ld_word4(p + 4, w.sys);
@@ -330,6 +334,9 @@ struct AttnSplit {
   __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
     P = G >= heads ? G / heads : 0;
     if (P > kMaxParts) P = kMaxParts;
+    // A short context has no use for all of them (8 heads, 100 tokens): one CTA's warps take up to kCW tiles side by side, and merging parts
+    // costs two trips through L2 (publishing and reading the partials); beyond, six tiles to a part.
+    if (P > 1) P = nt <= kCW ? 1 : (nt / 6 < P ? nt / 6 : P);
   }
   __device__ __forceinline__ void range(int cta, int& i0, int& i1) const {
     if (P > 0) {
@@ -382,6 +389,7 @@ __device__ void prefetch_op_l2(const MegaArgs& a, int l, int kind) {
     const AttnSplit split(a.heads, nt, G);
     int i0, i1;
     split.range(cta, i0, i1);
+#pragma unroll 1
     for (int i = i0; i < i1; ++i) {
       const int head = i / nt, j = i - head * nt;
       asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(
@@ -399,6 +407,7 @@ __device__ void prefetch_op_l2(const MegaArgs& a, int l, int kind) {
     proj_range(p, cta, G, i0, i1);
     const uint8_t* src = ly->w[map_index(kind)] + (size_t)i0 * kStageBytes;
     size_t bytes = (size_t)(i1 - i0) * kStageBytes;
+#pragma unroll 1
     while (bytes > 0) {
       const uint32_t n = bytes < 18432 ? static_cast<uint32_t>(bytes) : 18432u;
       bulk_prefetch_l2(src, n);
@@ -413,8 +422,10 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
   const uint64_t pol = policy_evict_first();
   Ring r{0, 0};
   const int nt = a.pos / kTile + 1;
+#pragma unroll 1
   for (int l = 0; l < a.n_layers; ++l) {
     const MegaLayer* ly = a.layers + l;
+#pragma unroll 1
     for (int kind = 0; kind < kOpsPerLayer; ++kind) {
       if (a.l2_ahead > 0) {
         // the op `l2_ahead` ops after this one
@@ -426,11 +437,14 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
         int ai0, ai1;
         split.range(cta, ai0, ai1);
         const Runs runs(ai0, ai1, nt);
+#pragma unroll 1
         for (int rr = 0; rr < runs.R; ++rr) {
           int head, lo, hi;
           runs.bounds(rr, head, lo, hi);
+#pragma unroll 1
           for (int i = lo; i < hi; ++i) {
             const int j = i - head * nt;
+#pragma unroll 1
             for (int kv = 0; kv < 2; ++kv) {
               // a producer whose wait ran out requests nothing more: stages it cannot know to be free stay
               // untouched, and no barrier sees an arrival its phase does not expect
@@ -452,8 +466,10 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
         // boxes are stored strip after strip: the CTA's boxes are one contiguous stream, cut into kCW
         // chunks (one per consumer warp); ring position kCW j + w takes box j of chunk w
         const int B = pi1 - pi0, qn = B / kCW, rn = B % kCW;
+#pragma unroll 1
         for (int j = 0; j * kCW < B; ++j) {
           const int nw = B - j * kCW < kCW ? B - j * kCW : kCW;
+#pragma unroll 1
           for (int cw = 0; cw < nw; ++cw) {
             const int i = pi0 + cw * qn + (cw < rn ? cw : rn) + j;
             if (!w.wait(&empty[r.stage], r.phase ^ 1, 11)) return;
@@ -519,6 +535,7 @@ __device__ void grid_barrier(Ctx& c, bool cross = false) {
       target = c.xbar_target + (unsigned long long)gridDim.x * c.a.world;
       // one system-scope fence (this CTA's stores, the peer stores among them, are performed), then the arrivals
       asm volatile("fence.acq_rel.sys;" ::: "memory");
+#pragma unroll 1
       for (int r = 0; r < c.a.world; ++r)
         asm volatile("red.relaxed.sys.global.add.u64 [%0], %1;" ::"l"(c.a.peers[r] + c.a.off_xbar), "l"(1ull) : "memory");
     } else {
@@ -526,6 +543,7 @@ __device__ void grid_barrier(Ctx& c, bool cross = false) {
     }
     if (!*c.w.s_fail) {
       const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
       for (;;) {
         unsigned long long v;
         if (cross)
@@ -546,17 +564,6 @@ __device__ void grid_barrier(Ctx& c, bool cross = false) {
   else
     c.bar_target += gridDim.x;
   consumer_bar();
-}
-
-// Between two ops: the grid barrier, or (tagged vectors) only this CTA's consumer warps, whose shared
-// buffers the next op reuses.
-__device__ __forceinline__ void op_boundary(Ctx& c, bool tagged, bool cross) {
-  if (tagged) {
-    consumer_bar();
-    if (threadIdx.x == 0) trace_mark(c, 6);
-  } else {
-    grid_barrier(c, cross);
-  }
 }
 
 // The digit scale of a unit of 32 inputs whose largest magnitude is amax: the smallest power of two s with
@@ -634,6 +641,7 @@ __device__ __forceinline__ void digitise_chunk(Ctx& c, int ci, const uint4& v) {
 // unit's integers), the nibble offset's share.
 __device__ void digitise_x(Ctx& c, int d) {
   const int chunks = (d + kBoxK - 1) / kBoxK * kBoxK / 8;  // 8 inputs (16 bytes) per thread and round
+#pragma unroll 1
   for (int ci = threadIdx.x; ci < chunks; ci += kCW * 32) {
     const uint4 v = *reinterpret_cast<const uint4*>(c.xs + ci * 8);
     __syncwarp();  // rounds are warp-uniform (whole boxes): the unit's four lanes have read before any rewrites
@@ -657,6 +665,7 @@ __device__ __forceinline__ uint4 fetch8(const Waiter& w, const Src& s, int i) {
   uint4 xv = __ldcg(reinterpret_cast<const uint4*>(s.x + i));
   if (s.partials == nullptr) return xv;
   float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
   for (int r = 0; r < s.world; ++r) {
     const float4 p0 = __ldcg(reinterpret_cast<const float4*>(s.partials + (size_t)r * s.stride + i));
     const float4 p1 = __ldcg(reinterpret_cast<const float4*>(s.partials + (size_t)r * s.stride + i + 4));
@@ -686,39 +695,46 @@ __device__ __forceinline__ float consumer_sum(Ctx& c, float v) {
 }
 
 // Loads the d-element input vector of a projection and leaves it digitised in xs (digitise_x).
-// NORM: the reference RMSNorm first, xs = fp16(v * rsqrt(mean(v^2) + eps) * gamma), fp32 statistics.
+// gamma != null: the reference RMSNorm first, xs = fp16(v * rsqrt(mean(v^2) + eps) * gamma), fp32 statistics.
 // Vectors of up to kRegChunks chunks per thread stay in registers between the passes.
-template <bool NORM>
-__device__ void load_x(Ctx& c, const Src& src, const __half* gamma, int d) {
+__device__ __forceinline__ void load_x(Ctx& c, const Src& src, const __half* gamma, int d) {
   const int padded = (d + kBoxK - 1) / kBoxK * kBoxK;
   const int chunks = padded / 8;
+  const auto sum_squares = [](const uint4& v, float ss) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h[j]);
+      ss += f.x * f.x + f.y * f.y;
+    }
+    return ss;
+  };
+  const auto normalise = [](uint4& v, const uint4& gv, float inv) {
+    __half2* h = reinterpret_cast<__half2*>(&v);
+    const __half2* gh = reinterpret_cast<const __half2*>(&gv);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h[j]);
+      const float2 g = __half22float2(gh[j]);
+      h[j] = __floats2half2_rn(f.x * inv * g.x, f.y * inv * g.y);
+    }
+  };
   if (chunks > kRegChunks * kCW * 32) {
     // general path through shared memory
     float ss = 0.0f;
+#pragma unroll 1
     for (int i = threadIdx.x * 8; i < padded; i += kCW * 32 * 8) {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (i < d) v = fetch8(c.w, src, i);
       *reinterpret_cast<uint4*>(c.xs + i) = v;
-      const __half2* h = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(h[j]);
-        ss += f.x * f.x + f.y * f.y;
-      }
+      ss = sum_squares(v, ss);
     }
-    if (NORM) {
+    if (gamma != nullptr) {
       const float inv = rsqrtf(consumer_sum(c, ss) / static_cast<float>(d) + c.a.rms_eps);
+#pragma unroll 1
       for (int i = threadIdx.x * 8; i < d; i += kCW * 32 * 8) {
         uint4 v = *reinterpret_cast<uint4*>(c.xs + i);
-        const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma + i));
-        __half2* h = reinterpret_cast<__half2*>(&v);
-        const __half2* gh = reinterpret_cast<const __half2*>(&gv);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(h[j]);
-          const float2 g = __half22float2(gh[j]);
-          h[j] = __floats2half2_rn(f.x * inv * g.x, f.y * inv * g.y);
-        }
+        normalise(v, __ldg(reinterpret_cast<const uint4*>(gamma + i)), inv);
         *reinterpret_cast<uint4*>(c.xs + i) = v;
       }
     }
@@ -727,45 +743,27 @@ __device__ void load_x(Ctx& c, const Src& src, const __half* gamma, int d) {
     consumer_bar();
     return;
   }
-  uint4 v[kRegChunks];
-  if (NORM) {
-    uint4 gv[kRegChunks];
+  uint4 v[kRegChunks], gv[kRegChunks];
+  // gamma is read once per step, so it comes from HBM: asked for before the wait for the vector, not after it
+#pragma unroll
+  for (int r = 0; r < kRegChunks; ++r) {
+    const int ci = threadIdx.x + r * kCW * 32;
+    gv[r] = make_uint4(0u, 0u, 0u, 0u);
+    if (gamma != nullptr && ci * 8 < d) gv[r] = __ldg(reinterpret_cast<const uint4*>(gamma + ci * 8));
+  }
+#pragma unroll
+  for (int r = 0; r < kRegChunks; ++r) {
+    const int ci = threadIdx.x + r * kCW * 32;
+    v[r] = make_uint4(0u, 0u, 0u, 0u);
+    if (ci * 8 < d) v[r] = fetch8(c.w, src, ci * 8);
+  }
+  if (gamma != nullptr) {
     float ss = 0.0f;
 #pragma unroll
-    for (int r = 0; r < kRegChunks; ++r) {
-      const int ci = threadIdx.x + r * kCW * 32;
-      v[r] = make_uint4(0u, 0u, 0u, 0u);
-      gv[r] = make_uint4(0u, 0u, 0u, 0u);
-      if (ci * 8 < d) {
-        v[r] = fetch8(c.w, src, ci * 8);
-        gv[r] = __ldg(reinterpret_cast<const uint4*>(gamma + ci * 8));
-      }
-      const __half2* h = reinterpret_cast<const __half2*>(&v[r]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(h[j]);
-        ss += f.x * f.x + f.y * f.y;
-      }
-    }
+    for (int r = 0; r < kRegChunks; ++r) ss = sum_squares(v[r], ss);
     const float inv = rsqrtf(consumer_sum(c, ss) / static_cast<float>(d) + c.a.rms_eps);
 #pragma unroll
-    for (int r = 0; r < kRegChunks; ++r) {
-      __half2* h = reinterpret_cast<__half2*>(&v[r]);
-      const __half2* gh = reinterpret_cast<const __half2*>(&gv[r]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(h[j]);
-        const float2 g = __half22float2(gh[j]);
-        h[j] = __floats2half2_rn(f.x * inv * g.x, f.y * inv * g.y);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < kRegChunks; ++r) {
-      const int ci = threadIdx.x + r * kCW * 32;
-      v[r] = make_uint4(0u, 0u, 0u, 0u);
-      if (ci * 8 < d) v[r] = fetch8(c.w, src, ci * 8);
-    }
+    for (int r = 0; r < kRegChunks; ++r) normalise(v[r], gv[r], inv);
   }
   // the digit scale is per unit of 32 inputs, found by the unit's own four lanes: no block-wide maximum
 #pragma unroll
@@ -871,9 +869,11 @@ __device__ __forceinline__ void store_out(const MegaArgs& a, const Dest& dst, in
   if (dst.tagged != nullptr) {
     st_tagged(dst.tagged + idx, v, dst.tag);
     if (dst.all)
+#pragma unroll 1
       for (int r = 0; r < a.world; ++r)
         if (r != a.rank) st_tagged_sys(peer_ptr(a, dst.tagged, r) + idx, v, dst.tag);
   } else if (dst.all) {
+#pragma unroll 1
     for (int r = 0; r < a.world; ++r) reinterpret_cast<__half*>(a.peers[r] + dst.off)[idx] = v;
   } else {
     dst.local[idx] = v;
@@ -888,6 +888,7 @@ __device__ __forceinline__ void finish_strip(const MegaArgs& a, int kind, int st
   const int n = strip * kStripN + lane;
   if (out.partial) {
     if (lane < kStripN)
+#pragma unroll 1
       for (int r = 0; r < a.world; ++r) reinterpret_cast<float*>(a.peers[r] + out.off)[n] = v;
     return;
   }
@@ -910,34 +911,53 @@ __device__ __forceinline__ int chunk_owner(int b, int qn, int rn) {
   return rn + static_cast<int>(static_cast<unsigned>(b - big) / static_cast<unsigned>(qn));  // qn > 0 here
 }
 
+// A CTA's and a warp's share of a projection.  The op's boxes are cut into kCW contiguous chunks, one per warp (lengths
+// differ by at most one), so that a warp meets few strips; ring position kCW j + w holds box j of warp w's chunk.
+// Worked out before the input vector is waited for: the divisions take longer than a box.
+struct ProjPlan {
+  int S, B;            // boxes per strip, boxes of this CTA
+  int strip0;          // its first strip
+  int qn, rn;          // chunk lengths: the first rn have qn + 1 boxes, the others qn
+  int start, len, sl;  // this warp's chunk and the strip (within the CTA's) that it begins in
+  int stage;           // ring stage of its first box, and that stage's phase
+  uint32_t phase;
+  __device__ __forceinline__ ProjPlan(const Ctx& c, int kind) {
+    const ProjShape p = proj_shape(c.a, kind);
+    const int warp = threadIdx.x >> 5;
+    int i0, i1;
+    proj_range(p, blockIdx.x, gridDim.x, i0, i1);
+    S = p.S;
+    B = i1 - i0;
+    strip0 = i0 / S;
+    qn = B / kCW;
+    rn = B % kCW;
+    len = qn + (warp < rn ? 1 : 0);
+    start = warp * qn + (warp < rn ? warp : rn);
+    sl = start / S;
+    const int pos = c.ring_base + warp;
+    stage = pos % c.a.stages;
+    phase = static_cast<uint32_t>(pos / c.a.stages) & 1u;
+  }
+};
+
 // resid / tresid: the vector added to the outputs (element 0 = output 0 of this rank's shard), as halves or as
 // tagged words written by the op with tag tresid_tag.
-__device__ void run_projection(Ctx& c, int kind, const __half* resid, const Dest& out, const uint32_t* tresid = nullptr,
-                               uint32_t tresid_tag = 0) {
+__device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int kind, const __half* resid, const Dest& out,
+                                               const uint32_t* tresid, uint32_t tresid_tag) {
   const MegaArgs& a = c.a;
-  const ProjShape p = proj_shape(a, kind);
-  const int cta = blockIdx.x, G = gridDim.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  int i0, i1;
-  proj_range(p, cta, G, i0, i1);
-  const int B = i1 - i0;
   long long waited = 0, boxed = 0, ea = 0, eb = 0, ec = 0;
   const bool tracing = MLD_TRACING(a) && lane == 0;  // every warp keeps its own clocks
-  // The op's boxes are cut into kCW contiguous chunks, one per warp (lengths differ by at most one), so
-  // that a warp meets few strips; ring position kCW j + w holds box j of warp w's chunk.
-  const int qn = B / kCW, rn = B % kCW;
-  const int len = qn + (warp < rn ? 1 : 0);
-  const int start = warp * qn + (warp < rn ? warp : rn);
-  int pos = c.ring_base + warp;
-  int stage = pos % a.stages;
-  uint32_t phase = static_cast<uint32_t>(pos / a.stages) & 1u;
-  int b = start;
-  const int b_stop = start + len;
+  const int qn = p.qn, rn = p.rn, start = p.start;
+  int stage = p.stage, sl = p.sl, b = start;
+  uint32_t phase = p.phase;
+  const int b_stop = start + p.len;
+#pragma unroll 1
   while (b < b_stop) {
-    const int sl = b / p.S;  // strip within the CTA's range
-    const int strip = i0 / p.S + sl;
+    const int strip = p.strip0 + sl;
     const int s_lo = sl * p.S, s_hi = s_lo + p.S;
+    ++sl;  // (a warp's boxes lie side by side: the next round of this loop is the next strip)
     const int b_end = b_stop < s_hi ? b_stop : s_hi;
     // the strip's residual values are fetched now: whichever warp completes the strip has them at hand
     __half rv = __float2half_rn(0.0f);
@@ -950,6 +970,7 @@ __device__ void run_projection(Ctx& c, int kind, const __half* resid, const Dest
       rv = __ldcg(resid + strip * kStripN + lane);
     }
     float tot[2] = {0.0f, 0.0f};
+#pragma unroll 1
     for (; b < b_end; ++b) {
       const long long w0 = tracing ? clock64() : 0;
       // A parity wait is only right while the barrier is at most one phase behind: the stage's previous
@@ -966,6 +987,7 @@ __device__ void run_projection(Ctx& c, int kind, const __half* resid, const Dest
       if (tracing) boxed += clock64() - b0;
       if (lane == 0) mbar_arrive_n(&c.empty[stage], kCW);
       stage += kCW;
+#pragma unroll 1
       while (stage >= a.stages) {
         stage -= a.stages;
         phase ^= 1u;
@@ -977,9 +999,7 @@ __device__ void run_projection(Ctx& c, int kind, const __half* resid, const Dest
     tot[0] += __shfl_xor_sync(0xffffffffu, tot[0], 2);
     tot[1] += __shfl_xor_sync(0xffffffffu, tot[1], 1);
     tot[1] += __shfl_xor_sync(0xffffffffu, tot[1], 2);
-    // the warps that hold boxes of this strip: w_lo .. w_hi
-    const int w_lo = chunk_owner(s_lo, qn, rn), w_hi = chunk_owner(s_hi - 1, qn, rn);
-    if (w_lo == w_hi) {
+    if (s_lo >= start && s_hi <= b_stop) {
       // the strip is this warp's alone: rows g and g+8 sit in lanes t == 0
       const float lo = __shfl_sync(0xffffffffu, tot[0], (lane & 7) * 4);
       const float hi = __shfl_sync(0xffffffffu, tot[1], (lane & 7) * 4);
@@ -987,6 +1007,8 @@ __device__ void run_projection(Ctx& c, int kind, const __half* resid, const Dest
       if (tracing) ec += clock64() - e0;
       continue;
     }
+    // the warps that hold boxes of this strip: w_lo .. w_hi
+    const int w_lo = chunk_owner(s_lo, qn, rn), w_hi = chunk_owner(s_hi - 1, qn, rn);
     // A warp shares at most two strips with others: the one its chunk begins in (share 0) and the one it
     // ends in (share 1, where it is w_lo).  Each share is written once per op, so nothing waits for a
     // place; the strip's arrivals are counted at w_lo.
@@ -1008,17 +1030,18 @@ __device__ void run_projection(Ctx& c, int kind, const __half* resid, const Dest
       // the last warp to get here sums the shares in the order of the inputs and completes the strip
       __threadfence_block();
       float v = c.dump[(w_lo * 2 + 1) * kStripN + (lane & 15)];
+#pragma unroll 1
       for (int w = w_lo + 1; w <= w_hi; ++w) v += c.dump[w * 2 * kStripN + (lane & 15)];
       if (lane == 0) c.proj_arrived()[w_lo] = 0;  // next used after the op's grid barrier
       finish_strip(a, kind, strip, v, resid != nullptr || tresid != nullptr, rv, out);
     }
     if (tracing) eb += clock64() - e3;
   }
-  c.ring_base += B;
+  c.ring_base += p.B;
   if (tracing && warp == 0) {
     unsigned long long* tr = a.trace + ((size_t)blockIdx.x * a.n_layers * kOpsPerLayer + c.op_index) * kTraceSlots;
     tr[4] = static_cast<unsigned long long>(waited);
-    tr[5] = static_cast<unsigned long long>(B);
+    tr[5] = static_cast<unsigned long long>(p.B);
     tr[7] = static_cast<unsigned long long>(boxed);
     // warp 0's clocks after its boxes: up to the arrival, after it (the sum, when it is the last), own strips
     tr[8] = static_cast<unsigned long long>(ea);
@@ -1052,7 +1075,7 @@ __device__ __forceinline__ uint32_t tile_offset(int row, int dim) {
 // every B column holds the same vector, every accumulator column holds the same
 // result and nothing has to be masked.  A warp keeps (max, sum, O[128]) over its
 // tiles; warps and finally CTAs are merged when the CTA's run over a head ends.
-__device__ void run_attention(Ctx& c, const MegaLayer* ly) {
+__device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
   const MegaArgs& a = c.a;
   const int cta = blockIdx.x, G = gridDim.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1076,6 +1099,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
   int stage = pos % a.stages;
   uint32_t phase = static_cast<uint32_t>(pos / a.stages) & 1u;
   int seq_lo = 0;
+#pragma unroll 1
   for (int rr = 0; rr < runs.R; ++rr) {
     int head, lo, hi;
     runs.bounds(rr, head, lo, hi);
@@ -1087,11 +1111,22 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
     if (q < seq_hi) {
       // rotary embedding of q (rope.cc:70-89), scaled and rounded to fp16 as the unfused graph stores it
       __syncwarp();
-      uint32_t qw[4] = {0u, 0u, 0u, 0u};
-      if (a.tagged) {  // all four words are asked for before any is looked at
+      uint32_t qw[4] = {0u, 0u, 0u, 0u}, kw[4] = {0u, 0u, 0u, 0u}, vw[4] = {0u, 0u, 0u, 0u};
+      if (a.tagged) {  // all the words are asked for before any is looked at
         const uint32_t* qp = a.tq + (size_t)head * kHeadDim;
 #pragma unroll
         for (int i = 0; i < 4; ++i) qw[i] = ld_word(qp + lane + 32 * (i >> 1) + (i & 1) * (kHeadDim / 2), false);
+        // the new token's k and v too, by the warp whose share of the run includes the head's last tile
+        const int ahead = nt - 1 - (j0 + (q - seq_lo));
+        if (hi == (head + 1) * nt && ahead % aw == 0) {
+          const uint32_t* tk = a.tq + (size_t)(a.heads + head) * kHeadDim;
+          const uint32_t* tv = a.tq + (size_t)(2 * a.heads + head) * kHeadDim;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            kw[i] = ld_word(tk + lane + 32 * (i >> 1) + (i & 1) * (kHeadDim / 2), false);
+            vw[i] = ld_word(tv + lane + 32 * (i >> 1) + (i & 1) * (kHeadDim / 2), false);
+          }
+        }
       }
 #pragma unroll
       for (int rep = 0; rep < 2; ++rep) {
@@ -1118,6 +1153,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
         qb[ks][0] = *reinterpret_cast<const uint32_t*>(sq + 16 * ks + 2 * t);
         qb[ks][1] = *reinterpret_cast<const uint32_t*>(sq + 16 * ks + 2 * t + 8);
       }
+#pragma unroll 1
       for (; q < seq_hi; q += aw) {
         const int j = j0 + (q - seq_lo);
         int vstage = stage + 1;
@@ -1143,16 +1179,6 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           const __half* vp = a.qkv + (size_t)(2 * a.heads + head) * kHeadDim;
           __half* kc = ly->kcache + (size_t)a.pos * width + head * kHeadDim;
           __half* vc = ly->vcache + (size_t)a.pos * width + head * kHeadDim;
-          uint32_t kw[4] = {0u, 0u, 0u, 0u}, vw[4] = {0u, 0u, 0u, 0u};
-          if (a.tagged) {
-            const uint32_t* tk = a.tq + (size_t)(a.heads + head) * kHeadDim;
-            const uint32_t* tv = a.tq + (size_t)(2 * a.heads + head) * kHeadDim;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              kw[i] = ld_word(tk + lane + 32 * (i >> 1) + (i & 1) * (kHeadDim / 2), false);
-              vw[i] = ld_word(tv + lane + 32 * (i >> 1) + (i & 1) * (kHeadDim / 2), false);
-            }
-          }
 #pragma unroll
           for (int rep = 0; rep < 2; ++rep) {
             const int e = lane + 32 * rep, half = kHeadDim / 2;
@@ -1184,8 +1210,11 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           }
           // rows past the new token are not tokens yet: whatever the cache holds there must not reach
           // the products (0 * NaN), so they read as zero
-          for (int zr = row + 1; zr < kTile; ++zr)
-            *reinterpret_cast<uint2*>(vt + tile_offset(zr, 4 * lane)) = make_uint2(0u, 0u);
+          if (lane > row) {  // (a lane per row)
+#pragma unroll 4
+            for (int i = 0; i < kHeadDim / 8; ++i)
+              *reinterpret_cast<uint4*>(vt + tile_offset(lane, 8 * i)) = make_uint4(0u, 0u, 0u, 0u);
+          }
           __syncwarp();
         }
         // ---- scores: two blocks of 16 tokens, eight steps of 16 dims
@@ -1271,6 +1300,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           mbar_arrive_n(&c.empty[vstage], kCW);
         }
         stage += 2 * aw;
+#pragma unroll 1
         while (stage >= a.stages) {
           stage -= a.stages;
           phase ^= 1u;
@@ -1347,10 +1377,12 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           write = false;
         } else {
           if (trs) trs[9] = globaltimer_ns();
+#pragma unroll 1
           for (int base = 0; base < pm; base += 32) {
             const int u = base + lane;
             if (u < pm && !*c.w.s_fail) {
               const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
               for (;;) {
                 unsigned fv;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(fv) : "l"(flags + u) : "memory");
@@ -1366,6 +1398,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           __syncwarp();
           if (trs) trs[10] = globaltimer_ns();
           float TM = -INFINITY, po[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pl = 0.0f;
+#pragma unroll 1
           for (int base = 0; base < pm; base += 8) {
             int myoff = -1;
             {
@@ -1427,6 +1460,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
         __syncwarp();
         // contributors: the CTAs first..lastc whose range is not empty; lane u looks at CTA base + u
         int need = 0;
+#pragma unroll 1
         for (int base = first; base <= lastc; base += 32) {
           const int cc = base + lane;
           bool has = false;
@@ -1450,6 +1484,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           float TM = -INFINITY;
           o[0] = o[1] = o[2] = o[3] = 0.0f;
           ls = 0.0f;
+#pragma unroll 1
           for (int base = first; base <= lastc; base += 8) {
             // lane u < 8 finds the partial of CTA base + u (offset in floats, -1 if none); all lanes then load
             int myoff = -1;
@@ -1511,6 +1546,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(dst), "r"(tg | (pk.x & 0xFFFFu)),
                        "r"(tg | (pk.x >> 16)), "r"(tg | (pk.y & 0xFFFFu)), "r"(tg | (pk.y >> 16))
                        : "memory");
+#pragma unroll 1
           for (int r = 0; r < a.world; ++r)
             if (r != a.rank)
               asm volatile("st.relaxed.sys.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(peer_ptr(a, dst, r)),
@@ -1521,6 +1557,7 @@ __device__ void run_attention(Ctx& c, const MegaLayer* ly) {
           *reinterpret_cast<uint2*>(a.attn + (size_t)head * kHeadDim + 4 * lane) = pk;
         } else {
           const size_t at = (size_t)a.rank * a.d_local + (size_t)head * kHeadDim + 4 * lane;
+#pragma unroll 1
           for (int r = 0; r < a.world; ++r)
             *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(a.peers[r] + a.off_attn) + at) = pk;
         }
@@ -1552,10 +1589,12 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+#pragma unroll 1
     for (int s = 0; s < a.stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], kCW);  // attention tiles are read by every warp; a weight box's one reader arrives kCW-fold
     }
+#pragma unroll 1
     for (int i = 0; i < kSharedInts; ++i) s_int[i] = 0;
     // Arrival count of the grid barrier when this launch began (a multiple of the grid size; read before
     // this CTA's first arrival it lies in [base, base + grid)).  base / grid numbers the barriers of all
@@ -1593,178 +1632,134 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
     // every launch completes at least one local barrier, so five epochs per barrier keep launches apart
     c.epoch_base = static_cast<unsigned>(c.bar_target / gridDim.x) * kOpsPerLayer * (a.tagged ? a.n_layers : 1);
     const int d = a.d_model;
-    const bool sharded = a.world > 1;
+    const bool sharded = a.world > 1, tg = a.tagged != 0, paired = a.paired != 0;
     const size_t shard = (size_t)a.rank * a.d_local;  // first output of this rank in h / x
-    if (!a.paired) {
-      for (int l = 0; l < a.n_layers; ++l) {
-        const MegaLayer* ly = a.layers + l;
-        const bool last = l + 1 == a.n_layers;
-        const __half* x_cur = l == 0 ? a.x_in : (((l - 1) & 1) ? a.xb : a.xa);
-        // the last layer writes the caller's vector directly, unless peers have to write it too
-        __half* x_next = (last && !sharded) ? a.x_out : ((l & 1) ? a.xb : a.xa);
-        Dest d_qkv{a.qkv, 0ull, false, false};
-        Dest d_h{a.h + shard, a.off_h + shard * 2, sharded, false};
-        Dest d_act{a.act + (size_t)a.rank * a.ffn_local, a.off_act + (size_t)a.rank * a.ffn_local * 2, sharded, false};
-        Dest d_x{x_next + shard, ((l & 1) ? a.off_xb : a.off_xa) + shard * 2, sharded, false};
-        Src s_x{x_cur, nullptr, 0, 0, nullptr}, s_attn{a.attn, nullptr, 0, 0, nullptr}, s_h{a.h, nullptr, 0, 0, nullptr},
-            s_act{a.act, nullptr, 0, 0, nullptr};
-        const uint32_t* tres_o = nullptr;
-        const uint32_t* tres_down = nullptr;
-        uint32_t tres_o_tag = 0, tres_down_tag = 0;
-        const bool tg = a.tagged != 0;
-        uint32_t* tx_next = (l & 1) ? a.txb : a.txa;
-        if (tg) {
-          // tagged vectors: every op's outputs carry the op's number, readers wait word by word
+    // Paired sharding: q/k/v and gate/up are split by outputs, o and down by inputs, so attention's output and the
+    // activations never leave the rank; o and down produce fp32 partial sums of the whole vector, stored on every rank,
+    // and the next vector load adds them up (rank order) onto the residual.  Two barriers of a layer span the ranks
+    // instead of four.
+    const float* ph = reinterpret_cast<const float*>(a.peers[a.rank] + a.off_ph);
+    const float* pd = reinterpret_cast<const float*>(a.peers[a.rank] + a.off_pd);
+    // One copy of the code for all four projections of every sharding: the loops stay rolled.  (With a copy per
+    // projection and sharding the kernel was 512 KB of instructions; every op began with instruction-cache misses, and a
+    // warp's only box took 2200 cycles where a warm one takes 850.  A step of 8 layers of 8 heads: 251 us before, 173
+    // now; of the 7B geometry at 2048 tokens: 1540 and 1397.)
+#pragma unroll 1
+    for (int l = 0; l < a.n_layers; ++l) {
+      const MegaLayer* ly = a.layers + l;
+      const bool last = l + 1 == a.n_layers;
+#pragma unroll 1
+      for (int kind = 0; kind < kOpsPerLayer; ++kind) {
+        c.op_index = l * kOpsPerLayer + kind;
+        trace_mark(c, 0);
+        if (kind == kAttn) {
+          run_attention(c, ly);
+        } else {
           const unsigned e0 = c.epoch_base + l * kOpsPerLayer;
-          d_qkv.tagged = a.tq, d_qkv.tag = op_tag(e0 + kQkv);
-          d_h.tagged = a.th + shard, d_h.tag = op_tag(e0 + kO);
-          d_act.tagged = a.tact + (size_t)a.rank * a.ffn_local, d_act.tag = op_tag(e0 + kGu);
-          // (one GPU: the last layer writes the caller's vector directly)
-          if (!last || sharded) d_x.tagged = tx_next + shard, d_x.tag = op_tag(e0 + kDown);
-          if (l > 0) {
-            s_x.tx = ((l - 1) & 1) ? a.txb : a.txa, s_x.tag = op_tag(e0 - 1);  // down of the layer before
-            tres_o = s_x.tx + shard, tres_o_tag = s_x.tag;
+          // the layer's input and output vectors (the last layer writes the caller's directly, unless peers have to
+          // write it too), as halves and as tagged words (tx_cur: null in the first layer)
+          const __half* x_cur = l == 0 ? a.x_in : (((l - 1) & 1) ? a.xb : a.xa);
+          __half* x_next = (last && !sharded) ? a.x_out : ((l & 1) ? a.xb : a.xa);
+          uint32_t* tx_cur = tg && l > 0 ? (((l - 1) & 1) ? a.txb : a.txa) : nullptr;
+          Src src{nullptr, nullptr, 0, 0, nullptr};
+          Dest out{nullptr, 0ull, false, false};
+          const __half *gamma = nullptr, *resid = nullptr;
+          const uint32_t* tres = nullptr;
+          uint32_t tres_tag = 0;
+          int len = d;
+          if (kind == kQkv) {
+            gamma = ly->norm1;
+            out.local = a.qkv;
+            src.x = x_cur;
+            if (paired && l > 0) src = Src{a.h, pd, a.world, d, a.xa};  // h of the layer before plus its down partials
+            if (tg) {
+              src.tx = tx_cur, src.tag = op_tag(e0 - 1);  // down of the layer before
+              out.tagged = a.tq;
+            }
+          } else if (kind == kO) {
+            src.x = a.attn;
+            if (paired) {
+              len = a.d_local;
+              out = Dest{nullptr, a.off_ph + (size_t)a.rank * d * 4, true, true};
+            } else {
+              out = Dest{a.h + shard, a.off_h + shard * 2, sharded, false};
+              resid = x_cur + shard;
+            }
+            if (tg) {
+              src.tx = a.tattn, src.tag = op_tag(e0 + kAttn);
+              out.tagged = a.th + shard;
+              if (tx_cur != nullptr) tres = tx_cur + shard, tres_tag = op_tag(e0 - 1), resid = nullptr;
+            }
+          } else if (kind == kGu) {
+            gamma = ly->norm2;
+            src.x = a.h;
+            if (paired) {
+              src = Src{l == 0 ? a.x_in : a.xa, ph, a.world, d, a.h};  // h = x + o
+              out.local = a.act;
+            } else {
+              out = Dest{a.act + (size_t)a.rank * a.ffn_local, a.off_act + (size_t)a.rank * a.ffn_local * 2, sharded, false};
+            }
+            if (tg) {
+              src.tx = a.th, src.tag = op_tag(e0 + kO);
+              out.tagged = a.tact + (size_t)a.rank * a.ffn_local;
+            }
+          } else {
+            src.x = a.act;
+            len = paired ? a.ffn_local : a.ffn;
+            if (paired) {
+              out = Dest{nullptr, a.off_pd + (size_t)a.rank * d * 4, true, true};
+            } else {
+              out = Dest{x_next + shard, ((l & 1) ? a.off_xb : a.off_xa) + shard * 2, sharded, false};
+              resid = a.h + shard;
+            }
+            if (tg) {
+              src.tx = a.tact, src.tag = op_tag(e0 + kGu);
+              tres = a.th + shard, tres_tag = op_tag(e0 + kO), resid = nullptr;
+              if (!last || sharded) out.tagged = ((l & 1) ? a.txb : a.txa) + shard;
+            }
           }
-          s_attn.tx = a.tattn, s_attn.tag = op_tag(e0 + kAttn);
-          s_h.tx = a.th, s_h.tag = op_tag(e0 + kO);
-          s_act.tx = a.tact, s_act.tag = op_tag(e0 + kGu);
-          tres_down = a.th + shard, tres_down_tag = s_h.tag;
-        }
-        // With tagged vectors a CTA without strips of a projection has no business with its input vector
-        // (with barriers every CTA keeps the same sequence of block-wide steps).
-        auto has_items = [&](int kind) {
-          if (!tg) return true;
-          int j0, j1;
-          proj_range(proj_shape(a, kind), blockIdx.x, gridDim.x, j0, j1);
-          return j1 > j0;
-        };
-        c.op_index = l * kOpsPerLayer;
-        trace_mark(c, 0);
-        if (has_items(kQkv)) {
-          load_x<true>(c, s_x, ly->norm1, d);
-          trace_mark(c, 1);
-          run_projection(c, kQkv, nullptr, d_qkv);
-        }
-        trace_mark(c, 2);
-        op_boundary(c, tg, false);  // q, k, v stay on this rank
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        run_attention(c, ly);
-        trace_mark(c, 2);
-        op_boundary(c, tg, true);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        if (has_items(kO)) {
-          load_x<false>(c, s_attn, nullptr, d);
-          trace_mark(c, 1);
-          run_projection(c, kO, tres_o != nullptr ? nullptr : x_cur + shard, d_h, tres_o, tres_o_tag);
-        }
-        trace_mark(c, 2);
-        op_boundary(c, tg, true);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        if (has_items(kGu)) {
-          load_x<true>(c, s_h, ly->norm2, d);
-          trace_mark(c, 1);
-          run_projection(c, kGu, nullptr, d_act);
-        }
-        trace_mark(c, 2);
-        op_boundary(c, tg, true);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        if (has_items(kDown)) {
-          load_x<false>(c, s_act, nullptr, a.ffn);
-          trace_mark(c, 1);
-          run_projection(c, kDown, tg ? nullptr : a.h + shard, d_x, tres_down, tres_down_tag);
-        }
-        trace_mark(c, 2);
-        if (tg && last)
-          grid_barrier(c);  // one barrier per launch keeps the launches' op numbers apart
-        else
-          op_boundary(c, tg, true);
-        trace_mark(c, 3);
-        if (last && sharded && blockIdx.x == 0) {
-          // the step's result, assembled from all ranks' shards, goes to the caller's vector
-          for (int i = threadIdx.x * 8; i < d; i += kCW * 32 * 8) {
-            if (tg)
-              *reinterpret_cast<uint4*>(a.x_out + i) = ld_tagged8(c.w, tx_next + i, d_x.tag);
-            else
-              *reinterpret_cast<uint4*>(a.x_out + i) = __ldcg(reinterpret_cast<const uint4*>(x_next + i));
+          out.tag = op_tag(e0 + kind);
+          // With tagged vectors a CTA without strips of a projection has no business with its input vector
+          // (with barriers every CTA keeps the same sequence of block-wide steps).
+          const ProjPlan plan(c, kind);
+          if (!tg || plan.B > 0) {
+            load_x(c, src, gamma, len);
+            trace_mark(c, 1);
+            run_projection(c, plan, kind, resid, out, tres, tres_tag);
           }
         }
-      }
-    } else {
-      // Paired sharding: q/k/v and gate/up are split by outputs, o and down by inputs, so attention's
-      // output and the activations never leave the rank; o and down produce fp32 partial sums of the
-      // whole vector, stored on every rank, and the next vector load adds them up (rank order) onto the
-      // residual.  Two barriers of a layer span the ranks instead of four.
-      const float* ph = reinterpret_cast<const float*>(a.peers[a.rank] + a.off_ph);
-      const float* pd = reinterpret_cast<const float*>(a.peers[a.rank] + a.off_pd);
-      const Dest d_qkv{a.qkv, 0ull, false, false};
-      const Dest d_act{a.act, 0ull, false, false};
-      const Dest d_ph{nullptr, a.off_ph + (size_t)a.rank * d * 4, true, true};
-      const Dest d_pd{nullptr, a.off_pd + (size_t)a.rank * d * 4, true, true};
-      for (int l = 0; l < a.n_layers; ++l) {
-        const MegaLayer* ly = a.layers + l;
-        // layer input: the caller's vector, or h of the layer before (a.h) plus its down partials; kept in
-        // a.xa because it is the residual of this layer's h
-        const Src s_x = l == 0 ? Src{a.x_in, nullptr, 0, 0, nullptr} : Src{a.h, pd, a.world, d, a.xa};
-        const __half* x_res = l == 0 ? a.x_in : a.xa;
-        c.op_index = l * kOpsPerLayer;
-        trace_mark(c, 0);
-        load_x<true>(c, s_x, ly->norm1, d);
-        trace_mark(c, 1);
-        run_projection(c, kQkv, nullptr, d_qkv);
         trace_mark(c, 2);
-        grid_barrier(c);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        run_attention(c, ly);
-        trace_mark(c, 2);
-        grid_barrier(c);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        load_x<false>(c, Src{a.attn, nullptr, 0, 0, nullptr}, nullptr, a.d_local);
-        trace_mark(c, 1);
-        run_projection(c, kO, nullptr, d_ph);
-        trace_mark(c, 2);
-        grid_barrier(c, true);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        load_x<true>(c, Src{x_res, ph, a.world, d, a.h}, ly->norm2, d);  // h = x + o
-        trace_mark(c, 1);
-        run_projection(c, kGu, nullptr, d_act);
-        trace_mark(c, 2);
-        grid_barrier(c);
-        trace_mark(c, 3);
-
-        c.op_index += 1;
-        trace_mark(c, 0);
-        load_x<false>(c, Src{a.act, nullptr, 0, 0, nullptr}, nullptr, a.ffn_local);
-        trace_mark(c, 1);
-        run_projection(c, kDown, nullptr, d_pd);
-        trace_mark(c, 2);
-        grid_barrier(c, true);
+        // q, k, v stay on this rank (paired: only o and down leave it); with tagged vectors one barrier per launch keeps
+        // the launches' op numbers apart
+        const bool cross = paired ? kind == kO || kind == kDown : kind != kQkv;
+        const bool whole_grid = !tg || (last && kind == kDown);
+        if (whole_grid) {
+          grid_barrier(c, !tg && cross);
+        } else {
+          consumer_bar();  // only this CTA's consumer warps, whose shared buffers the next op reuses
+          if (threadIdx.x == 0) trace_mark(c, 6);
+        }
         trace_mark(c, 3);
       }
+    }
+    if (paired) {
       if (blockIdx.x == 0) {
         // the step's result: h of the last layer plus its down partials
         const Src s_out{a.h, pd, a.world, d, a.x_out};
+#pragma unroll 1
         for (int i = threadIdx.x * 8; i < d; i += kCW * 32 * 8) fetch8(c.w, s_out, i);
+      }
+    } else if (sharded && blockIdx.x == 0) {
+      // the step's result, assembled from all ranks' shards, goes to the caller's vector
+      const int l = a.n_layers - 1;
+      const uint32_t* tx = (l & 1) ? a.txb : a.txa;
+      const __half* x = (l & 1) ? a.xb : a.xa;
+#pragma unroll 1
+      for (int i = threadIdx.x * 8; i < d; i += kCW * 32 * 8) {
+        if (tg)
+          *reinterpret_cast<uint4*>(a.x_out + i) = ld_tagged8(c.w, tx + i, op_tag(c.epoch_base + l * kOpsPerLayer + kDown));
+        else
+          *reinterpret_cast<uint4*>(a.x_out + i) = __ldcg(reinterpret_cast<const uint4*>(x + i));
       }
     }
   }
