@@ -32,6 +32,8 @@ __device__ __forceinline__ float load_param(const void* p, size_t i, int f16) {
 }
 
 __global__ void __launch_bounds__(256) embedding_lookup_kernel(EmbedArgs a) {
+  pdl_launch_dependents();  // (the kernel behind it may begin: what reads dst waits for this one's end)
+  pdl_wait();
   const int S = blockIdx.x * blockDim.x + threadIdx.x;
   const int tok = blockIdx.y;
   if (S >= a.src_slices) return;
@@ -124,7 +126,7 @@ extern "C" int mld_embedding_lookup(const mld_embed_desc* d, const int32_t* ids,
   a.f16 = d->f16 ? 1 : 0;
   a.dst_layout = d->dst_layout;
   dim3 grid(div_up(a.src_slices, 256), tokens);
-  embedding_lookup_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  MLD_CUDA_CHECK(launch_overlapped(embedding_lookup_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), a));
   MLD_LAUNCH_CHECK();
   return MLD_OK;
 }

@@ -48,6 +48,8 @@ constexpr int kGenPhases = 32 / kGenSlices;  // input-slice phases of a warp
 template <typename T, int BITS>
 __global__ void __launch_bounds__(kGenWarps * 32) fc_generic_kernel(GenericArgs a) {
   __shared__ float part[kGenWarps][kGenSlices][kGenTokens][4];
+  pdl_launch_dependents();  // launched with programmatic serialization: a small matrix takes no longer than a launch
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ds = lane % kGenSlices, sp = lane / kGenSlices;
   const int dst_raw = blockIdx.x * kGenSlices + ds;
@@ -195,17 +197,9 @@ __global__ void __launch_bounds__(kGenWarps * 32) fc_generic_kernel(GenericArgs 
 int launch_fc_generic(const GenericArgs& a, int bits, bool f32, cudaStream_t stream) {
   const int grid = div_up(a.dst_slices, kGenSlices);
   if (grid == 0 || a.M == 0) return MLD_OK;
-  if (f32) {
-    if (bits == 8)
-      fc_generic_kernel<float, 8><<<grid, kGenWarps * 32, 0, stream>>>(a);
-    else
-      fc_generic_kernel<float, 4><<<grid, kGenWarps * 32, 0, stream>>>(a);
-  } else {
-    if (bits == 8)
-      fc_generic_kernel<__half, 8><<<grid, kGenWarps * 32, 0, stream>>>(a);
-    else
-      fc_generic_kernel<__half, 4><<<grid, kGenWarps * 32, 0, stream>>>(a);
-  }
+  void (*kern)(GenericArgs) = f32 ? (bits == 8 ? fc_generic_kernel<float, 8> : fc_generic_kernel<float, 4>)
+                                  : (bits == 8 ? fc_generic_kernel<__half, 8> : fc_generic_kernel<__half, 4>);
+  MLD_CUDA_CHECK(launch_overlapped(kern, dim3(grid), dim3(kGenWarps * 32), 0, stream, a));
   MLD_LAUNCH_CHECK();
   return MLD_OK;
 }
