@@ -78,6 +78,12 @@ def lib() -> C.CDLL:
         L.mld_packed_size_bytes.restype = C.c_size_t
         L.mld_fc_plan_workspace_bytes.restype = C.c_size_t
         L.mld_decoder_scratch_bytes.restype = C.c_size_t
+        # the calls of a token loop: declared arguments, so that plain addresses are passed without a wrapper each
+        p, i = C.c_void_p, C.c_int32
+        L.mld_fc_run.argtypes = [p, p, p, p, p, p, p, i, p]
+        L.mld_attn_decode.argtypes = [p, p, p, p, i, i, i, p]
+        L.mld_decoder_step.argtypes = [p, p, p, i, p]
+        L.mld_decoder_step_host.argtypes = [p, p, p, i, p]
         _lib = L
     return _lib
 
@@ -91,9 +97,21 @@ def _ptr(t):
     return C.c_void_p(0 if t is None else t.data_ptr())
 
 
+def _addr(t):
+    return None if t is None else t.data_ptr()
+
+
 def _stream(stream=None):
-    s = torch.cuda.current_stream() if stream is None else stream
-    return C.c_void_p(s.cuda_stream)
+    return C.c_void_p(_stream_addr(stream))
+
+
+def _stream_addr(stream=None):
+    """The CUDA stream handle of `stream`, or of the current stream (without building a torch.cuda.Stream for it)."""
+    if stream is not None:
+        return stream.cuda_stream
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def kernel_launch_count() -> int:
@@ -203,8 +221,10 @@ class FullyConnectedPlan:
         return code.value
 
     def run(self, src, weights, scale, dst, tokens, zero_point=None, bias=None, stream=None):
-        _check(lib().mld_fc_run(self._h, _ptr(src), _ptr(weights), _ptr(scale), _ptr(zero_point), _ptr(bias),
-                                _ptr(dst), tokens, _stream(stream)), "mld_fc_run")
+        rc = (_lib or lib()).mld_fc_run(self._h, _addr(src), _addr(weights), _addr(scale), _addr(zero_point), _addr(bias),
+                                        _addr(dst), tokens, _stream_addr(stream))
+        if rc != OK:
+            _check(rc, "mld_fc_run")
 
     def close(self):
         if self._h:
@@ -355,8 +375,8 @@ def attn_decode_static(q, kcache, vcache, out, heads, n_tokens, head_dim=128, st
 
 
 def attn_decode(q, kcache, vcache, out, heads, n_tokens, head_dim=128, stream=None):
-    _check(lib().mld_attn_decode(_ptr(q), _ptr(kcache), _ptr(vcache), _ptr(out), heads, head_dim, n_tokens,
-                                 _stream(stream)), "mld_attn_decode")
+    _check(lib().mld_attn_decode(_addr(q), _addr(kcache), _addr(vcache), _addr(out), heads, head_dim, n_tokens,
+                                 _stream_addr(stream)), "mld_attn_decode")
 
 
 def comm_unique_id() -> bytes:
@@ -415,11 +435,11 @@ class Decoder:
                "mld_decoder_ipc_import")
 
     def step(self, x_in, x_out, pos, stream=None):
-        _check(lib().mld_decoder_step(self._h, _ptr(x_in), _ptr(x_out), pos, _stream(stream)), "mld_decoder_step")
+        _check(lib().mld_decoder_step(self._h, _addr(x_in), _addr(x_out), pos, _stream_addr(stream)), "mld_decoder_step")
 
     def step_host(self, x_host, y_host, pos, stream=None):
         """x_host / y_host: pinned CPU fp16 tensors; includes both copies and a stream sync."""
-        _check(lib().mld_decoder_step_host(self._h, _ptr(x_host), _ptr(y_host), pos, _stream(stream)),
+        _check(lib().mld_decoder_step_host(self._h, _addr(x_host), _addr(y_host), pos, _stream_addr(stream)),
                "mld_decoder_step_host")
 
     def scratch_bytes(self):
