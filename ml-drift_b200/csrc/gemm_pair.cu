@@ -288,6 +288,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           ok = false;
           break;
         }
+        if (lane == 0) __stcg(slot_flag, 0u);  // its one reader takes it back: a replayed graph has the same epoch again
         tr_flag += MLD_PAIR_CLOCK() - tg0;
       }
       const int m = mi * 2 * kRowsPerCta + static_cast<int>(rank) * kRowsPerCta + quad * 32 + lane;

@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         atomicExch(a.error, kErrWtBase + 8);
         return false;
       }
+      // each flag has this one reader, which takes it back: a replayed graph launches with the same epoch again
+      for (int o = lane; o < others; o += 32) __stcg(flag_of(pair + 1 + o), 0u);
     }
     const int n = tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows + quad * 32 + lane;  // output channel
     const int m_first = (sg.tile % a.m_tiles) * wa.tile_tok;

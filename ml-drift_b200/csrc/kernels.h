@@ -196,8 +196,8 @@ struct PairGeometry {
 // Workspace through which two SM pairs that share a tile combine their partial sums.
 struct PairSplit {
   float* ws;         // pair_split_bytes(sms) bytes
-  uint32_t* flags;   // pair_split_flags(sms) words, zeroed once
-  uint32_t epoch;    // a value no earlier launch on this workspace used (never 0)
+  uint32_t* flags;   // pair_split_flags(sms) words, zeroed once; each is cleared by the warp that waited for it
+  uint32_t epoch;    // a value no earlier call on this workspace used (never 0); the replays of a captured call repeat it
 };
 inline size_t pair_split_bytes(int sms) { return (size_t)(sms / 2 > 0 ? sms / 2 : 1) * 2 * 4 * 8 * 8 * 32 * 16; }
 inline size_t pair_split_flags(int sms) { return (size_t)(sms / 2 > 0 ? sms / 2 : 1) * 2 * 4 * 8; }

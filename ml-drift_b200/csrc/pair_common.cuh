@@ -159,8 +159,8 @@ struct PairArgs {
   // (shared_tiles = 0: whole tiles only.)
   int shared_tiles, units_per_pair;
   float* split_ws;            // [pairs][2 CTAs][4 warps][8 chunks][8][32 lanes] x 16 bytes of raw accumulators
-  uint32_t* split_flags;      // [pairs][2 CTAs][4 warps]: = epoch once that warp's share of the slot is written
-  uint32_t epoch;             // differs from launch to launch, so the flags never need clearing
+  uint32_t* split_flags;      // [pairs][2 CTAs][4 warps]: = epoch from when that warp's share of the slot is written to when it is read
+  uint32_t epoch;             // differs from call to call (a replayed graph repeats its own)
   long long* trace;           // tuning builds only: [grid][8] cycle counts per role (waiting / working)
   int skip_transform;         // tuning builds only: leave the operand tiles unwritten (timing of the rest)
 };

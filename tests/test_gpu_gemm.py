@@ -277,3 +277,38 @@ def test_tiles_cut_along_k(mld, oracle, bits, M, K, N):
     # not fuse it into the addition of the offset (the restatement never does): up to 0.05 / 35 of the largest output,
     # and the output's own rounding
     assert _rel(y, ref) <= (1e-3 if bits == 4 else 0.05 / 35 + 2.0 ** -11)
+
+
+@pytest.mark.parametrize("bits,M,K,N,act_quant", [
+    (4, 77, 4096, 11008, 0), (8, 40, 8192, 1024, 0),  # lone CTAs: every tile cut along K
+    (4, 500, 4096, 264, 0),                           # pairs, fewer tiles than pairs
+    (8, 1100, 2048, 8192, 2)])                        # the pair GEMM, its last waves cut
+def test_cut_tiles_in_a_replayed_graph(mld, bits, M, K, N, act_quant):
+    # replays launch with the same flag values: each must wait for its own parts and not find those of the one before
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    w = torch.randn(N, K, generator=gen, device="cuda") * 0.02
+    block = 32 if bits == 4 else 0
+    q, s = mld.quantize_weights(w, bits, block)
+    packed, sums = mld.pack_weights(q, (N, 1, 1, K), bits, want_sum=True)
+    scale = mld.pack_scales(s, True)
+    plan = mld.FullyConnectedPlan(N, K, bits, scale_mode=mld.SCALE_BLOCK if block else mld.SCALE_PER_CHANNEL,
+                                  groups=K // block if block else 1, max_tokens=M, prefill_act_quant=act_quant)
+    if act_quant == 2:
+        plan.set_weights_sum(sums)
+    xs = [torch.randn(K // 4, M, 4, generator=gen, device="cuda").half() for _ in range(4)]
+    x, y = xs[0].clone(), torch.empty(-(-N // 4), M, 4, dtype=torch.float16, device="cuda")
+    plan.run(x, packed, scale, y, M)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.run(x, packed, scale, y, M)
+    for _ in range(3):
+        for xi in xs:
+            x.copy_(xi)
+            y.zero_()
+            graph.replay()
+            replayed = y.clone()
+            plan.run(x, packed, scale, y, M)
+            assert torch.equal(replayed, y)  # (the sums are taken in a fixed order)
+    assert plan.device_status() == 0
+    plan.close()
