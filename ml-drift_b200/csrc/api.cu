@@ -409,6 +409,7 @@ static int run_generic(mld_fc_plan* p, const void* src, const void* weights, con
   a.has_zp = d.has_zero_point;
   a.src_layout = d.src_layout;
   a.dst_layout = d.dst_layout;
+  a.pdl = p->pdl ? 1 : 0;
   return launch_fc_generic(a, d.weight_bits, d.precision == MLD_PRECISION_F32, stream);
 }
 

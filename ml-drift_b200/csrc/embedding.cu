@@ -32,8 +32,9 @@ __device__ __forceinline__ float load_param(const void* p, size_t i, int f16) {
 }
 
 __global__ void __launch_bounds__(256) embedding_lookup_kernel(EmbedArgs a) {
-  pdl_launch_dependents();  // (the kernel behind it may begin: what reads dst waits for this one's end)
+  // (a launch behind this one may begin when everything ahead of it is done; what reads dst waits for its end)
   pdl_wait();
+  pdl_launch_dependents();
   const int S = blockIdx.x * blockDim.x + threadIdx.x;
   const int tok = blockIdx.y;
   if (S >= a.src_slices) return;

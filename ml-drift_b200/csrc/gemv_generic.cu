@@ -48,8 +48,11 @@ constexpr int kGenPhases = 32 / kGenSlices;  // input-slice phases of a warp
 template <typename T, int BITS>
 __global__ void __launch_bounds__(kGenWarps * 32) fc_generic_kernel(GenericArgs a) {
   __shared__ float part[kGenWarps][kGenSlices][kGenTokens][4];
-  pdl_launch_dependents();  // launched with programmatic serialization: a small matrix takes no longer than a launch
+  // Launched with programmatic serialization (unless the plan forbids it): a small matrix takes no longer than a launch.
+  // In this order, so that a launch behind this one that waits for nothing but its own input (independent_io) begins
+  // only when everything ahead of this one is done.
   pdl_wait();
+  if (a.pdl) pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ds = lane % kGenSlices, sp = lane / kGenSlices;
   const int dst_raw = blockIdx.x * kGenSlices + ds;
@@ -199,7 +202,11 @@ int launch_fc_generic(const GenericArgs& a, int bits, bool f32, cudaStream_t str
   if (grid == 0 || a.M == 0) return MLD_OK;
   void (*kern)(GenericArgs) = f32 ? (bits == 8 ? fc_generic_kernel<float, 8> : fc_generic_kernel<float, 4>)
                                   : (bits == 8 ? fc_generic_kernel<__half, 8> : fc_generic_kernel<__half, 4>);
-  MLD_CUDA_CHECK(launch_overlapped(kern, dim3(grid), dim3(kGenWarps * 32), 0, stream, a));
+  if (a.pdl) {
+    MLD_CUDA_CHECK(launch_overlapped(kern, dim3(grid), dim3(kGenWarps * 32), 0, stream, a));
+  } else {
+    kern<<<grid, kGenWarps * 32, 0, stream>>>(a);
+  }
   MLD_LAUNCH_CHECK();
   return MLD_OK;
 }

@@ -32,6 +32,7 @@ struct GenericArgs {
   float scalar_scale, scalar_zp;
   int has_zp;
   int src_layout, dst_layout;
+  int pdl;  // launch with programmatic stream serialization
 };
 int launch_fc_generic(const GenericArgs& a, int bits, bool f32, cudaStream_t stream);
 
