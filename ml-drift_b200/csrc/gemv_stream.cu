@@ -193,7 +193,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // ZP: a zero point per scale; a second box of the scales' shape follows them in the stage.  (u - 8 - z) s x summed
 // over a group is s (sum(u x) - (1 + z / 8) 8 sum(x)), so the zero point only scales the offset term, in fp32
 // (2048 x 4096 INT4, 12 tokens: 9.2 us; the general kernel, which took such weights before, 45.8).
-template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT>
+// INTERLEAVE: the passes of all strips lie side by side (StripGeometry::interleave).  A form of its own, because the steps
+// and box counts that only it has, worked out at run time, cost every other launch 0.3 to 0.8 us (14208 x 2432 INT4, one
+// token 13.6 against 12.9; 4096 x 11008 10.9 against 10.2).
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE>
 __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     fc_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                     const __grid_constant__ CUtensorMap tmap_z, StripArgs a) {
@@ -222,9 +225,9 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   const int64_t u_lo = (int64_t)strip * a.units / a.strips, u_hi = (int64_t)(strip + 1) * a.units / a.strips;
   // (interleaved: the passes of all strips side by side, pass p of strip s being the grid's (p strips + s)-th box or
   // pair of boxes, so that what the SMs read at a time is one contiguous piece of every weight row)
-  const int cs = a.interleave ? strip * W * 8 : static_cast<int>(u_lo) * a.gran;
-  const int ce = a.interleave ? a.units * a.gran : static_cast<int>(u_hi) * a.gran;
-  const int pass_step = a.interleave ? a.strips * W * 8 : W * 8;
+  const int cs = INTERLEAVE ? strip * W * 8 : static_cast<int>(u_lo) * a.gran;
+  const int ce = INTERLEAVE ? a.units * a.gran : static_cast<int>(u_hi) * a.gran;
+  const int pass_step = INTERLEAVE ? a.strips * W * 8 : W * 8;
   const int passes = (ce - cs + pass_step - 1) / pass_step;
   const int r_lo = kr * a.rows_per_split;
   const int r_hi = min(a.src_slices, r_lo + a.rows_per_split);
@@ -270,9 +273,9 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         const int row0 = r_lo + si * kStageRows;
         const int rows = min(kStageRows, r_hi - row0);
         const int chunk0 = cs + pass * pass_step;
-        // (boxes past the end of the strip, in its last pass, are not fetched: their sums, of whatever the stage held, are
+        // (boxes past the end of the matrix, in the last pass, are not fetched: their sums, of whatever the stage held, are
         // not stored)
-        const int boxes = min(W, (ce - chunk0 + 7) / 8);
+        const int boxes = INTERLEAVE ? min(W, (ce - chunk0 + 7) / 8) : W;
         mbar_arrive_expect_tx(&full[stage], boxes * kBoxBytes + s_bytes +
                                                 (DIGITS ? 0u : static_cast<uint32_t>(rows) * a.M_total * 8u));
 #pragma unroll
@@ -445,7 +448,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       for (int f = 0; f < F::NF; ++f)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) tot[b][f][j] = 0.0f;
-    [[maybe_unused]] const int boxes = min(W, (ce - cs - pass * pass_step + 7) / 8);  // of this pass
+    [[maybe_unused]] const int boxes = INTERLEAVE ? min(W, (ce - cs - pass * pass_step + 7) / 8) : W;  // of this pass
 
     for (int si = 0; si < n_st; ++si) {
 #ifdef MLD_TRACE
@@ -812,10 +815,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   }
 }
 
-template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false, bool ZP = false, bool SPLIT = false>
-int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE>
+int launch_strip_f(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
                    const StripGeometry& gm, cudaStream_t stream) {
-  auto kern = fc_strip_kernel<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT>;
+  auto kern = fc_strip_kernel<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, INTERLEAVE>;
   static bool configured[kMaxDevices];  // per instantiation and device
   int dev;
   if (needs_configure(configured, &dev)) {
@@ -846,6 +849,15 @@ int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorM
   MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tw, ts, tz, a));
   count_launch();
   return MLD_OK;
+}
+
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false, bool ZP = false, bool SPLIT = false>
+int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
+                   const StripGeometry& gm, cudaStream_t stream) {
+  if constexpr (W == 2) {  // (strips of several passes with pdl are two boxes wide)
+    if (gm.interleave) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, true>(tw, ts, tz, a, gm, stream);
+  }
+  return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, false>(tw, ts, tz, a, gm, stream);
 }
 
 template <int BITS, int W, bool ZP>
@@ -958,7 +970,7 @@ int launch_fc_strip(int bits, bool subnormal, const CUtensorMap& tw, const CUten
 #define MLD_WZ(B, WV) \
   case WV:            \
     return launch_strip_w<B, WV, true>(subnormal, mone, tw, ts, *tz, a, gm, stream)
-  if (tz != nullptr) {  // (zero points: strips of up to two boxes, see strip_serves)
+  if (tz != nullptr) {  // (zero points are taken with pdl only, whose strips have two boxes at most)
     if (bits == 4) {
       switch (gm.w) {
         MLD_WZ(4, 1);

@@ -88,7 +88,6 @@ struct StripArgs {
   int red_m;          // token stride of the reduction buffer (one token tile)
   int peer_m;         // token stride of the cluster partner's sums
   int ts_shift;       // 2^ts_shift warps split a launch's tokens
-  int interleave;     // a strip's passes lie a grid's width apart instead of side by side
   int dst_layout;
   int epilogue;       // mld_epilogue
   float scalar_scale;
@@ -106,7 +105,8 @@ struct StripGeometry {
   int rows_per_split;
   int scale_rows, group_slices, gs_shift;
   int scale_stage_bytes, zp_off, stage_bytes, stages, red_m, peer_m, stage_rows;
-  int ts_shift, launch_tokens, interleave;
+  int ts_shift, launch_tokens;
+  int interleave;  // a strip's passes lie a grid's width apart instead of side by side
   int xdig_bytes;  // shared memory kept for the digitised activation vector (4-bit weights), else 0
   size_t smem_bytes;
 };
