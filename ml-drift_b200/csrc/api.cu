@@ -485,6 +485,7 @@ static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, 
   a.red_m = gm.red_m;
   a.peer_m = gm.peer_m;
   a.ts_shift = gm.ts_shift;
+  a.interleave = gm.interleave;
   a.dst_layout = d.dst_layout;
   a.epilogue = d.epilogue;
   a.scalar_scale = d.scalar_scale;

@@ -195,7 +195,8 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // (2048 x 4096 INT4, 12 tokens: 9.2 us; the general kernel, which took such weights before, 45.8).
 // INTERLEAVE: the passes of all strips lie side by side (StripGeometry::interleave).  A form of its own, because the steps
 // and box counts that only it has, worked out at run time, cost every other launch 0.3 to 0.8 us (14208 x 2432 INT4, one
-// token 13.6 against 12.9; 4096 x 11008 10.9 against 10.2).
+// token 13.6 against 12.9; 4096 x 11008 10.9 against 10.2).  Several tokens through strips of two boxes take this form always:
+// there it is the faster one (4096 x 11008, 5 tokens: 15.0 against 15.4).
 template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE>
 __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     fc_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
@@ -225,9 +226,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   const int64_t u_lo = (int64_t)strip * a.units / a.strips, u_hi = (int64_t)(strip + 1) * a.units / a.strips;
   // (interleaved: the passes of all strips side by side, pass p of strip s being the grid's (p strips + s)-th box or
   // pair of boxes, so that what the SMs read at a time is one contiguous piece of every weight row)
-  const int cs = INTERLEAVE ? strip * W * 8 : static_cast<int>(u_lo) * a.gran;
-  const int ce = INTERLEAVE ? a.units * a.gran : static_cast<int>(u_hi) * a.gran;
-  const int pass_step = INTERLEAVE ? a.strips * W * 8 : W * 8;
+  const bool interleave = INTERLEAVE && a.interleave;
+  const int cs = interleave ? strip * W * 8 : static_cast<int>(u_lo) * a.gran;
+  const int ce = interleave ? a.units * a.gran : static_cast<int>(u_hi) * a.gran;
+  const int pass_step = interleave ? a.strips * W * 8 : W * 8;
   const int passes = (ce - cs + pass_step - 1) / pass_step;
   const int r_lo = kr * a.rows_per_split;
   const int r_hi = min(a.src_slices, r_lo + a.rows_per_split);
@@ -855,9 +857,9 @@ template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false, bool 
 int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
                    const StripGeometry& gm, cudaStream_t stream) {
   if constexpr (W == 2) {  // (strips of several passes with pdl are two boxes wide)
-    if (gm.interleave) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, true>(tw, ts, tz, a, gm, stream);
+    if (!MONE || gm.interleave) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, true>(tw, ts, tz, a, gm, stream);
   }
-  return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, false>(tw, ts, tz, a, gm, stream);
+  if constexpr (W != 2 || MONE) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, false>(tw, ts, tz, a, gm, stream);
 }
 
 template <int BITS, int W, bool ZP>

@@ -88,6 +88,7 @@ struct StripArgs {
   int red_m;          // token stride of the reduction buffer (one token tile)
   int peer_m;         // token stride of the cluster partner's sums
   int ts_shift;       // 2^ts_shift warps split a launch's tokens
+  int interleave;     // a strip's passes lie a grid's width apart instead of side by side
   int dst_layout;
   int epilogue;       // mld_epilogue
   float scalar_scale;
