@@ -907,7 +907,7 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
   if (gm.ksplit == 1 && w_max <= 2 && C > 8 * w_max * sms) {
     // More columns than one pass of one CTA per SM: two CTAs share each SM, so that one streams while the other is in a
     // pass's epilogue (151936 x 2048 INT8, one token: 17 passes of a lone CTA 85.8 us, 9 of two 69.7; with the passes of
-    // all strips side by side 64.0, and with the integer digits 54.7, against 47.6 for the bytes at the copy rate).
+    // all strips side by side 64.0, with the integer digits 52.0, against 47.6 for the bytes at the copy rate).
     strips = 2 * sms;
     gm.interleave = C > 8 * w_max * strips ? 1 : 0;
   }
