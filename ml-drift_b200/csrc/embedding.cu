@@ -32,9 +32,9 @@ __device__ __forceinline__ float load_param(const void* p, size_t i, int f16) {
 }
 
 __global__ void __launch_bounds__(256) embedding_lookup_kernel(EmbedArgs a) {
-  // (a launch behind this one may begin when everything ahead of it is done; what reads dst waits for its end)
+  // Overlaps the launch ahead with its own start, but lets no launch begin before its end: a streaming projection behind it
+  // triggers the next launch before it waits, and that one, if its plan has independent_io, reads dst without a wait.
   pdl_wait();
-  pdl_launch_dependents();
   const int S = blockIdx.x * blockDim.x + threadIdx.x;
   const int tok = blockIdx.y;
   if (S >= a.src_slices) return;

@@ -49,10 +49,8 @@ template <typename T, int BITS>
 __global__ void __launch_bounds__(kGenWarps * 32) fc_generic_kernel(GenericArgs a) {
   __shared__ float part[kGenWarps][kGenSlices][kGenTokens][4];
   // Launched with programmatic serialization (unless the plan forbids it): a small matrix takes no longer than a launch.
-  // In this order, so that a launch behind this one that waits for nothing but its own input (independent_io) begins
-  // only when everything ahead of this one is done.
+  // It lets no launch begin before its end (see embedding_lookup_kernel).
   pdl_wait();
-  if (a.pdl) pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ds = lane % kGenSlices, sp = lane / kGenSlices;
   const int dst_raw = blockIdx.x * kGenSlices + ds;

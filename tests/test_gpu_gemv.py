@@ -259,6 +259,54 @@ def test_independent_launches_overlap_and_finish_in_stream_order(mld, oracle):
     ref_plan.close()
 
 
+@pytest.mark.parametrize("writer", ["general", "embedding"])
+def test_independent_launch_behind_the_writer_of_its_input(mld, writer):
+    """x is written by a launch that is not a streaming one, read by an ordinary projection and then by an independent
+    one: the latter does not wait, so the writer must be done before the projection between them lets it begin."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    K, N, K0, rows = 2048, 1024, 8196, 64
+
+    def weights(n, k, bits, block):
+        q, s = mld.quantize_weights(torch.randn(n, k, device="cuda", generator=g) * 0.02, bits, block)
+        return mld.pack_weights(q, (n, 1, 1, k), bits)[0], mld.pack_scales(s, True)
+
+    source = weights(K, K0, 8, 0) if writer == "general" else weights(4096, K, 8, 0)
+    if writer == "general":
+        writes = mld.FullyConnectedPlan(K, K0, 8)          # input channels not a multiple of 8: the general kernel
+        inputs = [torch.randn(K0, device="cuda", generator=g).half() for _ in range(2)]
+        x = torch.zeros(K, dtype=torch.float16, device="cuda")
+    else:
+        inputs = [torch.randint(0, 4096, (rows,), device="cuda", generator=g, dtype=torch.int32) for _ in range(2)]
+        table = torch.zeros((rows, K), dtype=torch.float16, device="cuda")
+        x = table[rows - 1]
+    between = mld.FullyConnectedPlan(N, K, 4, scale_mode=mld.SCALE_BLOCK, groups=K // 32)
+    behind = mld.FullyConnectedPlan(N, K, 4, scale_mode=mld.SCALE_BLOCK, groups=K // 32, independent_io=True)
+    w = [weights(N, K, 4, 32) for _ in range(2)]
+    y = [torch.zeros(N, dtype=torch.float16, device="cuda") for _ in range(2)]
+
+    def chain(i, wait):
+        if writer == "general":
+            writes.run(inputs[i], *source, x, 1)
+            assert writes.last_route() == mld.ROUTE_DECODE_GENERAL
+        else:
+            mld.embedding_lookup(inputs[i], *source, table, 4096, K, 8, scale_mode=mld.SCALE_PER_CHANNEL)
+        for plan, p, out in zip((between, behind), w, y):
+            if wait:
+                torch.cuda.synchronize()
+            plan.run(x, *p, out, 1)
+
+    want = []
+    for i in range(2):
+        chain(i, wait=True)
+        torch.cuda.synchronize()
+        want.append([t.clone() for t in y])
+    assert not torch.equal(want[0][1], want[1][1])
+    for r in range(40):
+        chain(r % 2, wait=False)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(y, want[r % 2]))
+
+
 @pytest.mark.parametrize("K,N,block", [(2048, 1024, 32), (40, 64, 0), (200, 328, 0), (4096, 512, 64), (1032, 1160, 0),
                                        (11008, 256, 128)])
 @pytest.mark.parametrize("outliers", [False, True])
