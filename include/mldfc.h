@@ -287,11 +287,16 @@ typedef struct mld_fc_desc {
                                 (programmatic dependent launch off) */
   int32_t smem_limit_kb;     /* > 0: shared-memory budget of the stage ring */
   int32_t independent_io;    /* 1: the caller promises that neither src nor dst of a
-                                call is written or read by the launch ahead of it on
-                                the stream (projections of one input, benchmarks over
-                                rotating tensors): consecutive decode launches then
-                                overlap completely instead of handing over at the
-                                activation load; stream order of completion is kept */
+                                call is written, nor dst read, by the launch ahead of
+                                it on the stream, nor by any launch that may still be
+                                running when that one begins: the decode launches of
+                                this operator begin while the one ahead still runs.
+                                (Projections of one input that a launch from outside
+                                this library, an embedding lookup or a copy has
+                                written; benchmarks over rotating tensors.)  The
+                                decode launches of this plan then overlap completely
+                                instead of handing over at the activation load; stream
+                                order of completion is kept */
 } mld_fc_desc;
 
 typedef struct mld_fc_plan mld_fc_plan;
@@ -348,7 +353,12 @@ MLD_API int mld_fc_plan_prefetch_next(mld_fc_plan* plan, const void* next_weight
  * Small token counts run the decode dequant-GEMV
  * (GetFullyConnectedKernelCode, fully_connected.cc:623-942); larger ones the
  * prefill dequant-GEMM the reference builds from WeightsConverter + ConvGeneric
- * (common/gpu_model_builder.cc:1110-1276). */
+ * (common/gpu_model_builder.cc:1110-1276).
+ * A decode call of up to 8 tokens (16 in MLD_PRECISION_F16) over weights without
+ * zero points asks for weights and scales while the launches of this library
+ * ahead of it may still run (no_overlap = 1 prevents that): those launches must
+ * not be the ones that write them.  The conversion functions above are not such
+ * launches, and every other call reads nothing before the launch ahead is done. */
 MLD_API int mld_fc_run(mld_fc_plan* plan, const void* src, const void* weights,
                        const void* scale, const void* zero_point,
                        const void* bias, void* dst, int32_t tokens,

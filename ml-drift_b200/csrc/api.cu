@@ -420,7 +420,7 @@ static StripGeometry strip_geometry_of(const mld_fc_plan* p, int tokens) {
 }
 
 static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, const void* weights, const void* scale,
-                      const void* zp, const void* bias, void* dst, int tokens, cudaStream_t stream,
+                      const void* zp, const void* bias, void* dst, int tokens, bool wait_first, cudaStream_t stream,
                       const PeerScatter* scatter, const PeerWait* wait) {
   const mld_fc_desc& d = p->d;
   const int N4 = align_n(d.n, 4), SS = div_up(d.k, 4), DS = N4 / 4;
@@ -489,7 +489,9 @@ static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, 
   a.dst_layout = d.dst_layout;
   a.epilogue = d.epilogue;
   a.scalar_scale = d.scalar_scale;
-  a.pdl = p->pdl ? (d.independent_io != 0 && scatter == nullptr && wait == nullptr ? 2 : 1) : 0;
+  a.pdl = !p->pdl ? kPdlOff
+          : wait_first ? kPdlWaitFirst
+          : d.independent_io != 0 && scatter == nullptr && wait == nullptr ? kPdlIndependent : kPdlOverlap;
   a.trace = g_trace_buffer;
   a.trace_skip_math = 0;
 #ifdef MLD_TRACE
@@ -654,7 +656,7 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
     const StripGeometry gm = strip_geometry_of(plan, tokens);
     if (gm.stages >= 2) {
       plan->last_route = MLD_ROUTE_DECODE_STREAMING;
-      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, stream, nullptr, nullptr);
+      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, true, stream, nullptr, nullptr);
     }
   }
   if (path == 2) {
@@ -681,7 +683,7 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
     const StripGeometry gm = strip_geometry_of(plan, tokens);
     if (gm.stages >= 2) {
       plan->last_route = MLD_ROUTE_DECODE_STREAMING;
-      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, stream, scatter, wait);
+      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, d.has_zero_point || tokens > 16, stream, scatter, wait);
     }
   }
   if (d.epilogue != MLD_EPILOGUE_NONE) {

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   }
   // cluster partners: arrive now, wait only before the first remote access
   if (a.ksplit > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  if (a.pdl) pdl_launch_dependents();
+  if (a.pdl == kPdlOverlap || a.pdl == kPdlIndependent) pdl_launch_dependents();
 
   if (warp == kConsumerWarps) {
     // ------------------------------------------------------------ producer
@@ -301,19 +301,20 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       };
       // weights and scales are constants: the first ring-full of them is
       // requested before waiting for the preceding kernel; activations after.
-      // Launches that overlap completely request the whole ring at once, one lane per stage.  A launch that
+      // Launches that overlap completely, or not at all, request the whole ring at once, one lane per stage.  A launch that
       // hands over at the activation load requests it stage by stage: measured, its burst only gets in the way
       // of the launch ahead of it, which is still streaming.
       const int head = total < a.stages ? total : a.stages;
-      if (a.pdl == 2) {
+      if (a.pdl >= kPdlIndependent) {
+        if (a.pdl == kPdlWaitFirst) pdl_wait();
         if (lane < head) issue_weights(lane, lane);
         __syncwarp();
       }
       if (lane != 0) return;
-      if (a.pdl != 2)
+      if (a.pdl < kPdlIndependent)
         for (int it = 0; it < head; ++it) issue_weights(it, it);
       if (tr) tr[1] = globaltimer_ns();
-      if (a.pdl == 1) pdl_wait();  // pdl == 2: the caller declared x and y untouched by the launch before
+      if (a.pdl == kPdlOverlap) pdl_wait();  // (independent: the caller declared x and y untouched by the launch before)
       if (a.wait.world > 1) {
         const unsigned seq = static_cast<unsigned>(*a.wait.step * a.wait.seq_per_step + a.wait.seq_off);
         if (!wait_peer_flags(a.wait.flags, a.wait.world, seq, a.wait.limit_ns)) atomicExch(a.error, kErrPeerWait);
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       // share of the next projection's weights into L2.
       // Launches that did not wait above still complete in stream order: the grid is not done before the
       // grid ahead of it is.
-      if (a.pdl == 2) pdl_wait();
+      if (a.pdl == kPdlIndependent) pdl_wait();
       if (a.next_w != nullptr) {
         const unsigned long long per = ((a.next_w_bytes / gridDim.x) + 127ull) & ~127ull;
         unsigned long long lo = per * blockIdx.x, hi = lo + per;

@@ -67,6 +67,14 @@ struct PeerOutputs {
 };
 
 constexpr int kStripTokens = 32;  // tokens of one launch of the streaming kernel at most
+// How a launch of the streaming kernel meets its neighbours on the stream; all but the first are launched with
+// programmatic serialization.
+enum StripPdl {
+  kPdlOff = 0,
+  kPdlOverlap = 1,      // weights and scales are asked for at once, x after the launch ahead; the next may begin at once
+  kPdlIndependent = 2,  // nothing waits but the end (mld_fc_desc.independent_io)
+  kPdlWaitFirst = 3,    // nothing is read before the launch ahead is done, and the next begins at this one's end
+};
 struct StripArgs {
   const void* x;      // fp16, sliced [K/4][M_total][4] (for one token a plain vector)
   const void* bias;   // fp16 [N4] or null
@@ -92,7 +100,7 @@ struct StripArgs {
   int dst_layout;
   int epilogue;       // mld_epilogue
   float scalar_scale;
-  int pdl;            // launched with programmatic stream serialization
+  int pdl;            // StripPdl
   PeerScatter scatter;  // world <= 1: outputs go to y only
   PeerWait wait;        // world <= 1: no flag wait before the activations are read
   const void* next_w;  // optional: weights of the projection that runs next, pulled into L2 behind this one

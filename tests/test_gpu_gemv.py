@@ -307,6 +307,37 @@ def test_independent_launch_behind_the_writer_of_its_input(mld, writer):
         assert all(torch.equal(a, b) for a, b in zip(y, want[r % 2]))
 
 
+@pytest.mark.parametrize("tokens,use_zp,forced", [(12, False, False), (1, True, False), (40, True, False), (20, False, True)])
+def test_scales_written_by_the_launch_ahead(mld, tokens, use_zp, forced):
+    """Calls that the general kernel or the GEMM used to serve read their weights' parameters after the launch ahead."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    K, N, K0 = 512, 1024, 16384
+    q0, s0 = mld.quantize_weights(torch.randn(N, K0, device="cuda", generator=g) * 0.02, 4, 32)
+    w0 = (mld.pack_weights(q0, (N, 1, 1, K0), 4)[0], mld.pack_scales(s0, True))
+    ahead = mld.FullyConnectedPlan(N, K0, 4, scale_mode=mld.SCALE_BLOCK, groups=K0 // 32)
+    q, _ = mld.quantize_weights(torch.randn(N, K, device="cuda", generator=g), 4, 0)
+    w, _ = mld.pack_weights(q, (N, 1, 1, K), 4)
+    plan = mld.FullyConnectedPlan(N, K, 4, has_zero_point=use_zp, max_tokens=tokens, force_path=mld.PATH_GEMV if forced else 0)
+    x = torch.randn(K // 4, tokens, 4, device="cuda", generator=g).half()
+    inputs = [torch.randn(K0, device="cuda", generator=g).half() for _ in range(2)]
+    params = torch.zeros(N, dtype=torch.float16, device="cuda")
+    y = torch.zeros(N // 4, tokens, 4, dtype=torch.float16, device="cuda")
+
+    def chain(i, wait):
+        ahead.run(inputs[i], *w0, params, 1)
+        if wait:
+            torch.cuda.synchronize()
+        plan.run(x, w, params, y, tokens, zero_point=params if use_zp else None)
+        assert plan.last_route() == mld.ROUTE_DECODE_STREAMING
+        torch.cuda.synchronize()
+        return y.clone()
+
+    want = [chain(i, True) for i in range(2)]
+    assert not torch.equal(*want)
+    for r in range(20):
+        assert torch.equal(chain(r % 2, False), want[r % 2])
+
+
 @pytest.mark.parametrize("K,N,block", [(2048, 1024, 32), (40, 64, 0), (200, 328, 0), (4096, 512, 64), (1032, 1160, 0),
                                        (11008, 256, 128)])
 @pytest.mark.parametrize("outliers", [False, True])
