@@ -675,7 +675,7 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
     plan->last_route = MLD_ROUTE_DECODE_GENERAL;
     return run_generic(plan, src, weights, scale, zp, b, dst, tokens, stream);
   }
-  if (d.epilogue != MLD_EPILOGUE_NONE && !(path == 1 && plan->stream_ok && tokens <= 16)) {
+  if (d.epilogue != MLD_EPILOGUE_NONE && !(path == 1 && plan->stream_ok && !d.has_zero_point && tokens <= 16)) {
     set_last_error_text("the fused SiLU*mul write is available on the streaming decode kernel only");
     return MLD_UNIMPLEMENTED;
   }

@@ -417,6 +417,17 @@ def test_errors(mld):
         plan.run(x, x, None, x, 1)       # per-channel scale tensor missing
 
 
+def test_fused_write_refuses_zero_points(mld):
+    plan = mld.FullyConnectedPlan(64, 256, 4, scale_mode=mld.SCALE_BLOCK, groups=8, has_zero_point=True,
+                                  epilogue=mld.EPILOGUE_SWIGLU_PAIRS)
+    x = torch.zeros(256, dtype=torch.float16, device="cuda")
+    w = torch.zeros(64 * 128, dtype=torch.uint8, device="cuda")
+    s = torch.zeros(8 * 64, dtype=torch.float16, device="cuda")
+    with pytest.raises(mld.MldError) as e:
+        plan.run(x, w, s, torch.zeros(64, dtype=torch.float16, device="cuda"), 1, zero_point=s)
+    assert e.value.status == mld.UNIMPLEMENTED
+
+
 # ------------------------------------------------- the streaming kernel over its token and scale-layout range
 def _exact_fc(x, q, scale, zp=None):
     """[M][N] in 64 bits from fp16 activations, integers [N][K], fp16 scales and zero points [N][G]"""
