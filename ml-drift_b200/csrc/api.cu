@@ -640,6 +640,10 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
 
   int path = d.force_path;
   if (path == 0) path = mld_fc_is_gemv_recommended(d.precision, tokens) ? 1 : 2;
+  if (d.epilogue != MLD_EPILOGUE_NONE && !(path == 1 && plan->stream_ok && !d.has_zero_point && tokens <= 16)) {
+    set_last_error_text("the fused SiLU*mul write is available on the streaming decode kernel only");
+    return MLD_UNIMPLEMENTED;
+  }
   const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(scale) & 15) == 0 &&
                        (reinterpret_cast<uintptr_t>(zp) & 15) == 0;
   const bool layout_ok = d.src_layout == MLD_LAYOUT_SLICED || tokens == 1;
@@ -651,8 +655,7 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
   // tokens as two launches hold.
   const bool few = d.force_path == 0 && d.prefill_act_quant == 0 && d.prefill_route == MLD_PREFILL_ROUTE_AUTO &&
                    d.cache_prepared_weights == 0 && outs == nullptr && tokens <= 16;
-  if (streams && path == 2 && (d.has_zero_point ? tokens <= 2 * kStripTokens : few && plan->pdl && plan->subnormal) &&
-      d.epilogue == MLD_EPILOGUE_NONE) {
+  if (streams && path == 2 && (d.has_zero_point ? tokens <= 2 * kStripTokens : few && plan->pdl && plan->subnormal)) {
     const StripGeometry gm = strip_geometry_of(plan, tokens);
     if (gm.stages >= 2) {
       plan->last_route = MLD_ROUTE_DECODE_STREAMING;
@@ -674,10 +677,6 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
     }
     plan->last_route = MLD_ROUTE_DECODE_GENERAL;
     return run_generic(plan, src, weights, scale, zp, b, dst, tokens, stream);
-  }
-  if (d.epilogue != MLD_EPILOGUE_NONE && !(path == 1 && plan->stream_ok && !d.has_zero_point && tokens <= 16)) {
-    set_last_error_text("the fused SiLU*mul write is available on the streaming decode kernel only");
-    return MLD_UNIMPLEMENTED;
   }
   if (streams && tokens <= (plan->pdl && plan->subnormal ? 2 * kStripTokens : 16)) {
     const StripGeometry gm = strip_geometry_of(plan, tokens);

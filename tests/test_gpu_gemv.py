@@ -428,6 +428,19 @@ def test_fused_write_refuses_zero_points(mld):
     assert e.value.status == mld.UNIMPLEMENTED
 
 
+@pytest.mark.parametrize("tokens,path", [(12, 0), (1, 2)])
+def test_fused_write_refuses_the_prefill_route(mld, tokens, path):
+    # (dst holds half of the rows; the GEMM would write all of them)
+    plan = mld.FullyConnectedPlan(64, 256, 4, scale_mode=mld.SCALE_BLOCK, groups=8, max_tokens=tokens, force_path=path,
+                                  epilogue=mld.EPILOGUE_SWIGLU_PAIRS)
+    x = torch.zeros(256 * tokens, dtype=torch.float16, device="cuda")
+    w = torch.zeros(64 * 128, dtype=torch.uint8, device="cuda")
+    s = torch.zeros(8 * 64, dtype=torch.float16, device="cuda")
+    with pytest.raises(mld.MldError) as e:
+        plan.run(x, w, s, torch.zeros(64 * tokens, dtype=torch.float16, device="cuda"), tokens)
+    assert e.value.status == mld.UNIMPLEMENTED
+
+
 # ------------------------------------------------- the streaming kernel over its token and scale-layout range
 def _exact_fc(x, q, scale, zp=None):
     """[M][N] in 64 bits from fp16 activations, integers [N][K], fp16 scales and zero points [N][G]"""
