@@ -178,21 +178,25 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 
 // W: weight boxes per stage (strip width up to W * 128 bytes per pass).
 // MONE: single-token launch (only token column 0 is kept).
-// DIGITS (one token, a one-token activation vector): integer MMAs instead.  The whole
-// activation vector is fetched once, and before the first stage is consumed the warps turn every unit
-// of 32 inputs into 16-bit fixed point with a power-of-two scale of its own, x ~ s (256 hi + lo).  One
-// m16n8k32 u8 x s8 MMA per 16 outputs and unit then multiplies the stored weights (4 bits: as the bytes of the
-// reference layout, which hold two outputs each; 8 bits: bytes of a block turned round) by the unit's two digits; four
-// units share accumulators (their digits sit in different B columns).  A 4-bit stage costs 64 MMAs where the fp16 form
-// needs 144, an 8-bit stage 32 against 96, and an fp16 MMA occupies the pipe twice as long: the 8-bit form was bound by
-// it (151936 x 2048: 64.0 us before).  Everything is exact in int32; the error is that of the fixed point, at most
-// 2^-16 of the unit's largest input per input.
+// DIGITS (one token): integer MMAs instead.  The whole activation vector is fetched once, and before the first stage is
+// consumed the warps turn every unit of 32 inputs into fixed point with a power-of-two scale of its own, in signed 8-bit
+// digits.  One m16n8k32 u8 x s8 MMA per 16 outputs and unit then multiplies the stored weights (4 bits: as the bytes of the
+// reference layout, which hold two outputs each; 8 bits: bytes of a block turned round) by the unit's digits, a B column
+// each, so that four (two) units share accumulators.  A 4-bit stage costs 64 MMAs where the fp16 form needs 144, an 8-bit
+// stage 32 against 96, and an fp16 MMA occupies the pipe twice as long.  Products and sums of a unit are exact in int32.
+//  * 4-bit weights: 16-bit fixed point, x ~ s (256 hi + lo), an input's error at most 2^-15 of the unit's largest.
+//  * 8-bit weights: 32-bit fixed point in four digits, an input's error at most 2^-31 of the unit's largest, which is below
+//    what the fp32 sums of the fp16 form lose (its terms are up to 255 x, their offset 128 x taken off at the end).  2048
+//    inputs, one in 32 of them 300 with zero weights: error against 64 bits 2.1e-4, the rounding of the output; two digits
+//    4.5e-3, the fp16 form 2.2e-4.  151936 x 2048 in a graph: 49.1 us; two digits 47.3, the fp16 form 55.8.
 // SPLIT: more than eight tokens (an MMA's columns) are split over the warps: 2^ts_shift warps share 8 << ts_shift k-slice rows
 // of a stage and take eight tokens each.  They unpack the same weights, which costs less than the MMAs, and a lane's
 // accumulators stay eight tokens wide, so that two CTAs still fit an SM.
 // ZP: a zero point per scale; a second box of the scales' shape follows them in the stage.  (u - 8 - z) s x summed
 // over a group is s (sum(u x) - (1 + z / 8) 8 sum(x)), so the zero point only scales the offset term, in fp32
-// (2048 x 4096 INT4, 12 tokens: 9.2 us; the general kernel, which took such weights before, 45.8).
+// (2048 x 4096 INT4, 12 tokens: 10.3 us; the general kernel, which took such weights before, 45.8).  One token stays in the
+// fp16 form: these launches wait before they read anything, so the digits have no stream to hide behind (2048 x 4096 in a
+// graph 6.0 us, two digits 6.2, four 6.5).
 // INTERLEAVE: the passes of all strips lie side by side (StripGeometry::interleave).  A form of its own, because the steps
 // and box counts that only it has, worked out at run time, cost every other launch 0.3 to 0.8 us (14208 x 2432 INT4, one
 // token 13.6 against 12.9; 4096 x 11008 10.9 against 10.2).  Several tokens through strips of two boxes take this form always:
@@ -205,6 +209,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   static_assert(!ZP || SUBNORMAL, "the offset term comes from the constant operand of the subnormal form");
   constexpr int WT = W * F::BOX_N;       // outputs per pass
   constexpr int NJ = MONE ? 2 : 4;       // accumulator values kept per fragment
+  constexpr int ND = BITS == 4 ? 2 : 4;  // DIGITS: digits of an activation
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* red = reinterpret_cast<float*>(smem + (size_t)a.stages * a.stage_bytes);  // [warps][WT][red_m]
@@ -212,11 +217,13 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   uint64_t* full = reinterpret_cast<uint64_t*>(peer + ((WT * a.peer_m + 1) & ~1));
   uint64_t* empty = full + a.stages;
   uint64_t* peer_bar = empty + a.stages;
-  // DIGITS: the activation vector of this CTA's K range, digitised in place ([unit][hi: 8 words][lo: 8 words],
-  // word j = the four inputs of k-slice j), then per unit {bits of the digit scale, 8 x the sum of its integers}
+  // DIGITS: the activation vector of this CTA's K range as digits ([unit][digit, the highest first][8 words], word j = the
+  // four inputs of k-slice j), the vector itself (two digits take its place), then per unit and pair of digits {bits of
+  // the pair's scale, its offset: 8 (128) x the sum of the pair's integers}
   uint64_t* xbar = peer_bar + 1;
   uint8_t* xdig = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(xbar + 1) + 15) & ~uintptr_t(15));
-  uint2* xmeta = reinterpret_cast<uint2*>(xdig + (size_t)a.rows_per_split * 8);
+  uint8_t* xraw = ND == 4 ? xdig + (size_t)a.rows_per_split * 16 : xdig;
+  uint2* xmeta = reinterpret_cast<uint2*>(xraw + (size_t)a.rows_per_split * 8);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kr = a.ksplit > 1 ? static_cast<int>(cluster_ctarank()) : 0;
@@ -323,7 +330,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       if constexpr (DIGITS) {
         const uint32_t xbytes = static_cast<uint32_t>(r_hi - r_lo) * 8u;
         mbar_arrive_expect_tx(xbar, xbytes);
-        bulk_load_1d(xdig, static_cast<const uint8_t*>(a.x) + (size_t)r_lo * 8, xbytes, xbar);
+        bulk_load_1d(xraw, static_cast<const uint8_t*>(a.x) + (size_t)r_lo * 8, xbytes, xbar);
       }
       for (int it = 0; it < head; ++it) issue_x(it, it);
       int stage = head == a.stages ? 0 : head;
@@ -386,7 +393,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         const int row = r_lo + u * 8 + 2 * q;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (have && row < r_hi) {
-          v = *reinterpret_cast<const uint4*>(xdig + (size_t)u * 64 + q * 16);
+          v = *reinterpret_cast<const uint4*>(xraw + (size_t)u * 64 + q * 16);
           if (row + 1 >= r_hi) v.z = v.w = 0u;
         }
         __syncwarp();  // the unit's four lanes have read before any of them rewrites it
@@ -414,29 +421,63 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         unsigned bad = (non_finite(v.x) || non_finite(v.y) || non_finite(v.z) || non_finite(v.w)) ? 1u : 0u;
         bad |= __shfl_xor_sync(0xffffffffu, bad, 1);
         bad |= __shfl_xor_sync(0xffffffffu, bad, 2);
-        // z = round(x / s) + 128 in the low 16 bits of the sum's mantissa: byte 1 = high digit, byte 0 ^ 0x80 = low digit
-        uint32_t z[8];
+        if constexpr (ND == 4) {
+          // x 65536 / s rounded (|.| <= 127 x 2^24), plus 2^7, 2^15 and 2^23: its bytes are the digits, the lower three ^ 0x80
+          uint32_t w[2][4];  // [k-slice][byte]: the four inputs of that byte
 #pragma unroll
-        for (int i = 0; i < 8; ++i) z[i] = __float_as_uint(fmaf(xf[i], inv, 12583040.0f));
-        uint32_t hiw[2], low[2];
+          for (int e = 0; e < 2; ++e) {
+            uint32_t z[4];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const uint32_t h01 = prmt(z[4 * e], z[4 * e + 1], 0x0051u), h23 = prmt(z[4 * e + 2], z[4 * e + 3], 0x0051u);
-          const uint32_t l01 = prmt(z[4 * e], z[4 * e + 1], 0x0040u), l23 = prmt(z[4 * e + 2], z[4 * e + 3], 0x0040u);
-          hiw[e] = prmt(h01, h23, 0x5410u);
-          low[e] = prmt(l01, l23, 0x5410u) ^ 0x80808080u;
-        }
-        int isum = __dp4a(static_cast<int>(hiw[0]), 0x01010101, 0);
-        isum = __dp4a(static_cast<int>(hiw[1]), 0x01010101, isum) * 256;
-        isum = __dp4a(static_cast<int>(low[0]), 0x01010101, isum);
-        isum = __dp4a(static_cast<int>(low[1]), 0x01010101, isum);
-        isum += __shfl_xor_sync(0xffffffffu, isum, 1);
-        isum += __shfl_xor_sync(0xffffffffu, isum, 2);
-        if (have) {
-          uint32_t* ud = reinterpret_cast<uint32_t*>(xdig + (size_t)u * 64);
-          *reinterpret_cast<uint2*>(ud + 2 * q) = make_uint2(hiw[0], hiw[1]);
-          *reinterpret_cast<uint2*>(ud + 8 + 2 * q) = make_uint2(low[0], low[1]);
-          if (q == 0) xmeta[u] = make_uint2(bad ? 0x7FC00000u : sbits, static_cast<uint32_t>((BITS == 4 ? 8 : 128) * isum));  // (stored weights = weights + 8, + 128)
+            for (int i = 0; i < 4; ++i) z[i] = static_cast<uint32_t>(__float2int_rn(xf[4 * e + i] * inv * 65536.0f)) + 0x00808080u;
+            transpose_bytes(make_uint4(z[0], z[1], z[2], z[3]), w[e]);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) w[e][b] ^= 0x80808080u;
+          }
+          int isum[2];  // of the high pair of digits and of the low one
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int b = 3 - 2 * h;
+            int v2 = __dp4a(static_cast<int>(w[0][b]), 0x01010101, 0);
+            v2 = __dp4a(static_cast<int>(w[1][b]), 0x01010101, v2) * 256;
+            v2 = __dp4a(static_cast<int>(w[0][b - 1]), 0x01010101, v2);
+            v2 = __dp4a(static_cast<int>(w[1][b - 1]), 0x01010101, v2);
+            v2 += __shfl_xor_sync(0xffffffffu, v2, 1);
+            isum[h] = v2 + __shfl_xor_sync(0xffffffffu, v2, 2);
+          }
+          if (have) {
+            uint32_t* ud = reinterpret_cast<uint32_t*>(xdig + (size_t)u * 128);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) *reinterpret_cast<uint2*>(ud + (3 - b) * 8 + 2 * q) = make_uint2(w[0][b], w[1][b]);
+            if (q == 0) {
+              xmeta[2 * u] = make_uint2(bad ? 0x7FC00000u : sbits, static_cast<uint32_t>(128 * isum[0]));
+              xmeta[2 * u + 1] = make_uint2(sbits - (16u << 23), static_cast<uint32_t>(128 * isum[1]));  // (bytes = weights + 128)
+            }
+          }
+        } else {
+          // z = round(x / s) + 128 in the low 16 bits of the sum's mantissa: byte 1 = high digit, byte 0 ^ 0x80 = low digit
+          uint32_t z[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) z[i] = __float_as_uint(fmaf(xf[i], inv, 12583040.0f));
+          uint32_t hiw[2], low[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const uint32_t h01 = prmt(z[4 * e], z[4 * e + 1], 0x0051u), h23 = prmt(z[4 * e + 2], z[4 * e + 3], 0x0051u);
+            const uint32_t l01 = prmt(z[4 * e], z[4 * e + 1], 0x0040u), l23 = prmt(z[4 * e + 2], z[4 * e + 3], 0x0040u);
+            hiw[e] = prmt(h01, h23, 0x5410u);
+            low[e] = prmt(l01, l23, 0x5410u) ^ 0x80808080u;
+          }
+          int isum = __dp4a(static_cast<int>(hiw[0]), 0x01010101, 0);
+          isum = __dp4a(static_cast<int>(hiw[1]), 0x01010101, isum) * 256;
+          isum = __dp4a(static_cast<int>(low[0]), 0x01010101, isum);
+          isum = __dp4a(static_cast<int>(low[1]), 0x01010101, isum);
+          isum += __shfl_xor_sync(0xffffffffu, isum, 1);
+          isum += __shfl_xor_sync(0xffffffffu, isum, 2);
+          if (have) {
+            uint32_t* ud = reinterpret_cast<uint32_t*>(xdig + (size_t)u * 64);
+            *reinterpret_cast<uint2*>(ud + 2 * q) = make_uint2(hiw[0], hiw[1]);
+            *reinterpret_cast<uint2*>(ud + 8 + 2 * q) = make_uint2(low[0], low[1]);
+            if (q == 0) xmeta[u] = make_uint2(bad ? 0x7FC00000u : sbits, static_cast<uint32_t>(8 * isum));  // (nibbles = weights + 8)
+          }
         }
       }
     }
@@ -480,7 +521,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       const uint8_t* xs = st + W * kBoxBytes + a.scale_stage_bytes;
       const int row0 = r_lo + si * kStageRows;
       if constexpr (DIGITS) {
-        static_assert(!DIGITS || MONE, "the digit form is for one token");
+        static_assert(MONE && !ZP, "the digit form is for one token and weights without zero points");
         // A stage is 2 W tasks: (half of its 64 k-slice rows = four units) x (box of 64 outputs).  The four
         // units of a task share accumulators: B column 2 j holds the high and 2 j + 1 the low digits of unit j
         // (lanes g supply column g, zero for the other units), so after the units' MMAs lane t holds both
@@ -491,19 +532,26 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         const int task = warp % T, tb = task >> 1, hq = task & 1;
         if (tb < boxes && si % GC == warp / T) {
           const int ubase = si * 8 + hq * 4;  // the task's first unit within the CTA's K range
-          const uint32_t* ud = reinterpret_cast<const uint32_t*>(xdig + (size_t)(ubase + (g >> 1)) * 64) + 8 * (g & 1);
-          const uint32_t bm0 = ud[t], bm1 = ud[4 + t];
-          int acc[F::NF][4];
+          constexpr int U = 8 / ND;  // units that share a set of accumulators
+          uint32_t bm[4 / U][2];
+          int accs[4 / U][F::NF][4];
 #pragma unroll
-          for (int f = 0; f < F::NF; ++f) acc[f][0] = acc[f][1] = acc[f][2] = acc[f][3] = 0;
+          for (int p = 0; p < 4 / U; ++p) {
+            const uint32_t* ud = reinterpret_cast<const uint32_t*>(xdig) + ((size_t)(ubase + p * U + g / ND) * ND + g % ND) * 8;
+            bm[p][0] = ud[t];
+            bm[p][1] = ud[4 + t];
+#pragma unroll
+            for (int f = 0; f < F::NF; ++f) accs[p][f][0] = accs[p][f][1] = accs[p][f][2] = accs[p][f][3] = 0;
+          }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             // k-slice rows ra and ra + 4 of unit j are what lane t feeds the MMA's K with
             const int ra = 32 * hq + 8 * j + t, rb = ra + 4;
             const uint4 qa = *reinterpret_cast<const uint4*>(st + tb * kBoxBytes + ra * 128 + ((g ^ (ra & 7)) << 4));
             const uint4 qb = *reinterpret_cast<const uint4*>(st + tb * kBoxBytes + rb * 128 + ((g ^ (rb & 7)) << 4));
-            const bool mine = (g >> 1) == j;
-            const uint32_t b0 = mine ? bm0 : 0u, b1 = mine ? bm1 : 0u;
+            const bool mine = g / ND == j % U;
+            const uint32_t b0 = mine ? bm[j / U][0] : 0u, b1 = mine ? bm[j / U][1] : 0u;
+            int(&acc)[F::NF][4] = accs[j / U];
             if constexpr (BITS == 4) {
 #pragma unroll
               for (int f = 0; f < 4; ++f) {
@@ -528,52 +576,44 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
               }
             }
           }
-          // lane t finishes unit t: its digit scale and offset, the weight scales of its group
-          const uint2 meta = xmeta[ubase + t];
-          const float sx = __uint_as_float(meta.x);
-          const int off = static_cast<int>(meta.y);
-          float sc[F::NPL], zo[F::NPL];
-          const int gidx = a.gs_shift >= 0 ? ((32 * hq + 8 * t) >> a.gs_shift) : 0;
-          const auto load_params = [&](const uint8_t* box, float (&v)[F::NPL]) {
-            const __half* p = reinterpret_cast<const __half*>(box) + gidx * WT + tb * F::BOX_N + F::NPL * g;
+          // lane t finishes columns 2t and 2t + 1, a pair of digits of one unit: the pair's scale and offset, the weight
+          // scales of the unit's group
 #pragma unroll
-            for (int i = 0; i < F::NPL / 4; ++i) {
-              const uint2 w = reinterpret_cast<const uint2*>(p)[i];
-              const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
-              const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-              v[4 * i] = f0.x; v[4 * i + 1] = f0.y; v[4 * i + 2] = f1.x; v[4 * i + 3] = f1.y;
+          for (int p = 0; p < 4 / U; ++p) {
+            const int unit = p * U + 2 * t / ND, pair = t % (ND / 2);  // of the task's four
+            const int(&acc)[F::NF][4] = accs[p];
+            const uint2 meta = xmeta[(ubase + unit) * (ND / 2) + pair];
+            const float sx = __uint_as_float(meta.x);
+            const int off = static_cast<int>(meta.y);
+            float sc[F::NPL];
+            const int gidx = a.gs_shift >= 0 ? ((32 * hq + 8 * unit) >> a.gs_shift) : 0;
+            if (a.scale_rows > 0) {
+              const __half* sp = reinterpret_cast<const __half*>(st + W * kBoxBytes) + gidx * WT + tb * F::BOX_N + F::NPL * g;
+#pragma unroll
+              for (int i = 0; i < F::NPL / 4; ++i) {
+                const uint2 w = reinterpret_cast<const uint2*>(sp)[i];
+                const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
+                const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+                sc[4 * i] = f0.x; sc[4 * i + 1] = f0.y; sc[4 * i + 2] = f1.x; sc[4 * i + 3] = f1.y;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < F::NPL; ++i) sc[i] = a.scalar_scale;
             }
-          };
-          if (a.scale_rows > 0) {
-            load_params(st + W * kBoxBytes, sc);
-          } else {
+            // acc: {row g high digit, row g low, row g + 8 high, row g + 8 low} of the pair
 #pragma unroll
-            for (int i = 0; i < F::NPL; ++i) sc[i] = a.scalar_scale;
-          }
-          if constexpr (ZP) {  // the zero point's share of the unit, z sum(x), in units of the digit scale
-            load_params(st + W * kBoxBytes + a.zp_off, zo);
-            const float isum = static_cast<float>(off) * (BITS == 4 ? 0.125f : 0.0078125f);
-#pragma unroll
-            for (int i = 0; i < F::NPL; ++i) zo[i] *= isum;
-          }
-          // acc: {row g high digit, row g low, row g + 8 high, row g + 8 low} of unit t
-#pragma unroll
-          for (int f = 0; f < F::NF; ++f) {
-            int even, odd;
-            if constexpr (BITS == 4) {
-              even = (acc[f][0] - acc[f][2]) * 256 + (acc[f][1] - acc[f][3]) - off;
-              odd = ((acc[f][2] * 256 + acc[f][3]) >> 4) - off;
-            } else {  // (|sum| <= 32 * 255 * 32640 < 2^28)
-              even = acc[f][0] * 256 + acc[f][1] - off;
-              odd = acc[f][2] * 256 + acc[f][3] - off;
+            for (int f = 0; f < F::NF; ++f) {
+              int even, odd;
+              if constexpr (BITS == 4) {
+                even = (acc[f][0] - acc[f][2]) * 256 + (acc[f][1] - acc[f][3]) - off;
+                odd = ((acc[f][2] * 256 + acc[f][3]) >> 4) - off;
+              } else {  // (|sum| <= 32 * 255 * 32640 < 2^28)
+                even = acc[f][0] * 256 + acc[f][1] - off;
+                odd = acc[f][2] * 256 + acc[f][3] - off;
+              }
+              tot[0][f][0] = fmaf(sc[2 * f] * sx, static_cast<float>(even), tot[0][f][0]);
+              tot[0][f][1] = fmaf(sc[2 * f + 1] * sx, static_cast<float>(odd), tot[0][f][1]);
             }
-            float ev = static_cast<float>(even), od = static_cast<float>(odd);
-            if constexpr (ZP) {
-              ev -= zo[2 * f];
-              od -= zo[2 * f + 1];
-            }
-            tot[0][f][0] = fmaf(sc[2 * f] * sx, ev, tot[0][f][0]);
-            tot[0][f][1] = fmaf(sc[2 * f + 1] * sx, od, tot[0][f][1]);
           }
         }
       } else {
@@ -870,8 +910,9 @@ int launch_strip_w(bool subnormal, bool mone, const CUtensorMap& tw, const CUten
     if (gm.ts_shift > 0) return launch_strip_t<BITS, W, true, false, false, ZP, true>(tw, ts, tz, a, gm, stream);
   }
   if (ZP || subnormal) {
-    if (mone && a.M_total == 1 && gm.xdig_bytes > 0)
-      return launch_strip_t<BITS, W, true, true, true, ZP>(tw, ts, tz, a, gm, stream);
+    if constexpr (!ZP) {
+      if (gm.xdig_bytes > 0) return launch_strip_t<BITS, W, true, true, true>(tw, ts, tz, a, gm, stream);
+    }
     if (mone) return launch_strip_t<BITS, W, true, true, false, ZP>(tw, ts, tz, a, gm, stream);
     return launch_strip_t<BITS, W, true, false, false, ZP>(tw, ts, tz, a, gm, stream);
   }
@@ -946,15 +987,29 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
   gm.stage_bytes = align_n(gm.w * kBoxBytes + gm.scale_stage_bytes + x_bytes, 1024);
   gm.red_m = m_total < 8 ? m_total : 8;
   gm.peer_m = gm.ksplit == 1 ? 0 : m_total < gm.launch_tokens ? m_total : gm.launch_tokens;
-  // 4-bit weights: room for a one-token activation vector of this CTA's K range as digits (8 bytes per k-slice,
-  // 8 per unit of eight k-slices, a barrier)
-  gm.xdig_bytes = m_total == 1 ? gm.rows_per_split * 9 + 48 : 0;
-  const int fixed = (kConsumerWarps * gm.red_m + gm.peer_m) * wt * 4 + 8 + (2 * 16 + 1) * 8 + gm.xdig_bytes + 1024 + 64;
   gm.stage_rows = kStageRows;
   // With programmatic dependent launch two consecutive GEMVs share an SM while
   // one drains and the next prefetches, so each takes at most half of it.
   int budget = pdl ? 112 * 1024 : 224 * 1024;
   if (smem_limit_kb >= 32 && smem_limit_kb <= 224) budget = smem_limit_kb * 1024;
+  int fixed = (kConsumerWarps * gm.red_m + gm.peer_m) * wt * 4 + 8 + (2 * 16 + 1) * 8 + 1024 + 64;
+  // One token as digits: room for the activation vector of this CTA's K range (per k-slice 8 bytes, 4 digits 16 more; per
+  // unit of eight k-slices 8 bytes for every two digits; a barrier).
+  if (m_total == 1 && split && !zero_point) {
+    const int xdig = gm.rows_per_split * (bits == 4 ? 9 : 26) + 48;
+    if (bits == 4) {
+      gm.xdig_bytes = xdig;
+    } else {
+      // 8-bit weights take four digits where a CTA multiplies enough by them to pay for turning the whole vector into them,
+      // and only as long as the ring keeps three stages beside them.  us in a graph, fp16 form / digits: 151936 x 2048 55.8 /
+      // 49.1, 65536 x 2048 28.1 / 24.8, 12288 x 4096 14.8 / 13.8, 12288 x 8192 27.7 / 25.4; below the first line 12288 x 1024
+      // 6.0 / 6.4, 32000 x 640 7.5 / 8.1, 8192 x 4096 9.4 / 9.9; below the second 16384 x 11008 36.6 / 42.9.
+      const int passes = gm.interleave ? div_up(C, strips * gm.w * 8) : div_up(max_width, gm.w * 8);
+      const bool pays = strips > sms && passes * (gm.rows_per_split / kStageRows) >= 16;
+      gm.xdig_bytes = pays && (budget - fixed - xdig) / gm.stage_bytes >= 3 ? xdig : 0;
+    }
+    fixed += gm.xdig_bytes;
+  }
   int stages = (budget - fixed) / gm.stage_bytes;
   if (stages > 16) stages = 16;
   if (stages < 2) stages = (227 * 1024 - fixed) / gm.stage_bytes;

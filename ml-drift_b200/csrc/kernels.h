@@ -116,7 +116,7 @@ struct StripGeometry {
   int scale_stage_bytes, zp_off, stage_bytes, stages, red_m, peer_m, stage_rows;
   int ts_shift, launch_tokens;
   int interleave;  // a strip's passes lie a grid's width apart instead of side by side
-  int xdig_bytes;  // shared memory kept for the digitised activation vector (4-bit weights), else 0
+  int xdig_bytes;  // shared memory kept for the digitised activation vector; 0: the fp16 form
   size_t smem_bytes;
 };
 StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slices, int scale_mode, int sms,

@@ -371,6 +371,40 @@ def test_one_token_int4_digit_route(mld, oracle, K, N, block, outliers):
         assert not np.isfinite(y).any()
 
 
+@pytest.mark.parametrize("use_zp", [False, True])
+@pytest.mark.parametrize("K,N", [(4096, 9600), (2056, 32000), (1032, 40968), (2048, 1024), (9088, 9480), (640, 65544)])
+def test_one_token_int8_loses_nothing_beside_outliers(mld, oracle, K, N, use_zp):
+    """One input in 32 is 300 and meets weights of zero, so only its 31 neighbours make the output: what a unit's scale
+    costs them is the error.  The fp16 form and the 32-bit digits (wide matrices) leave the rounding of the output, 2^-11
+    of the largest, and fp32 sums: 6e-4."""
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    q = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda", generator=g)
+    scale = (torch.rand((N, 1), device="cuda", generator=g) + 0.5) / 4096
+    zp = torch.randint(-100, 100, (N, 1), device="cuda", generator=g).float()
+    q[:, 5::32] = zp.to(torch.int8) if use_zp else 0
+    x = torch.randn(K, device="cuda", generator=g)
+    x[5::32] = 300.0
+    x = x.half()
+    packed, _ = mld.pack_weights(q, (N, 1, 1, K), 8)
+    w = q.double() - (zp.double() if use_zp else 0.0)
+    want = (w @ x.double()) * scale.half().double()[:, 0]
+
+    def run(x, exact_operands=False):
+        plan = mld.FullyConnectedPlan(N, K, 8, has_zero_point=use_zp, exact_operands=exact_operands)
+        y = torch.full((N,), float("nan"), dtype=torch.float16, device="cuda")
+        plan.run(x, packed, mld.pack_scales(scale, True), y, 1, zero_point=mld.pack_scales(zp, True) if use_zp else None)
+        torch.cuda.synchronize()
+        assert plan.device_status() == 0
+        return y.double()
+
+    top = want.abs().max()
+    assert (run(x) - want).abs().max() <= 6e-4 * top
+    if not use_zp:
+        assert (run(x, exact_operands=True) - want).abs().max() <= 6e-4 * top
+    x[K // 2] = float("inf")
+    assert not torch.isfinite(run(x)).any()
+
+
 def test_row_major_single_token(mld, oracle):
     rng = np.random.default_rng(6)
     K, N = 1024, 512
@@ -455,7 +489,8 @@ def _exact_fc(x, q, scale, zp=None):
                                             (8, 1032, 520, 0), (8, 512, 9600, 0), (4, 256, 19008, 64)])
 @pytest.mark.parametrize("use_zp", [False, True])
 def test_streaming_token_ranges(mld, oracle, M, bits, K, N, block, use_zp):
-    # the dispatch's own choice; rounding to fp16 once (2^-11) and the digits' 2^-16: 1e-3 of the largest output
+    # the dispatch's own choice; rounding to fp16 once (2^-11) and the digits' 2^-15 of a unit's largest: 1e-3 of the
+    # largest output
     if M > 16 and not use_zp:
         pytest.skip("served by the GEMM: test_gpu_gemm.py")
     rng = np.random.default_rng(M * 7 + K + N)
