@@ -362,8 +362,19 @@ __global__ void sum_i_kernel(const int8_t* src, int O, int64_t hwi, int32_t* sum
   }
 }
 
-// [O][G] fp32 -> [G][O4] fp16/fp32, zero padded (OHIToHOIO4 in buffer storage).
-// [O][G] -> [G][O4] through a 32 x 32 tile in shared memory, so that both sides are read and written along their rows
+// [O][G] fp32 -> [G][O4] fp16/fp32, zero padded (OHIToHOIO4 in buffer storage), a thread per value written.  For few
+// groups, where a row of the source is a fraction of a tile's 32 columns (see pack_scales_impl).
+__global__ void __launch_bounds__(256) pack_few_scales_kernel(const float* src, int O, int G, int O4, int dst_f16, void* dst) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (int64_t)G * O4) return;
+  const int g = static_cast<int>(idx / O4), o = static_cast<int>(idx % O4);
+  const float v = o < O ? src[(int64_t)o * G + g] : 0.0f;
+  if (dst_f16)
+    reinterpret_cast<__half*>(dst)[idx] = __float2half_rn(v);
+  else
+    reinterpret_cast<float*>(dst)[idx] = v;
+}
+// The same through a 32 x 32 tile in shared memory, so that both sides are read and written along their rows
 // (14336 x 128: 5.2 us; a thread per output value, reading down a column, fetched every sector of the source eight times
 // and took 11.5).
 __global__ void __launch_bounds__(256) pack_scales_kernel(const float* src, int O, int G, int O4, int dst_f16, void* dst) {
@@ -576,8 +587,13 @@ int pack_scales_impl(const float* src, int32_t o, int32_t g, int32_t dst_f16, vo
   const int O4 = align_n(o, 4);
   const int64_t n = (int64_t)g * O4;
   if (n == 0) return MLD_OK;
-  pack_scales_kernel<<<static_cast<unsigned>((int64_t)div_up(O4, 32) * div_up(g, 32)), 256, 0, stream>>>(src, o, g, O4,
-                                                                                                     dst_f16, dst);
+  // A tile has 32 groups: with one, one lane of 32 loads and one warp of eight stores.  us, a value per thread / tiles:
+  // 151936 x 1 1.7 / 5.7, x 4 3.5 / 6.6, x 16 9.0 / 7.1; 14336 x 1 1.5 / 1.7, x 4 1.6 / 1.7, x 8 1.8 / 1.7, x 128 10.4 / 4.5.
+  if (g <= 4)
+    pack_few_scales_kernel<<<static_cast<unsigned>(div_up64(n, 256)), 256, 0, stream>>>(src, o, g, O4, dst_f16, dst);
+  else
+    pack_scales_kernel<<<static_cast<unsigned>((int64_t)div_up(O4, 32) * div_up(g, 32)), 256, 0, stream>>>(src, o, g, O4,
+                                                                                                       dst_f16, dst);
   MLD_LAUNCH_CHECK();
   return MLD_OK;
 }

@@ -173,3 +173,14 @@ def test_pack_wide_stores(mld, oracle, O, I, bits, offset):
     got = buf.cpu().numpy()
     assert rc == 0 and np.array_equal(got[offset:offset + ref.size], ref.reshape(-1))
     assert (got[:offset] == 0x5A).all() and (got[offset + ref.size:] == 0x5A).all()
+
+
+@pytest.mark.parametrize("O,G", [(1, 1), (533, 1), (4099, 4), (130, 5), (31, 33), (4096, 32), (151936, 1)])
+@pytest.mark.parametrize("f16", [True, False])
+def test_pack_scales_shapes(mld, oracle, O, G, f16):
+    # few groups (a value per thread) and more (tiles of 32 x 32), ragged on both sides
+    s = np.random.default_rng(O + G).standard_normal((O, G)).astype(np.float32)
+    got = mld.pack_scales(_dev(s), f16).cpu().numpy()
+    ref = oracle.scale_layout(s, f16)
+    assert np.array_equal(got.view(np.uint16 if f16 else np.uint32).reshape(-1),
+                          ref.view(np.uint16 if f16 else np.uint32).reshape(-1))
