@@ -84,7 +84,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  // (numbered backwards: a pair waits for the one after it, whose blocks have then begun before its own, whatever else is
+  // on the GPU; blocks begin in the order of their numbers)
+  const int n_pairs = gridDim.x >> 1, pair = n_pairs - 1 - (static_cast<int>(blockIdx.x) >> 1);
   WorkList work0;
   {
     const int shared_units = a.shared_tiles * a.k_blocks;

@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
-  const int pair = blockIdx.x / CTAS, n_pairs = gridDim.x / CTAS;  // ("pair": whoever works on a tile)
+  // ("pair": whoever works on a tile; numbered backwards, so that the pairs another one waits for began before it)
+  const int n_pairs = gridDim.x / CTAS, pair = n_pairs - 1 - static_cast<int>(blockIdx.x) / CTAS;
   WorkList work0;
   {
     const int shared_units = a.shared_tiles * a.k_blocks;
@@ -204,7 +205,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   // accumulator buffer is being read): pieces of 16 token columns, part, part + kDrainParts, ...  A tile cut
   // along K: a pair whose share does not begin with the tile's first k-block (always the first of its segments, so that
   // nothing it waits for comes before) leaves its raw accumulators in its own workspace slot; the pair that has the
-  // first k-block adds the following pairs' slots to its own accumulators, in order, and writes the outputs.
+  // first k-block adds the following pairs' slots to its own accumulators, in order, and writes the outputs.  Blocks begin
+  // in the order of their numbers, so those pairs hold SMs already, whatever else is on the GPU.
   auto drain = [&](const Segment& sg, int part) -> bool {
     const int quad = warp & 3;  // TMEM lanes 32*quad .. 32*quad+31 belong to this warp
     const bool hands_over = sg.kb0 > 0, takes_over = !hands_over && sg.kb1 < a.k_blocks;

@@ -312,3 +312,29 @@ def test_cut_tiles_in_a_replayed_graph(mld, bits, M, K, N, act_quant):
             assert torch.equal(replayed, y)  # (the sums are taken in a fixed order)
     assert plan.device_status() == 0
     plan.close()
+
+
+def test_cut_tiles_beside_another_stream(mld):
+    # two operators on streams of different priority: launches that find only some of the SMs free, whose tiles' parts wait
+    # for one another, give what they give alone
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    cases = []
+    for (M, K, N), priority in (((77, 4096, 11008), 0), ((128, 8192, 1024), -1), ((300, 4096, 1100), 0)):
+        q, s = mld.quantize_weights(torch.randn(N, K, generator=gen, device="cuda") * 0.02, 4, 32)
+        plan = mld.FullyConnectedPlan(N, K, 4, scale_mode=mld.SCALE_BLOCK, groups=K // 32, max_tokens=M)
+        x = torch.randn(K // 4, M, 4, generator=gen, device="cuda").half()
+        args = (x, mld.pack_weights(q, (N, 1, 1, K), 4)[0], mld.pack_scales(s, True))
+        y = torch.empty(N // 4, M, 4, dtype=torch.float16, device="cuda")
+        plan.run(*args, y, M)
+        torch.cuda.synchronize()
+        cases.append((plan, args, y.clone(), y, M, torch.cuda.Stream(priority=priority)))
+    for _ in range(50):
+        for plan, args, want, y, M, stream in cases:
+            y.zero_()
+        torch.cuda.synchronize()
+        for _ in range(4):
+            for plan, args, want, y, M, stream in cases:
+                plan.run(*args, y, M, stream=stream)
+        torch.cuda.synchronize()
+        for plan, args, want, y, M, stream in cases:
+            assert plan.device_status() == 0 and torch.equal(y, want)
