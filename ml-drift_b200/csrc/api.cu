@@ -31,6 +31,16 @@ int sm_count(int device) {
   return n;
 }
 
+cudaError_t zero_now(void* p, size_t bytes) {
+  cudaStream_t s;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(p, 0, bytes, s);
+  const cudaError_t done = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  return e != cudaSuccess ? e : done;
+}
+
 encode_tiled_fn get_encode_tiled() {
   static encode_tiled_fn fn = nullptr;
   static std::once_flag once;
@@ -301,7 +311,7 @@ int mld_fc_plan_create(const mld_fc_desc* d, mld_fc_plan** out) {
   {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaMalloc(&p->error, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(p->error, 0, sizeof(int));
+    if (e == cudaSuccess) e = zero_now(p->error, sizeof(int));
     if (e != cudaSuccess) {
       set_last_error("plan workspace", e);
       if (p->error) cudaFree(p->error);
@@ -331,7 +341,7 @@ int mld_fc_plan_create(const mld_fc_desc* d, mld_fc_plan** out) {
     const size_t sb = pair_split_bytes(p->sms), fb = pair_split_flags(p->sms) * sizeof(uint32_t);
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->split.ws), sb);
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->split.flags), fb);
-    if (e == cudaSuccess) e = cudaMemset(p->split.flags, 0, fb);
+    if (e == cudaSuccess) e = zero_now(p->split.flags, fb);
     if (e != cudaSuccess) {
       set_last_error("prefill workspace", e);
       mld_fc_plan_destroy(p);

@@ -46,6 +46,9 @@ static inline int64_t div_up64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline int align_n(int a, int n) { return div_up(a, n) * n; }
 
 int sm_count(int device);
+// Zeroes device memory and waits for it, whatever the legacy stream has to do: an object that is created with it can be
+// used on any stream at once.
+cudaError_t zero_now(void* p, size_t bytes);
 
 // Function attributes such as the dynamic shared-memory limit are per device: a kernel is configured
 // once on every device it is launched on.  `done` is a zero-initialised table owned by the caller (one

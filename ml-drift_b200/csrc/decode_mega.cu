@@ -1987,13 +1987,12 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
   }
   if (cudaMalloc(&m->scratch, scratch_bytes) != cudaSuccess || cudaMalloc(&m->xchg, xchg_bytes) != cudaSuccess ||
       cudaMalloc(&m->d_layers, sizeof(MegaLayer) * cfg.layers) != cudaSuccess ||
-      cudaMalloc(&m->prepared, m->layer_bytes * cfg.layers) != cudaSuccess) {
+      cudaMalloc(&m->prepared, m->layer_bytes * cfg.layers) != cudaSuccess ||
+      zero_now(m->scratch, scratch_bytes) != cudaSuccess || zero_now(m->xchg, xchg_bytes) != cudaSuccess) {
     set_last_error_text("persistent step kernel: device allocation failed");
     mega_destroy(m);
     return MLD_CUDA_ERROR;
   }
-  cudaMemset(m->scratch, 0, scratch_bytes);
-  cudaMemset(m->xchg, 0, xchg_bytes);
   m->peers[cfg.rank] = m->xchg;
   m->qkv = reinterpret_cast<__half*>(m->scratch + o_qkv);
   m->attn = reinterpret_cast<__half*>(m->xchg + m->off_attn);

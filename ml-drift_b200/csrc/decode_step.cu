@@ -662,7 +662,7 @@ int mld_decoder_create(const mld_decoder_desc* d, const void* nccl_id128, mld_de
   for (int r = 0; r < 8; ++r) dec->xchg_peers[r] = nullptr;
   dec->p_qkv = dec->p_o = dec->p_gu = dec->p_down = nullptr;
   int rc = MLD_OK;
-  if (cudaMalloc(&dec->error, sizeof(int)) != cudaSuccess || cudaMemset(dec->error, 0, sizeof(int)) != cudaSuccess ||
+  if (cudaMalloc(&dec->error, sizeof(int)) != cudaSuccess || zero_now(dec->error, sizeof(int)) != cudaSuccess ||
       cudaHostAlloc(&dec->error_host, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
     set_last_error_text("decoder status word allocation failed");
     rc = MLD_CUDA_ERROR;
@@ -701,7 +701,11 @@ int mld_decoder_create(const mld_decoder_desc* d, const void* nccl_id128, mld_de
     mld_decoder_destroy(dec);
     return rc;
   }
-  cudaMemset(dec->scratch, 0, total);
+  if (zero_now(dec->scratch, total) != cudaSuccess) {
+    set_last_error_text("decoder scratch could not be cleared");
+    mld_decoder_destroy(dec);
+    return MLD_CUDA_ERROR;
+  }
   size_t off = 0;
   auto take = [&](size_t bytes) {
     uint8_t* p = dec->scratch + off;
@@ -743,8 +747,11 @@ int mld_decoder_create(const mld_decoder_desc* d, const void* nccl_id128, mld_de
       mld_decoder_destroy(dec);
       return MLD_CUDA_ERROR;
     }
-    cudaMemset(dec->xchg, 0, xo);
-    cudaMemset(dec->peer_tickets, 0, 256);
+    if (zero_now(dec->xchg, xo) != cudaSuccess || zero_now(dec->peer_tickets, 256) != cudaSuccess) {
+      set_last_error_text("decoder exchange block could not be cleared");
+      mld_decoder_destroy(dec);
+      return MLD_CUDA_ERROR;
+    }
     dec->xchg_peers[d->rank] = dec->xchg;
     dec->attn_full = reinterpret_cast<__half*>(dec->xchg + dec->off_attn);
     dec->h = reinterpret_cast<__half*>(dec->xchg + dec->off_h);

@@ -125,12 +125,12 @@ int mld_shard_group_create(int32_t rank, int32_t world, int32_t device, size_t o
   g->peers_ready = world == 1;
   g->comm = nullptr;
   g->limit_ns = 2000ull * 1000ull * 1000ull;
-  if (cudaMalloc(&g->block, g->block_bytes) != cudaSuccess) {
+  if (cudaMalloc(&g->block, g->block_bytes) != cudaSuccess || zero_now(g->block + g->off_flags, 256) != cudaSuccess) {
     set_last_error_text("shard group: device allocation failed");
+    if (g->block != nullptr) cudaFree(g->block);
     delete g;
     return MLD_CUDA_ERROR;
   }
-  cudaMemset(g->block + g->off_flags, 0, 256);
   g->peers[rank] = g->block;
   if (world > 1 && nccl_id128 != nullptr) {
     if (!nccl().load()) {

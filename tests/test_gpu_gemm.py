@@ -338,3 +338,29 @@ def test_cut_tiles_beside_another_stream(mld):
         torch.cuda.synchronize()
         for plan, args, want, y, M, stream in cases:
             assert plan.device_status() == 0 and torch.equal(y, want)
+
+
+def test_operator_is_ready_when_created(mld):
+    # created while the legacy stream is busy and used on a stream that does not wait for that one: nothing of the
+    # operator's workspace (flags of cut tiles, error word) may still be waiting to be cleared
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    M, K, N = 77, 4096, 2048
+    q, s = mld.quantize_weights(torch.randn(N, K, generator=gen, device="cuda") * 0.02, 4, 32)
+    x = torch.randn(K // 4, M, 4, generator=gen, device="cuda").half()
+    args = (x, mld.pack_weights(q, (N, 1, 1, K), 4)[0], mld.pack_scales(s, True))
+    y = torch.empty(N // 4, M, 4, dtype=torch.float16, device="cuda")
+
+    def plan():
+        return mld.FullyConnectedPlan(N, K, 4, scale_mode=mld.SCALE_BLOCK, groups=K // 32, max_tokens=M)
+
+    plan().run(*args, y, M)
+    torch.cuda.synchronize()
+    want, side = y.clone(), torch.cuda.Stream()
+    for _ in range(4):
+        torch.cuda._sleep(20_000_000)                 # about 10 ms on the legacy stream
+        p = plan()
+        for _ in range(1500):                         # past the end of that
+            p.run(*args, y, M, stream=side)
+        side.synchronize()
+        torch.cuda.synchronize()
+        assert p.device_status() == 0 and torch.equal(y, want)
