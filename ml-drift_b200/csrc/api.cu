@@ -658,13 +658,17 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
                        (reinterpret_cast<uintptr_t>(zp) & 15) == 0;
   const bool layout_ok = d.src_layout == MLD_LAYOUT_SLICED || tokens == 1;
   const bool streams = plan->stream_ok && aligned && layout_ok && (!d.has_zero_point || zp != nullptr);
-  // The streaming kernel beyond the decode rule's tokens.  Up to 16 its MMAs take no longer than the GEMM does (us a
-  // call, INT4, streaming / GEMM: 4096 x 4096, 9 tokens 12.4 / 17.0, 16 tokens 14.0 / 17.1; 4096 x 11008 27.2 / 27.9
-  // and 28.4 / 28.1; 8192 x 28672 80 / 104 and 82 / 104; at 24 tokens it loses, 47 / 29 on 4096 x 11008).  With zero
-  // points the alternative is the general kernel (2048 x 4096, 12 tokens: 48 against 9.5 us), so there it takes as many
-  // tokens as two launches hold.
+  // The streaming kernel beyond the decode rule's tokens.  Up to 16 it takes less time than the GEMM on most matrices (us
+  // in a graph, streaming / GEMM, 9 and 16 tokens; 15 matrices of 512..14336 inputs and 1024..28672 outputs were measured
+  // for each of INT4 block 32, INT4 and INT8 per channel.  INT4 block 32: 4096 -> 4096 13.7 / 17.4, 15.0 / 17.6;
+  // 4096 -> 14336 27.5 / 33.9, 28.9 / 34.0; 8192 -> 28672 82 / 105, 83 / 105.  INT8: 2048 -> 2048 8.0 / 12.3, 8.4 / 12.3;
+  // 8192 -> 8192 33.1 / 36.5, 34.1 / 36.5) and is even or up to a tenth slower where strips leave their boxes half empty
+  // (4096 -> 11008 INT4 27.0 / 28.6, 28.2 / 28.6, INT8 29.1 / 28.1, 29.6 / 28.1; 4096 -> 1024 INT4 13.1 / 12.6, 13.8 /
+  // 12.5).  At 24 tokens it loses (4096 -> 11008: 47 / 29).  With zero points the alternative is the general kernel (2048
+  // -> 4096, 12 tokens: 48 against 10.4 us), so there it takes as many tokens as two launches hold.
   const bool few = d.force_path == 0 && d.prefill_act_quant == 0 && d.prefill_route == MLD_PREFILL_ROUTE_AUTO &&
-                   d.cache_prepared_weights == 0 && outs == nullptr && tokens <= 16;
+                   d.cache_prepared_weights == 0 && outs == nullptr && tokens <= 16 &&
+                   (reinterpret_cast<uintptr_t>(b) & 7) == 0;  // (the GEMM refuses such a bias)
   if (streams && path == 2 && (d.has_zero_point ? tokens <= 2 * kStripTokens : few && plan->pdl && plan->subnormal)) {
     const StripGeometry gm = strip_geometry_of(plan, tokens);
     if (gm.stages >= 2) {

@@ -475,6 +475,17 @@ def test_fused_write_refuses_the_prefill_route(mld, tokens, path):
     assert e.value.status == mld.UNIMPLEMENTED
 
 
+@pytest.mark.parametrize("tokens", [12, 40])
+def test_misaligned_bias_is_refused_beyond_the_decode_tokens(mld, tokens):
+    plan = mld.FullyConnectedPlan(64, 256, 4, scale_mode=mld.SCALE_BLOCK, groups=8, has_bias=True, max_tokens=tokens)
+    x, y = (torch.zeros(n * tokens, dtype=torch.float16, device="cuda") for n in (256, 64))
+    w = torch.zeros(64 * 128, dtype=torch.uint8, device="cuda")
+    s = torch.zeros(8 * 64, dtype=torch.float16, device="cuda")
+    with pytest.raises(mld.MldError) as e:
+        plan.run(x, w, s, y, tokens, bias=s[1:65])
+    assert e.value.status == mld.INVALID_ARGUMENT
+
+
 # ------------------------------------------------- the streaming kernel over its token and scale-layout range
 def _exact_fc(x, q, scale, zp=None):
     """[M][N] in 64 bits from fp16 activations, integers [N][K], fp16 scales and zero points [N][G]"""
