@@ -136,19 +136,29 @@ def test_full_size_packing_roundtrip(mld):
     assert torch.equal(sums, q.to(torch.int32).sum(dim=1).to(torch.int32))
 
 
+@pytest.mark.parametrize("I", [256, 384])
 @pytest.mark.parametrize("bits,block", [(8, 0), (4, 32), (4, 0), (4, 128)])
-def test_quantiser_next_to_ties_and_extremes(mld, oracle, bits, block):
-    # values a few ulps around every halfway point, rows whose scale is tiny, huge or subnormal
+def test_quantiser_next_to_ties_and_extremes(mld, oracle, bits, block, I):
+    # groups of four values a few ulps around halfway points (divided), groups just far enough from them to be decided by
+    # the product with the reciprocal (2^-15 of a step), rows whose scale is tiny, huge or subnormal
     rng = np.random.default_rng(bits * 1000 + block)
-    O, I, top = 64, 256, 127 if bits == 8 else 7
+    O, top = 64, 127 if bits == 8 else 7
     bound = np.float32(10.0) ** rng.uniform(-6, 6, (O, 1)).astype(np.float32)
     bound[0], bound[1], bound[2], bound[3] = 1e-42, 3e-38, 3e38, 0.0
     sc = (bound / np.float32(top)).astype(np.float32)
     k = rng.integers(-top, top, (O, I)) + 0.5
-    w = (k * sc).astype(np.float32)
-    w = (w.view(np.int32) + rng.integers(-3, 4, (O, I)) * (w != 0)).view(np.float32)
+    near = (k * sc).astype(np.float32)
+    near = (near.view(np.int32) + rng.integers(-3, 4, (O, I), dtype=np.int32) * (near != 0).astype(np.int32)).view(np.float32)
+    beside = ((k + rng.choice((-1.0, 1.0), (O, I)) * 2.0 ** rng.uniform(-14.9, -13.0, (O, I))) * sc).astype(np.float32)
+    w = np.where(np.arange(I) // 4 % 2 == 0, near, beside)
     w = np.clip(w, -bound, bound).astype(np.float32)
     w[:, ::32] = bound
+    assert w.shape == (O, I) and np.isfinite(w).all()
+    t = w[4:] * (np.float32(1) / sc[4:])
+    decided = (np.abs(t - np.rint(t)) < 0.5 - 2.0 ** -15).reshape(O - 4, -1, 4).all(-1)
+    # the groups of `beside`, but for a few: at 127 steps w and t are rounded by up to 2^-17 of a step each, which takes some
+    # of the offsets between 2^-14.9 and 2^-14.6 (a ninth of the range) back over the line
+    assert 0.4 < decided.mean() < 0.55
     q, s = mld.quantize_weights(_dev(w), bits, block)
     qr, sr = oracle.quantize_int8_sym(w) if bits == 8 else oracle.quantize_int4_sym(w, block)
     assert np.array_equal(q.cpu().numpy(), qr)
