@@ -97,7 +97,6 @@ struct TmapEntry {
   const void* w;
   const void* s;
   const void* z;
-  int boxes;  // width of the scale box, in weight boxes
   CUtensorMap tw, ts, tz;
 };
 
@@ -124,7 +123,8 @@ struct mld_fc_plan {
   bool pair_ok;          // the prefill GEMM can read the packed weights directly (tensor-map pitch rule)
   const void* next_w;    // one-shot L2 prefetch hint for the next mld_fc_run on this plan
   size_t next_w_bytes;
-  std::vector<TmapEntry> tmaps;  // tensor maps keyed by the (weights, scale) pointers last seen
+  // tensor maps keyed by the (weights, scale, zero point) pointers last seen (the boxes do not depend on the token count)
+  std::vector<TmapEntry> tmaps;
   std::mutex mu;
 };
 
@@ -439,13 +439,12 @@ static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, 
     std::lock_guard<std::mutex> lock(p->mu);
     const TmapEntry* te = nullptr;
     for (const TmapEntry& e : p->tmaps)
-      if (e.w == weights && e.s == scale && e.z == zp && e.boxes == gm.w) te = &e;
+      if (e.w == weights && e.s == scale && e.z == zp) te = &e;
     if (te == nullptr) {
       TmapEntry e;
       e.w = weights;
       e.s = scale;
       e.z = zp;
-      e.boxes = gm.w;
       memset(&e.tz, 0, sizeof e.tz);
       const uint64_t blk = d.weight_bits == 4 ? 8 : 16;
       int rc = make_tmap_2d(&e.tw, weights, (uint64_t)DS * blk, SS, (uint64_t)DS * blk, 128, gm.stage_rows, 1,

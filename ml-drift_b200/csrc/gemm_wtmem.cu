@@ -675,7 +675,8 @@ WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share
   const long tiles = (long)g.n_tiles * g.tok_tiles;
   // The last whole wave of tiles and the remainder are cut along K and dealt out evenly; so are the tiles of a launch
   // that has fewer of them than pairs (43 tiles of 4096 x 11008 left 31 of 74 pairs without work), into parts of eight
-  // stages or more and no more than eight of them: the pair that completes a tile reads the other parts' accumulators
+  // stages or more, of an eighth of a tile at least (a tile that does not begin with a part has nine): the pair that
+  // completes a tile reads the other parts' accumulators
   // one after another, which costs about as much as a few stages.
   const bool few = tiles < pairs;
   g.shares_tiles = may_share && tiles % pairs != 0;

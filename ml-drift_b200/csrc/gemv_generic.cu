@@ -1,6 +1,7 @@
 // Decode-stage dequant-GEMV, general form: covers every case of the operator
-// the streaming kernel does not take (fp32 tensors, zero points, ragged shapes,
-// odd scale-group sizes, row-major multi-token activations) with plain loads.
+// the streaming kernel does not take (fp32 tensors, ragged shapes, odd
+// scale-group sizes, row-major multi-token activations, zero points of a scalar
+// scale, beyond 64 tokens or with its tuning switches) with plain loads.
 // A CTA owns four output slices (16 outputs); a lane owns one of them and every
 // 128th input slice, so that four lanes read 64 (32) neighbouring bytes of a
 // weight row and even a 2048 x 2048 matrix is spread over 128 CTAs of 16 warps; a

@@ -152,14 +152,17 @@ struct PairArgs {
   int* error;
   PeerOutputs outs;           // world > 1: the block is stored into every rank's tensor instead of y
   // Work split.  The first shared_tiles tiles are cut into k-block units, in the order (tile 0, k-block 0),
-  // (tile 0, k-block 1), ..., and SM pair p takes the units [p * units_per_pair, (p + 1) * units_per_pair): a
-  // range that is not a whole number of tiles makes the pair share its first and / or last tile with a
-  // neighbour (each tile with at most one: a range is never shorter than a tile); the partial sums meet
-  // through split_ws.  After that the pair takes whole tiles shared_tiles + p, + p + pairs, ...
-  // (shared_tiles = 0: whole tiles only.)
+  // (tile 0, k-block 1), ..., and SM pair p (the tensor-memory kernel's lone CTA p) takes the units
+  // [p * units_per_pair, (p + 1) * units_per_pair).  A range that is not a whole number of tiles makes it share its
+  // first and / or last tile; the partial sums meet through split_ws.  After that it takes whole tiles
+  // shared_tiles + p, + p + pairs, ...  (shared_tiles = 0: whole tiles only.)
+  // gemm_pair_kernel: a range is never shorter than a tile, so a tile has two parts at most; the pair with its tail
+  // writes the slot of the pair before, which has its head.  gemm_wtmem_kernel: a tile may have up to nine parts; all but
+  // the one with its head write their own slots.
   int shared_tiles, units_per_pair;
-  float* split_ws;            // [pairs][2 CTAs][4 warps][8 chunks][8][32 lanes] x 16 bytes of raw accumulators
-  uint32_t* split_flags;      // [pairs][2 CTAs][4 warps]: = epoch from when that warp's share of the slot is written to when it is read
+  float* split_ws;            // [pair and CTA, or lone CTA][4 warps][8 chunks][8][32 lanes] x 16 bytes of raw accumulators
+  uint32_t* split_flags;      // [pair and CTA, or lone CTA][4 warps][shares of a quarter: 4; gemm_wtmem_kernel 8]: = epoch
+                              // from when that share of the slot is written to when it is read
   uint32_t epoch;             // differs from call to call (a replayed graph repeats its own)
   long long* trace;           // tuning builds only: [grid][8] cycle counts per role (waiting / working)
   int skip_transform;         // tuning builds only: leave the operand tiles unwritten (timing of the rest)
