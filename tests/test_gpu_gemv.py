@@ -372,25 +372,34 @@ def test_one_token_int4_digit_route(mld, oracle, K, N, block, outliers):
 
 
 @pytest.mark.parametrize("use_zp", [False, True])
-@pytest.mark.parametrize("K,N", [(4096, 9600), (2056, 32000), (1032, 40968), (2048, 1024), (9088, 9480), (640, 65544)])
-def test_one_token_int8_loses_nothing_beside_outliers(mld, oracle, K, N, use_zp):
+@pytest.mark.parametrize("K,N,scales", [(4096, 9600, 0), (2056, 32000, 0), (1032, 40968, 0), (2048, 1024, 0), (9088, 9480, 0),
+                                        (640, 65544, 0), (2048, 32000, 32), (4096, 9600, 256), (2080, 19000, None)])
+def test_one_token_int8_loses_nothing_beside_outliers(mld, oracle, K, N, scales, use_zp):
     """One input in 32 is 300 and meets weights of zero, so only its 31 neighbours make the output: what a unit's scale
     costs them is the error.  The fp16 form and the 32-bit digits (wide matrices) leave the rounding of the output, 2^-11
-    of the largest, and fp32 sums: 6e-4."""
+    of the largest, and fp32 sums: 6e-4.  scales: inputs to a scale, 0 = per channel, None = one for all."""
+    if scales is None and use_zp:
+        pytest.skip("served by the general kernel")
     g = torch.Generator(device="cuda").manual_seed(K + N)
+    G = K // scales if scales else 1
     q = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda", generator=g)
-    scale = (torch.rand((N, 1), device="cuda", generator=g) + 0.5) / 4096
-    zp = torch.randint(-100, 100, (N, 1), device="cuda", generator=g).float()
-    q[:, 5::32] = zp.to(torch.int8) if use_zp else 0
+    scale = (torch.rand((N, G), device="cuda", generator=g) + 0.5) / 4096
+    if scales is None:
+        scale[:] = 2.0 ** -12
+    zp = torch.randint(-100, 100, (N, G), device="cuda", generator=g).float() * use_zp
+    groups = torch.arange(K, device="cuda") // (K // G)
+    q[:, 5::32] = zp[:, groups[5::32]].to(torch.int8)
     x = torch.randn(K, device="cuda", generator=g)
     x[5::32] = 300.0
     x = x.half()
     packed, _ = mld.pack_weights(q, (N, 1, 1, K), 8)
-    w = q.double() - (zp.double() if use_zp else 0.0)
-    want = (w @ x.double()) * scale.half().double()[:, 0]
+    sums = ((q.double().view(N, G, -1) - zp.double()[..., None]) * x.double().view(G, -1)).sum(-1)
+    want = (sums * scale.half().double()).sum(1)
+    mode = mld.SCALE_SCALAR if scales is None else mld.SCALE_BLOCK if scales else mld.SCALE_PER_CHANNEL
 
     def run(x, exact_operands=False):
-        plan = mld.FullyConnectedPlan(N, K, 8, has_zero_point=use_zp, exact_operands=exact_operands)
+        plan = mld.FullyConnectedPlan(N, K, 8, scale_mode=mode, groups=G, scalar_scale=2.0 ** -12, has_zero_point=use_zp,
+                                      exact_operands=exact_operands)
         y = torch.full((N,), float("nan"), dtype=torch.float16, device="cuda")
         plan.run(x, packed, mld.pack_scales(scale, True), y, 1, zero_point=mld.pack_scales(zp, True) if use_zp else None)
         torch.cuda.synchronize()
