@@ -281,10 +281,10 @@ typedef struct mld_fc_desc {
                                 0: 4-bit weights without zero points and one token
                                 multiply the nibbles by the activations as 16-bit
                                 fixed point (one power-of-two scale per 32 inputs) in
-                                integer MMAs; the other cases feed the raw nibbles /
-                                bytes as fp16 subnormals, or (8-bit weights, one
-                                token) multiply by 32-bit fixed point (same results
-                                up to fp32 summation order).  An infinity or NaN among
+                                integer MMAs; the other decode calls feed the raw
+                                nibbles / bytes as fp16 subnormals, or (8-bit weights,
+                                one token) multiply by 32-bit fixed point (same
+                                results up to fp32 summation order).  An infinity or NaN among
                                 a token's activations makes its outputs NaN */
   int32_t no_overlap;        /* 1: do not let consecutive launches overlap
                                 (programmatic dependent launch off) */

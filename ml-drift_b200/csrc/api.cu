@@ -435,7 +435,7 @@ static StripGeometry strip_geometry_of(const mld_fc_plan* p, int tokens) {
 }
 
 static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, const void* weights, const void* scale,
-                      const void* zp, const void* bias, void* dst, int tokens, bool wait_first, cudaStream_t stream,
+                      const void* zp, const void* bias, void* dst, int tokens, bool wait_first, bool exact, cudaStream_t stream,
                       const PeerScatter* scatter, const PeerWait* wait) {
   const mld_fc_desc& d = p->d;
   const int N4 = align_n(d.n, 4), SS = div_up(d.k, 4), DS = N4 / 4;
@@ -521,7 +521,7 @@ static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, 
   for (int tok0 = 0; tok0 < tokens; tok0 += gm.launch_tokens) {
     a.tok0 = tok0;
     a.M = tokens - tok0 < gm.launch_tokens ? tokens - tok0 : gm.launch_tokens;
-    const int rc = launch_fc_strip(d.weight_bits, p->subnormal, tw, ts, zp != nullptr ? &tz : nullptr, a, gm, stream);
+    const int rc = launch_fc_strip(d.weight_bits, p->subnormal && !exact, tw, ts, zp != nullptr ? &tz : nullptr, a, gm, stream);
     if (rc != MLD_OK) return rc;
   }
   return MLD_OK;
@@ -662,22 +662,23 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
                        (reinterpret_cast<uintptr_t>(zp) & 15) == 0;
   const bool layout_ok = d.src_layout == MLD_LAYOUT_SLICED || tokens == 1;
   const bool streams = plan->stream_ok && aligned && layout_ok && (!d.has_zero_point || zp != nullptr);
-  // The streaming kernel beyond the decode rule's tokens.  Up to 16 it takes less time than the GEMM on most matrices (us
-  // in a graph, streaming / GEMM, 9 and 16 tokens; 15 matrices of 512..14336 inputs and 1024..28672 outputs were measured
-  // for each of INT4 block 32, INT4 and INT8 per channel.  INT4 block 32: 4096 -> 4096 13.7 / 17.4, 15.0 / 17.6;
-  // 4096 -> 14336 27.5 / 33.9, 28.9 / 34.0; 8192 -> 28672 82 / 105, 83 / 105.  INT8: 2048 -> 2048 8.0 / 12.3, 8.4 / 12.3;
-  // 8192 -> 8192 33.1 / 36.5, 34.1 / 36.5) and is even or up to a tenth slower where strips leave their boxes half empty
-  // (4096 -> 11008 INT4 27.0 / 28.6, 28.2 / 28.6, INT8 29.1 / 28.1, 29.6 / 28.1; 4096 -> 1024 INT4 13.1 / 12.6, 13.8 /
-  // 12.5).  At 24 tokens it loses (4096 -> 11008: 47 / 29).  With zero points the alternative is the general kernel (2048
-  // -> 4096, 12 tokens: 48 against 10.4 us), so there it takes as many tokens as two launches hold.
+  // The streaming kernel beyond the decode rule's tokens.  Up to 16, with exact operands (the GEMM multiplies dequantised
+  // weights: inputs that meet zero weights must cost nothing here either), it takes less time than the GEMM where its boxes
+  // are filled or the inputs are few.  us in a graph, streaming / GEMM, 9 and 16 tokens (30 matrices measured for each of
+  // INT4 block 32, INT4 and INT8 per channel): INT4 block 32, 4096 -> 4096 13.6 / 17.5, 14.9 / 17.6; 4096 -> 14336
+  // 29.4 / 33.8, 30.9 / 34.0; 2048 -> 11008 17.5 / 19.7, 18.6 / 19.6; INT8 2048 -> 2048 7.8 / 12.3, 7.9 / 12.3; and on the
+  // other side of the line, with boxes filled to 58 and 65 per cent, 8192 -> 11008 52.5 / 46.2, 53.7 / 46.6; 4096 -> 11008
+  // 29.0 / 28.6, 30.2 / 28.7; 8192 -> 12288 53.6 / 51.4, 54.5 / 51.4.  At 24 tokens it loses (4096 -> 11008: 47 / 29).
+  // With zero points the alternative is the general kernel (2048 -> 4096, 12 tokens: 48 against 10.4 us), so there it takes
+  // as many tokens as two launches hold.
   const bool few = d.force_path == 0 && d.prefill_act_quant == 0 && d.prefill_route == MLD_PREFILL_ROUTE_AUTO &&
-                   d.cache_prepared_weights == 0 && outs == nullptr && tokens <= 16 &&
+                   d.cache_prepared_weights == 0 && outs == nullptr && tokens <= 16 && plan->pdl && plan->subnormal &&
                    (reinterpret_cast<uintptr_t>(b) & 7) == 0;  // (the GEMM refuses such a bias)
-  if (streams && path == 2 && (d.has_zero_point ? tokens <= 2 * kStripTokens : few && plan->pdl && plan->subnormal)) {
+  if (streams && path == 2 && (d.has_zero_point ? tokens <= 2 * kStripTokens : few)) {
     const StripGeometry gm = strip_geometry_of(plan, tokens);
-    if (gm.stages >= 2) {
+    if (gm.stages >= 2 && (d.has_zero_point || d.k <= 2048 || gm.fill >= 75)) {
       plan->last_route = MLD_ROUTE_DECODE_STREAMING;
-      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, true, stream, nullptr, nullptr);
+      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, true, !d.has_zero_point, stream, nullptr, nullptr);
     }
   }
   if (path == 2) {
@@ -700,7 +701,8 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
     const StripGeometry gm = strip_geometry_of(plan, tokens);
     if (gm.stages >= 2) {
       plan->last_route = MLD_ROUTE_DECODE_STREAMING;
-      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, d.has_zero_point || tokens > 16, stream, scatter, wait);
+      return run_stream(plan, gm, src, weights, scale, zp, b, dst, tokens, d.has_zero_point || tokens > 16, false, stream,
+                        scatter, wait);
     }
   }
   if (d.epilogue != MLD_EPILOGUE_NONE) {

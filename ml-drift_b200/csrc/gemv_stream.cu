@@ -907,6 +907,9 @@ template <int BITS, int W, bool ZP>
 int launch_strip_w(bool subnormal, bool mone, const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz,
                    const StripArgs& a, const StripGeometry& gm, cudaStream_t stream) {
   if constexpr (W <= 2) {
+    if constexpr (!ZP) {
+      if (gm.ts_shift > 0 && !subnormal) return launch_strip_t<BITS, W, false, false, false, false, true>(tw, ts, tz, a, gm, stream);
+    }
     if (gm.ts_shift > 0) return launch_strip_t<BITS, W, true, false, false, ZP, true>(tw, ts, tz, a, gm, stream);
   }
   if (ZP || subnormal) {
@@ -967,6 +970,8 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
     w = div_up(div_up(gm.units, strips) * gm.gran, 8);
   }
   gm.w = w > w_max ? w_max : w;
+  const int passes = gm.interleave ? div_up(C, strips * gm.w * 8) : div_up(max_width, gm.w * 8);
+  gm.fill = 100 * C / (strips * passes * gm.w * 8);
   gm.rows_per_split = gm.ksplit == 1 ? align_n(SS, kStageRows) : align_n(div_up(SS, 2), kStageRows);
   if (scale_mode == MLD_SCALE_SCALAR) {
     gm.scale_rows = 0;
@@ -1004,7 +1009,6 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
       // and only as long as the ring keeps three stages beside them.  us in a graph, fp16 form / digits: 151936 x 2048 55.8 /
       // 49.1, 65536 x 2048 28.1 / 24.8, 12288 x 4096 14.8 / 13.8, 12288 x 8192 27.7 / 25.4; below the first line 12288 x 1024
       // 6.0 / 6.4, 32000 x 640 7.5 / 8.1, 8192 x 4096 9.4 / 9.9; below the second 16384 x 11008 36.6 / 42.9.
-      const int passes = gm.interleave ? div_up(C, strips * gm.w * 8) : div_up(max_width, gm.w * 8);
       const bool pays = strips > sms && passes * (gm.rows_per_split / kStageRows) >= 16;
       gm.xdig_bytes = pays && (budget - fixed - xdig) / gm.stage_bytes >= 3 ? xdig : 0;
     }

@@ -116,6 +116,7 @@ struct StripGeometry {
   int scale_stage_bytes, zp_off, stage_bytes, stages, red_m, peer_m, stage_rows;
   int ts_shift, launch_tokens;
   int interleave;  // a strip's passes lie a grid's width apart instead of side by side
+  int fill;        // per cent of the columns of all boxes that are columns of the matrix
   int xdig_bytes;  // shared memory kept for the digitised activation vector; 0: the fp16 form
   size_t smem_bytes;
 };

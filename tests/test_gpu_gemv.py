@@ -414,6 +414,29 @@ def test_one_token_int8_loses_nothing_beside_outliers(mld, oracle, K, N, scales,
     assert not torch.isfinite(run(x)).any()
 
 
+@pytest.mark.parametrize("bits,K,N,M,streams", [(4, 4096, 4096, 12, True), (4, 2048, 11008, 9, True), (4, 4096, 11008, 16, False),
+                                                (8, 4096, 2048, 16, True), (8, 1032, 520, 10, True), (8, 4096, 11008, 9, False)])
+def test_few_tokens_in_place_of_the_gemm(mld, bits, K, N, M, streams):
+    """9 to 16 tokens: one input in 32 is 300 and meets zero weights, which costs the GEMM's dequantised weights nothing;
+    the exact operands of the streaming kernel leave the rounding of the output, 2^-11 of the largest, and fp32 sums."""
+    g = torch.Generator(device="cuda").manual_seed(K + N + M)
+    q = torch.randint(-7, 8, (N, K), dtype=torch.int8, device="cuda", generator=g)
+    q[:, 5::32] = 0
+    scale = (torch.rand((N, 1), device="cuda", generator=g) + 0.5) / 256
+    x = torch.randn(M, K, device="cuda", generator=g)
+    x[:, 5::32] = 300.0
+    x = x.half()
+    plan = mld.FullyConnectedPlan(N, K, bits, max_tokens=M)
+    y = torch.full((N // 4, M, 4), float("nan"), dtype=torch.float16, device="cuda")
+    plan.run(x.view(M, K // 4, 4).permute(1, 0, 2).contiguous(), mld.pack_weights(q, (N, 1, 1, K), bits)[0],
+             mld.pack_scales(scale, True), y, M)
+    torch.cuda.synchronize()
+    assert (plan.last_route() == mld.ROUTE_DECODE_STREAMING) == streams and plan.device_status() == 0
+    want = x.double() @ (q.double() * scale.half().double()).T
+    if streams:
+        assert (y.permute(1, 0, 2).reshape(M, N).double() - want).abs().max() <= 6e-4 * want.abs().max()
+
+
 def test_row_major_single_token(mld, oracle):
     rng = np.random.default_rng(6)
     K, N = 1024, 512
