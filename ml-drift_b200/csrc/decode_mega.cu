@@ -1642,8 +1642,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
     const float* pd = reinterpret_cast<const float*>(a.peers[a.rank] + a.off_pd);
     // One copy of the code for all four projections of every sharding: the loops stay rolled.  (With a copy per
     // projection and sharding the kernel was 512 KB of instructions; every op began with instruction-cache misses, and a
-    // warp's only box took 2200 cycles where a warm one takes 850.  A step of 8 layers of 8 heads: 251 us before, 173
-    // now; of the 7B geometry at 2048 tokens: 1540 and 1397.)
+    // warp's only box took 2200 cycles, 970 now.  A step of 8 layers of 8 heads with host vectors: 247 us before, 170 now;
+    // of the 7B geometry at 2048 tokens: 1510 and 1394.)
 #pragma unroll 1
     for (int l = 0; l < a.n_layers; ++l) {
       const MegaLayer* ly = a.layers + l;

@@ -126,7 +126,7 @@ struct WtArgs {
 // tokens: no transformed stage has to be announced to another SM (a remote arrival takes about 800 cycles, which bounds a
 // pair's rate of stages), at the price of every CTA fetching all of the tile's tokens.  Bound by the MMAs: a stage's four
 // take about 740 cycles whatever the number of tokens, on one accumulator or several, from one issuing thread or two.
-// 77 tokens, 4096 x 11008 INT4: 41.1 us a call with pairs and whole tiles, 32.3 with lone CTAs and tiles cut along K.
+// 77 tokens, 4096 x 11008 INT4: 41.1 us a call with pairs and whole tiles, 31.9 with lone CTAs and tiles cut along K.
 template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kPairThreads, 1)
     gemm_wtmem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, WtArgs wa) {

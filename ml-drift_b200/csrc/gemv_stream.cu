@@ -200,7 +200,8 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // INTERLEAVE: the passes of all strips lie side by side (StripGeometry::interleave).  A form of its own, because the steps
 // and box counts that only it has, worked out at run time, cost every other launch 0.3 to 0.8 us (14208 x 2432 INT4, one
 // token 13.6 against 12.9; 4096 x 11008 10.9 against 10.2).  Several tokens through strips of two boxes take this form always:
-// there it is the faster one (4096 x 11008, 5 tokens: 15.0 against 15.4).
+// they have nothing to interleave, but the compiler's schedule of it is the faster one (4096 x 11008, 5 tokens: 15.0 against
+// 15.4).
 template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE>
 __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     fc_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
@@ -951,8 +952,8 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
   int strips = sms / gm.ksplit;
   if (gm.ksplit == 1 && w_max <= 2 && C > 8 * w_max * sms) {
     // More columns than one pass of one CTA per SM: two CTAs share each SM, so that one streams while the other is in a
-    // pass's epilogue (151936 x 2048 INT8, one token: 17 passes of a lone CTA 85.8 us, 9 of two 69.7; with the passes of
-    // all strips side by side 64.0, with the integer digits 52.0, against 47.6 for the bytes at the copy rate).
+    // pass's epilogue (151936 x 2048 INT8, one token, fp16 form: 17 passes of a lone CTA 85.8 us, 9 of two 69.7; with the
+    // passes of all strips side by side 64.0, against 47.6 for the bytes at the copy rate).
     strips = 2 * sms;
     gm.interleave = C > 8 * w_max * strips ? 1 : 0;
   }
