@@ -334,9 +334,11 @@ struct AttnSplit {
   __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
     P = G >= heads ? G / heads : 0;
     if (P > kMaxParts) P = kMaxParts;
-    // A short context has no use for all of them (8 heads, 100 tokens): one CTA's warps take up to kCW tiles side by side, and merging parts
-    // costs two trips through L2 (publishing and reading the partials); beyond, six tiles to a part.
-    if (P > 1) P = nt <= kCW ? 1 : (nt / 6 < P ? nt / 6 : P);
+    // A short context has no use for parts: one CTA's warps take up to kCW tiles side by side, and merging parts costs two
+    // trips through L2 (publishing and reading the partials).  us a step of 8 (32 heads: 4) layers, all parts / one: 10
+    // tiles 4 heads 169.6 / 159.4, 8 heads 165.1 / 151.8, 16 heads 197.3 / 187.2, 32 heads 157.0 / 152.7; 13 tiles 169.8 /
+    // 178.8, 165.1 / 167.0, 197.6 / 202.9, 157.2 / 158.2.
+    if (nt <= kCW && P > 1) P = 1;
   }
   __device__ __forceinline__ void range(int cta, int& i0, int& i1) const {
     if (P > 0) {
