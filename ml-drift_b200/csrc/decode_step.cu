@@ -11,6 +11,7 @@
 // full-width consumer (after attention, o_proj, SiLU*mul and down_proj).
 #include <cuda_fp16.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -95,8 +96,8 @@ __device__ __forceinline__ void st_cta0_f32(const float* local, float v) {
 // (256 bytes) and folds them into its running max / sum / output with one rescale.
 // A cluster of up to 16 CTAs shares a head and cuts its tokens into even parts; the parts' results meet in the shared
 // memory of the cluster's first CTA, so no scratch in global memory and no second kernel are needed, and calls on
-// several streams share nothing.  32 heads x 8191 tokens, launch after launch: 32.0 us (48.0 with K, then V a token at a
-// time and a launch of its own for the merge).
+// several streams share nothing.  32 heads x 8191 tokens, launch after launch: 23.4 us, 0.88 of the copy rate (32.0 with
+// clusters that did not all fit at once; 48.0 with K, then V a token at a time and a launch of its own for the merge).
 constexpr int kAttnAhead = 4;
 constexpr int kMaxAttnParts = 16;
 template <int WARPS>
@@ -464,47 +465,75 @@ int attn_splits(int heads, int sms) {
   return splits;
 }
 
+// Fills in the launch of attn_decode_kernel<WARPS> with `parts` CTAs to a head; attrs has room for two.
 template <int WARPS>
-int launch_attn_decode_t(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
-                         int parts, cudaStream_t stream) {
-  auto kern = attn_decode_kernel<WARPS>;
+int attn_config(int heads, int parts, cudaStream_t stream, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attrs) {
   static bool configured[kMaxDevices];
   int dev;
   if (needs_configure(configured, &dev)) {
-    MLD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    MLD_CUDA_CHECK(cudaFuncSetAttribute(attn_decode_kernel<WARPS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (dev >= 0) configured[dev] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(heads) * parts);
-  cfg.blockDim = dim3(WARPS * 32);
-  cfg.stream = stream;
-  cudaLaunchAttribute attrs[2];
+  *cfg = {};
+  cfg->gridDim = dim3(static_cast<unsigned>(heads) * parts);
+  cfg->blockDim = dim3(WARPS * 32);
+  cfg->stream = stream;
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[0].val.programmaticStreamSerializationAllowed = 1;
   attrs[1].id = cudaLaunchAttributeClusterDimension;
   attrs[1].val.clusterDim.x = parts;
   attrs[1].val.clusterDim.y = 1;
   attrs[1].val.clusterDim.z = 1;
-  cfg.attrs = attrs;
-  cfg.numAttrs = parts > 1 ? 2 : 1;
-  MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, q, kcache, vcache, out, heads, n_tokens, parts));
+  cfg->attrs = attrs;
+  cfg->numAttrs = parts > 1 ? 2 : 1;
+  return MLD_OK;
+}
+
+// How many heads the device holds at once with `parts` (two or more) CTAs each.  A cluster lies within one GPC and GPCs
+// differ in size, so this is asked of the runtime, once per device and cluster size.
+template <int WARPS>
+int attn_resident_heads(int parts) {
+  static std::atomic<int> known[kMaxDevices][kMaxAttnParts + 1];  // the answer + 1; 0: not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  int n = known[dev][parts].load(std::memory_order_relaxed) - 1;
+  if (n >= 0) return n;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attrs[2];
+  if (attn_config<WARPS>(1, parts, nullptr, &cfg, attrs) != MLD_OK ||
+      cudaOccupancyMaxActiveClusters(&n, attn_decode_kernel<WARPS>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  known[dev][parts].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+template <int WARPS>
+int launch_attn_decode_t(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
+                         int max_parts, cudaStream_t stream) {
+  int parts = div_up(n_tokens, WARPS * 4 * kAttnAhead);  // no more than each has tokens for one round of its warps
+  if (parts > max_parts) parts = max_parts;
+  while (parts > 1 && attn_resident_heads<WARPS>(parts) < heads) --parts;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attrs[2];
+  const int rc = attn_config<WARPS>(heads, parts, stream, &cfg, attrs);
+  if (rc != MLD_OK) return rc;
+  MLD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<WARPS>, q, kcache, vcache, out, heads, n_tokens, parts));
   count_launch();
   return MLD_OK;
 }
 
-// CTAs that share a head: all of the launch resident at once with room for whole clusters in every GPC (3.5 CTAs of
-// four warps per SM of the four that fit; 16 heads and fewer take CTAs of eight warps, since 16 parts of four would
-// leave SMs short of loads in flight), and no more parts than each has tokens for one round of its warps.
+// CTAs that share a head: as many as let the whole launch be resident at once, because a head that has to wait for another
+// one's cluster costs a second wave.  us in a graph, K and V from HBM, eight warps: 32 heads of 8191 tokens in 7 / 8 / 10 /
+// 16 parts 24.6 / 23.3 / 32.9 / 32.2, 40 heads in 6 / 7 28.2 / 40.4, 16 heads in 8 / 12 / 16 17.6 / 16.0 / 20.1, 12 heads
+// 15.4 / 14.9 / 12.8.  CTAs of eight warps beat those of four with long caches (64 heads 41.3 / 42.2, 32 heads 23.3 / 31.9);
+// up to 512 tokens, eight rounds of four warps, the smaller CTAs start and merge sooner (16 heads: 64 tokens 2.6 / 3.3, 200
+// tokens 3.6 / 3.9, 500 tokens 4.7 / 4.7).
 int launch_attn_decode(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
-                       int sms, cudaStream_t stream) {
-  const int warps = heads <= 16 ? 8 : 4;
-  int parts = 7 * sms * 2 / warps / heads;
-  const int rounds = div_up(n_tokens, warps * 4 * kAttnAhead);
-  if (parts > rounds) parts = rounds;
-  if (parts > kMaxAttnParts) parts = kMaxAttnParts;
-  if (parts < 1) parts = 1;
-  if (warps == 8) return launch_attn_decode_t<8>(q, kcache, vcache, out, heads, n_tokens, parts, stream);
-  return launch_attn_decode_t<4>(q, kcache, vcache, out, heads, n_tokens, parts, stream);
+                       cudaStream_t stream) {
+  if (n_tokens <= 8 * 4 * 4 * kAttnAhead) return launch_attn_decode_t<4>(q, kcache, vcache, out, heads, n_tokens, 8, stream);
+  return launch_attn_decode_t<8>(q, kcache, vcache, out, heads, n_tokens, kMaxAttnParts, stream);
 }
 
 }  // namespace
@@ -610,7 +639,7 @@ static int attn_decode(const void* q, const void* kcache, const void* vcache, vo
   MLD_REQUIRE(device < 64, "device ordinal too large");
   return launch_attn_decode(static_cast<const __half*>(q), static_cast<const __half*>(kcache),
                             static_cast<const __half*>(vcache), static_cast<__half*>(out), heads, n_tokens,
-                            sm_count(device), static_cast<cudaStream_t>(stream));
+                            static_cast<cudaStream_t>(stream));
 }
 
 int mld_attn_decode(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads, int32_t head_dim,

@@ -429,6 +429,13 @@ def test_attention_decode_parts(mld, heads, n_tokens):
     assert (out.double() - ref).abs().max() <= 2.0 ** -10 * ref.abs().max()
 
 
+@pytest.mark.parametrize("heads,n_tokens", [
+    (8, 512), (8, 513), (64, 500), (40, 513),                                     # the last of four warps, the first of eight
+    (12, 4096), (16, 4096), (20, 4097), (30, 2500), (36, 2047), (48, 3000), (200, 600)])  # 16 parts to a head down to one
+def test_attention_decode_resident_parts(mld, heads, n_tokens):
+    test_attention_decode_parts(mld, heads, n_tokens)
+
+
 def test_attention_decode_on_two_streams(mld):
     g = torch.Generator(device="cuda").manual_seed(3)
     cases = []
