@@ -683,6 +683,53 @@ __device__ __forceinline__ uint4 fetch8(const Waiter& w, const Src& s, int i) {
 
 constexpr int kRegChunks = 4;  // chunks of 8 inputs a thread can hold: vectors up to 4 * 8 * 32 * kCW inputs
 
+// This thread's chunks of a tagged vector of d values (chunk r: values 8 (threadIdx.x + 32 kCW r) ..), waited for
+// (bounded; code 22).  All chunks are asked for at once and the missing ones together again, so that the wait ends one
+// trip to L2 after the last word was written, however many chunks a thread has.
+__device__ __forceinline__ void fetch_tagged(const Waiter& w, const uint32_t* tx, uint32_t tag, int d, uint4 (&v)[kRegChunks]) {
+  const uint32_t want = tag * 0x00010001u;  // the tag in both halves of a word
+  uint4 lo[kRegChunks], hi[kRegChunks];
+  unsigned missing = 0;
+#pragma unroll
+  for (int r = 0; r < kRegChunks; ++r) {
+    lo[r] = hi[r] = make_uint4(0u, 0u, 0u, 0u);
+    if ((static_cast<int>(threadIdx.x) + r * kCW * 32) * 8 < d) missing |= 1u << r;
+  }
+  const auto ask = [&]() {
+#pragma unroll
+    for (int r = 0; r < kRegChunks; ++r) {
+      if (missing & (1u << r)) {
+        const uint32_t* p = tx + (threadIdx.x + r * kCW * 32) * 8;
+        lo[r] = ld_word4(p, w.sys);
+        hi[r] = ld_word4(p + 4, w.sys);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRegChunks; ++r)
+      if (__byte_perm(lo[r].x, lo[r].y, 0x7632) == want && __byte_perm(lo[r].z, lo[r].w, 0x7632) == want &&
+          __byte_perm(hi[r].x, hi[r].y, 0x7632) == want && __byte_perm(hi[r].z, hi[r].w, 0x7632) == want)
+        missing &= ~(1u << r);
+  };
+  ask();
+  if (missing != 0 && !*w.s_fail) {
+    const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
+    for (;;) {
+      ask();
+      if (missing == 0 || *w.s_fail) break;
+      if (globaltimer_ns() - t0 > w.limit) {
+        *w.s_fail = 1;
+        atomicExch(w.error, 22);
+        break;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRegChunks; ++r)
+    v[r] = make_uint4(__byte_perm(lo[r].x, lo[r].y, 0x5410), __byte_perm(lo[r].z, lo[r].w, 0x5410),
+                      __byte_perm(hi[r].x, hi[r].y, 0x5410), __byte_perm(hi[r].z, hi[r].w, 0x5410));
+}
+
 // Block-wide sum of one float per thread over the consumer warps.
 __device__ __forceinline__ float consumer_sum(Ctx& c, float v) {
 #pragma unroll
@@ -753,11 +800,15 @@ __device__ __forceinline__ void load_x(Ctx& c, const Src& src, const __half* gam
     gv[r] = make_uint4(0u, 0u, 0u, 0u);
     if (gamma != nullptr && ci * 8 < d) gv[r] = __ldg(reinterpret_cast<const uint4*>(gamma + ci * 8));
   }
+  if (src.tx != nullptr) {
+    fetch_tagged(c.w, src.tx, src.tag, d, v);
+  } else {
 #pragma unroll
-  for (int r = 0; r < kRegChunks; ++r) {
-    const int ci = threadIdx.x + r * kCW * 32;
-    v[r] = make_uint4(0u, 0u, 0u, 0u);
-    if (ci * 8 < d) v[r] = fetch8(c.w, src, ci * 8);
+    for (int r = 0; r < kRegChunks; ++r) {
+      const int ci = threadIdx.x + r * kCW * 32;
+      v[r] = make_uint4(0u, 0u, 0u, 0u);
+      if (ci * 8 < d) v[r] = fetch8(c.w, src, ci * 8);
+    }
   }
   if (gamma != nullptr) {
     float ss = 0.0f;
