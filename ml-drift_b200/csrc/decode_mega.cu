@@ -75,7 +75,7 @@ constexpr int kAttnSlots = 2;                // head runs likewise
 constexpr int kAttDump = kHeadDim + 4;       // 128 outputs, then max and sum (padded: rows stay 16-byte aligned)
 constexpr int kDumpFloats = 2 * kCW * kStripN > kAttnSlots * kCW * kAttDump ? 2 * kCW * kStripN : kAttnSlots * kCW * kAttDump;
 constexpr int kWarpScratch = 3 * kHeadDim;   // attention: rotated q, new k, new v (floats) per warp
-constexpr int kMaxParts = 8;                 // CTAs that share a head at most: the merging part reads all partials in one round
+constexpr int kMaxParts = 8;                 // CTAs that share a head at most: the merging part reads the others in two rounds
 constexpr int kTraceSlots = 12;              // per (CTA, op): 4 timestamps, warp 0's clocks, all-warps-done, last load issued
 enum { kQkv = 0, kAttn = 1, kO = 2, kGu = 3, kDown = 4, kOpsPerLayer = 5 };
 
@@ -118,9 +118,8 @@ struct MegaArgs {
   int tagged;
   uint32_t *tq, *tattn, *th, *tact, *txa, *txb;
   unsigned long long wait_limit_ns;  // bound on every wait of this launch
-  float* att_part;     // [grid][kAttSlots][kAttDump]
+  float* att_part;     // [grid][kAttSlots][kAttDump], or (parts of a head on several CTAs) a record of words per CTA
   int* att_tickets;    // [heads]
-  unsigned* att_flags; // [heads][grid / heads]: epoch of the attention whose partial the part has published
   unsigned* bar;       // 64-bit arrival counter of the grid barrier (8-byte aligned)
   int* error;
   unsigned long long* trace;  // optional [grid][ops][kTraceSlots]
@@ -202,6 +201,13 @@ __device__ __forceinline__ uint4 ld_word4(const uint32_t* p, bool sys) {
   else
     asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
+}
+// Two 64-bit words that carry their own validity (16-byte aligned; each word is read and written whole).
+__device__ __forceinline__ void st_words2(unsigned long long* p, unsigned long long x, unsigned long long y) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
+}
+__device__ __forceinline__ void ld_words2(const unsigned long long* p, unsigned long long& x, unsigned long long& y) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
 }
 // One tagged value, waited for (bounded; code 22).
 __device__ __forceinline__ __half ld_tagged(const Waiter& w, const uint32_t* p, uint32_t tag) {
@@ -1411,71 +1417,64 @@ __device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
       split.contributors(head, first, lastc);
       bool write = true;
       if (split.P > 1 && lastc > first) {
-        // The head's parts publish their partial and a flag; the part with the last tile (which also has
-        // the new token, so the most to do) waits for them and merges: parts in order, its own last.
+        // The parts publish their partial as 64-bit words of a value and the op's epoch, so that a word says itself whether
+        // it is there: no flag, and no fence that a flag would wait for.  The part with the last tile (which also has the
+        // new token, so the most to do) reads the others' words until they are all there and merges: parts in order, its
+        // own last.
         const unsigned epoch = c.epoch_base + static_cast<unsigned>(c.op_index) + 1u;
         const int part = cta - first, pm = lastc - first;  // pm: the part with the head's last tile
-        unsigned* flags = a.att_flags + (size_t)head * split.P;
+        const auto record = [&](int who) {
+          return reinterpret_cast<unsigned long long*>(a.att_part + (size_t)who * kAttSlots * kAttDump);
+        };
         if (part < pm) {
-          float* pp = a.att_part + (size_t)cta * kAttSlots * kAttDump;
-          *reinterpret_cast<float4*>(pp + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
-          if (lane == 0) {
-            pp[kHeadDim] = M;
-            pp[kHeadDim + 1] = ls;
-          }
+          unsigned long long* pp = record(cta);
+          const auto word = [&](float v) { return static_cast<unsigned long long>(epoch) << 32 | __float_as_uint(v); };
+          st_words2(pp + 4 * lane, word(o[0]), word(o[1]));
+          st_words2(pp + 4 * lane + 2, word(o[2]), word(o[3]));
+          if (lane == 0) st_words2(pp + kHeadDim, word(M), word(ls));
           if (trs) trs[9] = globaltimer_ns();
-          __syncwarp();  // the release below is cumulative over the other lanes' stores
-          if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + part), "r"(epoch) : "memory");
-          if (trs) trs[10] = globaltimer_ns();
           write = false;
         } else {
           if (trs) trs[9] = globaltimer_ns();
+          float TM = -INFINITY, po[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pl = 0.0f;
+          constexpr int kAtOnce = 4;
 #pragma unroll 1
-          for (int base = 0; base < pm; base += 32) {
-            const int u = base + lane;
-            if (u < pm && !*c.w.s_fail) {
-              const unsigned long long t0 = globaltimer_ns();
+          for (int base = 0; base < pm; base += kAtOnce) {
+            float mc[kAtOnce], lc[kAtOnce];
+            float4 oc[kAtOnce];
+            const unsigned long long t0 = globaltimer_ns();
 #pragma unroll 1
-              for (;;) {
-                unsigned fv;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(fv) : "l"(flags + u) : "memory");
-                if (fv == epoch) break;
-                if (globaltimer_ns() - t0 > c.w.limit || *c.w.s_fail) {
-                  *c.w.s_fail = 1;
-                  atomicCAS(a.error, 0, 21);
-                  break;
+            for (;;) {
+              bool all = true;
+#pragma unroll
+              for (int u = 0; u < kAtOnce; ++u) {
+                mc[u] = -INFINITY;
+                lc[u] = 0.0f;
+                oc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (base + u < pm) {
+                  const unsigned long long* pp = record(first + base + u);
+                  unsigned long long w[6];
+                  ld_words2(pp + 4 * lane, w[0], w[1]);
+                  ld_words2(pp + 4 * lane + 2, w[2], w[3]);
+                  ld_words2(pp + kHeadDim, w[4], w[5]);
+#pragma unroll
+                  for (int i = 0; i < 6; ++i) all = all && static_cast<unsigned>(w[i] >> 32) == epoch;
+                  const auto value = [](unsigned long long x) { return __uint_as_float(static_cast<unsigned>(x)); };
+                  oc[u] = make_float4(value(w[0]), value(w[1]), value(w[2]), value(w[3]));
+                  mc[u] = value(w[4]);
+                  lc[u] = value(w[5]);
                 }
               }
-            }
-          }
-          __syncwarp();
-          if (trs) trs[10] = globaltimer_ns();
-          float TM = -INFINITY, po[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pl = 0.0f;
-#pragma unroll 1
-          for (int base = 0; base < pm; base += 8) {
-            int myoff = -1;
-            {
-              const int u = base + (lane & 7);
-              if (u < pm) myoff = (first + u) * kAttSlots * kAttDump;
-            }
-            float mc[8], lc[8];
-            float4 oc[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int off = __shfl_sync(0xffffffffu, myoff, u);
-              mc[u] = -INFINITY;
-              lc[u] = 0.0f;
-              oc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-              if (off >= 0) {
-                const float* pp = a.att_part + off;
-                mc[u] = __ldcg(pp + kHeadDim);
-                lc[u] = __ldcg(pp + kHeadDim + 1);
-                oc[u] = __ldcg(reinterpret_cast<const float4*>(pp + 4 * lane));
+              if (__all_sync(0xffffffffu, all || *c.w.s_fail)) break;
+              if (globaltimer_ns() - t0 > c.w.limit) {
+                *c.w.s_fail = 1;
+                atomicCAS(a.error, 0, 21);
               }
             }
+            if (trs) trs[10] = globaltimer_ns();
             float NM = TM;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) NM = fmaxf(NM, mc[u]);
+            for (int u = 0; u < kAtOnce; ++u) NM = fmaxf(NM, mc[u]);
             const float resc = TM == -INFINITY ? 0.0f : __expf(TM - NM);
             po[0] *= resc;
             po[1] *= resc;
@@ -1483,7 +1482,7 @@ __device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
             po[3] *= resc;
             pl *= resc;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < kAtOnce; ++u) {
               const float wc = mc[u] == -INFINITY ? 0.0f : __expf(mc[u] - NM);
               po[0] = fmaf(wc, oc[u].x, po[0]);
               po[1] = fmaf(wc, oc[u].y, po[1]);
@@ -1897,7 +1896,7 @@ struct MegaDecoder {
   uint8_t* scratch;
   int tagged;
   uint32_t *tq, *tattn, *th, *tact, *txa, *txb;  // tagged-word vectors (tq in scratch, the others in xchg)
-  size_t off_tagged, tagged_bytes, tq_bytes, flags_bytes;
+  size_t off_tagged, tagged_bytes, tq_bytes, part_bytes;
   uint8_t* xchg;              // exchange block (vectors every rank needs + the cross-rank barrier counter)
   uint8_t* peers[8];          // every rank's exchange block as mapped here (own entry = xchg)
   size_t off_attn, off_h, off_act, off_xa, off_xb, off_xbar, off_ph, off_pd;
@@ -1909,7 +1908,6 @@ struct MegaDecoder {
   __half *qkv, *attn, *h, *act, *xa, *xb;
   float* att_part;
   int *att_tickets, *error;
-  unsigned* att_flags;
   unsigned* bar;
   unsigned long long* trace;
 };
@@ -2008,7 +2006,7 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
   };
   const int dl = m->d_local, fl = m->ffn_local;
   const size_t o_qkv = take((size_t)3 * dl * 2), o_ap = take((size_t)m->grid * kAttSlots * kAttDump * 4),
-               o_at = take((size_t)m->heads_local * 4), o_af = take((size_t)(m->grid + m->heads_local) * 4),
+               o_at = take((size_t)m->heads_local * 4),
                o_bar = take(8), o_err = take(4);
   // the op-to-op vectors as tagged words unless the descriptor asks for grid barriers (the split of o and down
   // by input columns exchanges fp32 partial sums and keeps the barriers)
@@ -2060,10 +2058,9 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
   m->tact = reinterpret_cast<uint32_t*>(m->xchg + o_tact);
   m->txa = reinterpret_cast<uint32_t*>(m->xchg + o_txa);
   m->txb = reinterpret_cast<uint32_t*>(m->xchg + o_txb);
-  m->flags_bytes = (size_t)(m->grid + m->heads_local) * 4;
+  m->part_bytes = (size_t)m->grid * kAttSlots * kAttDump * 4;
   m->att_part = reinterpret_cast<float*>(m->scratch + o_ap);
   m->att_tickets = reinterpret_cast<int*>(m->scratch + o_at);
-  m->att_flags = reinterpret_cast<unsigned*>(m->scratch + o_af);
   m->bar = reinterpret_cast<unsigned*>(m->scratch + o_bar);
   m->error = reinterpret_cast<int*>(m->scratch + o_err);
   m->h_layers.resize(cfg.layers);
@@ -2148,7 +2145,7 @@ int mega_grid(const MegaDecoder* m) { return m->grid; }
 
 const int* mega_error_word(const MegaDecoder* m) { return m->error; }
 
-// Back to the state after creation: counters zero, no tagged word or flag valid.  (Tags and flag epochs
+// Back to the state after creation: counters zero, no tagged word or record valid.  (Tags and record epochs
 // derive from the launch counter; restarting it is safe only because everything that carries a tag or an
 // epoch is cleared with it.)
 int mega_reset(MegaDecoder* m) {
@@ -2156,7 +2153,7 @@ int mega_reset(MegaDecoder* m) {
   MLD_CUDA_CHECK(cudaMemset(m->bar, 0, 8));
   MLD_CUDA_CHECK(cudaMemset(m->xchg + m->off_xbar, 0, 8));
   MLD_CUDA_CHECK(cudaMemset(m->att_tickets, 0, (size_t)m->heads_local * 4));
-  MLD_CUDA_CHECK(cudaMemset(m->att_flags, 0, m->flags_bytes));
+  MLD_CUDA_CHECK(cudaMemset(m->att_part, 0, m->part_bytes));
   if (m->tagged) {
     MLD_CUDA_CHECK(cudaMemset(m->tq, 0, m->tq_bytes));
     MLD_CUDA_CHECK(cudaMemset(m->xchg + m->off_tagged, 0, m->tagged_bytes));
@@ -2224,7 +2221,6 @@ int mega_step(MegaDecoder* m, const void* x_in, void* x_out, int pos, cudaStream
   a.xb = m->xb;
   a.att_part = m->att_part;
   a.att_tickets = m->att_tickets;
-  a.att_flags = m->att_flags;
   a.bar = m->bar;
   a.error = m->error;
   a.trace = m->trace;
