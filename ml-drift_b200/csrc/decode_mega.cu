@@ -4,7 +4,7 @@
 // projection drains its TMA pipeline, the next one fills it again, and the
 // weights of a projection (8-45 MB) stream for only a few microseconds.  Here
 // one cooperative grid of one CTA per SM runs all layers:
-//   * a producer thread per CTA walks the step's whole list of weight boxes and
+//   * a producer warp per CTA walks the step's whole list of weight boxes and
 //     KV-cache tiles this CTA will need, in order, and keeps a ring of 9 KB
 //     stages (about 170 KB) full.  Nothing it loads depends on the step's
 //     activations, so it runs ahead across op and layer boundaries;
@@ -92,7 +92,6 @@ struct MegaArgs {
   const MegaLayer* layers;
   int n_layers, d_model, heads, ffn, pos;
   int stages;          // ring depth
-  int l2_ahead;        // ops by which the L2 prefetch runs ahead of the ring's loads (0 = none)
   int xs_bytes;        // shared-memory bytes of the input-vector / attention scratch area
   int us_floats;       // entries of the per-32-input sums of the input vector
   float rms_eps, min_ts, max_ts, q_scale;
@@ -376,70 +375,70 @@ struct AttnSplit {
 };
 
 // ------------------------------------------------------------------ producer
-struct Ring {
-  int stage;
-  uint32_t phase;
-  __device__ __forceinline__ void advance(int stages) {
-    if (++stage == stages) {
-      stage = 0;
-      phase ^= 1;
-    }
-  }
-};
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 
-// Asks L2 for this CTA's whole share of an op: HBM then runs an op ahead of the
-// ring, which only has to cover the L2 -> shared memory latency.
-__device__ void prefetch_op_l2(const MegaArgs& a, int l, int kind) {
-  const int cta = blockIdx.x, G = gridDim.x;
-  const MegaLayer* ly = a.layers + l;
-  if (kind == kAttn) {
-    const int nt = a.pos / kTile + 1;
-    const AttnSplit split(a.heads, nt, G);
-    int i0, i1;
-    split.range(cta, i0, i1);
+// The whole producer warp: a lane per ring stage, up to `width` of them at a time, each of which waits for its own stage and
+// asks for its own box as soon as that is free.  (One lane going through the stages, a few hundred cycles each, refilled an
+// emptied ring of 21 too slowly: 7B step 1256 us, 1236 with this and the residuals off the boxes' path.)  A pass never laps the ring: the use of a stage before a lane's was
+// asked for in an earlier pass, so its release is what the parity of the lane's wait tells apart.
+// Calls ask(i, stage) for i = 0 .. n - 1; false when a wait ran out.
+template <typename Ask>
+__device__ __forceinline__ bool produce(const MegaArgs& a, uint64_t* empty, const Waiter& w, unsigned& pos, int n, int code,
+                                        const Ask& ask) {
+  const int lane = threadIdx.x & 31, width = a.stages < 32 ? a.stages : 32;
 #pragma unroll 1
-    for (int i = i0; i < i1; ++i) {
-      const int head = i / nt, j = i - head * nt;
-      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(
-                       reinterpret_cast<uint64_t>(&ly->kc)),
-                   "r"(head * kHeadDim), "r"(j * kTile)
-                   : "memory");
-      asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(
-                       reinterpret_cast<uint64_t>(&ly->vc)),
-                   "r"(head * kHeadDim), "r"(j * kTile)
-                   : "memory");
-    }
-  } else {
-    const ProjShape p = proj_shape(a, kind);
-    int i0, i1;
-    proj_range(p, cta, G, i0, i1);
-    const uint8_t* src = ly->w[map_index(kind)] + (size_t)i0 * kStageBytes;
-    size_t bytes = (size_t)(i1 - i0) * kStageBytes;
+  for (int base = 0; base < n; base += width) {
+    const int i = base + lane;
+    bool pending = lane < width && i < n;
+    const unsigned at = pos + i;
+    const int stage = static_cast<int>(at % static_cast<unsigned>(a.stages));
+    const uint32_t parity = (at / static_cast<unsigned>(a.stages) & 1u) ^ 1u;
+    unsigned long long t0 = 0;
 #pragma unroll 1
-    while (bytes > 0) {
-      const uint32_t n = bytes < 18432 ? static_cast<uint32_t>(bytes) : 18432u;
-      bulk_prefetch_l2(src, n);
-      src += n;
-      bytes -= n;
+    for (int polls = 1;; ++polls) {
+      if (pending && mbar_test_wait(&empty[stage], parity)) {
+        ask(i, stage);
+        pending = false;
+      }
+      if (!__any_sync(0xffffffffu, pending)) break;
+      if ((polls & 63) == 0) {
+        // a producer whose wait ran out requests nothing more: stages it cannot know to be free stay
+        // untouched, and no barrier sees an arrival its phase does not expect
+        const unsigned long long now = globaltimer_ns();
+        if (t0 == 0) t0 = now;
+        const bool late = now - t0 > w.limit;
+        if (late && pending && !*w.s_fail) {
+          *w.s_fail = 1;
+          atomicExch(w.error, code);
+        }
+        if (__any_sync(0xffffffffu, late || *w.s_fail)) return false;
+      }
     }
   }
+  pos += n;
+  return true;
 }
 
 __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, uint64_t* empty, const Waiter& w) {
   const int cta = blockIdx.x, G = gridDim.x;
   const uint64_t pol = policy_evict_first();
-  Ring r{0, 0};
+  unsigned pos = 0;  // ring stages asked for so far
   const int nt = a.pos / kTile + 1;
 #pragma unroll 1
   for (int l = 0; l < a.n_layers; ++l) {
     const MegaLayer* ly = a.layers + l;
 #pragma unroll 1
     for (int kind = 0; kind < kOpsPerLayer; ++kind) {
-      if (a.l2_ahead > 0) {
-        // the op `l2_ahead` ops after this one
-        const int o = l * kOpsPerLayer + kind + a.l2_ahead;
-        if (o < a.n_layers * kOpsPerLayer) prefetch_op_l2(a, o / kOpsPerLayer, o % kOpsPerLayer);
-      }
       if (kind == kAttn) {
         const AttnSplit split(a.heads, nt, G);
         int ai0, ai1;
@@ -449,47 +448,35 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
         for (int rr = 0; rr < runs.R; ++rr) {
           int head, lo, hi;
           runs.bounds(rr, head, lo, hi);
-#pragma unroll 1
-          for (int i = lo; i < hi; ++i) {
-            const int j = i - head * nt;
-#pragma unroll 1
-            for (int kv = 0; kv < 2; ++kv) {
-              // a producer whose wait ran out requests nothing more: stages it cannot know to be free stay
-              // untouched, and no barrier sees an arrival its phase does not expect
-              if (!w.wait(&empty[r.stage], r.phase ^ 1, 10)) return;
-              uint8_t* st = ring + (size_t)r.stage * kStageBytes;
-              mbar_arrive_expect_tx(&full[r.stage], kBox);
-              const CUtensorMap* map = kv == 0 ? &ly->kc : &ly->vc;
-              tma_load_2d_hint(st, map, &full[r.stage], head * kHeadDim, j * kTile, pol);
-              tma_load_2d_hint(st + 4096, map, &full[r.stage], head * kHeadDim + 64, j * kTile, pol);
-              r.advance(a.stages);
-            }
-          }
+          const int j0 = lo - head * nt;
+          // an item is a K tile and a V tile
+          if (!produce(a, empty, w, pos, 2 * (hi - lo), 10, [&](int i, int stage) {
+                const CUtensorMap* map = (i & 1) == 0 ? &ly->kc : &ly->vc;
+                uint8_t* st = ring + (size_t)stage * kStageBytes;
+                mbar_arrive_expect_tx(&full[stage], kBox);
+                tma_load_2d_hint(st, map, &full[stage], head * kHeadDim, (j0 + (i >> 1)) * kTile, pol);
+                tma_load_2d_hint(st + 4096, map, &full[stage], head * kHeadDim + 64, (j0 + (i >> 1)) * kTile, pol);
+              }))
+            return;
         }
       } else {
         const ProjShape p = proj_shape(a, kind);
-        const uint8_t* wbase = ly->w[map_index(kind)];
         int pi0, pi1;
         proj_range(p, cta, G, pi0, pi1);
         // boxes are stored strip after strip: the CTA's boxes are one contiguous stream, cut into kCW
         // chunks (one per consumer warp); ring position kCW j + w takes box j of chunk w
+        const uint8_t* boxes = ly->w[map_index(kind)] + (size_t)pi0 * kStageBytes;
         const int B = pi1 - pi0, qn = B / kCW, rn = B % kCW;
-#pragma unroll 1
-        for (int j = 0; j * kCW < B; ++j) {
-          const int nw = B - j * kCW < kCW ? B - j * kCW : kCW;
-#pragma unroll 1
-          for (int cw = 0; cw < nw; ++cw) {
-            const int i = pi0 + cw * qn + (cw < rn ? cw : rn) + j;
-            if (!w.wait(&empty[r.stage], r.phase ^ 1, 11)) return;
-            uint8_t* st = ring + (size_t)r.stage * kStageBytes;
-            mbar_arrive_expect_tx(&full[r.stage], kStageBytes);
-            bulk_load_1d_hint(st, wbase + (size_t)i * kStageBytes, kStageBytes, &full[r.stage], pol);
-            r.advance(a.stages);
-          }
-        }
+        if (!produce(a, empty, w, pos, B, 11, [&](int i, int stage) {
+              const int j = i / kCW, cw = i - j * kCW;
+              mbar_arrive_expect_tx(&full[stage], kStageBytes);
+              bulk_load_1d_hint(ring + (size_t)stage * kStageBytes, boxes + (size_t)(cw * qn + (cw < rn ? cw : rn) + j) * kStageBytes,
+                                kStageBytes, &full[stage], pol);
+            }))
+          return;
       }
       // when this op's last load was issued
-      if (MLD_TRACING(a) && kind != kAttn)
+      if (MLD_TRACING(a) && kind != kAttn && (threadIdx.x & 31) == 0)
         a.trace[((size_t)blockIdx.x * a.n_layers * kOpsPerLayer + l * kOpsPerLayer + kind) * kTraceSlots + 11] = globaltimer_ns();
     }
   }
@@ -1018,13 +1005,13 @@ __device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int ki
     const int s_lo = sl * p.S, s_hi = s_lo + p.S;
     ++sl;  // (a warp's boxes lie side by side: the next round of this loop is the next strip)
     const int b_end = b_stop < s_hi ? b_stop : s_hi;
-    // the strip's residual values are fetched now: whichever warp completes the strip has them at hand
+    // the strip's residual values are asked for now: whichever warp completes the strip has them at hand then (tagged words
+    // are looked at only there, so that nothing waits for them before the boxes)
     __half rv = __float2half_rn(0.0f);
-    if (tresid != nullptr) {
-      if (lane < kStripN) {
-        const uint32_t* rp = tresid + strip * kStripN + lane;
-        rv = tagged_value(c.w, rp, tresid_tag, ld_word(rp, c.w.sys));
-      }
+    uint32_t rw = 0;
+    const uint32_t* const rp = tresid != nullptr ? tresid + strip * kStripN + (lane & (kStripN - 1)) : nullptr;
+    if (rp != nullptr) {
+      rw = ld_word(rp, c.w.sys);
     } else if (resid != nullptr && lane < kStripN) {
       rv = __ldcg(resid + strip * kStripN + lane);
     }
@@ -1062,6 +1049,7 @@ __device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int ki
       // the strip is this warp's alone: rows g and g+8 sit in lanes t == 0
       const float lo = __shfl_sync(0xffffffffu, tot[0], (lane & 7) * 4);
       const float hi = __shfl_sync(0xffffffffu, tot[1], (lane & 7) * 4);
+      if (rp != nullptr) rv = tagged_value(c.w, rp, tresid_tag, rw);
       finish_strip(a, kind, strip, (lane & 8) ? hi : lo, resid != nullptr || tresid != nullptr, rv, out);
       if (tracing) ec += clock64() - e0;
       continue;
@@ -1092,6 +1080,7 @@ __device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int ki
 #pragma unroll 1
       for (int w = w_lo + 1; w <= w_hi; ++w) v += c.dump[w * 2 * kStripN + (lane & 15)];
       if (lane == 0) c.proj_arrived()[w_lo] = 0;  // next used after the op's grid barrier
+      if (rp != nullptr) rv = tagged_value(c.w, rp, tresid_tag, rw);
       finish_strip(a, kind, strip, v, resid != nullptr || tresid != nullptr, rv, out);
     }
     if (tracing) eb += clock64() - e3;
@@ -1638,7 +1627,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
   uint64_t* full = reinterpret_cast<uint64_t*>(rope + kHeadDim / 2);
   uint64_t* empty = full + a.stages;
   int* s_int = reinterpret_cast<int*>(empty + a.stages);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
 
   if (threadIdx.x == 0) {
 #pragma unroll 1
@@ -1676,7 +1665,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_mega_kernel(const __grid_c
   Waiter w{s_int, a.error, a.wait_limit_ns, a.world > 1};
 
   if (warp == kCW) {
-    if (lane == 0) producer_loop(a, ring, full, empty, w);
+    producer_loop(a, ring, full, empty, w);
   } else {
     Ctx c{a, ring, full, empty, xs, reinterpret_cast<int*>(us), rope, dump, s_int, w, 0, 0, 0ull, 0ull, 0u, 0};
     c.bar_target = *reinterpret_cast<const unsigned long long*>(s_int + kSharedInts + 1);
@@ -1888,7 +1877,7 @@ __global__ void __launch_bounds__(256) retile_weights_kernel(const uint8_t* __re
 // ------------------------------------------------------------------ host side
 struct MegaDecoder {
   MegaConfig cfg;
-  int sms, grid, stages, xs_bytes, us_floats, l2_ahead;
+  int sms, grid, stages, xs_bytes, us_floats;
   size_t smem_bytes;
   MegaLayer* d_layers;
   std::vector<MegaLayer> h_layers;
@@ -1970,7 +1959,6 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
     return MLD_UNIMPLEMENTED;
   }
   m->stages = stages;
-  m->l2_ahead = 0;  // measured: asking L2 for the next op ahead of the ring's loads slows the step down
   m->smem_bytes = (size_t)fixed + (size_t)stages * (kStageBytes + 16);
   cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(m->smem_bytes));
@@ -2196,7 +2184,6 @@ int mega_step(MegaDecoder* m, const void* x_in, void* x_out, int pos, cudaStream
   a.off_xbar = m->off_xbar;
   a.pos = pos;
   a.stages = m->stages;
-  a.l2_ahead = m->l2_ahead;
   a.xs_bytes = m->xs_bytes;
   a.us_floats = m->us_floats;
   a.rms_eps = c.rms_eps;
