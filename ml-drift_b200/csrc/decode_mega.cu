@@ -608,14 +608,13 @@ __device__ __forceinline__ void digitise_chunk(Ctx& c, int ci, const uint4& v) {
   sum = __dp4a(static_cast<int>(low[1]), 0x01010101, sum);
   sum += __shfl_xor_sync(0xffffffffu, sum, 1);
   sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  // chunk q of the unit holds inputs 8q..8q+7: half q >> 1, lanes t = 2 (q & 1) and 2 (q & 1) + 1
+  // chunk q of the unit holds inputs 8q..8q+7, which MMA q of the unit's set takes: [digit][first or second four][q]
   const int unit = ci >> 2, q = ci & 3;
   uint32_t* ub = reinterpret_cast<uint32_t*>(c.xs + unit * 32);
-  const int w0 = 2 * (2 * (q & 1)) + (q >> 1);  // word index of (t, half): 2 t + half
-  ub[w0] = hiw[0];
-  ub[w0 + 2] = hiw[1];
-  ub[8 + w0] = low[0];
-  ub[8 + w0 + 2] = low[1];
+  ub[q] = hiw[0];
+  ub[4 + q] = hiw[1];
+  ub[8 + q] = low[0];
+  ub[12 + q] = low[1];
   if (q == 0) {
     // |8 sum| <= 8 * 32 * 32512 < 2^23: the offset term and the scale's exponent share one word
     const int m = unit & 31;
@@ -631,7 +630,8 @@ __device__ __forceinline__ void digitise_chunk(Ctx& c, int ci, const uint4& v) {
 // channel costs its 31 neighbours nothing worth naming and the rest of the
 // vector nothing at all.  The unit (64 bytes either way) is rewritten as
 // [hi: 32 bytes][lo: 32 bytes], each in the order the B fragments take them
-// (8 bytes per lane t: inputs 4t..4t+3 and 16+4t..16+4t+3).
+// (inputs 8q..8q+3 for q = 0..3, then 8q+4..8q+7: a lane's words for the four
+// MMAs of a set lie side by side).
 // isum[box][t][set] = the scale's exponent bits | 23 bits of 8 * (sum of the
 // unit's integers), the nibble offset's share.
 __device__ void digitise_x(Ctx& c, int d) {
@@ -826,53 +826,82 @@ __device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], ui
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// One box (16 outputs x 1024 inputs) by one warp.  Lane = 4g + t.  A unit of 32
-// inputs (one scale per output) is exactly one integer MMA m16n8k32.  A 32-bit
+__device__ __forceinline__ void mma_u8s8_first(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+}
+// Four words of shared memory for the lanes with on != 0; the others keep what they have.
+template <int OFFSET>
+__device__ __forceinline__ void lds_if(uint32_t (&v)[4], uint32_t addr, uint32_t on) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+%6];\n\t}"
+      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])
+      : "r"(addr), "r"(on), "n"(OFFSET));
+}
+// The digits that a lane feeds its box's MMAs (see consume_box); all zero between boxes where the lane's are.
+struct Digits {
+  uint32_t b0[2][4], b1[2][4];
+  __device__ __forceinline__ Digits() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) b0[i >> 2][i & 3] = b1[i >> 2][i & 3] = 0u;
+  }
+};
+
+// One box (16 outputs x 1024 inputs) by one warp.  Lane = 4g + t.  A 32-bit
 // word of the re-tiled weights holds four inputs of row g in its low nibbles
 // and of row g+8 in its high nibbles; A's rows g take the word as it is (bytes
 // u_g + 16 u_g8) and its rows g+8 the word with the low nibbles cleared (bytes
 // 16 u_g8), so that row g's sum is the difference of the two results and the
 // nibbles are never shifted apart.  B = the digitised inputs; everything is
-// exact in int32.  The 32 units of a box go in eight sets
-// of four; B column 2j holds the high digit and 2j + 1 the low digit of unit j
-// of the set (lane g supplies column g, zero for the other units), so a lane
-// ends a set with both digits of unit t for rows g and g+8, combines them,
-// takes off the nibble offset and applies the unit's scale.
-__device__ __forceinline__ void consume_box(const Ctx& c, const uint8_t* st, int kb, float (&tot)[2]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  // this lane's digit bytes for the eight sets: unit 4 set + (g >> 1), digit g & 1, inputs 4t.. and 16+4t..
-  const uint2* xd = reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(c.xs) + (size_t)kb * 2 * kBoxK) + lane;
-  uint2 xb[8];
+// exact in int32.  The 32 units of a box (32 inputs, one scale per output) go
+// in eight sets of four, a set in four MMAs m16n8k32 of which each takes eight
+// inputs of every unit: K row r of MMA m is input 8m + r % 8 of unit r / 8.  B
+// column 2j holds the high digit and 2j + 1 the low digit of unit j's inputs and
+// zeros in the K rows of the other units, so a lane ends a set with both digits
+// of unit t for rows g and g+8, combines them, takes off the nibble offset and
+// applies the unit's scale.  With units spread over K that way, a lane's B words
+// are zero, or the unit's, for all MMAs alike: nothing is selected per MMA, the
+// lanes concerned just load (a unit per MMA, where the lanes of the other
+// columns had to put zeros in place, took two selects each: 7B step 1236 us,
+// 1224 without).
+template <int BT>
+__device__ __forceinline__ void box_sets(const uint4* wl, uint32_t xaddr, uint32_t on0, uint32_t on1, Digits& x, int (&acc)[8][4]) {
+  uint4 wv[4];
 #pragma unroll
-  for (int sidx = 0; sidx < 8; ++sidx) xb[sidx] = xd[32 * sidx];
-  const uint4* wl = reinterpret_cast<const uint4*>(st) + lane;  // load j of the box: wl[32 j], units 2j and 2j + 1
-  int acc[8][4];
+  for (int i = 0; i < 4; ++i) wv[i] = wl[32 * (4 * BT + i)];
+  lds_if<512 * BT>(x.b0[0], xaddr, on0);
+  lds_if<512 * BT>(x.b1[0], xaddr, on1);
+  lds_if<512 * BT + 256>(x.b0[1], xaddr, on0);
+  lds_if<512 * BT + 256>(x.b1[1], xaddr, on1);
 #pragma unroll
-  for (int sidx = 0; sidx < 8; ++sidx) acc[sidx][0] = acc[sidx][1] = acc[sidx][2] = acc[sidx][3] = 0;
-  uint4 wbuf[2][4];
+  for (int m = 0; m < 4; ++m) {
 #pragma unroll
-  for (int jj = 0; jj < 4; ++jj) wbuf[0][jj] = wl[32 * jj];
-#pragma unroll
-  for (int bt = 0; bt < 4; ++bt) {  // four loads = eight units = two sets per batch, fetched a batch ahead
-    if (bt + 1 < 4) {
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) wbuf[(bt + 1) & 1][jj] = wl[32 * (4 * (bt + 1) + jj)];
-    }
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const uint4 wv = wbuf[bt & 1][jj];
-      const int sidx = 2 * bt + (jj >> 1);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int us = 2 * (jj & 1) + h;  // unit within the set
-        const uint32_t w0 = h ? wv.z : wv.x, w1 = h ? wv.w : wv.y;
-        // rows g: the whole byte (row g's nibble + 16 x row g+8's); rows g+8: 16 x row g+8's nibble
-        const uint32_t af[4] = {w0, w0 & 0xF0F0F0F0u, w1, w1 & 0xF0F0F0F0u};
-        const bool mine = (g >> 1) == us;
-        mma_u8s8(acc[sidx], af, mine ? xb[sidx].x : 0u, mine ? xb[sidx].y : 0u);
-      }
+    for (int ss = 0; ss < 2; ++ss) {
+      const uint4 q = wv[2 * ss + (m >> 1)];
+      const uint32_t w0 = (m & 1) ? q.z : q.x, w1 = (m & 1) ? q.w : q.y;
+      // rows g: the whole byte (row g's nibble + 16 x row g+8's); rows g+8: 16 x row g+8's nibble
+      const uint32_t af[4] = {w0, w0 & 0xF0F0F0F0u, w1, w1 & 0xF0F0F0F0u};
+      if (m == 0)
+        mma_u8s8_first(acc[2 * BT + ss], af, x.b0[ss][m], x.b1[ss][m]);
+      else
+        mma_u8s8(acc[2 * BT + ss], af, x.b0[ss][m], x.b1[ss][m]);
     }
   }
+}
+__device__ __forceinline__ void consume_box(const Ctx& c, const uint8_t* st, int kb, Digits& x, float (&tot)[2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  // this lane's column is digit g & 1 of unit j of the set; K rows 4t.. are inputs of unit t / 2, rows 16 + 4t.. of unit
+  // 2 + t / 2, of each the first or second four of the MMA's eight
+  const int j = g >> 1;
+  const uint32_t on0 = j == (t >> 1), on1 = j == 2 + (t >> 1);
+  const uint32_t xaddr = smem_u32(c.xs) + kb * 2 * kBoxK + (g * 8 + (t & 1) * 4) * 4;
+  const uint4* wl = reinterpret_cast<const uint4*>(st) + lane;  // load i of the box: wl[32 i], MMAs 2 (i % 2) and + 1 of set i / 2
+  int acc[8][4];
+  box_sets<0>(wl, xaddr, on0, on1, x, acc);
+  box_sets<1>(wl, xaddr, on0, on1, x, acc);
+  box_sets<2>(wl, xaddr, on0, on1, x, acc);
+  box_sets<3>(wl, xaddr, on0, on1, x, acc);
   // unit 4 set + t: scales of rows g and g+8 (16 halves per lane: [set][row]) and the offset term
   const uint4 sc0 = *reinterpret_cast<const uint4*>(st + kBox + lane * 32);
   const uint4 sc1 = *reinterpret_cast<const uint4*>(st + kBox + lane * 32 + 16);
@@ -999,6 +1028,7 @@ __device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int ki
   int stage = p.stage, sl = p.sl, b = start;
   uint32_t phase = p.phase;
   const int b_stop = start + p.len;
+  Digits digits;
 #pragma unroll 1
   while (b < b_stop) {
     const int strip = p.strip0 + sl;
@@ -1028,7 +1058,7 @@ __device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int ki
       c.w.wait(&c.full[stage], phase, 12);
       if (tracing) waited += clock64() - w0;
       const long long b0 = tracing ? clock64() : 0;
-      consume_box(c, c.ring + (size_t)stage * kStageBytes, b - s_lo, tot);
+      consume_box(c, c.ring + (size_t)stage * kStageBytes, b - s_lo, digits, tot);
       __syncwarp();
       if (tracing) boxed += clock64() - b0;
       if (lane == 0) mbar_arrive_n(&c.empty[stage], kCW);
@@ -1831,15 +1861,16 @@ __global__ void __launch_bounds__(256) retile_weights_kernel(const uint8_t* __re
     const int strip = static_cast<int>(box / S), kb = static_cast<int>(box - (int64_t)strip * S);
     uint32_t word = 0;
     if (wi < kBox / 4) {
-      // weights: word = [load j][lane][q]; unit 2j + (q >> 1) of the box, inputs 16 (q & 1) + 4t + {0..3} of the
-      // unit: byte b = input b, low nibble row g, high nibble row g + 8
+      // weights: word = [load j][lane][q]; MMA m = 2 (j & 1) + (q >> 1) of set j >> 1, K rows 16 (q & 1) + 4t + {0..3}:
+      // unit 2 (q & 1) + (t >> 1) of the set, inputs 8m + 4 (t & 1) + {0..3} of the unit; byte b = input b, low nibble row g,
+      // high nibble row g + 8
       const int j = wi >> 7, lane = (wi >> 2) & 31, q = wi & 3;
       const int g = lane >> 2, t = lane & 3;
-      const int unit = 2 * j + (q >> 1);
+      const int unit = 4 * (j >> 1) + 2 * (q & 1) + (t >> 1), m = 2 * (j & 1) + (q >> 1);
 #pragma unroll
       for (int nib = 0; nib < 8; ++nib) {
         const int row = (nib & 1) ? g + 8 : g;
-        const int k = kb * kBoxK + unit * 32 + (q & 1) * 16 + 4 * t + (nib >> 1);
+        const int k = kb * kBoxK + unit * 32 + 8 * m + 4 * (t & 1) + (nib >> 1);
         const int n = strip * kStripN + row;
         uint32_t v = 0;
         if (k < K) {
