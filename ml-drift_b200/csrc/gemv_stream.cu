@@ -45,6 +45,13 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same from other accumulators: d = a b + c.
+__device__ __forceinline__ void mma_f16_from(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
 __device__ __forceinline__ void mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
@@ -84,7 +91,8 @@ struct Frag {
 // subtract, giving the signed weight exactly (x16 for high nibbles).
 // SUBNORMAL operands: the raw masked bits, i.e. fp16 subnormals u * 2^-24 (x16
 // for high nibbles); the "- shift * sum(x)" term comes from one extra MMA per
-// step against a constant operand, and results carry a 2^-24 factor.
+// step against a constant operand, whose result the products are then added to,
+// and results carry a 2^-24 factor.
 // The A operand of MMA f from a lane's 16 bytes (f is a constant wherever this is inlined).
 template <int BITS, bool SUBNORMAL>
 __device__ __forceinline__ void unpack(const uint4& q, int f, uint32_t (&a)[4]) {
@@ -369,7 +377,8 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
 
   // -------------------------------------------------------------- consumers
   const int g = lane >> 2, t = lane & 3;
-  constexpr uint32_t kOnesA = BITS == 4 ? 0x00080008u : 0x00800080u;  // subnormal 8 / 128
+  // minus the offset as a subnormal: -8 / -128 against rows g; rows g + 8 (high nibbles) carry it x16
+  constexpr uint32_t kOffsetA = BITS == 4 ? 0x80088008u : 0x80808080u, kOffsetA16 = 0x80808080u;
   constexpr float kOdd = BITS == 4 ? 0.0625f : 1.0f;                  // high nibbles are carried x16
   constexpr float kOutScale = (SUBNORMAL && !DIGITS) ? 16777216.0f : 1.0f;
   int stage = 0;
@@ -633,18 +642,19 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
             bx[p][1] = xv.y;
           }
         }
-        float ones[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        // minus the offset times the sum of the inputs, x16 for the rows of high nibbles: what the products are added to
+        // (zero points: what is added to them, times a factor of each output's own)
+        float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float offset[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if constexpr (SUBNORMAL) {
-          const uint32_t oa[4] = {kOnesA, kOnesA, kOnesA, kOnesA};
-          mma_f16(ones, oa, bx[0][0], bx[0][1]);
-          mma_f16(ones, oa, bx[1][0], bx[1][1]);
+          const uint32_t oa[4] = {kOffsetA, kOffsetA16, kOffsetA, kOffsetA16};
+          mma_f16_from(offset, oa, bx[0][0], bx[0][1], zero);
+          mma_f16(offset, oa, bx[1][0], bx[1][1]);
         }
         const int gidx = a.gs_shift >= 0 ? (rbase >> a.gs_shift) : 0;
 #pragma unroll
         for (int b = 0; b < W; ++b) {
           float grp[F::NF][4];
-#pragma unroll
-          for (int f = 0; f < F::NF; ++f) grp[f][0] = grp[f][1] = grp[f][2] = grp[f][3] = 0.0f;
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
             const int r = rbase + 2 * t + p;
@@ -653,7 +663,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
             for (int f = 0; f < F::NF; ++f) {
               uint32_t av[4];
               unpack<BITS, SUBNORMAL>(q, f, av);
-              mma_f16(grp[f], av, bx[p][0], bx[p][1]);
+              if (p == 0)
+                mma_f16_from(grp[f], av, bx[p][0], bx[p][1], ZP ? zero : offset);
+              else
+                mma_f16(grp[f], av, bx[p][0], bx[p][1]);
             }
           }
           // scales (and zero points) of this lane's outputs for the group these eight rows are in
@@ -686,22 +699,20 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
 #pragma unroll
             for (int i = 0; i < F::NPL; ++i) zf[i] = fmaf(zf[i], BITS == 4 ? 0.125f : 0.0078125f, 1.0f);
           }
+          if constexpr (BITS == 4) {
+#pragma unroll
+            for (int f = 0; f < F::NF; ++f) sc[2 * f + 1] *= kOdd;
+          }
           // row g of MMA f is output 2f, row g+8 is output 2f+1
 #pragma unroll
           for (int f = 0; f < F::NF; ++f) {
 #pragma unroll
             for (int jj = 0; jj < NJ; ++jj) {
               const int j = MONE ? 2 * jj : jj;  // MONE keeps (row g, token 2t) and (row g+8, token 2t)
-              const bool odd = (j & 2) != 0;
+              const int o = 2 * f + (j >> 1);
               float v = grp[f][j];
-              if constexpr (SUBNORMAL) {
-                float offset = ones[j & 1];
-                if constexpr (ZP) offset *= zf[2 * f + (odd ? 1 : 0)];
-                v = odd ? fmaf(v, kOdd, -offset) : (v - offset);
-              } else {
-                if (odd) v *= kOdd;
-              }
-              tot[b][f][jj] = fmaf(sc[2 * f + (odd ? 1 : 0)], v, tot[b][f][jj]);
+              if constexpr (ZP) v = fmaf(offset[j], zf[o], v);
+              tot[b][f][jj] = fmaf(sc[o], v, tot[b][f][jj]);
             }
           }
         }
