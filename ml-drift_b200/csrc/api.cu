@@ -112,9 +112,10 @@ static int gm_stage_rows() { return strip_geometry(4, 64, 64, 1, 8, MLD_SCALE_BL
 
 // ------------------------------------------------------------------ plan type
 struct TmapEntry {
-  const void* w;
+  const void* wt;
   const void* s;
   const void* z;
+  int w;  // boxes of a strip: the scale box is as wide
   CUtensorMap tw, ts, tz;
 };
 
@@ -141,7 +142,8 @@ struct mld_fc_plan {
   bool pair_ok;          // the prefill GEMM can read the packed weights directly (tensor-map pitch rule)
   const void* next_w;    // one-shot L2 prefetch hint for the next mld_fc_run on this plan
   size_t next_w_bytes;
-  // tensor maps keyed by the (weights, scale, zero point) pointers last seen (the boxes do not depend on the token count)
+  // tensor maps keyed by the (weights, scale, zero point) pointers last seen and the strip width, which is all that the
+  // token count changes about the boxes
   std::vector<TmapEntry> tmaps;
   std::mutex mu;
 };
@@ -457,10 +459,11 @@ static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, 
     std::lock_guard<std::mutex> lock(p->mu);
     const TmapEntry* te = nullptr;
     for (const TmapEntry& e : p->tmaps)
-      if (e.w == weights && e.s == scale && e.z == zp) te = &e;
+      if (e.wt == weights && e.s == scale && e.z == zp && e.w == gm.w) te = &e;
     if (te == nullptr) {
       TmapEntry e;
-      e.w = weights;
+      e.wt = weights;
+      e.w = gm.w;
       e.s = scale;
       e.z = zp;
       memset(&e.tz, 0, sizeof e.tz);

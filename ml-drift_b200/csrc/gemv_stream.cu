@@ -6,9 +6,9 @@
 //  * the grid is one CTA per SM (two for matrices of several passes); each CTA
 //    owns a strip of output columns (16-byte granularity, so the strips balance
 //    to within one chunk) and streams every K row of that strip - no split-K
-//    traffic through global memory.  When the matrix is too narrow for 148 useful strips, two CTAs of
-//    a thread-block cluster share a strip, take half of K each and combine
-//    through distributed shared memory;
+//    traffic through global memory.  When the matrix is too narrow for 148 useful strips, the CTAs of
+//    a thread-block cluster (two, or up to eight for one token) share a strip, take an even part of K each
+//    and combine through distributed shared memory;
 //  * packed weights (128-byte-swizzled boxes), block scales and activations are
 //    staged by TMA / bulk copies into a ring of shared-memory stages, all
 //    completing on one mbarrier per stage;
@@ -210,7 +210,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // token 13.6 against 12.9; 4096 x 11008 10.9 against 10.2).  Several tokens through strips of two boxes take this form always:
 // they have nothing to interleave, but the compiler's schedule of it is the faster one (4096 x 11008, 5 tokens: 15.0 against
 // 15.4).
-template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE>
+// CUT: clusters of more than two CTAs cut K (StripGeometry::ksplit).  A form of its own likewise: adding up any number of
+// partners' sums cost launches of one or two CTAs to a strip 0.1 to 0.3 us (896 x 12288 4.15 / 4.35, 2432 x 6048 INT8 6.05 /
+// 6.47).
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE, bool CUT>
 __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     fc_strip_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s,
                     const __grid_constant__ CUtensorMap tmap_z, StripArgs a) {
@@ -222,8 +225,9 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* red = reinterpret_cast<float*>(smem + (size_t)a.stages * a.stage_bytes);  // [warps][WT][red_m]
-  float* peer = red + kConsumerWarps * WT * a.red_m;                                // [WT][peer_m]
-  uint64_t* full = reinterpret_cast<uint64_t*>(peer + ((WT * a.peer_m + 1) & ~1));
+  float* peer = red + kConsumerWarps * WT * a.red_m;                                // [partners][WT][peer_m]
+  const int partners = CUT ? a.ksplit - 1 : 1;
+  uint64_t* full = reinterpret_cast<uint64_t*>(peer + ((partners * WT * a.peer_m + 1) & ~1));
   uint64_t* empty = full + a.stages;
   uint64_t* peer_bar = empty + a.stages;
   // DIGITS: the activation vector of this CTA's K range as digits ([unit][digit, the highest first][8 words], word j = the
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         mbar_init(&full[s], 1);
         mbar_init(&empty[s], kConsumerWarps);
       }
-      mbar_init(peer_bar, kConsumerWarps * 32);
+      mbar_init(peer_bar, partners * kConsumerWarps * 32);
       if constexpr (DIGITS) mbar_init(xbar, 1);
       fence_barrier_init();
     }
@@ -776,8 +780,8 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
     }
     MLD_CONSUMER_BARRIER();
     if (a.ksplit > 1 && pass == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (a.ksplit > 1 && kr == 1) {
-      peer_remote = map_to_rank(smem_u32(peer), 0);
+    if (CUT ? kr > 0 : a.ksplit > 1 && kr == 1) {
+      peer_remote = map_to_rank(smem_u32(CUT ? peer + (kr - 1) * WT * a.peer_m : peer), 0);
       bar_remote = map_to_rank(smem_u32(peer_bar), 0);
     }
     if (a.ksplit > 1 && kr == 0) {
@@ -797,8 +801,13 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       }
       return v;
     };
-    if (a.ksplit > 1 && kr == 1) {
-      // upper half of K: hand the sums to the partner
+    // CUT: the other CTAs' sums of an output onto this one's, in the order of their parts of K
+    [[maybe_unused]] const auto add_peers = [&](float v, int n_local, int tok) {
+      for (int r = 0; r < partners; ++r) v += peer[(r * WT + n_local) * a.peer_m + tok];
+      return v;
+    };
+    if (CUT ? kr > 0 : a.ksplit > 1 && kr == 1) {
+      // a later part of K: hand the sums to the cluster's first CTA
       for (int idx = threadIdx.x; idx < WT * a.M && !failed; idx += kConsumerWarps * 32) {
         const int n_local = idx / a.M, tok = idx - n_local * a.M;
         st_cluster_f32(peer_remote + (n_local * a.peer_m + tok) * 4, warp_sum(n_local, tok));
@@ -809,7 +818,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
       for (int idx = threadIdx.x; idx < (WT / 2) * a.M && !failed; idx += kConsumerWarps * 32) {
         const int p_local = idx / a.M, tok = idx - p_local * a.M;
         float sg = warp_sum(2 * p_local, tok), su = warp_sum(2 * p_local + 1, tok);
-        if (a.ksplit > 1) {
+        if constexpr (CUT) {
+          sg = add_peers(sg, 2 * p_local, tok);
+          su = add_peers(su, 2 * p_local + 1, tok);
+        } else if (a.ksplit > 1) {
           sg += peer[(2 * p_local) * a.peer_m + tok];
           su += peer[(2 * p_local + 1) * a.peer_m + tok];
         }
@@ -834,7 +846,11 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         const int n = n0 + n_local;
         if (n >= n_end) continue;
         float s = warp_sum(n_local, tok);
-        if (a.ksplit > 1) s += peer[n_local * a.peer_m + tok];  // fixed order: lower half of K first
+        if constexpr (CUT) {
+          s = add_peers(s, n_local, tok);
+        } else if (a.ksplit > 1) {
+          s += peer[n_local * a.peer_m + tok];  // fixed order: lower half of K first
+        }
         __half r = __float2half_rn(s * kOutScale);
         if (a.bias != nullptr) r = __hadd(r, static_cast<const __half*>(a.bias)[n]);
         const int tk_out = a.tok0 + tok;
@@ -849,7 +865,7 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
         }
       }
     }
-    if (a.ksplit > 1 && kr == 1) mbar_arrive_cluster(bar_remote);  // release: the stores above are visible
+    if (CUT ? kr > 0 : a.ksplit > 1 && kr == 1) mbar_arrive_cluster(bar_remote);  // release: the stores above are visible
     MLD_CONSUMER_BARRIER();
     if (tr && threadIdx.x == 0) tr[5] = globaltimer_ns();
   }
@@ -870,10 +886,10 @@ __global__ void __launch_bounds__((kConsumerWarps + 1) * 32, W <= 2 ? 2 : 1)
   }
 }
 
-template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE>
+template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS, bool ZP, bool SPLIT, bool INTERLEAVE, bool CUT = false>
 int launch_strip_f(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
                    const StripGeometry& gm, cudaStream_t stream) {
-  auto kern = fc_strip_kernel<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, INTERLEAVE>;
+  auto kern = fc_strip_kernel<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, INTERLEAVE, CUT>;
   static bool configured[kMaxDevices];  // per instantiation and device
   int dev;
   if (needs_configure(configured, &dev)) {
@@ -909,6 +925,9 @@ int launch_strip_f(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorM
 template <int BITS, int W, bool SUBNORMAL, bool MONE, bool DIGITS = false, bool ZP = false, bool SPLIT = false>
 int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tz, const StripArgs& a,
                    const StripGeometry& gm, cudaStream_t stream) {
+  if constexpr (W == 2 && MONE && !SPLIT) {  // (one token, strips of two whole boxes)
+    if (gm.ksplit > 2) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, false, true>(tw, ts, tz, a, gm, stream);
+  }
   if constexpr (W == 2) {  // (strips of several passes with pdl are two boxes wide)
     if (!MONE || gm.interleave) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, true>(tw, ts, tz, a, gm, stream);
   }
@@ -981,10 +1000,47 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
     gm.grid = strips;
     w = div_up(div_up(gm.units, strips) * gm.gran, 8);
   }
+  // One token: strips that fill their boxes, where the rule above leaves part of them empty or splits what is small already.
+  // us in a graph, INT4 block 32 unless said otherwise, the rule above / as here.
+  if (m_total == 1 && w_max == 2) {
+    const int n_st = div_up(SS, kStageRows), most = sms + sms * 73 / 100;
+    int S = 0, boxes = 2;
+    if (C < 8 * sms && n_st <= 8) {
+      // up to 2048 inputs the stages of a whole strip take less time than the cluster's meeting: 2048 x 4096 4.5 / 4.3,
+      // 1024 x 3072 4.0 / 3.4, 1024 x 1024 4.0 / 3.0 (4096 x 4096, on the other side of the line: 5.5 / 6.5)
+      S = 1;
+      boxes = 1;
+    } else if (C <= 16 * most) {
+      // Strips of two whole boxes.  As many as SMs or more, or K cut so that a CTA has up to eight stages (it also turns that
+      // much of the vector into digits) where clusters of that size are all resident at once and every SM has work: 4096 x
+      // 11008 10.0 / 9.0 (2 x 86 CTAs; 3 x 86 9.2), 4096 x 14336 10.0 / 9.5, 14336 x 4096 12.9 / 9.9, 8192 x 8192 11.0 / 10.2
+      // (4 x 64), 4096 x 22016 14.8 / 13.1, 1536 x 21568 8.9 / 6.7, INT8 4096 x 11008 13.9 / 12.8.  On the other side of the
+      // line: clusters of three (4736 x 8320 7.6 / 8.7), fewer than sixteen stages to cut (INT8 2432 x 6048 6.0 / 6.4) and
+      // idle SMs (2048 x 16384 6.2 / 7.6).
+      const int full = div_up(C, 16);
+      if (full >= sms) {
+        S = 1;
+      } else if (n_st >= 16) {
+        for (int s = 2; s <= 8 && full * s <= most; ++s) {
+          if (s == 3) continue;
+          S = s;
+          if (div_up(n_st, s) <= 8) break;
+        }
+        if (full * S < sms) S = 0;
+      }
+    }
+    if (S > 0) {
+      gm.interleave = 0;
+      gm.ksplit = S;
+      gm.strips = strips = div_up(C, 8 * boxes);
+      gm.grid = strips * S;
+      w = div_up(div_up(gm.units, strips) * gm.gran, 8);
+    }
+  }
   gm.w = w > w_max ? w_max : w;
   const int passes = gm.interleave ? div_up(C, strips * gm.w * 8) : div_up(max_width, gm.w * 8);
   gm.fill = 100 * C / (strips * passes * gm.w * 8);
-  gm.rows_per_split = gm.ksplit == 1 ? align_n(SS, kStageRows) : align_n(div_up(SS, 2), kStageRows);
+  gm.rows_per_split = align_n(div_up(SS, gm.ksplit), kStageRows);
   if (scale_mode == MLD_SCALE_SCALAR) {
     gm.scale_rows = 0;
     gm.group_slices = 1;
@@ -1009,7 +1065,7 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
   // one drains and the next prefetches, so each takes at most half of it.
   int budget = pdl ? 112 * 1024 : 224 * 1024;
   if (smem_limit_kb >= 32 && smem_limit_kb <= 224) budget = smem_limit_kb * 1024;
-  int fixed = (kConsumerWarps * gm.red_m + gm.peer_m) * wt * 4 + 8 + (2 * 16 + 1) * 8 + 1024 + 64;
+  int fixed = (kConsumerWarps * gm.red_m + (gm.ksplit - 1) * gm.peer_m) * wt * 4 + 8 + (2 * 16 + 1) * 8 + 1024 + 64;
   // One token as digits: room for the activation vector of this CTA's K range (per k-slice 8 bytes, 4 digits 16 more; per
   // unit of eight k-slices 8 bytes for every two digits; a barrier).
   if (m_total == 1 && split && !zero_point) {

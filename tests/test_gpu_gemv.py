@@ -571,3 +571,30 @@ def test_streaming_many_passes(mld, oracle):
             plan.run(_dev(oracle.to_sliced(x.astype(np.float32)).astype(np.float16)), packed, sc, y, M)
             torch.cuda.synchronize()
             assert _rel(oracle.from_sliced(y.float().cpu().numpy(), N), _exact_fc(x, q, scale)) <= 1e-3
+
+
+@pytest.mark.parametrize("bits,K,N,block,use_zp", [
+    (4, 8192, 4744, 32, False), (4, 10240, 3848, 128, False), (4, 13312, 2704, 0, False), (4, 14592, 2440, 64, False),
+    (4, 4104, 9480, 0, False), (8, 12800, 1352, 0, False), (4, 8192, 4744, 128, True),  # K cut into 2 to 8 parts
+    (4, 512, 19008, 32, False), (8, 1032, 1160, 0, False), (4, 2048, 9464, 32, True)])  # whole strips of two boxes and one
+def test_one_token_whole_strips(mld, oracle, bits, K, N, block, use_zp):
+    # one plan and one set of weights at one and at five tokens, whose strips differ; 1e-3 as in test_streaming_token_ranges
+    rng = np.random.default_rng(K + N)
+    G = K // block if block else 1
+    lo, hi = (-128, 128) if bits == 8 else (-8, 8)
+    q = rng.integers(lo, hi, size=(N, K), dtype=np.int8)
+    scale = (rng.uniform(0.5, 1.5, (N, G)) / hi / 16).astype(np.float32)
+    zp = rng.integers(lo, hi, size=(N, G)).astype(np.float32) if use_zp else None
+    packed = _dev(oracle.rearrange_int8_as_uint8(q) if bits == 8 else oracle.rearrange_int8_as_uint4(q))
+    params = [_dev(oracle.scale_layout(t, True).view(np.float16)) if t is not None else None for t in (scale, zp)]
+    plan = mld.FullyConnectedPlan(N, K, bits, scale_mode=mld.SCALE_BLOCK if block else mld.SCALE_PER_CHANNEL, groups=G,
+                                  has_zero_point=use_zp, precision=mld.F32F16, max_tokens=5)
+    x = rng.standard_normal((5, K)).astype(np.float16)
+    want = _exact_fc(x, q, scale, zp)
+    for M in (1, 5, 1):
+        y = torch.full(((N + 3) // 4, M, 4), float("nan"), dtype=torch.float16, device="cuda")
+        plan.run(_dev(oracle.to_sliced(x[:M].astype(np.float32)).astype(np.float16)), packed, params[0], y, M,
+                 zero_point=params[1])
+        torch.cuda.synchronize()
+        assert plan.last_route() == mld.ROUTE_DECODE_STREAMING and plan.device_status() == 0
+        assert _rel(oracle.from_sliced(y.float().cpu().numpy(), N), want[:M]) <= 1e-3
