@@ -10,6 +10,7 @@ namespace mld {
 
 namespace {
 
+constexpr int kPackBlocks = 256;                 // blocks that pack_rows_kernel's grid has at least, where the rows allow
 constexpr int kTileSlices = 32;                  // 32 x 32 blocks of 4x4 per CTA
 constexpr int kTileCh = kTileSlices * 4;         // 128 channels each way
 constexpr int kRowPitch = kTileSlices * 16 + 4;  // bytes per src-slice row of the staged tile (+4: bank spread)
@@ -190,8 +191,8 @@ __device__ __forceinline__ void st_global_32b(uint8_t* p, const uint32_t (&a)[4]
                : "memory");
 }
 
-// The common case without shared memory: int8 source, one output group (the FullyConnected choice), input
-// channels a multiple of 16, 16-byte aligned rows.  A warp takes 16 output rows x 128 input channels.  Per
+// The common case without staging in shared memory: int8 source, one output group (the FullyConnected choice), input
+// channels a multiple of 16, 16-byte aligned rows.  A warp takes 16 output rows x 128 input channels at a time.  Per
 // step it reads four rows, eight lanes to a row and 16 bytes to a lane; the four lanes that hold the same 16
 // input channels of the four rows exchange words so that each ends up with the four rows of ONE group of four
 // input channels, i.e. one 4x4 block, which it transposes byte-wise in registers.  After four steps a lane
@@ -200,83 +201,114 @@ __device__ __forceinline__ void st_global_32b(uint8_t* p, const uint32_t (&a)[4]
 // A lane's run is stored 32 bytes at a time where every run starts on a 32-byte boundary (WIDE: whole groups of four
 // output slices and of 16 outputs): one whole sector per store instead of four quarter-filled requests.  14336 x 4096 to
 // INT4: 47.2 us, 38.3 with these stores, and 16 less with the exchange of words free of branches.
+// 2^across_shift of the block's eight warps lie side by side along the input channels and gridDim.x such blocks take turns
+// along them, the other warps take further rows.  The sums of a row's weights stay in registers until a block is through;
+// where one block covers all of a row it writes them, and neither atomics nor a fill ahead of the kernel are needed.
 template <int BITS, bool WIDE>
-__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a) {
+__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_shift) {
+  pdl_wait();
+  __shared__ int32_t sums[8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hw = blockIdx.z;
+  const int across = 1 << across_shift, part = warp & (across - 1);
   const int r = lane >> 3, c = lane & 7;                 // row of the step's four, 16-byte chunk of the 128 inputs
-  const int i0 = blockIdx.x * 128 + c * 16;              // first input channel of this lane's chunk
-  const int o0 = (blockIdx.y * 8 + warp) * 16;           // first of the warp's 16 output rows
-  if (o0 >= a.dst_slices * 4) return;
+  const int o0 = (blockIdx.y * (8 >> across_shift) + (warp >> across_shift)) * 16;  // first of the warp's 16 output rows
   const int8_t* src = reinterpret_cast<const int8_t*>(a.src);
   const uint32_t padw = (a.pad & 0xFFu) * 0x01010101u;
-  uint32_t blk[4][4];                                     // [step = output slice][word k = input channel of the block]
-#pragma unroll
-  for (int st = 0; st < 4; ++st) {
-    const int o = o0 + st * 4 + r;
-    uint4 v = make_uint4(padw, padw, padw, padw);
-    int32_t rowsum = 0;
-    if (o < a.O && i0 < a.I) {
-      v = *reinterpret_cast<const uint4*>(src + ((int64_t)o * a.HW + hw) * a.I + i0);
-      rowsum = __dp4a(static_cast<int>(v.x), 0x01010101, 0);
-      rowsum = __dp4a(static_cast<int>(v.y), 0x01010101, rowsum);
-      rowsum = __dp4a(static_cast<int>(v.z), 0x01010101, rowsum);
-      rowsum = __dp4a(static_cast<int>(v.w), 0x01010101, rowsum);
-      // q + shift, byte-wise: +128 is a flip of the top bit; +8 on values in [-8, 7] likewise, kept to 4 bits
-      const uint32_t flip = BITS == 8 ? 0x80808080u : 0x08080808u, keep = BITS == 8 ? 0xFFFFFFFFu : 0x0F0F0F0Fu;
-      v.x = (v.x ^ flip) & keep;
-      v.y = (v.y ^ flip) & keep;
-      v.z = (v.z ^ flip) & keep;
-      v.w = (v.w ^ flip) & keep;
-    }
-    if (a.sum_i != nullptr) {
-      rowsum += __shfl_xor_sync(0xffffffffu, rowsum, 1);
-      rowsum += __shfl_xor_sync(0xffffffffu, rowsum, 2);
-      rowsum += __shfl_xor_sync(0xffffffffu, rowsum, 4);
-      if (c == 0 && o < a.O && o < a.sum_len && rowsum != 0) atomicAdd(a.sum_i + o, rowsum);
-    }
-    // lane (r, c) collects word r of the rows 0..3 held by lanes (0..3, c)
-    uint32_t rows[4] = {v.x, v.y, v.z, v.w};
-    exchange_words(rows, r);
-    // rows[n] = bytes (k = 0..3) of output n; the block wants word k = bytes (n = 0..3)
-    const uint32_t t0 = __byte_perm(rows[0], rows[1], 0x5140), t1 = __byte_perm(rows[2], rows[3], 0x5140);
-    const uint32_t t2 = __byte_perm(rows[0], rows[1], 0x7362), t3 = __byte_perm(rows[2], rows[3], 0x7362);
-    blk[st][0] = __byte_perm(t0, t1, 0x5410);
-    blk[st][1] = __byte_perm(t0, t1, 0x7632);
-    blk[st][2] = __byte_perm(t2, t3, 0x5410);
-    blk[st][3] = __byte_perm(t2, t3, 0x7632);
-  }
-  const int s = (i0 >> 2) + r;                             // this lane's input slice
-  if (s >= a.src_slices) return;
-  const int ds0 = o0 >> 2;
-  const int64_t block_index = ((int64_t)hw * a.src_slices + s) * a.group + ds0;
-  if (BITS == 8 && WIDE) {
-    uint8_t* dst = a.dst + block_index * 16;
-    st_global_32b(dst, blk[0], blk[1]);
-    st_global_32b(dst + 32, blk[2], blk[3]);
-  } else if (BITS == 8) {
-    uint4* dst = reinterpret_cast<uint4*>(a.dst + block_index * 16);
-#pragma unroll
-    for (int st = 0; st < 4; ++st)
-      if (ds0 + st < a.total_ds) dst[st] = make_uint4(blk[st][0], blk[st][1], blk[st][2], blk[st][3]);
-  } else {
-    uint32_t run[8];
+  int32_t rowsum[4] = {0, 0, 0, 0};
+  for (int base = (blockIdx.x * across + part) * 128; base < a.I && o0 < a.dst_slices * 4; base += gridDim.x * across * 128) {
+    const int i0 = base + c * 16;                          // first input channel of this lane's chunk
+    uint32_t blk[4][4];                                    // [step = output slice][word k = input channel of the block]
+    uint4 v4[4];
 #pragma unroll
     for (int st = 0; st < 4; ++st) {
-      // bytes v0 v1 v2 v3 of a word (each < 16) -> v0 | v1 << 4, v2 | v3 << 4
-      const uint32_t y0 = blk[st][0] | (blk[st][0] >> 4), y1 = blk[st][1] | (blk[st][1] >> 4);
-      const uint32_t y2 = blk[st][2] | (blk[st][2] >> 4), y3 = blk[st][3] | (blk[st][3] >> 4);
-      run[2 * st] = __byte_perm(y0, y1, 0x6420);
-      run[2 * st + 1] = __byte_perm(y2, y3, 0x6420);
+      const int o = o0 + st * 4 + r;
+      v4[st] = make_uint4(0u, 0u, 0u, 0u);
+      if (o < a.O && i0 < a.I) v4[st] = *reinterpret_cast<const uint4*>(src + ((int64_t)o * a.HW + hw) * a.I + i0);
     }
-    if (WIDE) {
-      st_global_32b(a.dst + block_index * 8, *reinterpret_cast<uint32_t(*)[4]>(&run[0]),
-                    *reinterpret_cast<uint32_t(*)[4]>(&run[4]));
-    } else {
-      uint2* dst = reinterpret_cast<uint2*>(a.dst + block_index * 8);
 #pragma unroll
-      for (int st = 0; st < 4; ++st)
-        if (ds0 + st < a.total_ds) dst[st] = make_uint2(run[2 * st], run[2 * st + 1]);
+    for (int st = 0; st < 4; ++st) {
+      const int o = o0 + st * 4 + r;
+      uint4 v = v4[st];
+      if (o < a.O && i0 < a.I) {
+        rowsum[st] = __dp4a(static_cast<int>(v.x), 0x01010101, rowsum[st]);
+        rowsum[st] = __dp4a(static_cast<int>(v.y), 0x01010101, rowsum[st]);
+        rowsum[st] = __dp4a(static_cast<int>(v.z), 0x01010101, rowsum[st]);
+        rowsum[st] = __dp4a(static_cast<int>(v.w), 0x01010101, rowsum[st]);
+        // q + shift, byte-wise: +128 is a flip of the top bit; +8 on values in [-8, 7] likewise, kept to 4 bits
+        const uint32_t flip = BITS == 8 ? 0x80808080u : 0x08080808u, keep = BITS == 8 ? 0xFFFFFFFFu : 0x0F0F0F0Fu;
+        v.x = (v.x ^ flip) & keep;
+        v.y = (v.y ^ flip) & keep;
+        v.z = (v.z ^ flip) & keep;
+        v.w = (v.w ^ flip) & keep;
+      } else {
+        v = make_uint4(padw, padw, padw, padw);
+      }
+      // lane (r, c) collects word r of the rows 0..3 held by lanes (0..3, c)
+      uint32_t rows[4] = {v.x, v.y, v.z, v.w};
+      exchange_words(rows, r);
+      // rows[n] = bytes (k = 0..3) of output n; the block wants word k = bytes (n = 0..3)
+      const uint32_t t0 = __byte_perm(rows[0], rows[1], 0x5140), t1 = __byte_perm(rows[2], rows[3], 0x5140);
+      const uint32_t t2 = __byte_perm(rows[0], rows[1], 0x7362), t3 = __byte_perm(rows[2], rows[3], 0x7362);
+      blk[st][0] = __byte_perm(t0, t1, 0x5410);
+      blk[st][1] = __byte_perm(t0, t1, 0x7632);
+      blk[st][2] = __byte_perm(t2, t3, 0x5410);
+      blk[st][3] = __byte_perm(t2, t3, 0x7632);
+    }
+    const int s = (i0 >> 2) + r;                           // this lane's input slice
+    const int ds0 = o0 >> 2;
+    const int64_t block_index = ((int64_t)hw * a.src_slices + s) * a.group + ds0;
+    if (s < a.src_slices) {
+      if (BITS == 8 && WIDE) {
+        uint8_t* dst = a.dst + block_index * 16;
+        st_global_32b(dst, blk[0], blk[1]);
+        st_global_32b(dst + 32, blk[2], blk[3]);
+      } else if (BITS == 8) {
+        uint4* dst = reinterpret_cast<uint4*>(a.dst + block_index * 16);
+#pragma unroll
+        for (int st = 0; st < 4; ++st)
+          if (ds0 + st < a.total_ds) dst[st] = make_uint4(blk[st][0], blk[st][1], blk[st][2], blk[st][3]);
+      } else {
+        uint32_t run[8];
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+          // bytes v0 v1 v2 v3 of a word (each < 16) -> v0 | v1 << 4, v2 | v3 << 4
+          const uint32_t y0 = blk[st][0] | (blk[st][0] >> 4), y1 = blk[st][1] | (blk[st][1] >> 4);
+          const uint32_t y2 = blk[st][2] | (blk[st][2] >> 4), y3 = blk[st][3] | (blk[st][3] >> 4);
+          run[2 * st] = __byte_perm(y0, y1, 0x6420);
+          run[2 * st + 1] = __byte_perm(y2, y3, 0x6420);
+        }
+        if (WIDE) {
+          st_global_32b(a.dst + block_index * 8, *reinterpret_cast<uint32_t(*)[4]>(&run[0]),
+                        *reinterpret_cast<uint32_t(*)[4]>(&run[4]));
+        } else {
+          uint2* dst = reinterpret_cast<uint2*>(a.dst + block_index * 8);
+#pragma unroll
+          for (int st = 0; st < 4; ++st)
+            if (ds0 + st < a.total_ds) dst[st] = make_uint2(run[2 * st], run[2 * st + 1]);
+        }
+      }
+    }
+  }
+  if (a.sum_i == nullptr) return;
+#pragma unroll
+  for (int st = 0; st < 4; ++st) {
+    int32_t v = rowsum[st];
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    if (c == 0) sums[warp][st * 4 + r] = v;
+  }
+  __syncthreads();
+  if (part == 0 && lane < 16) {
+    const int o = o0 + lane;
+    int32_t v = 0;
+    for (int w = 0; w < across; ++w) v += sums[warp + w][lane];
+    if (o < a.O && o < a.sum_len) {
+      if (gridDim.x == 1 && gridDim.z == 1)
+        a.sum_i[o] = v;
+      else if (v != 0)
+        atomicAdd(a.sum_i + o, v);
     }
   }
 }
@@ -365,6 +397,7 @@ __global__ void sum_i_kernel(const int8_t* src, int O, int64_t hwi, int32_t* sum
 // [O][G] fp32 -> [G][O4] fp16/fp32, zero padded (OHIToHOIO4 in buffer storage), a thread per value written.  For few
 // groups, where a row of the source is a fraction of a tile's 32 columns (see pack_scales_impl).
 __global__ void __launch_bounds__(256) pack_few_scales_kernel(const float* src, int O, int G, int O4, int dst_f16, void* dst) {
+  pdl_wait();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)G * O4) return;
   const int g = static_cast<int>(idx / O4), o = static_cast<int>(idx % O4);
@@ -378,6 +411,7 @@ __global__ void __launch_bounds__(256) pack_few_scales_kernel(const float* src, 
 // (14336 x 128: 4.5 us; a thread per output value, reading down a column, fetches every sector of the source eight times
 // and takes 10.4).
 __global__ void __launch_bounds__(256) pack_scales_kernel(const float* src, int O, int G, int O4, int dst_f16, void* dst) {
+  pdl_wait();
   __shared__ float tile[32][33];
   const int o_tiles = (O4 + 31) / 32;
   const int o0 = blockIdx.x % o_tiles * 32, g0 = blockIdx.x / o_tiles * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
@@ -405,6 +439,7 @@ __global__ void __launch_bounds__(256) pack_scales_kernel(const float* src, int 
 __global__ void __launch_bounds__(128) quantize_kernel(const float* w, int O, int I, int block, int G,
                                                        float qmax, float qlo, float qhi, int8_t* q,
                                                        float* scale) {
+  pdl_wait();
   const int o = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   for (int g = warp + blockIdx.y * nwarps; g < G; g += nwarps * gridDim.y) {
@@ -460,6 +495,7 @@ template <int LPB>
 __global__ void __launch_bounds__(256) quantize_blocks_kernel(const float* __restrict__ w, int64_t chunks, float qmax,
                                                               float qlo, float qhi, int8_t* __restrict__ q,
                                                               float* __restrict__ scale) {
+  pdl_wait();
   const int64_t ch0 = (int64_t)blockIdx.x * 512 + threadIdx.x;
   float4 v[2][2];
 #pragma unroll
@@ -493,6 +529,7 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const float* __res
 // L2 / L1, 16 bytes per lane.
 __global__ void __launch_bounds__(256) quantize_rows_kernel(const float* __restrict__ w, int I, float qmax, float qlo,
                                                             float qhi, int8_t* __restrict__ q, float* __restrict__ scale) {
+  pdl_wait();
   __shared__ float red[8];
   const float* row = w + (int64_t)blockIdx.x * I;
   float bound = 0.0f;
@@ -537,28 +574,32 @@ int pack_weights_impl(const mld_pack_desc* d, const void* src, void* dst, int32_
   a.shift = d->bits == 8 ? 128 : 8;
   a.pad = d->pad_value;
   a.swap_dims = d->swap_dims;
-  if (sum_i != nullptr) {
-    const int n = sum_len < d->o ? sum_len : d->o;
-    if (n > 0) MLD_CUDA_CHECK(cudaMemsetAsync(sum_i, 0, sizeof(int32_t) * n, stream));
-  }
   dim3 grid(div_up(a.src_slices, kTileSlices), div_up(a.total_ds, kTileSlices), a.HW);
-  if (grid.x == 0 || grid.y == 0 || grid.z == 0) return MLD_OK;
+  const int n_sums = sum_i == nullptr ? 0 : sum_len < d->o ? sum_len : d->o;
+  const auto clear_sums = [&]() { return n_sums > 0 ? cudaMemsetAsync(sum_i, 0, sizeof(int32_t) * n_sums, stream) : cudaSuccess; };
+  if (grid.x == 0 || grid.y == 0 || grid.z == 0) {
+    MLD_CUDA_CHECK(clear_sums());
+    return MLD_OK;
+  }
   const bool rows_fit = d->source == MLD_SRC_INT8 && a.I % 16 == 0 && a.group == a.dst_slices &&
                         (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+  if (!rows_fit) MLD_CUDA_CHECK(clear_sums());
   if (rows_fit) {
-    dim3 rgrid(div_up(a.I, 128), div_up(a.dst_slices * 4, 128), a.HW);
+    // Warps side by side along a row as far as it has 128 channels for them; blocks beside them only where there are too few
+    // rows to keep the SMs busy (512 rows of 11008: 32 blocks of eight warps otherwise).
+    const int chunks = div_up(a.I, 128);
+    int across_shift = 0;
+    while (across_shift < 3 && (2 << across_shift) <= chunks) ++across_shift;
+    const int rows = 16 * (8 >> across_shift), blocks = div_up(a.dst_slices * 4, rows) * a.HW;
+    const int most = div_up(chunks, 1 << across_shift);
+    int beside = div_up(kPackBlocks, blocks);
+    if (beside > most) beside = most;
+    dim3 rgrid(beside, div_up(a.dst_slices * 4, rows), a.HW);
+    if (beside > 1 || a.HW > 1) MLD_CUDA_CHECK(clear_sums());
     const bool wide = a.dst_slices % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
-    if (d->bits == 8) {
-      if (wide)
-        pack_rows_kernel<8, true><<<rgrid, 256, 0, stream>>>(a);
-      else
-        pack_rows_kernel<8, false><<<rgrid, 256, 0, stream>>>(a);
-    } else {
-      if (wide)
-        pack_rows_kernel<4, true><<<rgrid, 256, 0, stream>>>(a);
-      else
-        pack_rows_kernel<4, false><<<rgrid, 256, 0, stream>>>(a);
-    }
+    const auto kern = d->bits == 8 ? (wide ? pack_rows_kernel<8, true> : pack_rows_kernel<8, false>)
+                                   : (wide ? pack_rows_kernel<4, true> : pack_rows_kernel<4, false>);
+    MLD_CUDA_CHECK(launch_overlapped(kern, rgrid, dim3(256), 0, stream, a, across_shift));
   } else if (d->source == MLD_SRC_UINT4_PACKED && a.I % 32 == 0 && a.O % 4 == 0 && !a.swap_dims &&
              a.group == a.dst_slices && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
              (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
@@ -590,10 +631,11 @@ int pack_scales_impl(const float* src, int32_t o, int32_t g, int32_t dst_f16, vo
   // A tile has 32 groups: with one, one lane of 32 loads and one warp of eight stores.  us, a value per thread / tiles:
   // 151936 x 1 1.7 / 5.7, x 4 3.5 / 6.6, x 16 9.0 / 7.1; 14336 x 1 1.5 / 1.7, x 4 1.6 / 1.7, x 8 1.8 / 1.7, x 128 10.4 / 4.5.
   if (g <= 4)
-    pack_few_scales_kernel<<<static_cast<unsigned>(div_up64(n, 256)), 256, 0, stream>>>(src, o, g, O4, dst_f16, dst);
+    MLD_CUDA_CHECK(launch_overlapped(pack_few_scales_kernel, dim3(static_cast<unsigned>(div_up64(n, 256))), dim3(256), 0, stream,
+                                     src, o, g, O4, dst_f16, dst));
   else
-    pack_scales_kernel<<<static_cast<unsigned>((int64_t)div_up(O4, 32) * div_up(g, 32)), 256, 0, stream>>>(src, o, g, O4,
-                                                                                                       dst_f16, dst);
+    MLD_CUDA_CHECK(launch_overlapped(pack_scales_kernel, dim3(static_cast<unsigned>((int64_t)div_up(O4, 32) * div_up(g, 32))),
+                                     dim3(256), 0, stream, src, o, g, O4, dst_f16, dst));
   MLD_LAUNCH_CHECK();
   return MLD_OK;
 }
@@ -611,19 +653,18 @@ int quantize_weights_impl(const float* w, int32_t o, int32_t i, int32_t bits, in
   if (aligned && block % 8 == 0 && lpb >= 1 && lpb <= 32 && (lpb & (lpb - 1)) == 0) {
     const int64_t chunks = (int64_t)o * i / 8;
     const unsigned gb = static_cast<unsigned>(div_up64(chunks, 512));
-    switch (lpb) {
-      case 1: quantize_blocks_kernel<1><<<gb, 256, 0, stream>>>(w, chunks, qmax, qlo, qhi, q, scale); break;
-      case 2: quantize_blocks_kernel<2><<<gb, 256, 0, stream>>>(w, chunks, qmax, qlo, qhi, q, scale); break;
-      case 4: quantize_blocks_kernel<4><<<gb, 256, 0, stream>>>(w, chunks, qmax, qlo, qhi, q, scale); break;
-      case 8: quantize_blocks_kernel<8><<<gb, 256, 0, stream>>>(w, chunks, qmax, qlo, qhi, q, scale); break;
-      case 16: quantize_blocks_kernel<16><<<gb, 256, 0, stream>>>(w, chunks, qmax, qlo, qhi, q, scale); break;
-      default: quantize_blocks_kernel<32><<<gb, 256, 0, stream>>>(w, chunks, qmax, qlo, qhi, q, scale); break;
-    }
+    const auto kern = lpb == 1    ? quantize_blocks_kernel<1>
+                      : lpb == 2  ? quantize_blocks_kernel<2>
+                      : lpb == 4  ? quantize_blocks_kernel<4>
+                      : lpb == 8  ? quantize_blocks_kernel<8>
+                      : lpb == 16 ? quantize_blocks_kernel<16>
+                                  : quantize_blocks_kernel<32>;
+    MLD_CUDA_CHECK(launch_overlapped(kern, dim3(gb), dim3(256), 0, stream, w, chunks, qmax, qlo, qhi, q, scale));
   } else if (aligned && G == 1 && i % 4 == 0) {
-    quantize_rows_kernel<<<o, 256, 0, stream>>>(w, i, qmax, qlo, qhi, q, scale);
+    MLD_CUDA_CHECK(launch_overlapped(quantize_rows_kernel, dim3(o), dim3(256), 0, stream, w, i, qmax, qlo, qhi, q, scale));
   } else {
     dim3 grid(o, G >= 64 ? 4 : 1);
-    quantize_kernel<<<grid, 128, 0, stream>>>(w, o, i, block, G, qmax, qlo, qhi, q, scale);
+    MLD_CUDA_CHECK(launch_overlapped(quantize_kernel, grid, dim3(128), 0, stream, w, o, i, block, G, qmax, qlo, qhi, q, scale));
   }
   MLD_LAUNCH_CHECK();
   return MLD_OK;

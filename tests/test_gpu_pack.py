@@ -194,3 +194,20 @@ def test_pack_scales_shapes(mld, oracle, O, G, f16):
     ref = oracle.scale_layout(s, f16)
     assert np.array_equal(got.view(np.uint16 if f16 else np.uint32).reshape(-1),
                           ref.view(np.uint16 if f16 else np.uint32).reshape(-1))
+
+
+@pytest.mark.parametrize("shape", [(16, 1, 1, 4224), (500, 1, 1, 2064), (4112, 1, 1, 1040), (2040, 1, 1, 272), (48, 2, 1, 2064),
+                                   (1030, 1, 1, 128)])
+@pytest.mark.parametrize("bits", [8, 4])
+def test_pack_rows_sums(mld, oracle, shape, bits):
+    # blocks that cover all of a row, that share it (atomic sums) and that hold several groups of rows
+    O, H, W, I = shape
+    rng = np.random.default_rng(O + I)
+    lo, hi = (-128, 128) if bits == 8 else (-8, 8)
+    q = rng.integers(lo, hi, size=shape, dtype=np.int8)
+    ref = oracle.rearrange_int8_as_uint8(q) if bits == 8 else oracle.rearrange_int8_as_uint4(q)
+    for _ in range(2):
+        got, sums = mld.pack_weights(_dev(q), shape, bits, want_sum=True)
+        torch.cuda.synchronize()
+        assert np.array_equal(got.cpu().numpy(), ref)
+        assert np.array_equal(sums.cpu().numpy(), oracle.weights_sum_i(q))
