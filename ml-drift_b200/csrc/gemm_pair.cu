@@ -168,7 +168,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- MMA issuer
-    if (rank == 0 && lane == 0) {
+    // (the whole warp waits and one elected lane issues: see gemm_wtmem_kernel)
+    if (rank == 0) {
+      const auto wait_all = [](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_cluster(bar, parity)); };
       uint32_t idesc;
       if constexpr (I8)
         idesc = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(a.tile_n >> 3) << 17) | (16u << 24);
@@ -186,8 +188,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       for (; ok && work.next(sg); ++local) {
         const int acc = local & 1;
         const long long t0 = MLD_PAIR_CLOCK();
-        if (!wait_cluster(&tmem_empty[acc], (acc ? acc_phase1 : acc_phase0) ^ 1)) {
-          atomicExch(a.error, kErrPairBase + 2);
+        if (!wait_all(&tmem_empty[acc], (acc ? acc_phase1 : acc_phase0) ^ 1)) {
+          if (lane == 0) atomicExch(a.error, kErrPairBase + 2);
           ok = false;
           break;
         }
@@ -197,8 +199,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * 256);
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
           const long long t1 = MLD_PAIR_CLOCK();
-          if (!wait_cluster(&full_ab[stage], phase)) {
-            atomicExch(a.error, kErrPairBase + 3);
+          if (!wait_all(&full_ab[stage], phase)) {
+            if (lane == 0) atomicExch(a.error, kErrPairBase + 3);
             ok = false;
             break;
           }
@@ -206,21 +208,25 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           tc_after();
           const uint64_t da = make_desc(smem_u32(sA + (size_t)stage * kABytes));
           const uint64_t db = make_desc(smem_u32(sB + (size_t)stage * kBBytes));
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint64_t adv = static_cast<uint64_t>((k * 32) >> 4);  // 32 bytes of K per MMA inside the swizzle atom
-            umma_pair<I8>(tmem_d, da + adv, db + adv, idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t adv = static_cast<uint64_t>((k * 32) >> 4);  // 32 bytes of K per MMA inside the swizzle atom
+              umma_pair<I8>(tmem_d, da + adv, db + adv, idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
+            }
+            commit_pair(&empty[stage]);
           }
-          commit_pair(&empty[stage]);
+          __syncwarp();
           if (++stage == a.stages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) commit_pair(&tmem_full[acc]);
+        if (ok && elect_one()) commit_pair(&tmem_full[acc]);
+        __syncwarp();
       }
 #ifdef MLD_TRACE
-      if (a.trace != nullptr) {
+      if (a.trace != nullptr && lane == 0) {
         a.trace[blockIdx.x * 8 + 2] = tr_wait_acc;
         a.trace[blockIdx.x * 8 + 3] = tr_wait_ab;
         a.trace[blockIdx.x * 8 + 4] = MLD_PAIR_CLOCK() - tr_start;

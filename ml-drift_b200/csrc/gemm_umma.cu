@@ -465,8 +465,8 @@ __device__ __forceinline__ void transpose_sliced_tile(const __half* __restrict__
 
 __global__ void __launch_bounds__(256) transpose_x_kernel(const __half* __restrict__ x, int layout, int M, int K, int Kp,
                                                           __half* __restrict__ out) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // (after the wait: gemm_wtmem_kernel reads weights and scales as soon as it begins)
   const int Sp = Kp / 4;
   if (layout == MLD_LAYOUT_SLICED) {
     transpose_sliced_tile(x, M, K, Kp, out, blockIdx.x, blockIdx.y);

@@ -17,11 +17,13 @@
 // A cluster of two CTAs owns a tile of 256 output channels x tile_tok tokens (tile_tok <= 256).  Per CTA:
 //   warp 0       TMA producer of the activation tiles: this CTA's half of the tile's tokens, K-major rows of
 //                128 bytes in the 128-byte swizzle, eight stages
-//   warp 24      TMA producer of the packed weight boxes ([K/4] rows of 4x4 blocks) of this CTA's 128 channels
-//   warps 6..21  transform: two groups of eight warps on alternate stages; a thread owns one output channel
-//                (= one TMEM lane; a warp can only address the lane quarter 32 * (warp % 4)) and half of the
-//                stage's 64 input channels, dequantises them to 16 registers of two halves and stores them to
-//                the stage's 32 tensor-memory columns
+//   warp 24      TMA producer of the packed weight boxes ([K/4] rows of 4x4 blocks) of this CTA's 128 channels (a lone
+//                CTA: warp 22)
+//   warps 6..21  transform: four groups of four warps on every fourth stage; a thread owns one output channel
+//                (= one TMEM lane; a warp can only address the lane quarter 32 * (warp % 4)), dequantises the
+//                stage's 64 input channels to 32 registers of two halves and stores them to the stage's 32
+//                tensor-memory columns.  (Bound by the instructions that all warps issue: with eight warps to a
+//                stage, half the channels each, a third of them went into what a stage costs a warp anyway.)
 //   warps 22,23  forwarders: tell the pair's first CTA that this CTA's half of a stage is in place
 //   warp 1       tensor-memory owner; in the first CTA also the MMA issuer: four tcgen05.mma per stage (K = 16
 //                each, A = 8 TMEM columns, B = 32 bytes further into the swizzled rows)
@@ -29,13 +31,14 @@
 //                adds the bias, and four neighbouring lanes exchange values so that each holds the four channels
 //                of one output slice for two tokens, a 16-byte piece of the sliced output layout
 // Tensor memory: columns 0..255 accumulators (one buffer: reading a tile's accumulators is not overlapped with
-// the next tile's MMAs, so the transform warps, idle meanwhile, share the reading with the epilogue warps),
-// columns 256..511 the weight ring (8 stages x 32 columns).
+// the next tile's MMAs, so the transform warps, idle meanwhile, share the reading with the epilogue warps; a CTA that works
+// alone has two buffers of 128), columns 256..511 the weight ring (8 stages x 32 columns).
 // The split of the work over the pairs (tiles of the last wave shared along K) is gemm_pair_kernel's.
 // Every wait is bounded.
 #include <cuda_fp16.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "pair_common.cuh"
@@ -47,7 +50,10 @@ constexpr int kWtStages = 8;          // operand ring: activation tile in shared
 constexpr int kWtRows = 128;          // output channels per CTA
 constexpr int kWtTokBytes = 128 * kKBytes;  // up to 128 token rows per CTA and stage
 constexpr uint32_t kWtACol = 256;     // first TMEM column of the weight ring
+constexpr int kWtAccCols = 128;       // columns of each of a lone CTA's two sets of accumulators
 constexpr int kErrWtBase = 50;
+constexpr int kXfWarps = 4;            // transform warps that share a stage, one per quarter of the channels
+constexpr int kScaleAhead = 16;       // stages by which L2 is asked for the scales ahead of their use
 constexpr int kDrainParts = 5;        // warps that read one lane quarter's accumulators: one epilogue + four transform
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -114,6 +120,13 @@ __device__ __forceinline__ void tmem_dealloc_all(uint32_t taddr) {
   }
 }
 
+// (1024 + u) - (1024 + zero) is exact, so the dequantised weight is rounded once.  (The WeightsConverter rounds u s, zero s
+// and their difference, which is further from (u - zero) s and an instruction more.)
+__device__ __forceinline__ uint32_t dq_once(uint32_t biased, __half2 offset, __half2 s2) {
+  const __half2 r = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&biased), offset), s2);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
 struct WtArgs {
   PairArgs p;       // M, N, N4, k_blocks, scales, bias, y, dst_layout, error, outs, split, work list, w ring
   int tile_tok;     // tokens per tile (UMMA N), a multiple of 16
@@ -127,8 +140,10 @@ struct WtArgs {
 // pair's rate of stages), at the price of every CTA fetching all of the tile's tokens.  Bound by the MMAs: a stage's four
 // take about 740 cycles whatever the number of tokens, on one accumulator or several, from one issuing thread or two.
 // 77 tokens, 4096 x 11008 INT4: 41.1 us a call with pairs and whole tiles, 31.9 with lone CTAs and tiles cut along K.
+template <bool PAIR>
+constexpr int kWtThreads = PAIR ? kPairThreads : kPairThreads - 64;  // (a lone CTA has no forwarders: more registers a thread)
 template <int MODE, bool PAIR>
-__global__ void __launch_bounds__(kPairThreads, 1)
+__global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
     gemm_wtmem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, WtArgs wa) {
   const PairArgs& a = wa.p;
   constexpr int BLK = MODE == kModeInt4F16 ? 8 : 16;   // bytes of a packed 4x4 block
@@ -145,9 +160,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   uint64_t* w_empty = full_w + a.w_stages;            // [w_stages]: the transform warps have read the box
   uint64_t* full_ab = w_empty + a.w_stages;           // [stages], first CTA: tokens of both CTAs landed, weights of both in TMEM
   uint64_t* empty = full_ab + kWtStages;              // [stages]: the stage's MMAs have completed (arrives in both CTAs)
-  uint64_t* tmem_full = empty + kWtStages;            // [1], arrives in both CTAs
-  uint64_t* tmem_empty = tmem_full + 1;               // [1], first CTA: the epilogue warps of both CTAs have drained it
-  uint64_t* xf_done = tmem_empty + 1;                 // [stages]: this CTA's transform warps have stored their half
+  uint64_t* tmem_full = empty + kWtStages;            // [2] (accumulators; a pair has one), arrives in both CTAs
+  uint64_t* tmem_empty = tmem_full + 2;               // [2], first CTA: the warps that read it (of both CTAs) are done
+  uint64_t* xf_done = tmem_empty + 2;                 // [stages]: this CTA's transform warps have stored their half
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xf_done + kWtStages);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -169,16 +184,18 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.w_stages; ++s) {
       mbar_init(&full_w[s], 1);
-      mbar_init(&w_empty[s], kTransformWarps);
+      mbar_init(&w_empty[s], kXfWarps);
     }
     for (int s = 0; s < kWtStages; ++s) {
       // the producer's expect_tx, + one arrival per CTA for its weights (a lone CTA's transform warps arrive themselves)
-      mbar_init(&full_ab[s], PAIR ? 1 + 2 : 1 + kTransformWarps);
+      mbar_init(&full_ab[s], PAIR ? 1 + 2 : 1 + kXfWarps);
       mbar_init(&empty[s], 1);
-      mbar_init(&xf_done[s], kTransformWarps);
+      mbar_init(&xf_done[s], kXfWarps);
     }
-    mbar_init(tmem_full, 1);
-    mbar_init(tmem_empty, CTAS * 4 * kDrainParts);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tmem_full[b], 1);
+      mbar_init(&tmem_empty[b], PAIR ? CTAS * 4 * kDrainParts : 4);
+    }
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc_all<PAIR>(tmem_slot);
@@ -186,41 +203,45 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();  // the partner's barriers are initialised before anything arrives on them
   tc_after();
-  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t full_ab_lead = PAIR ? map_shared(smem_u32(full_ab), 0) : 0u;
   const uint32_t tmem_empty_lead = PAIR ? map_shared(smem_u32(tmem_empty), 0) : 0u;
-  auto release_tmem = [&]() {
+  auto release_tmem = [&](int part, int acc) {
     if constexpr (PAIR)
       arrive_remote(tmem_empty_lead);
-    else
-      mbar_arrive(tmem_empty);
+    else if (part == 0)
+      mbar_arrive(&tmem_empty[acc]);
   };
   // tile -> (token tile, channel tile): the token tiles of one channel tile follow each other
   auto tile_tok0 = [&](int tile) { return (tile % a.m_tiles) * wa.tile_tok; };
   auto tile_n0 = [&](int tile) { return (tile / a.m_tiles) * CTAS * kWtRows; };
 
-  // Accumulators -> outputs, the share `part` of kDrainParts of the warps that can address this lane quarter
-  // (one epilogue warp and the quarter's four transform warps, which have nothing to transform while the only
-  // accumulator buffer is being read): pieces of 16 token columns, part, part + kDrainParts, ...  A tile cut
-  // along K: a pair whose share does not begin with the tile's first k-block (always the first of its segments, so that
-  // nothing it waits for comes before) leaves its raw accumulators in its own workspace slot; the pair that has the
-  // first k-block adds the following pairs' slots to its own accumulators, in order, and writes the outputs.  Blocks begin
-  // in the order of their numbers, so those pairs hold SMs already, whatever else is on the GPU.
-  auto drain = [&](const Segment& sg, int part) -> bool {
+  // Accumulators -> outputs, the share `part` of `parts` of the warps that can address this lane quarter: pieces of 16 token
+  // columns, part, part + parts, ...  A pair has one set of accumulators, so the quarter's four transform warps, which have
+  // nothing to transform while it is being read, share the reading with its epilogue warp (five parts).  A lone CTA has two:
+  // the epilogue warp reads while the next tile's MMAs run, and the transform warps join in for the last.
+  // A tile cut along K: a pair (CTA) whose share does not begin with the tile's first k-block (always the first of its
+  // segments, so that nothing it waits for comes before) leaves its raw accumulators in its own workspace slot; the one that
+  // has the first k-block adds the following slots to its own accumulators, in order, and writes the outputs.  Blocks begin
+  // in the order of their numbers, so those it waits for hold SMs already, whatever else is on the GPU.  A slot has a flag
+  // per lane quarter and part (lone CTAs, whose writer and reader may be shared differently: per quarter and piece).
+  auto drain = [&](const Segment& sg, int part, int parts, int acc) -> bool {
     const int quad = warp & 3;  // TMEM lanes 32*quad .. 32*quad+31 belong to this warp
     const bool hands_over = sg.kb0 > 0, takes_over = !hands_over && sg.kb1 < a.k_blocks;
     const auto rows_of = [&](int slot) {
       return reinterpret_cast<uint4*>(a.split_ws) + ((size_t)(slot * CTAS + static_cast<int>(rank)) * 4 + quad) * (8 * 8 * 32) + lane;
     };
-    const auto flag_of = [&](int slot) { return a.split_flags + ((slot * CTAS + static_cast<int>(rank)) * 4 + quad) * 8 + part; };
+    const auto flag_of = [&](int slot, int i) {  // the i-th flag that this warp's share has
+      return a.split_flags + ((slot * CTAS + static_cast<int>(rank)) * 4 + quad) * 8 + (PAIR ? part : part + i * parts);
+    };
     // the pairs that hold the rest of a tile this pair completes
     const int others = takes_over ? ((sg.tile + 1) * a.k_blocks - 1) / a.units_per_pair - pair : 0;
-    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(PAIR ? 0 : acc * kWtAccCols);
     const int n_pieces = wa.tile_tok >> 4;
+    const int n_flags = PAIR ? 1 : part < n_pieces ? (n_pieces - part + parts - 1) / parts : 0;
     if (hands_over) {
       uint4* const slot_rows = rows_of(pair);
-      for (int pc = part; pc < n_pieces; pc += kDrainParts) {
+      for (int pc = part; pc < n_pieces; pc += parts) {
         uint32_t r[16];
         tmem_ld16(lane_base + static_cast<uint32_t>(16 * pc), r);
         tmem_ld_wait();
@@ -230,16 +251,14 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       __threadfence();
       tc_before();
       __syncwarp();
-      if (lane == 0) {
-        st_release_gpu(flag_of(pair), a.epoch);
-        release_tmem();
-      }
+      if (lane < n_flags) st_release_gpu(flag_of(pair, lane), a.epoch);
+      if (lane == 0) release_tmem(part, acc);
       return true;
     }
     if (takes_over) {
       bool seen = true;
-      for (int o = lane; o < others; o += 32) {  // a lane per slot
-        const uint32_t* flag = flag_of(pair + 1 + o);
+      for (int i = lane; i < others * n_flags; i += 32) {  // a lane per flag
+        const uint32_t* flag = flag_of(pair + 1 + i / n_flags, i % n_flags);
         const unsigned long long t0 = globaltimer_ns();
         uint32_t v;
         while ((v = ld_acquire_gpu(flag)) != a.epoch && globaltimer_ns() - t0 <= kWaitLimitNs) __nanosleep(32);
@@ -250,7 +269,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         return false;
       }
       // each flag has this one reader, which takes it back: a replayed graph launches with the same epoch again
-      for (int o = lane; o < others; o += 32) __stcg(flag_of(pair + 1 + o), 0u);
+      for (int i = lane; i < others * n_flags; i += 32) __stcg(flag_of(pair + 1 + i / n_flags, i % n_flags), 0u);
     }
     const int n = tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows + quad * 32 + lane;  // output channel
     const int m_first = (sg.tile % a.m_tiles) * wa.tile_tok;
@@ -258,7 +277,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     __half bias_h = __float2half_rn(0.0f);
     if (a.bias != nullptr && has_n) bias_h = static_cast<const __half*>(a.bias)[n];
     const int q = lane & 3;  // place among the four channels of the output slice n >> 2
-    for (int pc = part; pc < n_pieces; pc += kDrainParts) {
+    for (int pc = part; pc < n_pieces; pc += parts) {
       const int c0 = 16 * pc;
       uint32_t r[16];
       tmem_ld16(lane_base + static_cast<uint32_t>(c0), r);
@@ -348,63 +367,73 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
     tc_before();
     __syncwarp();
-    if (lane == 0) release_tmem();
+    if (lane == 0) release_tmem(part, acc);
     return true;
   };
 
   if (warp == 0) {
     // ------------------------------------------------ producer of the activation tiles
-    if (lane == 0) {
-      prefetch_tmap(&tmap_x);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      WorkList work = work0;
-      Segment sg;
-      while (ok && work.next(sg)) {
-        const int m0 = tile_tok0(sg.tile) + static_cast<int>(rank) * cta_tok;
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1)) {
-            atomicExch(a.error, kErrWtBase + 1);
-            ok = false;
-            break;
-          }
+    if (lane == 0) prefetch_tmap(&tmap_x);
+    // Everything else that this kernel reads was complete when the transposition ahead of it let it begin.
+    pdl_wait();
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    WorkList work = work0;
+    Segment sg;
+    while (ok && work.next(sg)) {
+      const int m0 = tile_tok0(sg.tile) + static_cast<int>(rank) * cta_tok;
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1))) {
+          if (lane == 0) atomicExch(a.error, kErrWtBase + 1);
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&full_ab[stage], static_cast<uint32_t>(wa.tile_tok) * kKBytes);
           if constexpr (PAIR)
             tma_load_2d_pair(sX + (size_t)stage * kWtTokBytes, &tmap_x, full_ab_lead + stage * 8, kb * 64, m0);
           else
             tma_load_2d(sX + (size_t)stage * kWtTokBytes, &tmap_x, &full_ab[stage], kb * 64, m0);
-          if (++stage == kWtStages) {
-            stage = 0;
-            phase ^= 1;
-          }
+        }
+        __syncwarp();
+        if (++stage == kWtStages) {
+          stage = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------- MMA issuer
-    if (rank == 0 && lane == 0) {
+    // The whole warp goes through the waits and one elected lane issues, so that the instructions' operands are uniform
+    // for the compiler: with a single lane in the loop a stage took 512 cycles of issuing alone, whatever the tile.
+    if (rank == 0) {
       const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(wa.tile_tok >> 3) << 17) | ((PAIR ? 16u : 8u) << 24);
       int stage = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      uint32_t phase = 0;
       bool ok = true;
+      const auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+        return __all_sync(0xffffffffu, PAIR ? wait_cluster(bar, parity) : mbar_wait(bar, parity));
+      };
       WorkList work = work0;
       Segment sg;
       [[maybe_unused]] long long tr_acc = 0, tr_ab = 0;
       [[maybe_unused]] const long long tr_start = MLD_PAIR_CLOCK();
-      while (ok && work.next(sg)) {
+      for (int nth = 0; ok && work.next(sg); ++nth) {
+        const int acc = PAIR ? 0 : nth & 1;
+        const uint32_t acc_phase = static_cast<uint32_t>(PAIR ? nth : nth >> 1) & 1u;
+        const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * kWtAccCols);
         [[maybe_unused]] const long long t0 = MLD_PAIR_CLOCK();
-        if (!wait_cluster(tmem_empty, acc_phase ^ 1)) {
-          atomicExch(a.error, kErrWtBase + 2);
+        if (!wait_all(&tmem_empty[acc], acc_phase ^ 1)) {
+          if (lane == 0) atomicExch(a.error, kErrWtBase + 2);
           break;
         }
         tr_acc += MLD_PAIR_CLOCK() - t0;
-        acc_phase ^= 1;
         tc_after();
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
           [[maybe_unused]] const long long t1 = MLD_PAIR_CLOCK();
-          if (!wait_cluster(&full_ab[stage], phase)) {
-            atomicExch(a.error, kErrWtBase + 3);
+          if (!wait_all(&full_ab[stage], phase)) {
+            if (lane == 0) atomicExch(a.error, kErrWtBase + 3);
             ok = false;
             break;
           }
@@ -412,20 +441,24 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           tc_after();
           const uint64_t db = make_desc(smem_u32(sX + (size_t)stage * kWtTokBytes));
           const uint32_t ta = tmem_base + kWtACol + static_cast<uint32_t>(stage * 32);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_ts<PAIR>(tmem_base, ta + 8u * k, db + static_cast<uint64_t>((k * 32) >> 4), idesc,
-                          (kb > sg.kb0 || k > 0) ? 1u : 0u);
-          commit<PAIR>(&empty[stage]);
+            for (int k = 0; k < 4; ++k)
+              umma_ts<PAIR>(tmem_d, ta + 8u * k, db + static_cast<uint64_t>((k * 32) >> 4), idesc,
+                            (kb > sg.kb0 || k > 0) ? 1u : 0u);
+            commit<PAIR>(&empty[stage]);
+          }
+          __syncwarp();
           if (++stage == kWtStages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) commit<PAIR>(tmem_full);
+        if (ok && elect_one()) commit<PAIR>(&tmem_full[acc]);
+        __syncwarp();
       }
 #ifdef MLD_TRACE
-      if (wa.trace != nullptr) {
+      if (wa.trace != nullptr && lane == 0) {
         wa.trace[blockIdx.x * 8 + 2] = tr_acc;
         wa.trace[blockIdx.x * 8 + 3] = tr_ab;
         wa.trace[blockIdx.x * 8 + 4] = MLD_PAIR_CLOCK() - tr_start;
@@ -434,42 +467,42 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
   } else if (warp < 6) {
     // --------------------------------------------------------------------- epilogue
-    uint32_t acc_phase = 0;
     WorkList work = work0;
     Segment sg;
-    while (work.next(sg)) {
-      if (!mbar_wait(tmem_full, acc_phase)) {
+    for (int nth = 0; work.next(sg); ++nth) {
+      const int acc = PAIR ? 0 : nth & 1;
+      if (!mbar_wait(&tmem_full[acc], static_cast<uint32_t>(PAIR ? nth : nth >> 1) & 1u)) {
         atomicExch(a.error, kErrWtBase + 4);
         break;
       }
-      acc_phase ^= 1;
       tc_after();
-      if (!drain(sg, 0)) break;
+      if (!drain(sg, 0, PAIR || work.done() ? kDrainParts : 1, acc)) break;
     }
     if (a.outs.world > 1) __threadfence_system();  // the peer stores are performed before the kernel ends
-  } else if (warp == 24) {
+  } else if (warp == (PAIR ? 24 : 22)) {
     // ------------------------------------------------- producer of the packed weight boxes
-    if (lane == 0) {
-      prefetch_tmap(&tmap_w);
-      int ws = 0;
-      uint32_t wphase = 0;
-      bool ok = true;
-      WorkList work = work0;
-      Segment sg;
-      while (ok && work.next(sg)) {
-        const int nb0 = (tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows) / 4 * BLK;  // byte column of the box
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          if (!mbar_wait(&w_empty[ws], wphase ^ 1)) {
-            atomicExch(a.error, kErrWtBase + 7);
-            ok = false;
-            break;
-          }
+    if (lane == 0) prefetch_tmap(&tmap_w);
+    int ws = 0;
+    uint32_t wphase = 0;
+    bool ok = true;
+    WorkList work = work0;
+    Segment sg;
+    while (ok && work.next(sg)) {
+      const int nb0 = (tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows) / 4 * BLK;  // byte column of the box
+      for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&w_empty[ws], wphase ^ 1))) {
+          if (lane == 0) atomicExch(a.error, kErrWtBase + 7);
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           mbar_arrive_expect_tx(&full_w[ws], static_cast<uint32_t>(w_stage));
           tma_load_2d(sW + (size_t)ws * w_stage, &tmap_w, &full_w[ws], nb0 / 4, kb * SLICES);  // 32-bit elements
-          if (++ws == a.w_stages) {
-            ws = 0;
-            wphase ^= 1;
-          }
+        }
+        __syncwarp();
+        if (++ws == a.w_stages) {
+          ws = 0;
+          wphase ^= 1;
         }
       }
     }
@@ -500,127 +533,136 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
   } else {
     // -------------------------------------------------------------------- transform
-    const int group = (warp - 6) >> 3;            // this group takes the iterations of its parity
-    const int half = ((warp - 6) & 7) >> 2;       // which 32 of the stage's 64 input channels
+    const int group = (warp - 6) >> 2;            // this group of four warps takes every fourth stage
     const int quad = warp & 3;                     // the TMEM lane quarter this warp can address
     const int row = quad * 32 + lane;              // output channel of the CTA's 128 = TMEM lane
     const int col4 = row & 3;                      // column of the row inside its 4x4 blocks
     const uint32_t sel8 = static_cast<uint32_t>(col4) | (static_cast<uint32_t>(4 + col4) << 8);
-    int stage = 0, ws = 0;
-    uint32_t phase = 0, wphase = 0;
-    auto advance = [&](int n) {
-      for (int i = 0; i < n; ++i) {
-        if (++stage == kWtStages) {
-          stage = 0;
-          phase ^= 1;
-        }
-        if (++ws == a.w_stages) {
-          ws = 0;
-          wphase ^= 1;
-        }
-      }
-    };
+    const __half2 offset = __float2half2_rn(MODE == kModeInt4F16 ? 1032.0f : 1152.0f);  // 1024 + the value of a zero
+    const int w_shift = __ffs(a.w_stages) - 1;
     bool ok = true;
-    int xf_iter = 0;
-    uint32_t acc_phase = 0;
+    int xf_iter = 0;  // stages before the segment
+    // A stage's stores are waited for and announced when the next stage's box has been asked for, so that the two trips
+    // overlap.
+    int stored = -1;
+    const auto announce = [&]() {
+      if (stored < 0) return;
+      tmem_st_wait();
+      tc_before();
+      __syncwarp();
+      if (lane == 0) {
+        if constexpr (PAIR)
+          mbar_arrive(&xf_done[stored]);  // local; a forwarder passes it on to the pair's first CTA
+        else
+          mbar_arrive(&full_ab[stored]);
+      }
+      stored = -1;
+    };
     WorkList work = work0;
     Segment sg;
     [[maybe_unused]] long long tr_wait = 0, tr_work = 0, tr_st = 0;
     [[maybe_unused]] const long long tr_start = MLD_PAIR_CLOCK();
-    while (ok && work.next(sg)) {
+    for (int nth = 0; ok && work.next(sg); ++nth) {
       const int n = tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows + row;
-      const bool has_n = n < a.N4;
-      // this thread's 32 input channels of a stage are one scale group whenever groups are whole multiples of 32
-      // inputs, the usual case: one load per stage then, issued a stage ahead
-      const bool one_group = a.scale_mode != MLD_SCALE_BLOCK || (a.group_slices & 7) == 0;
-      auto scale_at = [&](int slice) -> __half {
-        if (!has_n) return __float2half_rn(0.0f);
-        if (a.scale == nullptr) return __float2half_rn(a.scalar_scale);
-        int g = a.scale_mode != MLD_SCALE_BLOCK ? 0 : (a.gs_shift >= 0 ? slice >> a.gs_shift : slice / a.group_slices);
+      const bool scaled = n < a.N4 && a.scale != nullptr, blocks = a.scale_mode == MLD_SCALE_BLOCK;
+      // 32 input channels are one scale group whenever groups are whole multiples of 32 inputs, the usual case: two loads
+      // a stage then, issued when the group's stage before is begun
+      const bool one_group = !blocks || (a.group_slices & 7) == 0;
+      const __half fixed_scale = __float2half_rn(n < a.N4 ? a.scalar_scale : 0.0f);
+      const auto scale_ptr = [&](int slice) {
+        int g = !blocks ? 0 : (a.gs_shift >= 0 ? slice >> a.gs_shift : slice / a.group_slices);
         if (g >= a.G) g = a.G - 1;
-        return __ldg(a.scale + (size_t)g * a.N4 + n);
+        return a.scale + (size_t)g * a.N4 + n;
       };
-      int kb = sg.kb0 + ((xf_iter ^ group) & 1);
-      if (kb != sg.kb0) advance(1);  // skip the other group's stage
-      __half sc_next = __float2half_rn(0.0f);
-      if (kb < sg.kb1) sc_next = scale_at(kb * SLICES + 8 * half);
-      for (; kb < sg.kb1; kb += 2) {
-        const __half sc_cur = sc_next;
-        if (kb + 2 < sg.kb1) sc_next = scale_at((kb + 2) * SLICES + 8 * half);
-        // the packed box has landed, and the stage's tensor-memory columns are free again (their MMAs completed)
+      const auto scale_at = [&](int slice) -> __half { return scaled ? __ldg(scale_ptr(slice)) : fixed_scale; };
+      // (a stage takes less time than a trip to HBM: without this the loop waits for the scales)
+      const auto prefetch_scales = [&](int kb) {
+        if (scaled && blocks && kb < sg.kb1) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(scale_ptr(kb * SLICES)));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(scale_ptr(kb * SLICES + 8)));
+        }
+      };
+      int kb = sg.kb0 + ((group - xf_iter) & 3);
+      for (int ahead = 4; ahead < kScaleAhead; ahead += 4) prefetch_scales(kb + ahead);
+      __half next0 = fixed_scale, next1 = fixed_scale;
+      if (kb < sg.kb1) {
+        next0 = scale_at(kb * SLICES);
+        next1 = scale_at(kb * SLICES + 8);
+      }
+      for (; kb < sg.kb1; kb += 4) {
+        const int iter = xf_iter + kb - sg.kb0, stage = iter & (kWtStages - 1), ws = iter & (a.w_stages - 1);
+        const __half cur[2] = {next0, next1};
+        if (kb + 4 < sg.kb1) {
+          next0 = scale_at((kb + 4) * SLICES);
+          next1 = scale_at((kb + 4) * SLICES + 8);
+        }
+        prefetch_scales(kb + kScaleAhead);
+        // the packed box has landed (and, below, the stage's tensor-memory columns are free again: their MMAs completed)
         [[maybe_unused]] const long long t0 = MLD_PAIR_CLOCK();
-        if (!mbar_wait(&full_w[ws], wphase) || !mbar_wait(&empty[stage], phase ^ 1)) {
+        if (!mbar_wait(&full_w[ws], static_cast<uint32_t>(iter >> w_shift) & 1u)) {
           atomicExch(a.error, kErrWtBase + 5);
           ok = false;
           break;
         }
         [[maybe_unused]] const long long t1 = MLD_PAIR_CLOCK();
         tr_wait += t1 - t0;
-        tc_after();
         const uint8_t* wp = sW + (size_t)ws * w_stage + (row >> 2) * BLK;
-        const __half shift = __ushort2half_rn(static_cast<unsigned short>(MODE == kModeInt4F16 ? 8 : 128));
-        uint32_t o[16];  // o[j] = input channels 32 half + 2j, 2j + 1 of the stage
-        if constexpr (MODE == kModeInt4F16) {
-          uint2 blk[8];
+        const uint32_t columns = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kWtACol + static_cast<uint32_t>(stage * 32);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) blk[i] = *reinterpret_cast<const uint2*>(wp + (size_t)(8 * half + i) * w_pitch);
+        for (int half = 0; half < 2; ++half) {
+          using Block = typename std::conditional<MODE == kModeInt4F16, uint2, uint4>::type;
+          Block blk[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) blk[i] = *reinterpret_cast<const Block*>(wp + (size_t)(8 * half + i) * w_pitch);
+          if (half == 0) {
+            announce();
+            if (!mbar_wait(&empty[stage], (static_cast<uint32_t>(iter / kWtStages) & 1u) ^ 1u)) {
+              atomicExch(a.error, kErrWtBase + 5);
+              ok = false;
+              break;
+            }
+            tc_after();
+          }
+          uint32_t o[16];  // o[j] = input channels 32 half + 2j, 2j + 1 of the stage
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const __half scc = one_group ? sc_cur : scale_at(kb * SLICES + 2 * (4 * half + c));
-            const __half2 s2 = __half2half2(scc);
-            const __half2 b2 = __half2half2(__hmul(__hneg(scc), shift));
+            const __half2 s2 = __half2half2(one_group ? cur[half] : scale_at(kb * SLICES + 2 * (4 * half + c)));
 #pragma unroll
             for (int qq = 0; qq < 2; ++qq) {
-              // nibble (k % 4) * 4 + col4: k0, k1 in the halves of .x, k2, k3 in those of .y
-              o[4 * c + 2 * qq] = dq2(((blk[2 * c + qq].x >> (4 * col4)) & 0x000F000Fu) | 0x64006400u, s2, b2);
-              o[4 * c + 2 * qq + 1] = dq2(((blk[2 * c + qq].y >> (4 * col4)) & 0x000F000Fu) | 0x64006400u, s2, b2);
+              const Block v = blk[2 * c + qq];
+              if constexpr (MODE == kModeInt4F16) {
+                // nibble (k % 4) * 4 + col4: k0, k1 in the halves of .x, k2, k3 in those of .y
+                o[4 * c + 2 * qq] = dq_once(((v.x >> (4 * col4)) & 0x000F000Fu) | 0x64006400u, offset, s2);
+                o[4 * c + 2 * qq + 1] = dq_once(((v.y >> (4 * col4)) & 0x000F000Fu) | 0x64006400u, offset, s2);
+              } else {
+                o[4 * c + 2 * qq] = dq_once((__byte_perm(v.x, v.y, sel8) & 0x00FF00FFu) | 0x64006400u, offset, s2);
+                o[4 * c + 2 * qq + 1] = dq_once((__byte_perm(v.z, v.w, sel8) & 0x00FF00FFu) | 0x64006400u, offset, s2);
+              }
             }
           }
-        } else {
-          uint4 blk[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) blk[i] = *reinterpret_cast<const uint4*>(wp + (size_t)(8 * half + i) * w_pitch);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const __half scc = one_group ? sc_cur : scale_at(kb * SLICES + 2 * (4 * half + c));
-            const __half2 s2 = __half2half2(scc);
-            const __half2 b2 = __half2half2(__hmul(__hneg(scc), shift));
-#pragma unroll
-            for (int qq = 0; qq < 2; ++qq) {
-              const uint4 v = blk[2 * c + qq];
-              o[4 * c + 2 * qq] = dq2((__byte_perm(v.x, v.y, sel8) & 0x00FF00FFu) | 0x64006400u, s2, b2);
-              o[4 * c + 2 * qq + 1] = dq2((__byte_perm(v.z, v.w, sel8) & 0x00FF00FFu) | 0x64006400u, s2, b2);
-            }
-          }
+          tmem_st16(columns + static_cast<uint32_t>(16 * half), o);
         }
+        if (!ok) break;
         [[maybe_unused]] const long long t2 = MLD_PAIR_CLOCK();
         tr_work += t2 - t1;
-        tmem_st16(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kWtACol + static_cast<uint32_t>(stage * 32 + 16 * half), o);
-        tmem_st_wait();
-        tr_st += MLD_PAIR_CLOCK() - t2;
-        tc_before();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&w_empty[ws]);     // the box may be overwritten
-          if constexpr (PAIR)
-            mbar_arrive(&xf_done[stage]);  // local; a forwarder passes it on to the pair's first CTA
-          else
-            mbar_arrive(&full_ab[stage]);
-        }
-        advance(kb + 1 < sg.kb1 ? 2 : 1);
+        if (lane == 0) mbar_arrive(&w_empty[ws]);  // the box may be overwritten
+        stored = stage;
       }
+      announce();
       xf_iter += sg.kb1 - sg.kb0;
       if (!ok) break;
-      // This segment's accumulators: the transform warps share the reading with the epilogue warp of their
+      // A pair's segment, a lone CTA's last: the transform warps share the reading with the epilogue warp of their
       // quarter.  (Measured: reading them only when the ring is full and the next stage blocked, so that the next
       // tile's first stages are transformed beforehand, costs more in polling than the refill costs here.)
-      if (!mbar_wait(tmem_full, acc_phase)) {
+      if (!PAIR && !work.done()) continue;
+      const int acc = PAIR ? 0 : nth & 1;
+      if (!mbar_wait(&tmem_full[acc], static_cast<uint32_t>(PAIR ? nth : nth >> 1) & 1u)) {
         atomicExch(a.error, kErrWtBase + 9);
         break;
       }
-      acc_phase ^= 1;
       tc_after();
-      if (!drain(sg, 1 + group * 2 + half)) break;
+      if (!drain(sg, 1 + group, kDrainParts, acc)) break;
     }
 #ifdef MLD_TRACE
     if (wa.trace != nullptr && warp == 6 && lane == 0) {
@@ -696,10 +738,9 @@ WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share
   }
   const int blk = mode == kModeInt4F16 ? 8 : 16;
   const int w_stage = 16 * (kWtRows / 4) * blk;
-  const int fixed = 1024 + (2 * 24 + 3 * kWtStages + 2) * 8 + 64;
+  const int fixed = 1024 + (2 * 24 + 3 * kWtStages + 4) * 8 + 64;
   int ws = (226 * 1024 - fixed - kWtStages * kWtTokBytes) / w_stage;
-  if (ws > 16) ws = 16;
-  g.w_stages = ws;
+  g.w_stages = ws >= 16 ? 16 : 8;  // (a power of two; shared memory has room for twelve of the larger)
   g.smem_bytes = (size_t)kWtStages * kWtTokBytes + (size_t)ws * w_stage + fixed;
   return g;
 }
@@ -776,7 +817,7 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.grid, 1, 1);
-  cfg.blockDim = dim3(kPairThreads, 1, 1);
+  cfg.blockDim = dim3(g.ctas == 2 ? kWtThreads<true> : kWtThreads<false>, 1, 1);
   cfg.dynamicSmemBytes = g.smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];

@@ -204,6 +204,7 @@ struct WorkList {
     }
     return false;
   }
+  __device__ __forceinline__ bool done() const { return u >= u_end && tile >= tile_end; }
   __device__ __forceinline__ int stages_in_all() const {
     return (u_end - u) + (tile < tile_end ? (tile_end - tile + tile_step - 1) / tile_step : 0) * k_blocks;
   }
