@@ -17,14 +17,12 @@
 // A cluster of two CTAs owns a tile of 256 output channels x tile_tok tokens (tile_tok <= 256).  Per CTA:
 //   warp 0       TMA producer of the activation tiles: this CTA's half of the tile's tokens, K-major rows of
 //                128 bytes in the 128-byte swizzle, eight stages
-//   warp 24      TMA producer of the packed weight boxes ([K/4] rows of 4x4 blocks) of this CTA's 128 channels (a lone
-//                CTA: warp 22)
+//   warp 22      TMA producer of the packed weight boxes ([K/4] rows of 4x4 blocks) of this CTA's 128 channels
 //   warps 6..21  transform: four groups of four warps on every fourth stage; a thread owns one output channel
 //                (= one TMEM lane; a warp can only address the lane quarter 32 * (warp % 4)), dequantises the
 //                stage's 64 input channels to 32 registers of two halves and stores them to the stage's 32
 //                tensor-memory columns.  (Bound by the instructions that all warps issue: with eight warps to a
 //                stage, half the channels each, a third of them went into what a stage costs a warp anyway.)
-//   warps 22,23  forwarders: tell the pair's first CTA that this CTA's half of a stage is in place
 //   warp 1       tensor-memory owner; in the first CTA also the MMA issuer: four tcgen05.mma per stage (K = 16
 //                each, A = 8 TMEM columns, B = 32 bytes further into the swizzled rows)
 //   warps 2..5   epilogue: a thread reads its output channel's accumulators (one TMEM lane, a column per token),
@@ -92,6 +90,11 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
         : "memory");
   }
 }
+// Arrives on a barrier of the pair's first CTA.  What it orders is tensor memory, by tcgen05.wait and
+// fence::before_thread_sync ahead of it; releasing at cluster scope on top of that would take about 800 cycles.
+__device__ __forceinline__ void arrive_in_pair(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 // Arrives on the barrier (in both CTAs of a pair) once every MMA issued so far has completed.
 template <bool PAIR>
 __device__ __forceinline__ void commit(uint64_t* bar) {
@@ -136,14 +139,15 @@ struct WtArgs {
 };
 
 // PAIR: the two-CTA form described above.  Otherwise a CTA works alone on tiles of 128 output channels x up to 128
-// tokens: no transformed stage has to be announced to another SM (a remote arrival takes about 800 cycles, which bounds a
-// pair's rate of stages), at the price of every CTA fetching all of the tile's tokens.  Bound by the MMAs: a stage's four
-// take about 740 cycles whatever the number of tokens, on one accumulator or several, from one issuing thread or two.
-// 77 tokens, 4096 x 11008 INT4: 41.1 us a call with pairs and whole tiles, 31.9 with lone CTAs and tiles cut along K.
-template <bool PAIR>
-constexpr int kWtThreads = PAIR ? kPairThreads : kPairThreads - 64;  // (a lone CTA has no forwarders: more registers a thread)
+// tokens: twice as many, smaller tiles, at the price of every CTA fetching all of the tile's tokens.
+// Bound by the transformation (64 x 128 weights a stage and CTA at five instructions for two) beside whatever else the warps
+// issue: a pair's stage takes about 700 cycles, 512 of them its MMAs; a lone CTA's MMAs need 160 to 260.
+// 4096 x 11008 INT4, in a graph: 77 tokens 23.2 us (30.5 with eight warps to a stage and one set of accumulators, 41.1 with
+// pairs and whole tiles); 256 tokens 34.0, 512 48.3 (42.9, 66.7 with stages announced to the pair's first CTA by warps of
+// their own, whose release at cluster scope took longer than a stage).
+constexpr int kWtThreads = 23 * 32;
 template <int MODE, bool PAIR>
-__global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
+__global__ void __launch_bounds__(kWtThreads, 1)
     gemm_wtmem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, WtArgs wa) {
   const PairArgs& a = wa.p;
   constexpr int BLK = MODE == kModeInt4F16 ? 8 : 16;   // bytes of a packed 4x4 block
@@ -162,8 +166,7 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
   uint64_t* empty = full_ab + kWtStages;              // [stages]: the stage's MMAs have completed (arrives in both CTAs)
   uint64_t* tmem_full = empty + kWtStages;            // [2] (accumulators; a pair has one), arrives in both CTAs
   uint64_t* tmem_empty = tmem_full + 2;               // [2], first CTA: the warps that read it (of both CTAs) are done
-  uint64_t* xf_done = tmem_empty + 2;                 // [stages]: this CTA's transform warps have stored their half
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xf_done + kWtStages);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
@@ -187,10 +190,8 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
       mbar_init(&w_empty[s], kXfWarps);
     }
     for (int s = 0; s < kWtStages; ++s) {
-      // the producer's expect_tx, + one arrival per CTA for its weights (a lone CTA's transform warps arrive themselves)
-      mbar_init(&full_ab[s], PAIR ? 1 + 2 : 1 + kXfWarps);
+      mbar_init(&full_ab[s], 1 + CTAS * kXfWarps);  // the producer's expect_tx, the transform warps
       mbar_init(&empty[s], 1);
-      mbar_init(&xf_done[s], kXfWarps);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
   const uint32_t tmem_empty_lead = PAIR ? map_shared(smem_u32(tmem_empty), 0) : 0u;
   auto release_tmem = [&](int part, int acc) {
     if constexpr (PAIR)
-      arrive_remote(tmem_empty_lead);
+      arrive_in_pair(tmem_empty_lead);
     else if (part == 0)
       mbar_arrive(&tmem_empty[acc]);
   };
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
       uint32_t phase = 0;
       bool ok = true;
       const auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        return __all_sync(0xffffffffu, PAIR ? wait_cluster(bar, parity) : mbar_wait(bar, parity));
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity));
       };
       WorkList work = work0;
       Segment sg;
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
       if (!drain(sg, 0, PAIR || work.done() ? kDrainParts : 1, acc)) break;
     }
     if (a.outs.world > 1) __threadfence_system();  // the peer stores are performed before the kernel ends
-  } else if (warp == (PAIR ? 24 : 22)) {
+  } else if (warp == 22) {
     // ------------------------------------------------- producer of the packed weight boxes
     if (lane == 0) prefetch_tmap(&tmap_w);
     int ws = 0;
@@ -506,31 +507,6 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
         }
       }
     }
-  } else if (warp >= 22) {
-    if constexpr (!PAIR) {
-      // (a lone CTA has nobody to tell)
-    } else {
-    // ------------------------------------------------------------------- forwarders
-    if (lane == 0) {
-      const int parity_of_mine = warp - 22;  // stages of even / odd iterations
-      int stage = 0, iter = 0;
-      uint32_t phase = 0;
-      const int n_iter = work0.stages_in_all();
-      for (; iter < n_iter; ++iter) {
-        if ((iter & 1) == parity_of_mine) {
-          if (!mbar_wait(&xf_done[stage], phase)) {
-            atomicExch(a.error, kErrWtBase + 6);
-            break;
-          }
-          arrive_remote(full_ab_lead + stage * 8);
-        }
-        if (++stage == kWtStages) {
-          stage = 0;
-          phase ^= 1;
-        }
-      }
-    }
-    }
   } else {
     // -------------------------------------------------------------------- transform
     const int group = (warp - 6) >> 2;            // this group of four warps takes every fourth stage
@@ -552,7 +528,7 @@ __global__ void __launch_bounds__(kWtThreads<PAIR>, 1)
       __syncwarp();
       if (lane == 0) {
         if constexpr (PAIR)
-          mbar_arrive(&xf_done[stored]);  // local; a forwarder passes it on to the pair's first CTA
+          arrive_in_pair(full_ab_lead + stored * 8);
         else
           mbar_arrive(&full_ab[stored]);
       }
@@ -738,7 +714,7 @@ WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share
   }
   const int blk = mode == kModeInt4F16 ? 8 : 16;
   const int w_stage = 16 * (kWtRows / 4) * blk;
-  const int fixed = 1024 + (2 * 24 + 3 * kWtStages + 4) * 8 + 64;
+  const int fixed = 1024 + (2 * 24 + 2 * kWtStages + 4) * 8 + 64;
   int ws = (226 * 1024 - fixed - kWtStages * kWtTokBytes) / w_stage;
   g.w_stages = ws >= 16 ? 16 : 8;  // (a power of two; shared memory has room for twelve of the larger)
   g.smem_bytes = (size_t)kWtStages * kWtTokBytes + (size_t)ws * w_stage + fixed;
@@ -817,7 +793,7 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.grid, 1, 1);
-  cfg.blockDim = dim3(g.ctas == 2 ? kWtThreads<true> : kWtThreads<false>, 1, 1);
+  cfg.blockDim = dim3(kWtThreads, 1, 1);
   cfg.dynamicSmemBytes = g.smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
