@@ -544,10 +544,10 @@ static int run_stream(mld_fc_plan* p, const StripGeometry& gm, const void* src, 
 }
 
 // Prefill: the activations are brought into K-major order (and quantised per token for the int8 route),
-// then one tcgen05 GEMM.  By default the GEMM reads the packed weights as they are and dequantises them in
-// shared memory (gemm_pair_kernel); with cache_prepared_weights, or for a weight matrix whose row pitch a
-// tensor map cannot express, the weights are first expanded to a K-major copy (kept between calls when
-// cached) and a plain GEMM runs on that.
+// then one tcgen05 GEMM.  By default the GEMM reads the packed weights as they are and brings them, dequantised or as
+// bytes, into tensor memory (gemm_wtmem_kernel); with cache_prepared_weights, where convert_pays says so, or for a weight
+// matrix whose row pitch a tensor map cannot express, the weights are first expanded to a K-major copy (kept between calls
+// when cached) and a plain GEMM runs on that.
 static int run_gemm(mld_fc_plan* p, const void* src, const void* weights, const void* scale, const void* bias,
                     void* dst, int tokens, cudaStream_t stream, const PeerOutputs* outs, bool* outs_used) {
   const mld_fc_desc& d = p->d;
@@ -565,17 +565,22 @@ static int run_gemm(mld_fc_plan* p, const void* src, const void* weights, const 
   int rc;
   const bool convert = d.cache_prepared_weights != 0 || !p->pair_ok || d.prefill_route == MLD_PREFILL_ROUTE_CONVERT ||
                        (d.prefill_route == MLD_PREFILL_ROUTE_AUTO && convert_pays(tokens));  // (routes 1 and 3: inside)
-  if (!convert && !i8 && d.prefill_route != MLD_PREFILL_ROUTE_INLINE_SMEM) {
-    // float route: the dequantised weights go to tensor memory
+  if (!convert && d.prefill_route != MLD_PREFILL_ROUTE_INLINE_SMEM) {
+    // the weights, dequantised or as bytes, go to tensor memory
     p->last_route = MLD_ROUTE_PREFILL_INLINE;
-    const int mode = d.weight_bits == 4 ? 0 : 1;
+    const int mode = i8 ? 2 : d.weight_bits == 4 ? 0 : 1;
     const WtGeometry wg = wtmem_geometry(tokens, d.n, d.k, mode, p->sms, true);
     if (++p->split.epoch == 0) p->split.epoch = 1;
-    rc = launch_transpose_x(src, d.src_layout, tokens, d.k, wg.kp, p->x_kmajor, stream);
+    if (i8)
+      rc = launch_quantize_act(src, d.src_layout, tokens, d.k, wg.kp, d.prefill_act_quant == 1, p->x_kmajor, p->a_params,
+                               stream);
+    else
+      rc = launch_transpose_x(src, d.src_layout, tokens, d.k, wg.kp, p->x_kmajor, stream);
     if (rc != MLD_OK) return rc;
     return launch_gemm_wtmem(mode, p->x_kmajor, weights, wg, tokens, d.n, d.k, scale, d.scale_mode,
-                             d.scale_mode == MLD_SCALE_BLOCK ? d.groups : 1, p->group_slices, d.scalar_scale, bias, dst,
-                             d.dst_layout, err, stream, outs, &p->split);
+                             d.scale_mode == MLD_SCALE_BLOCK ? d.groups : 1, p->group_slices, d.scalar_scale, bias,
+                             p->a_params, d.prefill_act_quant == 2 ? p->w_sum : nullptr, dst, d.dst_layout, err, stream, outs,
+                             &p->split);
   }
   if (!convert) {
     p->last_route = MLD_ROUTE_PREFILL_INLINE;

@@ -497,8 +497,8 @@ __global__ void __launch_bounds__(256) transpose_x_kernel(const __half* __restri
 __global__ void __launch_bounds__(256) quantize_act_kernel(const __half* __restrict__ x, int layout, int M, int K, int Kp,
                                                            int symmetric, int8_t* __restrict__ xq,
                                                            float* __restrict__ params) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // (after the wait: see transpose_x_kernel)
   const int m = blockIdx.x;
   __shared__ float red[8], red2[8];
   __shared__ int redi[8];
@@ -626,8 +626,8 @@ __global__ void __launch_bounds__(256) act_quantize_sliced_kernel(const __half* 
                                                                   int symmetric, const float* __restrict__ part,
                                                                   float* __restrict__ params,
                                                                   int8_t* __restrict__ xq) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // (after the wait: see transpose_x_kernel)
   __shared__ uint32_t tile[32][33];
   const int S = (K + 3) / 4, Sp = Kp / 4;
   const int m0 = blockIdx.y * 32, s0 = blockIdx.x * 32;

@@ -8,6 +8,10 @@
 //
 //   Y^T[N x M] = W[N x K] X[M x K]^T
 //
+// With int8 activations (quantised per token by the kernel ahead) the weights go to tensor memory as signed bytes, exact
+// products are summed in int32, and the epilogue dequantises them.  8192 -> 3584, in a graph: 17 tokens 21 us (62 through
+// shared memory, 44 with a conversion pass), 512 46 (70, 51), 2048 92 (127, 96).
+//
 // The weights are the MMA's M-side operand and sit in tensor memory; the activations are the N-side operand in
 // shared memory.  A dequantised weight tile is then written once, by tcgen05.st, into the memory the tensor
 // core reads it from, instead of being written to shared memory by the transform warps and read back from
@@ -73,10 +77,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 // D[tmem_d] (+)= A[tmem_a] B[desc_b]^T over the pair (or by this CTA alone); A: 16 halves per lane in 8 columns of
 // tensor memory (of both CTAs').
-template <bool PAIR>
+template <bool PAIR, bool I8>
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
                                         uint32_t accumulate) {
-  if constexpr (PAIR) {
+  if constexpr (PAIR && I8) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+  } else if constexpr (I8) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+  } else if constexpr (PAIR) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
@@ -146,18 +162,48 @@ struct WtArgs {
 // pairs and whole tiles); 256 tokens 34.0, 512 48.3 (42.9, 66.7 with stages announced to the pair's first CTA by warps of
 // their own, whose release at cluster scope took longer than a stage).
 constexpr int kWtThreads = 23 * 32;
+template <int MODE>
+constexpr int kWtSlices = MODE == kModeInt8I8 ? 32 : 16;
+
+// The bytes of two 4x4 blocks turned round over the four lanes c = 0..3 that share them: lane c comes with word c (input
+// channel c, a byte per output) of each and leaves with output c's bytes of the four input channels, as signed numbers.
+// Two butterfly steps (lanes 2 apart, then 1), both blocks' halves in one shuffle.  (A lane reading whole blocks, of which
+// it needs a quarter, would take the shared memory twice the time of word and shuffle.)
+struct TurnSelectors {
+  uint32_t give2, keep2, give1, keep1, out0, out1;
+  __device__ __forceinline__ explicit TurnSelectors(int c) {
+    // step 1: bytes of outputs 2h, 2h + 1 stay with the lanes whose c / 2 is h
+    keep2 = (c & 2) ? 0x7632u : 0x5410u;
+    give2 = (c & 2) ? 0x5410u : 0x7632u;
+    // step 2, of {own, received}: bytes {block 0 own, block 0 received, block 1 own, block 1 received} of output c (c ^ 1)
+    keep1 = (c & 1) ? 0x7351u : 0x6240u;
+    give1 = (c & 1) ? 0x6240u : 0x7351u;
+    // then {kept, received} hold input channels c, c ^ 2 and c ^ 1, c ^ 3: in the order of the channels
+    uint32_t s = 0;
+    for (int k = 0; k < 4; ++k) s |= static_cast<uint32_t>(k == c ? 0 : k == (c ^ 2) ? 1 : k == (c ^ 1) ? 4 : 5) << (4 * k);
+    out0 = s;
+    out1 = s + 0x2222u;
+  }
+};
+__device__ __forceinline__ void turn_blocks(uint32_t w0, uint32_t w1, const TurnSelectors& t, uint32_t& o0, uint32_t& o1) {
+  const uint32_t k2 = __byte_perm(w0, w1, t.keep2), r2 = __shfl_xor_sync(0xffffffffu, __byte_perm(w0, w1, t.give2), 2);
+  const uint32_t k1 = __byte_perm(k2, r2, t.keep1), r1 = __shfl_xor_sync(0xffffffffu, __byte_perm(k2, r2, t.give1), 1);
+  o0 = __byte_perm(k1, r1, t.out0) ^ 0x80808080u;
+  o1 = __byte_perm(k1, r1, t.out1) ^ 0x80808080u;
+}
 template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kWtThreads, 1)
     gemm_wtmem_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, WtArgs wa) {
   const PairArgs& a = wa.p;
+  constexpr bool I8 = MODE == kModeInt8I8;
   constexpr int BLK = MODE == kModeInt4F16 ? 8 : 16;   // bytes of a packed 4x4 block
-  constexpr int SLICES = 16;                            // packed rows per stage (64 input channels)
+  constexpr int SLICES = kWtSlices<MODE>;               // packed rows per stage (64 input channels, 128 of a byte)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int CTAS = PAIR ? 2 : 1;                    // CTAs per tile
   const int cta_tok = wa.tile_tok / CTAS;               // token rows this CTA fetches
   constexpr int w_pitch = (kWtRows / 4) * BLK;          // bytes of one packed row of the box
-  constexpr int w_stage = SLICES * w_pitch;             // 4 KB / 8 KB
+  constexpr int w_stage = SLICES * w_pitch;             // 4 / 8 / 16 KB
   uint8_t* sX = smem;
   uint8_t* sW = sX + (size_t)kWtStages * kWtTokBytes;
   uint64_t* full_w = reinterpret_cast<uint64_t*>(sW + (size_t)a.w_stages * w_stage);  // [w_stages]
@@ -277,6 +323,14 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     const bool has_n = n < a.N4;
     __half bias_h = __float2half_rn(0.0f);
     if (a.bias != nullptr && has_n) bias_h = static_cast<const __half*>(a.bias)[n];
+    [[maybe_unused]] float w_scale = 0.0f, w_offset = 0.0f;  // int8 route: the channel's scale, the sum of its weights
+    if constexpr (I8) {
+      pdl_wait();  // (the tokens' parameters come from the kernel ahead; over by now, whoever waited first)
+      if (n < a.N) {
+        w_scale = __half2float(a.scale[n]);
+        if (a.w_sum != nullptr) w_offset = static_cast<float>(a.w_sum[n]);
+      }
+    }
     const int q = lane & 3;  // place among the four channels of the output slice n >> 2
     for (int pc = part; pc < n_pieces; pc += parts) {
       const int c0 = 16 * pc;
@@ -289,10 +343,28 @@ __global__ void __launch_bounds__(kWtThreads, 1)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint4 v = __ldcg(&slot_rows[(pc * 4 + j) * 32]);
-          r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + __uint_as_float(v.x));
-          r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + __uint_as_float(v.y));
-          r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + __uint_as_float(v.z));
-          r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + __uint_as_float(v.w));
+          if constexpr (I8) {
+            r[4 * j] += v.x, r[4 * j + 1] += v.y, r[4 * j + 2] += v.z, r[4 * j + 3] += v.w;
+          } else {
+            r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + __uint_as_float(v.x));
+            r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + __uint_as_float(v.y));
+            r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + __uint_as_float(v.z));
+            r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + __uint_as_float(v.w));
+          }
+        }
+      }
+      if constexpr (I8) {
+        // CreateDequantization (quantize_and_dequantize.cc:867-964):
+        //   res = float(acc) * (w_scale * src_scale) + w_scale * src_zero_point * weights_sum
+        // lanes 0..15 hold the scales of the piece's tokens, 16..31 their zero points
+        const int tok = m_first + c0 + (lane & 15);
+        const float mine = tok < a.M ? a.a_params[tok * 3 + (lane >> 4)] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float a_scale = __shfl_sync(0xffffffffu, mine, j), a_off = __shfl_sync(0xffffffffu, mine, 16 + j);
+          float v = static_cast<float>(static_cast<int32_t>(r[j])) * (w_scale * a_scale);
+          if (a.w_sum != nullptr) v += w_scale * a_off * w_offset;
+          r[j] = __float_as_uint(v);
         }
       }
       // token pairs as packed halves: h2[i] = tokens c0 + 2i, c0 + 2i + 1 of channel n
@@ -393,9 +465,9 @@ __global__ void __launch_bounds__(kWtThreads, 1)
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&full_ab[stage], static_cast<uint32_t>(wa.tile_tok) * kKBytes);
           if constexpr (PAIR)
-            tma_load_2d_pair(sX + (size_t)stage * kWtTokBytes, &tmap_x, full_ab_lead + stage * 8, kb * 64, m0);
+            tma_load_2d_pair(sX + (size_t)stage * kWtTokBytes, &tmap_x, full_ab_lead + stage * 8, kb * 4 * SLICES, m0);
           else
-            tma_load_2d(sX + (size_t)stage * kWtTokBytes, &tmap_x, &full_ab[stage], kb * 64, m0);
+            tma_load_2d(sX + (size_t)stage * kWtTokBytes, &tmap_x, &full_ab[stage], kb * 4 * SLICES, m0);
         }
         __syncwarp();
         if (++stage == kWtStages) {
@@ -409,7 +481,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     // The whole warp goes through the waits and one elected lane issues, so that the instructions' operands are uniform
     // for the compiler: with a single lane in the loop a stage took 512 cycles of issuing alone, whatever the tile.
     if (rank == 0) {
-      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(wa.tile_tok >> 3) << 17) | ((PAIR ? 16u : 8u) << 24);
+      const uint32_t idesc = (I8 ? (2u << 4) | (1u << 7) | (1u << 10) : 1u << 4) | (static_cast<uint32_t>(wa.tile_tok >> 3) << 17) | ((PAIR ? 16u : 8u) << 24);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -445,7 +517,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              umma_ts<PAIR>(tmem_d, ta + 8u * k, db + static_cast<uint64_t>((k * 32) >> 4), idesc,
+              umma_ts<PAIR, I8>(tmem_d, ta + 8u * k, db + static_cast<uint64_t>((k * 32) >> 4), idesc,
                             (kb > sg.kb0 || k > 0) ? 1u : 0u);
             commit<PAIR>(&empty[stage]);
           }
@@ -515,6 +587,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     const int col4 = row & 3;                      // column of the row inside its 4x4 blocks
     const uint32_t sel8 = static_cast<uint32_t>(col4) | (static_cast<uint32_t>(4 + col4) << 8);
     const __half2 offset = __float2half2_rn(MODE == kModeInt4F16 ? 1032.0f : 1152.0f);  // 1024 + the value of a zero
+    [[maybe_unused]] const TurnSelectors turn(col4);
     const int w_shift = __ffs(a.w_stages) - 1;
     bool ok = true;
     int xf_iter = 0;  // stages before the segment
@@ -540,7 +613,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     [[maybe_unused]] const long long tr_start = MLD_PAIR_CLOCK();
     for (int nth = 0; ok && work.next(sg); ++nth) {
       const int n = tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows + row;
-      const bool scaled = n < a.N4 && a.scale != nullptr, blocks = a.scale_mode == MLD_SCALE_BLOCK;
+      const bool scaled = !I8 && n < a.N4 && a.scale != nullptr, blocks = a.scale_mode == MLD_SCALE_BLOCK;
       // 32 input channels are one scale group whenever groups are whole multiples of 32 inputs, the usual case: two loads
       // a stage then, issued when the group's stage before is begun
       const bool one_group = !blocks || (a.group_slices & 7) == 0;
@@ -584,6 +657,28 @@ __global__ void __launch_bounds__(kWtThreads, 1)
         tr_wait += t1 - t0;
         const uint8_t* wp = sW + (size_t)ws * w_stage + (row >> 2) * BLK;
         const uint32_t columns = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + kWtACol + static_cast<uint32_t>(stage * 32);
+        if constexpr (I8) {
+          const uint32_t* ww = reinterpret_cast<const uint32_t*>(sW + (size_t)ws * w_stage) + row;  // input channel `col4` of the block
+          uint32_t in[16];
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) in[i] = ww[(16 * half + i) * (w_pitch / 4)];
+            if (half == 0) {
+              announce();
+              if (!mbar_wait(&empty[stage], (static_cast<uint32_t>(iter / kWtStages) & 1u) ^ 1u)) {
+                atomicExch(a.error, kErrWtBase + 5);
+                ok = false;
+                break;
+              }
+              tc_after();
+            }
+            uint32_t o[16];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) turn_blocks(in[i], in[i + 1], turn, o[i], o[i + 1]);
+            tmem_st16(columns + static_cast<uint32_t>(16 * half), o);
+          }
+        } else {
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           using Block = typename std::conditional<MODE == kModeInt4F16, uint2, uint4>::type;
@@ -617,6 +712,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
             }
           }
           tmem_st16(columns + static_cast<uint32_t>(16 * half), o);
+        }
         }
         if (!ok) break;
         [[maybe_unused]] const long long t2 = MLD_PAIR_CLOCK();
@@ -678,13 +774,14 @@ extern "C" __attribute__((visibility("default"))) void mld_debug_set_wt_trace(vo
 WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share) {
   WtGeometry g;
   const int N4 = align_n(N, 4);
-  g.kp = align_n(K, 8);
-  g.k_blocks = div_up(g.kp, 64);
+  const bool i8 = mode == kModeInt8I8;
+  g.kp = align_n(K, i8 ? 16 : 8);
+  g.k_blocks = div_up(g.kp, i8 ? 128 : 64);
   // Up to 128 tokens a CTA works alone; with more, pairs share the fetching of the tokens.
   g.ctas = M <= 128 || sms < 2 ? 1 : 2;
   g.n_tiles = div_up(N4, g.ctas * kWtRows);
   const int most = 128 * g.ctas;
-  g.tile_tok = M >= most ? most : align_n(M, 16);
+  g.tile_tok = M >= most ? most : align_n(M, i8 && g.ctas == 2 ? 32 : 16);
 #ifdef MLD_TRACE
   if (const char* e = getenv("MLD_WT_TOK")) g.tile_tok = atoi(e);
 #endif
@@ -713,19 +810,19 @@ WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share
     g.grid = g.ctas * static_cast<int>(few ? tiles : pairs);
   }
   const int blk = mode == kModeInt4F16 ? 8 : 16;
-  const int w_stage = 16 * (kWtRows / 4) * blk;
+  const int w_stage = (i8 ? 32 : 16) * (kWtRows / 4) * blk;
   const int fixed = 1024 + (2 * 24 + 2 * kWtStages + 4) * 8 + 64;
   int ws = (226 * 1024 - fixed - kWtStages * kWtTokBytes) / w_stage;
-  g.w_stages = ws >= 16 ? 16 : 8;  // (a power of two; shared memory has room for twelve of the larger)
+  g.w_stages = ws >= 16 ? 16 : ws >= 8 ? 8 : 4;  // (a power of two)
   g.smem_bytes = (size_t)kWtStages * kWtTokBytes + (size_t)ws * w_stage + fixed;
   return g;
 }
 
 int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const WtGeometry& g, int M, int N, int K,
                       const void* scale, int scale_mode, int G, int group_slices, float scalar_scale, const void* bias,
-                      void* y, int dst_layout, int* error, cudaStream_t stream, const PeerOutputs* outs,
-                      const PairSplit* split) {
-  if (mode != kModeInt4F16 && mode != kModeInt8F16) {
+                      const float* a_params, const int32_t* w_sum, void* y, int dst_layout, int* error, cudaStream_t stream,
+                      const PeerOutputs* outs, const PairSplit* split) {
+  if (mode != kModeInt4F16 && mode != kModeInt8F16 && mode != kModeInt8I8) {
     set_last_error_text("bad GEMM mode");
     return MLD_INVALID_ARGUMENT;
   }
@@ -736,13 +833,15 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   const int N4 = align_n(N, 4);
   const int blk = mode == kModeInt4F16 ? 8 : 16;
   const int SS = div_up(K, 4), DS = N4 / 4;
+  const bool i8 = mode == kModeInt8I8;
   CUtensorMap tx, tw;
   // activations: K-major rows [M][kp]; box = one swizzle atom of K x this CTA's half of the tile's tokens
-  int rc = make_tmap_2d(&tx, x_kmajor, (uint64_t)g.kp * 2, M, (uint64_t)g.kp * 2, kKBytes, g.tile_tok / g.ctas, 2,
-                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, true);
+  const int esz = i8 ? 1 : 2;
+  int rc = make_tmap_2d(&tx, x_kmajor, (uint64_t)g.kp * esz, M, (uint64_t)g.kp * esz, kKBytes, g.tile_tok / g.ctas, esz,
+                        CU_TENSOR_MAP_SWIZZLE_128B, i8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, true);
   if (rc != MLD_OK) return rc;
-  // packed weights: [K/4] rows of N4/4 blocks; box = one stage's 16 rows x the CTA's 32 blocks, in 32-bit elements
-  rc = make_tmap_2d(&tw, packed, (uint64_t)DS * blk, SS, (uint64_t)DS * blk, (kWtRows / 4) * blk, 16, 4,
+  // packed weights: [K/4] rows of N4/4 blocks; box = one stage's rows x the CTA's 32 blocks, in 32-bit elements
+  rc = make_tmap_2d(&tw, packed, (uint64_t)DS * blk, SS, (uint64_t)DS * blk, (kWtRows / 4) * blk, i8 ? 32 : 16, 4,
                     CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc != MLD_OK) return rc;
   WtArgs wa;
@@ -764,6 +863,8 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
     if ((1 << sh) == group_slices) a.gs_shift = sh;
   a.scalar_scale = scalar_scale;
   a.bias = bias;
+  a.a_params = a_params;
+  a.w_sum = w_sum;
   a.y = y;
   a.dst_layout = dst_layout;
   a.error = error;
@@ -782,9 +883,13 @@ int launch_gemm_wtmem(int mode, const void* x_kmajor, const void* packed, const 
   wa.trace_flags = getenv("MLD_WT_FLAGS") != nullptr ? atoi(getenv("MLD_WT_FLAGS")) : 0;
 #endif
   void (*kern)(CUtensorMap, CUtensorMap, WtArgs) =
-      g.ctas == 2 ? (mode == kModeInt4F16 ? gemm_wtmem_kernel<kModeInt4F16, true> : gemm_wtmem_kernel<kModeInt8F16, true>)
-                  : (mode == kModeInt4F16 ? gemm_wtmem_kernel<kModeInt4F16, false> : gemm_wtmem_kernel<kModeInt8F16, false>);
-  static bool configured[2][2][kMaxDevices];
+      g.ctas == 2 ? (mode == kModeInt4F16   ? gemm_wtmem_kernel<kModeInt4F16, true>
+                     : mode == kModeInt8F16 ? gemm_wtmem_kernel<kModeInt8F16, true>
+                                            : gemm_wtmem_kernel<kModeInt8I8, true>)
+                  : (mode == kModeInt4F16   ? gemm_wtmem_kernel<kModeInt4F16, false>
+                     : mode == kModeInt8F16 ? gemm_wtmem_kernel<kModeInt8F16, false>
+                                            : gemm_wtmem_kernel<kModeInt8I8, false>);
+  static bool configured[2][3][kMaxDevices];
   bool(&done)[kMaxDevices] = configured[g.ctas - 1][mode];
   int dev;
   if (needs_configure(done, &dev)) {

@@ -128,6 +128,13 @@ def test_w8a8_prefill_vs_oracle(mld, oracle, rule, route, cache, M, K, N):
     assert _rel(y, x16.astype(np.float32) @ w.T) < 3e-2
 
 
+@pytest.mark.parametrize("rule", ["symmetric", "asymmetric"])
+@pytest.mark.parametrize("M,K,N", [(17, 4160, 200), (77, 8192, 520), (128, 656, 20000),  # lone CTAs, tiles in parts and whole
+                                   (129, 4096, 264), (200, 1040, 2568), (257, 2064, 520)])  # pairs
+def test_w8a8_weights_in_tensor_memory(mld, oracle, rule, M, K, N):
+    test_w8a8_prefill_vs_oracle(mld, oracle, rule, "inline", False, M, K, N)
+
+
 def test_w8a8_shard_of_the_eight_way_split(mld, oracle):
     """One rank's share of the W8A8 prefill case that is split eight ways over N: M=2048, K=8192,
     N=3584 of 28672, asymmetric per-token activations.  Sampled tokens against the restated chain: the
