@@ -213,8 +213,7 @@ enum mld_prefill_route {
   MLD_PREFILL_ROUTE_INLINE = 1,
   MLD_PREFILL_ROUTE_CONVERT = 2,
   MLD_PREFILL_ROUTE_INLINE_SMEM = 3  /* inside the GEMM, through shared memory
-                                        instead of tensor memory (the form the
-                                        int8-activation route uses; kept
+                                        instead of tensor memory (kept
                                         selectable for comparison) */
 };
 
@@ -263,9 +262,9 @@ typedef struct mld_fc_desc {
                                 weights in a pass of their own when that costs
                                 little beside the product, dequantise inside
                                 the GEMM otherwise; with the costs measured
-                                for these kernels the pass pays above 512
-                                tokens, with the reference's constants above
-                                200), 1 = always inside the GEMM, 2 = always
+                                for these kernels the pass pays above 512 to
+                                4096 tokens, more the longer the inputs, with
+                                the reference's constants above 200), 1 = always inside the GEMM, 2 = always
                                 the separate pass */
   /* Features of the reference operator that this library does not serve: a
    * non-zero value makes mld_fc_plan_create return MLD_UNIMPLEMENTED and name

@@ -251,10 +251,22 @@ int mld_fc_is_gemv_recommended(int32_t precision, int32_t tokens) {
 
 // The builder's conversion-cost rule (gpu_model_builder.cc:1132-1173) weighs the bytes a separate conversion
 // pass reads and writes against the flops of the product and converts when the ratio is small, which with its
-// constants means from 200 tokens up.  The same rule with this library's measured costs (a 14336 x 4096 INT4
-// projection: dequantising inside the GEMM wins by 12 us up to 512 tokens, i.e. two token tiles, and loses by
-// 12 us from 640 on) puts the threshold at 512.
-static bool convert_pays(int tokens) { return tokens > 512; }
+// constants means from 200 tokens up.  The same rule with this library's measured costs: a pass costs more the more inputs a
+// channel has, dequantising inside the GEMM a little for every tile of 256 tokens.  us in a graph, inside / converted:
+//   float, K = 8192 and more: 8192 -> 8192 INT4 1024 tokens 97 / 144, 4096 384 / 388; 11008 -> 4096 4096 tokens 267 / 284
+//   float, K = 4096, N K from 32 M: 4096 -> 14336 1024 tokens 92 / 106, 2048 167 / 171, 3072 254 / 238; -> 11008 2048 tokens
+//     135 / 136; and below: 4096 -> 4096 INT4 640 tokens 35.8 / 35.0, 2048 -> 8192 520 tokens 48 / 44
+//   int8 activations: 8192 -> 28672 2048 tokens 379 / 402, 8192 -> 3584 2048 92 / 96, 4096 154 / 151; 4096 -> 14336 1024
+//     tokens 79 / 86, 2048 133 / 124; 4096 -> 4096 640 tokens 40 / 36
+static bool convert_pays(const mld_fc_desc& d, int tokens) {
+  const bool i8 = d.prefill_act_quant != 0;
+  int most = 512;
+  if (d.k >= 8192)
+    most = i8 ? 2048 : 4096;
+  else if (d.k >= 4096 && static_cast<int64_t>(d.n) * d.k >= 32 << 20)
+    most = i8 ? 1024 : 2048;
+  return tokens > most;
+}
 
 int mld_fc_plan_create(const mld_fc_desc* d, mld_fc_plan** out) {
   MLD_REQUIRE(d != nullptr && out != nullptr, "null argument");
@@ -352,7 +364,7 @@ int mld_fc_plan_create(const mld_fc_desc* d, mld_fc_plan** out) {
     const GemmGeometry gmax = gemm_geometry(d->max_tokens, d->n, d->k, i8, p->sms);
     // the K-major copy of the weights is needed only by the route that prepares them in a pass of its own
     const bool need_w = d->cache_prepared_weights != 0 || !p->pair_ok || d->prefill_route == MLD_PREFILL_ROUTE_CONVERT ||
-                        (d->prefill_route == MLD_PREFILL_ROUTE_AUTO && convert_pays(d->max_tokens));
+                        (d->prefill_route == MLD_PREFILL_ROUTE_AUTO && convert_pays(*d, d->max_tokens));
     const size_t wb = need_w ? (size_t)N4 * gmax.kp * esz : 0, xb = (size_t)d->max_tokens * gmax.kp * esz,
                  pb = (size_t)d->max_tokens * kActParamFloats * sizeof(float);
     cudaError_t e = need_w ? cudaMalloc(&p->w_kmajor, wb) : cudaSuccess;
@@ -564,7 +576,7 @@ static int run_gemm(mld_fc_plan* p, const void* src, const void* weights, const 
   }
   int rc;
   const bool convert = d.cache_prepared_weights != 0 || !p->pair_ok || d.prefill_route == MLD_PREFILL_ROUTE_CONVERT ||
-                       (d.prefill_route == MLD_PREFILL_ROUTE_AUTO && convert_pays(tokens));  // (routes 1 and 3: inside)
+                       (d.prefill_route == MLD_PREFILL_ROUTE_AUTO && convert_pays(d, tokens));  // (routes 1 and 3: inside)
   if (!convert && d.prefill_route != MLD_PREFILL_ROUTE_INLINE_SMEM) {
     // the weights, dequantised or as bytes, go to tensor memory
     p->last_route = MLD_ROUTE_PREFILL_INLINE;
