@@ -2026,7 +2026,7 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
   const int dl = m->d_local, fl = m->ffn_local;
   const size_t o_qkv = take((size_t)3 * dl * 2), o_ap = take((size_t)m->grid * kAttSlots * kAttDump * 4),
                o_at = take((size_t)m->heads_local * 4),
-               o_bar = take(8), o_err = take(4);
+               o_bar = take(8), o_res = take((size_t)d * 2 + sizeof(int));
   // the op-to-op vectors as tagged words unless the descriptor asks for grid barriers (the split of o and down
   // by input columns exchanges fp32 partial sums and keeps the barriers)
   m->tagged = (cfg.handover == 0 && !m->paired) ? 1 : 0;
@@ -2081,7 +2081,7 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
   m->att_part = reinterpret_cast<float*>(m->scratch + o_ap);
   m->att_tickets = reinterpret_cast<int*>(m->scratch + o_at);
   m->bar = reinterpret_cast<unsigned*>(m->scratch + o_bar);
-  m->error = reinterpret_cast<int*>(m->scratch + o_err);
+  m->error = reinterpret_cast<int*>(m->scratch + o_res + (size_t)d * 2);
   m->h_layers.resize(cfg.layers);
   m->layer_set.assign(cfg.layers, 0);
   *out = m;
@@ -2163,6 +2163,7 @@ int mega_read_trace(MegaDecoder* m, unsigned long long* out, size_t count) {
 int mega_grid(const MegaDecoder* m) { return m->grid; }
 
 const int* mega_error_word(const MegaDecoder* m) { return m->error; }
+void* mega_result(const MegaDecoder* m) { return reinterpret_cast<uint8_t*>(m->error) - (size_t)m->cfg.d_model * 2; }
 
 // Back to the state after creation: counters zero, no tagged word or record valid.  (Tags and record epochs
 // derive from the launch counter; restarting it is safe only because everything that carries a tag or an

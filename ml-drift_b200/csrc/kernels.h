@@ -160,6 +160,8 @@ int mega_step(MegaDecoder* m, const void* x_in, void* x_out, int pos, cudaStream
 // Reads (and clears) the kernel's error word: 0 = every wait of the last steps was satisfied.
 int mega_device_status(MegaDecoder* m, int* code);
 const int* mega_error_word(const MegaDecoder* m);
+// Room for a step's result vector with the error word right behind it, so that one copy brings both to the host.
+void* mega_result(const MegaDecoder* m);
 int mega_reset(MegaDecoder* m);
 void mega_set_wait_limit(MegaDecoder* m, int us);
 // Sharded: every rank exports its exchange block (64-byte IPC handle) and imports all of them (rank order).
