@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kWtThreads, 1)
   uint64_t* w_empty = full_w + a.w_stages;            // [w_stages]: the transform warps have read the box
   uint64_t* full_ab = w_empty + a.w_stages;           // [stages], first CTA: tokens of both CTAs landed, weights of both in TMEM
   uint64_t* empty = full_ab + kWtStages;              // [stages]: the stage's MMAs have completed (arrives in both CTAs)
-  uint64_t* tmem_full = empty + kWtStages;            // [2] (accumulators; a pair has one), arrives in both CTAs
-  uint64_t* tmem_empty = tmem_full + 2;               // [2], first CTA: the warps that read it (of both CTAs) are done
+  uint64_t* tmem_full = empty + kWtStages;            // [3] (see accumulators_ready), arrives in both CTAs
+  uint64_t* tmem_empty = tmem_full + 3;               // [2], first CTA: the warps that read it (of both CTAs) are done
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
       mbar_init(&full_ab[s], 1 + CTAS * kXfWarps);  // the producer's expect_tx, the transform warps
       mbar_init(&empty[s], 1);
     }
+    mbar_init(&tmem_full[2], 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
       mbar_init(&tmem_empty[b], PAIR ? CTAS * 4 * kDrainParts : 4);
@@ -262,6 +263,16 @@ __global__ void __launch_bounds__(kWtThreads, 1)
   // tile -> (token tile, channel tile): the token tiles of one channel tile follow each other
   auto tile_tok0 = [&](int tile) { return (tile % a.m_tiles) * wa.tile_tok; };
   auto tile_n0 = [&](int tile) { return (tile / a.m_tiles) * CTAS * kWtRows; };
+
+  // Who reads a segment's accumulators: all five warps that can address a lane quarter, or its epilogue warp alone.
+  const auto read_by_all = [&](const Segment&, bool last) { return PAIR || last; };
+  // The barrier that a segment's finished MMAs arrive on.  A wait tells one use of a barrier from the one before and no more, so
+  // nobody may miss a use of one that it waits on later: segments that the epilogue warp reads alone have barriers that it
+  // alone waits on, by accumulators, and those read by all have the third.  (With a segment of a few stages a transform
+  // warp is done while the MMAs of segments before it are still to come, since the ring holds eight stages.)
+  const auto accumulators_ready = [&](const Segment& sg, bool last, int nth) {
+    return &tmem_full[read_by_all(sg, last) ? 2 : PAIR ? 0 : nth & 1];
+  };
 
   // Accumulators -> outputs, the share `part` of `parts` of the warps that can address this lane quarter: pieces of 16 token
   // columns, part, part + parts, ...  A pair has one set of accumulators, so the quarter's four transform warps, which have
@@ -527,7 +538,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
             phase ^= 1;
           }
         }
-        if (ok && elect_one()) commit<PAIR>(&tmem_full[acc]);
+        if (ok && elect_one()) commit<PAIR>(accumulators_ready(sg, work.done(), nth));
         __syncwarp();
       }
 #ifdef MLD_TRACE
@@ -542,14 +553,17 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     // --------------------------------------------------------------------- epilogue
     WorkList work = work0;
     Segment sg;
+    int shared = 0;  // segments read by all so far
     for (int nth = 0; work.next(sg); ++nth) {
       const int acc = PAIR ? 0 : nth & 1;
-      if (!mbar_wait(&tmem_full[acc], static_cast<uint32_t>(PAIR ? nth : nth >> 1) & 1u)) {
+      const bool all = read_by_all(sg, work.done());
+      const int use = all ? shared++ : PAIR ? nth : nth >> 1;
+      if (!mbar_wait(accumulators_ready(sg, work.done(), nth), static_cast<uint32_t>(use) & 1u)) {
         atomicExch(a.error, kErrWtBase + 4);
         break;
       }
       tc_after();
-      if (!drain(sg, 0, PAIR || work.done() ? kDrainParts : 1, acc)) break;
+      if (!drain(sg, 0, all ? kDrainParts : 1, acc)) break;
     }
     if (a.outs.world > 1) __threadfence_system();  // the peer stores are performed before the kernel ends
   } else if (warp == 22) {
@@ -611,6 +625,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     Segment sg;
     [[maybe_unused]] long long tr_wait = 0, tr_work = 0, tr_st = 0;
     [[maybe_unused]] const long long tr_start = MLD_PAIR_CLOCK();
+    int shared = 0;  // segments read by all so far
     for (int nth = 0; ok && work.next(sg); ++nth) {
       const int n = tile_n0(sg.tile) + static_cast<int>(rank) * kWtRows + row;
       const bool scaled = !I8 && n < a.N4 && a.scale != nullptr, blocks = a.scale_mode == MLD_SCALE_BLOCK;
@@ -727,9 +742,9 @@ __global__ void __launch_bounds__(kWtThreads, 1)
       // A pair's segment, a lone CTA's last: the transform warps share the reading with the epilogue warp of their
       // quarter.  (Measured: reading them only when the ring is full and the next stage blocked, so that the next
       // tile's first stages are transformed beforehand, costs more in polling than the refill costs here.)
-      if (!PAIR && !work.done()) continue;
+      if (!read_by_all(sg, work.done())) continue;
       const int acc = PAIR ? 0 : nth & 1;
-      if (!mbar_wait(&tmem_full[acc], static_cast<uint32_t>(PAIR ? nth : nth >> 1) & 1u)) {
+      if (!mbar_wait(accumulators_ready(sg, work.done(), nth), static_cast<uint32_t>(shared++) & 1u)) {
         atomicExch(a.error, kErrWtBase + 9);
         break;
       }
@@ -811,7 +826,7 @@ WtGeometry wtmem_geometry(int M, int N, int K, int mode, int sms, bool may_share
   }
   const int blk = mode == kModeInt4F16 ? 8 : 16;
   const int w_stage = (i8 ? 32 : 16) * (kWtRows / 4) * blk;
-  const int fixed = 1024 + (2 * 24 + 2 * kWtStages + 4) * 8 + 64;
+  const int fixed = 1024 + (2 * 24 + 2 * kWtStages + 5) * 8 + 64;
   int ws = (226 * 1024 - fixed - kWtStages * kWtTokBytes) / w_stage;
   g.w_stages = ws >= 16 ? 16 : ws >= 8 ? 8 : 4;  // (a power of two)
   g.smem_bytes = (size_t)kWtStages * kWtTokBytes + (size_t)ws * w_stage + fixed;

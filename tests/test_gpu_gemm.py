@@ -286,6 +286,12 @@ def test_tiles_cut_along_k(mld, oracle, bits, M, K, N):
     assert _rel(y, ref) <= (1e-3 if bits == 4 else 0.05 / 35 + 2.0 ** -11)
 
 
+@pytest.mark.parametrize("M,K,N", [(77, 128, 57600), (20, 64, 80000), (128, 256, 19200), (300, 640, 11328)])
+def test_tiles_of_few_stages(mld, oracle, M, K, N):
+    # several tiles to a CTA (pair), all of their stages in the ring before the first MMA is issued
+    test_tiles_cut_along_k(mld, oracle, 4, M, K, N)
+
+
 @pytest.mark.parametrize("bits,M,K,N,act_quant", [
     (4, 77, 4096, 11008, 0), (8, 40, 8192, 1024, 0),  # lone CTAs: every tile cut along K
     (4, 500, 4096, 264, 0),                           # pairs, fewer tiles than pairs
