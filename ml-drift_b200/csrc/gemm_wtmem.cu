@@ -55,7 +55,6 @@ constexpr uint32_t kWtACol = 256;     // first TMEM column of the weight ring
 constexpr int kWtAccCols = 128;       // columns of each of a lone CTA's two sets of accumulators
 constexpr int kErrWtBase = 50;
 constexpr int kXfWarps = 4;            // transform warps that share a stage, one per quarter of the channels
-constexpr int kScaleAhead = 16;       // stages by which L2 is asked for the scales ahead of their use
 constexpr int kDrainParts = 5;        // warps that read one lane quarter's accumulators: one epilogue + four transform
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -639,28 +638,27 @@ __global__ void __launch_bounds__(kWtThreads, 1)
         return a.scale + (size_t)g * a.N4 + n;
       };
       const auto scale_at = [&](int slice) -> __half { return scaled ? __ldg(scale_ptr(slice)) : fixed_scale; };
-      // (a stage takes less time than a trip to HBM: without this the loop waits for the scales)
-      const auto prefetch_scales = [&](int kb) {
-        if (scaled && blocks && kb < sg.kb1) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(scale_ptr(kb * SLICES)));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(scale_ptr(kb * SLICES + 8)));
-        }
+      // Asked for a stage of the group ahead, four stages in all, which is more than a trip to HBM.  (The load by hand: it
+      // leaves the register alone where there is nothing to load, so that nothing looks at the value, and waits, before the
+      // stage that needs it.)
+      const auto ask_scale = [&](unsigned short& v, int slice) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.nc.u16 %0, [%1];\n\t}"
+                     : "+h"(v)
+                     : "l"(scale_ptr(slice)), "r"(scaled ? 1u : 0u));
       };
       int kb = sg.kb0 + ((group - xf_iter) & 3);
-      for (int ahead = 4; ahead < kScaleAhead; ahead += 4) prefetch_scales(kb + ahead);
-      __half next0 = fixed_scale, next1 = fixed_scale;
+      unsigned short next0 = __half_as_ushort(fixed_scale), next1 = next0;
       if (kb < sg.kb1) {
-        next0 = scale_at(kb * SLICES);
-        next1 = scale_at(kb * SLICES + 8);
+        ask_scale(next0, kb * SLICES);
+        ask_scale(next1, kb * SLICES + 8);
       }
       for (; kb < sg.kb1; kb += 4) {
         const int iter = xf_iter + kb - sg.kb0, stage = iter & (kWtStages - 1), ws = iter & (a.w_stages - 1);
-        const __half cur[2] = {next0, next1};
+        const unsigned short cur0 = next0, cur1 = next1;
         if (kb + 4 < sg.kb1) {
-          next0 = scale_at((kb + 4) * SLICES);
-          next1 = scale_at((kb + 4) * SLICES + 8);
+          ask_scale(next0, (kb + 4) * SLICES);
+          ask_scale(next1, (kb + 4) * SLICES + 8);
         }
-        prefetch_scales(kb + kScaleAhead);
         // the packed box has landed (and, below, the stage's tensor-memory columns are free again: their MMAs completed)
         [[maybe_unused]] const long long t0 = MLD_PAIR_CLOCK();
         if (!mbar_wait(&full_w[ws], static_cast<uint32_t>(iter >> w_shift) & 1u)) {
@@ -712,7 +710,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
           uint32_t o[16];  // o[j] = input channels 32 half + 2j, 2j + 1 of the stage
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const __half2 s2 = __half2half2(one_group ? cur[half] : scale_at(kb * SLICES + 2 * (4 * half + c)));
+            const __half2 s2 = __half2half2(one_group ? __ushort_as_half(half == 0 ? cur0 : cur1) : scale_at(kb * SLICES + 2 * (4 * half + c)));
 #pragma unroll
             for (int qq = 0; qq < 2; ++qq) {
               const Block v = blk[2 * c + qq];
