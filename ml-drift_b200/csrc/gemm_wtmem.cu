@@ -107,8 +107,8 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
 }
 // Arrives on a barrier of the pair's first CTA.  What it orders is tensor memory, by tcgen05.wait and
 // fence::before_thread_sync ahead of it; releasing at cluster scope on top of that would take about 800 cycles.
-__device__ __forceinline__ void arrive_in_pair(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+__device__ __forceinline__ void arrive_in_pair(uint32_t cluster_addr, uint32_t n = 1) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(n) : "memory");
 }
 // Arrives on the barrier (in both CTAs of a pair) once every MMA issued so far has completed.
 template <bool PAIR>
@@ -143,6 +143,11 @@ __device__ __forceinline__ void tmem_dealloc_all(uint32_t taddr) {
 __device__ __forceinline__ uint32_t dq_once(uint32_t biased, __half2 offset, __half2 s2) {
   const __half2 r = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&biased), offset), s2);
   return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// The piece after pc in a share of every `parts`-th unit of `unit` (1 or 2) pieces.
+__device__ __forceinline__ int next_piece(int pc, int unit, int parts) {
+  return unit == 2 && (pc & 1) == 0 ? pc + 1 : pc + 1 + (parts - 1) * unit;
 }
 
 struct WtArgs {
@@ -253,9 +258,10 @@ __global__ void __launch_bounds__(kWtThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t full_ab_lead = PAIR ? map_shared(smem_u32(full_ab), 0) : 0u;
   const uint32_t tmem_empty_lead = PAIR ? map_shared(smem_u32(tmem_empty), 0) : 0u;
-  auto release_tmem = [&](int part, int acc) {
+  // (a pair's accumulators are read by five warps of a quarter or by one, which then arrives for all)
+  auto release_tmem = [&](int part, int parts, int acc) {
     if constexpr (PAIR)
-      arrive_in_pair(tmem_empty_lead);
+      arrive_in_pair(tmem_empty_lead, kDrainParts / parts);
     else if (part == 0)
       mbar_arrive(&tmem_empty[acc]);
   };
@@ -263,8 +269,12 @@ __global__ void __launch_bounds__(kWtThreads, 1)
   auto tile_tok0 = [&](int tile) { return (tile % a.m_tiles) * wa.tile_tok; };
   auto tile_n0 = [&](int tile) { return (tile / a.m_tiles) * CTAS * kWtRows; };
 
-  // Who reads a segment's accumulators: all five warps that can address a lane quarter, or its epilogue warp alone.
-  const auto read_by_all = [&](const Segment&, bool last) { return PAIR || last; };
+  // Who reads a segment's accumulators: the quarter's epilogue warp alone, while the transform warps go on with the next
+  // tile, or all five warps that can address the quarter.  A lone CTA has a second set of accumulators, so that its MMAs go
+  // on, too: all join in for the last segment only.  A pair's MMAs wait for the reading, and the ring holds eight stages: one
+  // warp does for the raw sums that are handed over, but with whole tiles it takes longer than all five (4096 x 14336, 1024
+  // tokens 93.5 us against 86.8; 256 tokens, a handed-over part and a last one: 33.4 against 36.4).
+  const auto read_by_all = [&](const Segment& sg, bool last) { return last || (PAIR && sg.kb0 == 0); };
   // The barrier that a segment's finished MMAs arrive on.  A wait tells one use of a barrier from the one before and no more, so
   // nobody may miss a use of one that it waits on later: segments that the epilogue warp reads alone have barriers that it
   // alone waits on, by accumulators, and those read by all have the third.  (With a segment of a few stages a transform
@@ -273,15 +283,13 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     return &tmem_full[read_by_all(sg, last) ? 2 : PAIR ? 0 : nth & 1];
   };
 
-  // Accumulators -> outputs, the share `part` of `parts` of the warps that can address this lane quarter: pieces of 16 token
-  // columns, part, part + parts, ...  A pair has one set of accumulators, so the quarter's four transform warps, which have
-  // nothing to transform while it is being read, share the reading with its epilogue warp (five parts).  A lone CTA has two:
-  // the epilogue warp reads while the next tile's MMAs run, and the transform warps join in for the last.
+  // Accumulators -> outputs, the share `part` of `parts` of those warps: pieces of 16 token columns, every parts-th (pairs:
+  // two together).
   // A tile cut along K: a pair (CTA) whose share does not begin with the tile's first k-block (always the first of its
   // segments, so that nothing it waits for comes before) leaves its raw accumulators in its own workspace slot; the one that
   // has the first k-block adds the following slots to its own accumulators, in order, and writes the outputs.  Blocks begin
   // in the order of their numbers, so those it waits for hold SMs already, whatever else is on the GPU.  A slot has a flag
-  // per lane quarter and part (lone CTAs, whose writer and reader may be shared differently: per quarter and piece).
+  // per lane quarter and piece (two pieces), since its writer and reader may be shared differently.
   auto drain = [&](const Segment& sg, int part, int parts, int acc) -> bool {
     const int quad = warp & 3;  // TMEM lanes 32*quad .. 32*quad+31 belong to this warp
     const bool hands_over = sg.kb0 > 0, takes_over = !hands_over && sg.kb1 < a.k_blocks;
@@ -289,16 +297,17 @@ __global__ void __launch_bounds__(kWtThreads, 1)
       return reinterpret_cast<uint4*>(a.split_ws) + ((size_t)(slot * CTAS + static_cast<int>(rank)) * 4 + quad) * (8 * 8 * 32) + lane;
     };
     const auto flag_of = [&](int slot, int i) {  // the i-th flag that this warp's share has
-      return a.split_flags + ((slot * CTAS + static_cast<int>(rank)) * 4 + quad) * 8 + (PAIR ? part : part + i * parts);
+      return a.split_flags + ((slot * CTAS + static_cast<int>(rank)) * 4 + quad) * 8 + part + i * parts;
     };
     // the pairs that hold the rest of a tile this pair completes
     const int others = takes_over ? ((sg.tile + 1) * a.k_blocks - 1) / a.units_per_pair - pair : 0;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(PAIR ? 0 : acc * kWtAccCols);
+    constexpr int kUnit = PAIR ? 2 : 1;  // pieces that go together: a quarter has eight flags
     const int n_pieces = wa.tile_tok >> 4;
-    const int n_flags = PAIR ? 1 : part < n_pieces ? (n_pieces - part + parts - 1) / parts : 0;
+    const int n_units = (n_pieces + kUnit - 1) / kUnit, n_flags = part < n_units ? (n_units - part + parts - 1) / parts : 0;
     if (hands_over) {
       uint4* const slot_rows = rows_of(pair);
-      for (int pc = part; pc < n_pieces; pc += parts) {
+      for (int pc = kUnit * part; pc < n_pieces; pc = next_piece(pc, kUnit, parts)) {
         uint32_t r[16];
         tmem_ld16(lane_base + static_cast<uint32_t>(16 * pc), r);
         tmem_ld_wait();
@@ -309,7 +318,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
       tc_before();
       __syncwarp();
       if (lane < n_flags) st_release_gpu(flag_of(pair, lane), a.epoch);
-      if (lane == 0) release_tmem(part, acc);
+      if (lane == 0) release_tmem(part, parts, acc);
       return true;
     }
     if (takes_over) {
@@ -342,7 +351,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
       }
     }
     const int q = lane & 3;  // place among the four channels of the output slice n >> 2
-    for (int pc = part; pc < n_pieces; pc += parts) {
+    for (int pc = kUnit * part; pc < n_pieces; pc = next_piece(pc, kUnit, parts)) {
       const int c0 = 16 * pc;
       uint32_t r[16];
       tmem_ld16(lane_base + static_cast<uint32_t>(c0), r);
@@ -450,7 +459,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     }
     tc_before();
     __syncwarp();
-    if (lane == 0) release_tmem(part, acc);
+    if (lane == 0) release_tmem(part, parts, acc);
     return true;
   };
 
@@ -737,9 +746,6 @@ __global__ void __launch_bounds__(kWtThreads, 1)
       announce();
       xf_iter += sg.kb1 - sg.kb0;
       if (!ok) break;
-      // A pair's segment, a lone CTA's last: the transform warps share the reading with the epilogue warp of their
-      // quarter.  (Measured: reading them only when the ring is full and the next stage blocked, so that the next
-      // tile's first stages are transformed beforehand, costs more in polling than the refill costs here.)
       if (!read_by_all(sg, work.done())) continue;
       const int acc = PAIR ? 0 : nth & 1;
       if (!mbar_wait(accumulators_ready(sg, work.done(), nth), static_cast<uint32_t>(shared++) & 1u)) {
