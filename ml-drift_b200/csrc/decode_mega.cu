@@ -391,9 +391,13 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 // asks for its own box as soon as that is free.  (One lane going through the stages, a few hundred cycles each, refilled an
 // emptied ring of 21 too slowly: 7B step 1256 us, 1236 with this and the residuals off the boxes' path.)  A pass never laps the ring: the use of a stage before a lane's was
 // asked for in an earlier pass, so its release is what the parity of the lane's wait tells apart.
+// The first `ahead` boxes, which fill stages that an earlier op frees, are asked for one to a round of looking: nobody waits for
+// them yet, and bursts of them from every CTA are in the way of the boxes, tiles and vectors that the ops before are waiting for.
+// (32 heads, 8 layers: position 22 279.5 us without, 257.7 with this, 2047 312.6 and 293.6; 40 heads, position 300 380 and 356.
+// With the boxes that an op in progress waits for one by one as well it takes 265, 328 and 423.)
 // Calls ask(i, stage) for i = 0 .. n - 1; false when a wait ran out.
 template <typename Ask>
-__device__ __forceinline__ bool produce(const MegaArgs& a, uint64_t* empty, const Waiter& w, unsigned& pos, int n, int code,
+__device__ __forceinline__ bool produce(const MegaArgs& a, uint64_t* empty, const Waiter& w, unsigned& pos, int n, int ahead, int code,
                                         const Ask& ask) {
   const int lane = threadIdx.x & 31, width = a.stages < 32 ? a.stages : 32;
 #pragma unroll 1
@@ -406,10 +410,12 @@ __device__ __forceinline__ bool produce(const MegaArgs& a, uint64_t* empty, cons
     unsigned long long t0 = 0;
 #pragma unroll 1
     for (int polls = 1;; ++polls) {
-      if (pending && mbar_test_wait(&empty[stage], parity)) {
+      const unsigned ready = __ballot_sync(0xffffffffu, pending && mbar_test_wait(&empty[stage], parity));
+      if ((ready >> lane & 1u) != 0 && (i >= ahead || (ready & ((1u << lane) - 1u)) == 0)) {
         ask(i, stage);
         pending = false;
       }
+      __syncwarp();
       if (!__any_sync(0xffffffffu, pending)) break;
       if ((polls & 63) == 0) {
         // a producer whose wait ran out requests nothing more: stages it cannot know to be free stay
@@ -450,7 +456,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
           runs.bounds(rr, head, lo, hi);
           const int j0 = lo - head * nt;
           // an item is a K tile and a V tile
-          if (!produce(a, empty, w, pos, 2 * (hi - lo), 10, [&](int i, int stage) {
+          if (!produce(a, empty, w, pos, 2 * (hi - lo), 0, 10, [&](int i, int stage) {
                 const CUtensorMap* map = (i & 1) == 0 ? &ly->kc : &ly->vc;
                 uint8_t* st = ring + (size_t)stage * kStageBytes;
                 mbar_arrive_expect_tx(&full[stage], kBox);
@@ -467,7 +473,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
         // chunks (one per consumer warp); ring position kCW j + w takes box j of chunk w
         const uint8_t* boxes = ly->w[map_index(kind)] + (size_t)pi0 * kStageBytes;
         const int B = pi1 - pi0, qn = B / kCW, rn = B % kCW;
-        if (!produce(a, empty, w, pos, B, 11, [&](int i, int stage) {
+        if (!produce(a, empty, w, pos, B, a.stages, 11, [&](int i, int stage) {
               const int j = i / kCW, cw = i - j * kCW;
               mbar_arrive_expect_tx(&full[stage], kStageBytes);
               bulk_load_1d_hint(ring + (size_t)stage * kStageBytes, boxes + (size_t)(cw * qn + (cw < rn ? cw : rn) + j) * kStageBytes,
