@@ -76,6 +76,7 @@ constexpr int kAttDump = kHeadDim + 4;       // 128 outputs, then max and sum (p
 constexpr int kDumpFloats = 2 * kCW * kStripN > kAttnSlots * kCW * kAttDump ? 2 * kCW * kStripN : kAttnSlots * kCW * kAttDump;
 constexpr int kWarpScratch = 3 * kHeadDim;   // attention: rotated q, new k, new v (floats) per warp
 constexpr int kMaxParts = 8;                 // CTAs that share a head at most: the merging part reads the others in two rounds
+constexpr int kOneRound = 4;                 // parts that it reads in one (more, all in flight, cost the kernel registers)
 constexpr int kTraceSlots = 12;              // per (CTA, op): 4 timestamps, warp 0's clocks, all-warps-done, last load issued
 enum { kQkv = 0, kAttn = 1, kO = 2, kGu = 3, kDown = 4, kOpsPerLayer = 5 };
 
@@ -339,11 +340,14 @@ struct AttnSplit {
   __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
     P = G >= heads ? G / heads : 0;
     if (P > kMaxParts) P = kMaxParts;
-    // A short context has no use for parts: one CTA's warps take up to kCW tiles side by side, and merging parts costs two
-    // trips through L2 (publishing and reading the partials).  us a step of 8 (32 heads: 4) layers, all parts / one: 10
-    // tiles 4 heads 169.6 / 159.4, 8 heads 165.1 / 151.8, 16 heads 197.3 / 187.2, 32 heads 157.0 / 152.7; 13 tiles 169.8 /
-    // 178.8, 165.1 / 167.0, 197.6 / 202.9, 157.2 / 158.2.
-    if (nt <= kCW && P > 1) P = 1;
+    // No more parts than give each of a part's warps a tile, while the merging part can read the others in one round: warps
+    // take up to kCW tiles side by side, and merging costs two trips through L2 (publishing and reading the partials), a
+    // round more a third.  us a step of 8 layers with all 8 (24 heads: 6, 32 heads: 4) parts / as many as needed: 13 tiles
+    // 8 heads 169.4 / 154.1, 20 heads 221.9 / 202.8; 19 tiles 16 heads 192.7 / 182.0, 24 heads 232.4 / 221.1; 29 tiles 12 heads
+    // 185.9 / 174.9; 47 tiles 16 heads 194.8 / 187.6; 16 tiles 32 heads 271.3 / 270.0; with 6 of 8 parts for 63 tiles,
+    // 8 heads 168.1 / 172.2.
+    const int needed = (nt + kCW - 1) / kCW;
+    if (needed < P && needed <= kOneRound + 1) P = needed;
   }
   __device__ __forceinline__ void range(int cta, int& i0, int& i1) const {
     if (P > 0) {
@@ -1462,7 +1466,7 @@ __device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
         } else {
           if (trs) trs[9] = globaltimer_ns();
           float TM = -INFINITY, po[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pl = 0.0f;
-          constexpr int kAtOnce = 4;
+          constexpr int kAtOnce = kOneRound;
 #pragma unroll 1
           for (int base = 0; base < pm; base += kAtOnce) {
             float mc[kAtOnce], lc[kAtOnce];

@@ -33,7 +33,7 @@
 //                adds the bias, and four neighbouring lanes exchange values so that each holds the four channels
 //                of one output slice for two tokens, a 16-byte piece of the sliced output layout
 // Tensor memory: columns 0..255 accumulators (one buffer: reading a tile's accumulators is not overlapped with
-// the next tile's MMAs, so the transform warps, idle meanwhile, share the reading with the epilogue warps; a CTA that works
+// the next tile's MMAs, so the transform warps share the reading with the epilogue warps; a CTA that works
 // alone has two buffers of 128), columns 256..511 the weight ring (8 stages x 32 columns).
 // The split of the work over the pairs (tiles of the last wave shared along K) is gemm_pair_kernel's.
 // Every wait is bounded.
@@ -162,9 +162,10 @@ struct WtArgs {
 // tokens: twice as many, smaller tiles, at the price of every CTA fetching all of the tile's tokens.
 // Bound by the transformation (64 x 128 weights a stage and CTA at five instructions for two) beside whatever else the warps
 // issue: a pair's stage takes about 700 cycles, 512 of them its MMAs; a lone CTA's MMAs need 160 to 260.
-// 4096 x 11008 INT4, in a graph: 77 tokens 23.2 us (30.5 with eight warps to a stage and one set of accumulators, 41.1 with
-// pairs and whole tiles); 256 tokens 34.0, 512 48.3 (42.9, 66.7 with stages announced to the pair's first CTA by warps of
-// their own, whose release at cluster scope took longer than a stage).
+// 4096 x 11008 INT4, in a graph: 77 tokens 23.0 us (30.5 with eight warps to a stage and one set of accumulators, 41.1 with
+// pairs and whole tiles); 256 tokens 31.0, 512 45.6 (34.2, 48.5 with all five warps of a quarter reading the sums that are
+// handed over; 42.9, 66.7 with stages announced to the pair's first CTA by warps of their own as well, whose release at
+// cluster scope took longer than a stage).
 constexpr int kWtThreads = 23 * 32;
 template <int MODE>
 constexpr int kWtSlices = MODE == kModeInt8I8 ? 32 : 16;

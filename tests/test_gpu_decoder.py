@@ -113,6 +113,12 @@ def test_decode_step_matches_oracle(mld, oracle, mode, L, heads, ffn, T, pos, bl
 # Small grids reach the work splits a full B200 grid does not: fewer CTAs than heads (heads shared out
 # item by item, several heads per CTA, ticketed merge), a handful of CTAs per head, one CTA for everything;
 # and the last row of the cache (its tile is cut off by the end of the tensor).
+# Attention tiles of 32 tokens, the new token's among them: one part up to 11, two up to 22, ... five up to 55, then eight.
+@pytest.mark.parametrize("pos", [351, 352, 703, 704, 1055, 1056, 1407, 1408, 1759, 1760, 2047])
+def test_parts_of_a_head(mld, oracle, pos):
+    test_decode_step_matches_oracle(mld, oracle, "mega", 1, 2, 256, 2048, pos, 32)
+
+
 @pytest.mark.parametrize("grid,heads,ffn,T,pos", [
     (3, 4, 512, 200, 130),
     (2, 2, 256, 96, 95),
