@@ -253,18 +253,24 @@ int mld_fc_is_gemv_recommended(int32_t precision, int32_t tokens) {
 // pass reads and writes against the flops of the product and converts when the ratio is small, which with its
 // constants means from 200 tokens up.  The same rule with this library's measured costs: a pass costs more the more inputs a
 // channel has, dequantising inside the GEMM a little for every tile of 256 tokens.  us in a graph, inside / converted:
-//   float, K = 8192 and more: 8192 -> 8192 INT4 1024 tokens 97 / 144, 4096 384 / 388; 11008 -> 4096 4096 tokens 267 / 284
-//   float, K = 4096, N K from 32 M: 4096 -> 14336 1024 tokens 92 / 106, 2048 167 / 171, 3072 254 / 238; -> 11008 2048 tokens
-//     135 / 136; and below: 4096 -> 4096 INT4 640 tokens 35.8 / 35.0, 2048 -> 8192 520 tokens 48 / 44
-//   int8 activations: 8192 -> 28672 2048 tokens 379 / 402, 8192 -> 3584 2048 92 / 96, 4096 154 / 151; 4096 -> 14336 1024
-//     tokens 79 / 86, 2048 133 / 124; 4096 -> 4096 640 tokens 40 / 36
+//   float, K = 8192: 8192 -> 8192 INT4 1024 tokens 117 / 158, 2048 253 / 257, 4096 410 / 440
+//   float, K = 4096: 4096 -> 4096 INT4 1024 tokens 34.7 / 35.2, 2048 60.7 / 65.8, 3072 96 / 89; INT8 63 / 71, 92.5 / 91;
+//     -> 6144 INT4 2048 tokens 89.5 / 90.7, 3072 151 / 133; -> 14336 1024 tokens 97 / 118, 2048 159 / 168 (twenty calls in a row,
+//     under the power cap, 212 / 200), 3072 308 / 284
+//   float, K = 3072: -> 8192 INT4 1024 tokens 47.5 / 56.3, 2048 94 / 90; -> 3072 INT8 28.5 / 32.5, 42.5 / 42.3
+//   float below: 2048 -> 2048 INT4 520 tokens 35.3 / 33.7, 1024 23.9 / 23.2; -> 8192 39.1 / 38.5; 1024 -> 4096 21.8 / 20.2
+//   int8 activations: 8192 -> 28672 2048 tokens 371 / 402, 8192 -> 3584 2048 88 / 96, 4096 152 / 154; 4096 -> 14336 1024
+//     tokens 77 / 87, 2048 129 / 124; 4096 -> 4096 520 tokens 34.3 / 32.2, 1024 36.7 / 36.4
 static bool convert_pays(const mld_fc_desc& d, int tokens) {
-  const bool i8 = d.prefill_act_quant != 0;
   int most = 512;
-  if (d.k >= 8192)
-    most = i8 ? 2048 : 4096;
-  else if (d.k >= 4096 && static_cast<int64_t>(d.n) * d.k >= 32 << 20)
-    most = i8 ? 1024 : 2048;
+  if (d.prefill_act_quant != 0) {
+    if (d.k >= 8192)
+      most = 2048;
+    else if (d.k >= 4096 && static_cast<int64_t>(d.n) * d.k >= 32 << 20)
+      most = 1024;
+  } else {
+    most = d.k >= 8192 ? 4096 : d.k >= 4096 ? 2048 : d.k >= 3072 ? 1024 : 512;
+  }
   return tokens > most;
 }
 

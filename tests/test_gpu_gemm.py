@@ -225,6 +225,30 @@ def test_conversion_cost_rule_picks_the_route(mld, oracle):
     plan.close()
 
 
+@pytest.mark.parametrize("K,N,most,act_quant", [(3068, 64, 512, 0), (3072, 64, 1024, 0), (4096, 64, 2048, 0), (8192, 64, 4096, 0),
+                                                 (4096, 64, 512, 1), (4096, 8192, 1024, 1), (8192, 64, 2048, 1)])
+def test_conversion_cost_rule_by_size(mld, K, N, most, act_quant):
+    # the last number of tokens with the weights dequantised inside the GEMM and the first with a conversion pass; both
+    # round the same products to half and differ in the order of the sums only
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    q, s = mld.quantize_weights(torch.randn((N, K), generator=g, device="cuda") * 0.02, 8)
+    packed, _ = mld.pack_weights(q, (N, 1, 1, K), 8)
+    sc = mld.pack_scales(s, True)
+    x = torch.randn((K // 4, most + 1, 4), generator=g, device="cuda").half()
+    outs = []
+    for M, route in ((most, mld.ROUTE_PREFILL_INLINE), (most + 1, mld.ROUTE_PREFILL_CONVERTED)):
+        plan = mld.FullyConnectedPlan(N, K, 8, scale_mode=mld.SCALE_PER_CHANNEL, precision=mld.F32F16, max_tokens=M,
+                                      prefill_act_quant=act_quant)
+        y = torch.empty((N // 4, M, 4), dtype=torch.float16, device="cuda")
+        plan.run(x[:, :M].contiguous(), packed, sc, y, M)
+        torch.cuda.synchronize()
+        assert plan.last_route() == route and plan.device_status() == 0
+        outs.append(y[:, :most].float())
+        plan.close()
+    # (half(u * s) may be fused into the addition of the offset: see test_tiles_cut_along_k)
+    assert float((outs[0] - outs[1]).abs().max() / outs[1].abs().max()) <= 0.05 / 35 + 2.0 ** -11
+
+
 @pytest.mark.parametrize("route", ["auto", "inline"])
 def test_config3_full_size_sampled(mld, oracle, route):
     # the prefill benchmark case: M=1024, K=4096, N=14336, INT4 block 32; the oracle checks 8 sampled tokens
