@@ -48,6 +48,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "ring_order.h"
 
 namespace mld {
 
@@ -391,31 +392,35 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// The whole producer warp: a lane per ring stage, up to `width` of them at a time, each of which waits for its own stage and
-// asks for its own box as soon as that is free.  (One lane going through the stages, a few hundred cycles each, refilled an
-// emptied ring of 21 too slowly: 7B step 1256 us, 1236 with this and the residuals off the boxes' path.)  A pass never laps the ring: the use of a stage before a lane's was
-// asked for in an earlier pass, so its release is what the parity of the lane's wait tells apart.
+// The whole producer warp: a lane per ring stage, each of which waits for its own stage and asks for its own box as soon as
+// that is free.  (One lane going through the stages, a few hundred cycles each, refilled an emptied ring of 21 too slowly: 7B
+// step 1256 us, 1236 with this and the residuals off the boxes' path.)  A pass never laps the ring: the use of a stage before a
+// lane's was asked for in an earlier pass, so its release is what the parity of the lane's wait tells apart.  So that the
+// consumers' waits are as sure, a lane asks only when the lanes `distance` and more below it have found their stages free, too
+// (see ring_order.h; without, a warp that had run ahead of a slower one took the box before last of its stage for its own).
 // The first `ahead` boxes, which fill stages that an earlier op frees, are asked for one to a round of looking: nobody waits for
 // them yet, and bursts of them from every CTA are in the way of the boxes, tiles and vectors that the ops before are waiting for.
 // (32 heads, 8 layers: position 22 279.5 us without, 257.7 with this, 2047 312.6 and 293.6; 40 heads, position 300 380 and 356.
 // With the boxes that an op in progress waits for one by one as well it takes 265, 328 and 423.)
 // Calls ask(i, stage) for i = 0 .. n - 1; false when a wait ran out.
 template <typename Ask>
-__device__ __forceinline__ bool produce(const MegaArgs& a, uint64_t* empty, const Waiter& w, unsigned& pos, int n, int ahead, int code,
-                                        const Ask& ask) {
-  const int lane = threadIdx.x & 31, width = a.stages < 32 ? a.stages : 32;
+__device__ __forceinline__ bool produce(const MegaArgs& a, uint64_t* empty, const Waiter& w, unsigned& pos, int n, int ahead,
+                                        int distance, int code, const Ask& ask) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u, before = ring_lanes_before(lane, distance);
 #pragma unroll 1
-  for (int base = 0; base < n; base += width) {
+  for (int base = 0; base < n; base += a.stages) {
     const int i = base + lane;
-    bool pending = lane < width && i < n;
+    bool pending = lane < a.stages && i < n;
     const unsigned at = pos + i;
     const int stage = static_cast<int>(at % static_cast<unsigned>(a.stages));
     const uint32_t parity = (at / static_cast<unsigned>(a.stages) & 1u) ^ 1u;
     unsigned long long t0 = 0;
 #pragma unroll 1
     for (int polls = 1;; ++polls) {
-      const unsigned ready = __ballot_sync(0xffffffffu, pending && mbar_test_wait(&empty[stage], parity));
-      if ((ready >> lane & 1u) != 0 && (i >= ahead || (ready & ((1u << lane) - 1u)) == 0)) {
+      const bool mine = pending && mbar_test_wait(&empty[stage], parity);
+      const unsigned ready = __ballot_sync(0xffffffffu, mine), waiting = __ballot_sync(0xffffffffu, pending && !mine);
+      if (mine && (waiting & before) == 0 && (i >= ahead || (ready & below) == 0)) {
         ask(i, stage);
         pending = false;
       }
@@ -443,6 +448,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
   const int cta = blockIdx.x, G = gridDim.x;
   const uint64_t pol = policy_evict_first();
   unsigned pos = 0;  // ring stages asked for so far
+  const int proj_distance = ring_distance(a.stages, kCW), attn_distance = ring_attn_distance(a.stages, ring_attn_warps(a.stages, kCW));
   const int nt = a.pos / kTile + 1;
 #pragma unroll 1
   for (int l = 0; l < a.n_layers; ++l) {
@@ -460,7 +466,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
           runs.bounds(rr, head, lo, hi);
           const int j0 = lo - head * nt;
           // an item is a K tile and a V tile
-          if (!produce(a, empty, w, pos, 2 * (hi - lo), 0, 10, [&](int i, int stage) {
+          if (!produce(a, empty, w, pos, 2 * (hi - lo), 0, attn_distance, 10, [&](int i, int stage) {
                 const CUtensorMap* map = (i & 1) == 0 ? &ly->kc : &ly->vc;
                 uint8_t* st = ring + (size_t)stage * kStageBytes;
                 mbar_arrive_expect_tx(&full[stage], kBox);
@@ -477,7 +483,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
         // chunks (one per consumer warp); ring position kCW j + w takes box j of chunk w
         const uint8_t* boxes = ly->w[map_index(kind)] + (size_t)pi0 * kStageBytes;
         const int B = pi1 - pi0, qn = B / kCW, rn = B % kCW;
-        if (!produce(a, empty, w, pos, B, a.stages, 11, [&](int i, int stage) {
+        if (!produce(a, empty, w, pos, B, a.stages, proj_distance, 11, [&](int i, int stage) {
               const int j = i / kCW, cw = i - j * kCW;
               mbar_arrive_expect_tx(&full[stage], kStageBytes);
               bulk_load_1d_hint(ring + (size_t)stage * kStageBytes, boxes + (size_t)(cw * qn + (cw < rn ? cw : rn) + j) * kStageBytes,
@@ -1061,9 +1067,10 @@ __device__ __forceinline__ void run_projection(Ctx& c, const ProjPlan& p, int ki
       const long long w0 = tracing ? clock64() : 0;
       // A parity wait is only right while the barrier is at most one phase behind: the stage's previous
       // use must have been filled before its next filling is waited for.  Its having been released (what
-      // the producer also waits for) says so, and that wait cannot itself be a phase off, because
-      // everything up to a ring's length before this warp's previous box has been released.  The first
-      // ring's length of an op needs none of this: what came before it was used up before the op began.
+      // the producer also waits for) says so, and that wait cannot itself be a phase off, because the
+      // producer asked for this warp's previous box only when the use before that one had been released
+      // (ring_order.h).  The first ring's length of an op needs none of this: what came before it was used
+      // up before the op began.
       if ((b - start) * kCW + warp >= a.stages) wait_released(c.w, &c.empty[stage], phase ^ 1u, 17);
       c.w.wait(&c.full[stage], phase, 12);
       if (tracing) waited += clock64() - w0;
@@ -1181,7 +1188,7 @@ __device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
   // The first aw warps take every aw-th item of the op's sequence; an item is two ring stages.  A warp's
   // items lie 2 aw stages apart, which must not exceed the ring (2 kCW - 1 stages do for kCW warps: the
   // later stage of an item is waited for after the earlier one): shorter rings put fewer warps to work.
-  const int aw = a.stages >= 2 * kCW - 1 ? kCW : a.stages / 2;
+  const int aw = ring_attn_warps(a.stages, kCW);
   int q = warp < aw ? warp : (1 << 30);
   int pos = c.ring_base + 2 * (warp < aw ? warp : 0);
   int stage = pos % a.stages;
@@ -1993,7 +2000,7 @@ int mega_create(const MegaConfig& cfg, MegaDecoder** out) {
   cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg.device);
   int stages = (max_smem - fixed) / (kStageBytes + 16);
   if (cfg.ring_stages >= 2 && cfg.ring_stages < stages) stages = cfg.ring_stages;
-  if (stages > 64) stages = 64;
+  if (stages > 32) stages = 32;  // (a lane of the producer per stage)
   if (stages < kCW + 1) {  // every consumer warp needs a stage of its own in a round
     set_last_error_text("not enough shared memory for the persistent step kernel");
     mega_destroy(m);

@@ -147,7 +147,7 @@ def test_single_kernel_step_on_small_grids(mld, oracle, grid, heads, ffn, T, pos
 
 
 @pytest.mark.parametrize("stages", [12, 16, 20])
-def test_single_kernel_step_with_a_short_ring(mld, oracle, stages):
+def test_single_kernel_step_with_a_short_ring(mld, oracle, stages, grid=0):
     """Rings shorter than two stages per consumer warp (large vectors leave that little shared memory)
     put fewer warps on attention and must give the same step; the step is run several times so that
     consecutive launches, whose vectors carry different tags, are covered too."""
@@ -158,7 +158,7 @@ def test_single_kernel_step_with_a_short_ring(mld, oracle, stages):
     layers_ref, dec_tensors, kc, vc = build_small_decoder(mld, oracle, rng, L, heads, ffn, T, pos)
     x = rng.standard_normal(d).astype(np.float16)
     kcd, vcd = _dev(kc), _dev(vc)
-    dec = _make(mld, "mega", L, d, heads, ffn, T, 32, dec_tensors, kcd, vcd, ring_stages=stages)
+    dec = _make(mld, "mega", L, d, heads, ffn, T, 32, dec_tensors, kcd, vcd, ring_stages=stages, grid_limit=grid)
     y = torch.empty(d, dtype=torch.float16, device="cuda")
     xd = _dev(x)
     outs = []
@@ -174,6 +174,13 @@ def test_single_kernel_step_with_a_short_ring(mld, oracle, stages):
         assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) < 1e-2
     assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[1], outs[2])
     dec.close()
+
+
+# Three CTAs: up to 59 boxes and 86 tiles to one of them, more than twice any ring (0: as many stages as fit), so that a fast
+# warp could get two rings ahead of a slow one if boxes were asked for in any order (see test_ring_order.py).
+@pytest.mark.parametrize("stages", [12, 13, 16, 20, 21, 22, 0])
+def test_single_kernel_step_with_many_boxes_to_a_cta(mld, oracle, stages):
+    test_single_kernel_step_with_a_short_ring(mld, oracle, stages, grid=3)
 
 
 def test_single_kernel_step_ignores_uninitialised_cache_rows(mld, oracle):
