@@ -201,7 +201,7 @@ __device__ __forceinline__ void st_global_32b(uint8_t* p, const uint32_t (&a)[4]
 // A lane's run is stored 32 bytes at a time where every run starts on a 32-byte boundary (WIDE: whole groups of four
 // output slices and of 16 outputs): one whole sector per store instead of four quarter-filled requests.  14336 x 4096 to
 // INT4: 47.2 us, 38.3 with these stores, and 16 less with the exchange of words free of branches.
-// 2^across_shift of the block's eight warps lie side by side along the input channels and gridDim.x such blocks take turns
+// 2^across_shift of the block's eight warps lie side by side along the input channels and gridDim.y such blocks take turns
 // along them, the other warps take further rows.  The sums of a row's weights stay in registers until a block is through;
 // where one block covers all of a row it writes them, and neither atomics nor a fill ahead of the kernel are needed.
 template <int BITS, bool WIDE>
@@ -212,11 +212,11 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_s
   const int hw = blockIdx.z;
   const int across = 1 << across_shift, part = warp & (across - 1);
   const int r = lane >> 3, c = lane & 7;                 // row of the step's four, 16-byte chunk of the 128 inputs
-  const int o0 = (blockIdx.y * (8 >> across_shift) + (warp >> across_shift)) * 16;  // first of the warp's 16 output rows
+  const int o0 = (blockIdx.x * (8 >> across_shift) + (warp >> across_shift)) * 16;  // first of the warp's 16 output rows
   const int8_t* src = reinterpret_cast<const int8_t*>(a.src);
   const uint32_t padw = (a.pad & 0xFFu) * 0x01010101u;
   int32_t rowsum[4] = {0, 0, 0, 0};
-  for (int base = (blockIdx.x * across + part) * 128; base < a.I && o0 < a.dst_slices * 4; base += gridDim.x * across * 128) {
+  for (int base = (blockIdx.y * across + part) * 128; base < a.I && o0 < a.dst_slices * 4; base += gridDim.y * across * 128) {
     const int i0 = base + c * 16;                          // first input channel of this lane's chunk
     uint32_t blk[4][4];                                    // [step = output slice][word k = input channel of the block]
     uint4 v4[4];
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_s
     int32_t v = 0;
     for (int w = 0; w < across; ++w) v += sums[warp + w][lane];
     if (o < a.O && o < a.sum_len) {
-      if (gridDim.x == 1 && gridDim.z == 1)
+      if (gridDim.y == 1 && gridDim.z == 1)
         a.sum_i[o] = v;
       else if (v != 0)
         atomicAdd(a.sum_i + o, v);
@@ -594,7 +594,8 @@ int pack_weights_impl(const mld_pack_desc* d, const void* src, void* dst, int32_
     const int most = div_up(chunks, 1 << across_shift);
     int beside = div_up(kPackBlocks, blocks);
     if (beside > most) beside = most;
-    dim3 rgrid(beside, div_up(a.dst_slices * 4, rows), a.HW);
+    // (the rows along x, where a grid may have 2^31 blocks: a block has no more than 16 of them)
+    dim3 rgrid(div_up(a.dst_slices * 4, rows), beside, a.HW);
     if (beside > 1 || a.HW > 1) MLD_CUDA_CHECK(clear_sums());
     const bool wide = a.dst_slices % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
     const auto kern = d->bits == 8 ? (wide ? pack_rows_kernel<8, true> : pack_rows_kernel<8, false>)

@@ -211,3 +211,16 @@ def test_pack_rows_sums(mld, oracle, shape, bits):
         torch.cuda.synchronize()
         assert np.array_equal(got.cpu().numpy(), ref)
         assert np.array_equal(sums.cpu().numpy(), oracle.weights_sum_i(q))
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+def test_pack_rows_of_a_tall_matrix(mld, bits):
+    # more than 65535 blocks of rows (16 to a block from 1024 inputs on); the layout in plain torch: [I/4][O/4][4 inputs][4 outputs]
+    O, I = 16 * 65536, 1024
+    lo, hi = (-128, 128) if bits == 8 else (-8, 8)
+    q = torch.randint(lo, hi, (O, I), generator=torch.Generator(device="cuda").manual_seed(bits), device="cuda", dtype=torch.int8)
+    got, sums = mld.pack_weights(q, (O, 1, 1, I), bits, want_sum=True)
+    torch.cuda.synchronize()
+    assert torch.equal(sums, q.sum(1, dtype=torch.int32))
+    u = (q.to(torch.int16) - lo).to(torch.uint8).reshape(O // 4, 4, I // 4, 4).permute(2, 0, 3, 1).reshape(-1)
+    assert torch.equal(got.view(torch.uint8).reshape(-1), u if bits == 8 else u[0::2] | u[1::2] << 4)
