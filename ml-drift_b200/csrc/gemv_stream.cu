@@ -928,6 +928,10 @@ int launch_strip_t(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorM
   if constexpr (W == 2 && MONE && !SPLIT) {  // (one token, strips of two whole boxes)
     if (gm.ksplit > 2) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, false, true>(tw, ts, tz, a, gm, stream);
   }
+  if (gm.ksplit > 2) {  // (the other forms add up two parts and would drop the rest)
+    set_last_error_text("no form of the streaming kernel adds up more than two parts of K for these strips");
+    return MLD_UNIMPLEMENTED;
+  }
   if constexpr (W == 2) {  // (strips of several passes with pdl are two boxes wide)
     if (!MONE || gm.interleave) return launch_strip_f<BITS, W, SUBNORMAL, MONE, DIGITS, ZP, SPLIT, true>(tw, ts, tz, a, gm, stream);
   }
@@ -991,14 +995,15 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
   if (strips < 1) strips = 1;
   gm.strips = strips;
   gm.grid = strips * gm.ksplit;
-  const int max_width = div_up(gm.units, strips) * gm.gran;  // chunks
+  int max_width = div_up(gm.units, strips) * gm.gran;  // chunks
   int w = div_up(max_width, 8);
   if (gm.ksplit > 1 && w > w_max) {  // a cluster pair runs a single pass
     gm.ksplit = 1;
     strips = sms < gm.units ? sms : gm.units;
     gm.strips = strips;
     gm.grid = strips;
-    w = div_up(div_up(gm.units, strips) * gm.gran, 8);
+    max_width = div_up(gm.units, strips) * gm.gran;
+    w = div_up(max_width, 8);
   }
   // One token: strips that fill their boxes, where the rule above leaves part of them empty or splits what is small already.
   // us in a graph, INT4 block 32 unless said otherwise, the rule above / as here.
@@ -1017,10 +1022,11 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
       // (4 x 64), 4096 x 22016 14.8 / 13.1, 1536 x 21568 8.9 / 6.7, INT8 4096 x 11008 13.9 / 12.8.  On the other side of the
       // line: clusters of three (4736 x 8320 7.6 / 8.7), fewer than sixteen stages to cut (INT8 2432 x 6048 6.0 / 6.4) and
       // idle SMs (2048 x 16384 6.2 / 7.6).
+      // (Only where strips reach into their second box: the form for more than two parts has two.)
       const int full = div_up(C, 16);
       if (full >= sms) {
         S = 1;
-      } else if (n_st >= 16) {
+      } else if (n_st >= 16 && C > 8) {
         for (int s = 2; s <= 8 && full * s <= most; ++s) {
           if (s == 3) continue;
           S = s;
@@ -1034,7 +1040,8 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
       gm.ksplit = S;
       gm.strips = strips = div_up(C, 8 * boxes);
       gm.grid = strips * S;
-      w = div_up(div_up(gm.units, strips) * gm.gran, 8);
+      max_width = div_up(gm.units, strips) * gm.gran;
+      w = div_up(max_width, 8);
     }
   }
   gm.w = w > w_max ? w_max : w;
