@@ -442,6 +442,14 @@ def cpu_best_of(fn, reps=10, warm=3, budget_s=8.0):
     return best
 
 
+# The ways the operator serves a prefill call: prefill_route, cache_prepared_weights, and the route the label stands for, which
+# the run must have taken: the weights dequantised inside the GEMM, a conversion pass before a plain GEMM on every call, the
+# converted copy kept between calls, and what the conversion-cost rule picks at the entry's size (its "route" says which).
+PREFILL_ROUTES = {"dequantised_inside_gemm": (1, False, "inside"), "with_weight_conversion": (2, False, "converted"),
+                  "weights_prepared_once": (0, True, "cached"), "auto": (0, False, None)}
+PREFILL_ROUTE_NAMES = {3: "inside", 4: "converted", 5: "cached"}  # mld_fc_plan_last_route
+
+
 def side_benchmarks(mld, torch, peaks):
     """The kernel-level figures the metric also names, each kernel timed alone with CUDA events, with
     the CPU restatement of the same operation timed on the host's cores beside it."""
@@ -591,12 +599,7 @@ def side_benchmarks(mld, torch, peaks):
     yy = torch.empty((N // 4, M, 4), dtype=torch.float16, device="cuda")
     flops = 2.0 * M * K * N
     res = {}
-    # the three ways the operator serves a prefill call: the weights dequantised inside the GEMM (route 1),
-    # a conversion pass before a plain GEMM on every call (route 0: what the conversion-cost rule picks at
-    # this M), and the converted copy kept between calls
-    ROUTES = (("dequantised_inside_gemm", 1, False), ("with_weight_conversion", 0, False),
-              ("weights_prepared_once", 0, True))
-    for label, route, cache in ROUTES:
+    for label, (route, cache, kind) in PREFILL_ROUTES.items():
         plan = mld.FullyConnectedPlan(N, K, 4, scale_mode=mld.SCALE_BLOCK, groups=K // blk, precision=mld.F32F16,
                                       max_tokens=M, force_path=mld.PATH_GEMM, cache_prepared_weights=cache,
                                       prefill_route=route)
@@ -609,7 +612,10 @@ def side_benchmarks(mld, torch, peaks):
         e1.record()
         torch.cuda.synchronize()
         us = e0.elapsed_time(e1) * 1e3 / 20
-        res[label] = {"us": us, "TFLOPs": flops / us / 1e6}
+        took = PREFILL_ROUTE_NAMES.get(plan.last_route())
+        if kind not in (None, took):
+            raise RuntimeError(f"{label}: the plan took the {took} route")
+        res[label] = {"us": us, "TFLOPs": flops / us / 1e6, "route": took}
         plan.close()
     pk = peaks.get("bf16_tflops") or 1590.0
     # CPU restatement on a sample of the tokens (the work is linear in M)
@@ -635,7 +641,7 @@ def side_benchmarks(mld, torch, peaks):
     yy = torch.empty((N // 4, M, 4), dtype=torch.float16, device="cuda")
     ops = 2.0 * M * K * N
     res = {}
-    for label, route, cache in ROUTES:
+    for label, (route, cache, kind) in PREFILL_ROUTES.items():
         plan = mld.FullyConnectedPlan(N, K, 8, scale_mode=mld.SCALE_PER_CHANNEL, precision=mld.F32F16, max_tokens=M,
                                       force_path=mld.PATH_GEMM, prefill_act_quant=2, cache_prepared_weights=cache,
                                       prefill_route=route)
@@ -649,7 +655,10 @@ def side_benchmarks(mld, torch, peaks):
         e1.record()
         torch.cuda.synchronize()
         us = e0.elapsed_time(e1) * 1e3 / 20
-        res[label] = {"us": us, "TOPs": ops / us / 1e6}
+        took = PREFILL_ROUTE_NAMES.get(plan.last_route())
+        if kind not in (None, took):
+            raise RuntimeError(f"{label}: the plan took the {took} route")
+        res[label] = {"us": us, "TOPs": ops / us / 1e6, "route": took}
         plan.close()
     out["prefill_gemm_w8a8_shard"] = {
         "workload": "W8A8 GEMM M=2048 K=8192 N=3584 (one rank's eighth of N=28672): asymmetric per-token int8 "
