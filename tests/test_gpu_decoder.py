@@ -110,15 +110,40 @@ def test_decode_step_matches_oracle(mld, oracle, mode, L, heads, ffn, T, pos, bl
     dec.close()
 
 
-# Small grids reach the work splits a full B200 grid does not: fewer CTAs than heads (heads shared out
-# item by item, several heads per CTA, ticketed merge), a handful of CTAs per head, one CTA for everything;
-# and the last row of the cache (its tile is cut off by the end of the tensor).
 # Attention tiles of 32 tokens, the new token's among them: one part up to 11, two up to 22, ... five up to 55, then eight.
 @pytest.mark.parametrize("pos", [351, 352, 703, 704, 1055, 1056, 1407, 1408, 1759, 1760, 2047])
 def test_parts_of_a_head(mld, oracle, pos):
     test_decode_step_matches_oracle(mld, oracle, "mega", 1, 2, 256, 2048, pos, 32)
 
 
+@pytest.mark.parametrize("mode", ["mega", "mega_barriers"])
+def test_parts_of_a_head_change_from_step_to_step(mld, oracle, mode):
+    # one decoder over positions of one, two, five and eight parts, up and down: what parts of an earlier step left behind must
+    # not be taken for this step's
+    from oracle import decode_ref
+    rng = np.random.default_rng(3)
+    L, heads, ffn, T = 2, 2, 256, 2048
+    d = heads * 128
+    layers_ref, dec_tensors, kc, vc = build_small_decoder(mld, oracle, rng, L, heads, ffn, T, T - 1)
+    kcd, vcd, kref, vref = _dev(kc), _dev(vc), kc.astype(np.float32), vc.astype(np.float32)
+    dec = _make(mld, mode, L, d, heads, ffn, T, 32, dec_tensors, kcd, vcd)
+    steps = [351, 352, 703, 704, 1759, 1760, 353, 350, 1761, 705, 2047, 0, 1760, 352]
+    xs = rng.standard_normal((len(steps), d)).astype(np.float16)
+    xd, y = _dev(xs), torch.empty((len(steps), d), dtype=torch.float16, device="cuda")
+    for i, pos in enumerate(steps):
+        dec.step(xd[i], y[i], pos)
+    torch.cuda.synchronize()
+    assert dec.device_status() == 0
+    got = y.float().cpu().numpy()
+    for i, pos in enumerate(steps):
+        ref = decode_ref.decode_step(xs[i].astype(np.float32), layers_ref, kref, vref, pos, heads, 128, ffn)
+        assert np.isfinite(got[i]).all() and np.max(np.abs(got[i] - ref)) / np.max(np.abs(ref)) < 1e-2
+    dec.close()
+
+
+# Small grids reach the work splits a full B200 grid does not: fewer CTAs than heads (heads shared out
+# item by item, several heads per CTA, ticketed merge), a handful of CTAs per head, one CTA for everything;
+# and the last row of the cache (its tile is cut off by the end of the tensor).
 @pytest.mark.parametrize("grid,heads,ffn,T,pos", [
     (3, 4, 512, 200, 130),
     (2, 2, 256, 96, 95),

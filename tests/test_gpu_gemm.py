@@ -135,6 +135,13 @@ def test_w8a8_weights_in_tensor_memory(mld, oracle, rule, M, K, N):
     test_w8a8_prefill_vs_oracle(mld, oracle, rule, "inline", False, M, K, N)
 
 
+# ... and in shared memory, the form of prefill_route 3; the last as above
+@pytest.mark.parametrize("rule", ["symmetric", "asymmetric"])
+@pytest.mark.parametrize("M,K,N", [(64, 128, 32), (130, 1040, 264), (32, 8192, 96), (300, 2048, 520), (1100, 384, 4608)])
+def test_w8a8_weights_in_shared_memory(mld, oracle, rule, M, K, N):
+    test_w8a8_prefill_vs_oracle(mld, oracle, rule, "inline_smem", False, M, K, N)
+
+
 def test_w8a8_shard_of_the_eight_way_split(mld, oracle):
     """One rank's share of the W8A8 prefill case that is split eight ways over N: M=2048, K=8192,
     N=3584 of 28672, asymmetric per-token activations.  Sampled tokens against the restated chain: the
@@ -247,6 +254,28 @@ def test_conversion_cost_rule_by_size(mld, K, N, most, act_quant):
         plan.close()
     # (half(u * s) may be fused into the addition of the offset: see test_tiles_cut_along_k)
     assert float((outs[0] - outs[1]).abs().max() / outs[1].abs().max()) <= 0.05 / 35 + 2.0 ** -11
+
+
+@pytest.mark.parametrize("K,N,most", [(4096, 64, 512), (4096, 8192, 1024), (8192, 64, 2048)])
+def test_int8_activations_either_side_of_the_cost_rule(mld, K, N, most):
+    # symmetric per-token activations: the sums are exact integers on both routes and each output is one product of three
+    # factors taken in the same order, so the bits are the same
+    g = torch.Generator(device="cuda").manual_seed(K + N + most)
+    q, s = mld.quantize_weights(torch.randn((N, K), generator=g, device="cuda") * 0.02, 8)
+    packed, _ = mld.pack_weights(q, (N, 1, 1, K), 8)
+    sc = mld.pack_scales(s, True)
+    x = torch.randn((K // 4, most + 1, 4), generator=g, device="cuda").half()
+    outs = []
+    for M, route in ((most, mld.ROUTE_PREFILL_INLINE), (most + 1, mld.ROUTE_PREFILL_CONVERTED)):
+        plan = mld.FullyConnectedPlan(N, K, 8, scale_mode=mld.SCALE_PER_CHANNEL, precision=mld.F32F16, max_tokens=M,
+                                      prefill_act_quant=1)
+        y = torch.empty((N // 4, M, 4), dtype=torch.float16, device="cuda")
+        plan.run(x[:, :M].contiguous(), packed, sc, y, M)
+        torch.cuda.synchronize()
+        assert plan.last_route() == route and plan.device_status() == 0
+        outs.append(y[:, :most])
+        plan.close()
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
 
 
 @pytest.mark.parametrize("route", ["auto", "inline"])
