@@ -2179,7 +2179,6 @@ int mega_read_trace(MegaDecoder* m, unsigned long long* out, size_t count) {
 #endif
 int mega_grid(const MegaDecoder* m) { return m->grid; }
 
-const int* mega_error_word(const MegaDecoder* m) { return m->error; }
 void* mega_result(const MegaDecoder* m) { return reinterpret_cast<uint8_t*>(m->error) - (size_t)m->cfg.d_model * 2; }
 
 // Back to the state after creation: counters zero, no tagged word or record valid.  (Tags and record epochs

@@ -159,7 +159,6 @@ int mega_set_layer(MegaDecoder* m, int layer, const MegaLayerPtrs& p);
 int mega_step(MegaDecoder* m, const void* x_in, void* x_out, int pos, cudaStream_t stream);
 // Reads (and clears) the kernel's error word: 0 = every wait of the last steps was satisfied.
 int mega_device_status(MegaDecoder* m, int* code);
-const int* mega_error_word(const MegaDecoder* m);
 // Room for a step's result vector with the error word right behind it, so that one copy brings both to the host.
 void* mega_result(const MegaDecoder* m);
 int mega_reset(MegaDecoder* m);

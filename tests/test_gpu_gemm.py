@@ -1,9 +1,9 @@
 """Prefill dequant-GEMM (tcgen05) through the C ABI vs the CPU oracle.
 
-Every case runs on each route: "inline" (the GEMM reads the packed weights and dequantises them in shared
-tensor memory - or, "inline_smem", in shared memory; what the cost rule picks up to 512 tokens), "convert" (a conversion pass writes a K-major copy and
-a GEMM with both operands loaded by TMA follows; the rule's pick above 512 tokens) and "cached" (the
-same with the copy kept between calls).  All apply the same arithmetic to every weight.
+Every case runs on each route: "inline" (the GEMM reads the packed weights and dequantises them in
+tensor memory - or, "inline_smem", in shared memory; what the cost rule picks up to 512 to 4096 tokens, by the sizes),
+"convert" (a conversion pass writes a K-major copy and a GEMM with both operands loaded by TMA follows; the rule's pick
+above that) and "cached" (the same with the copy kept between calls).  All apply the same arithmetic to every weight.
 Float route: tolerance 1e-3 of max |ref| against the restated WeightsConverter + fp32-accumulate GEMM
 (fp16 operands, exact products).  Int8-activation route: the int32 accumulators are exact, so outputs
 agree with the restated Quantize -> int GEMM -> Dequantization chain to fp16 rounding."""
