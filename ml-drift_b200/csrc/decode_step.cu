@@ -509,11 +509,10 @@ int attn_resident_heads(int parts) {
   return n;
 }
 
+// Launches the parts asked for (see attn_shape), or fewer where the runtime has no room for that many clusters.
 template <int WARPS>
 int launch_attn_decode_t(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
-                         int max_parts, cudaStream_t stream) {
-  int parts = div_up(n_tokens, WARPS * 4 * kAttnAhead);  // no more than each has tokens for one round of its warps
-  if (parts > max_parts) parts = max_parts;
+                         int parts, cudaStream_t stream) {
   while (parts > 1 && attn_resident_heads<WARPS>(parts) < heads) --parts;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attrs[2];
@@ -524,19 +523,44 @@ int launch_attn_decode_t(const __half* q, const __half* kcache, const __half* vc
   return MLD_OK;
 }
 
-// CTAs that share a head: as many as let the whole launch be resident at once, because a head that has to wait for another
-// one's cluster costs a second wave.  us in a graph, K and V from HBM, eight warps: 32 heads of 8191 tokens in 7 / 8 / 10 /
-// 16 parts 24.6 / 23.3 / 32.9 / 32.2, 40 heads in 6 / 7 28.2 / 40.4, 16 heads in 8 / 12 / 16 17.6 / 16.0 / 20.1, 12 heads
-// 15.4 / 14.9 / 12.8.  CTAs of eight warps beat those of four with long caches (64 heads 41.3 / 42.2, 32 heads 23.3 / 31.9);
-// up to 512 tokens, eight rounds of four warps, the smaller CTAs start and merge sooner (16 heads: 64 tokens 2.6 / 3.3, 200
-// tokens 3.6 / 3.9, 500 tokens 4.7 / 4.7).
-int launch_attn_decode(const __half* q, const __half* kcache, const __half* vcache, __half* out, int heads, int n_tokens,
-                       cudaStream_t stream) {
-  if (n_tokens <= 8 * 4 * 4 * kAttnAhead) return launch_attn_decode_t<4>(q, kcache, vcache, out, heads, n_tokens, 8, stream);
-  return launch_attn_decode_t<8>(q, kcache, vcache, out, heads, n_tokens, kMaxAttnParts, stream);
-}
-
 }  // namespace
+
+// How many CTAs share a head, and of how many warps: as many as let the whole launch be resident at once, because a head that
+// has to wait for another one's cluster costs a second wave.  us in a graph, K and V from HBM, eight warps: 32 heads of 8191
+// tokens in 7 / 8 / 10 / 16 parts 24.6 / 23.3 / 32.9 / 32.2, 40 heads in 6 / 7 28.2 / 40.4, 12 heads in 8 / 12 / 16 15.4 / 14.9 /
+// 12.8.  The runtime's count of clusters that fit promises more than finds places: it has room for 56 clusters of five, but 56
+// heads of 2000 tokens take 18.7 us that way and 12.9 with four; 17 heads of 4000 tokens in 13 / 12 parts 12.3 / 10.6, 21 in
+// 12 / 11 14.3 / 11.2, 28 in 9 / 8 13.6 / 13.0; four warps, 400 tokens, 75 heads in 7 / 6 8.9 / 7.5, 112 heads in 5 / 4 11.4 /
+// 8.0.  So clusters of three to eight take seven eighths of the warps' places at most, those of nine to fifteen seven tenths;
+// of sixteen, which fit the GPCs by twos, the count is right (14 heads of 8000 tokens in 14 / 16 14.7 / 13.4, 15 heads 21.7 /
+// 19.5, and 14.6 in 13).
+// CTAs of eight warps beat those of four with long caches (64 heads 41.3 / 42.2, 32 heads 23.3 / 31.9) unless fewer warps come of
+// it (4000 tokens, eight / four: 96 heads in 2 / 5 34.1 / 33.0, 151 heads in 1 / 3 56.6 / 48.9) or they are not all resident (400
+// heads of 1000 tokens 38.3 / 34.2).  Up to 512 tokens, eight rounds of four warps, the smaller CTAs start and merge sooner
+// (16 heads: 64 tokens 2.6 / 3.3, 200 tokens 3.6 / 3.9, 500 tokens 4.7 / 4.7), but one CTA beats a cluster where a round of
+// eight warps does (8 heads: 100 tokens 3.2 / 3.5, 148 heads 4.4 / 5.1).
+AttnShape attn_shape(int heads, int n_tokens, int sms, int heads_by_16) {
+  const auto within = [](int v, int lo, int hi) { return v < lo ? lo : v > hi ? hi : v; };
+  const int four = within(7 * sms / 2 / heads, 1, 9);
+  int eight = heads <= sms ? within(7 * sms / 4 / heads, 2, kMaxAttnParts) : 1;
+  if (heads > heads_by_16 && eight > 15) eight = 15;
+  AttnShape s;
+  if (heads > 2 * sms)
+    s.warps = 4;
+  else if (n_tokens <= 8 * 4 * 4 * kAttnAhead)
+    s.warps = n_tokens > 4 * 4 * kAttnAhead && n_tokens <= 8 * 4 * kAttnAhead ? 8 : 4;
+  else
+    s.warps = 2 * eight >= four ? 8 : 4;
+  // no more than each has tokens for one round of its warps, and beyond eight none that saves no round (20 heads of 2000 tokens in
+  // 8 / 10 parts, two rounds each, 8.0 / 8.3)
+  const int rounds = div_up(n_tokens, s.warps * 4 * kAttnAhead);
+  s.parts = within(s.warps == 8 ? eight : four, 1, rounds);
+  if (s.warps == 8 && s.parts > 8 && s.parts < 16) {
+    s.parts = within(7 * sms / 5 / heads, 8, s.parts);
+    s.parts = within(div_up(rounds, div_up(rounds, s.parts)), 8, 15);
+  }
+  return s;
+}
 
 Nccl& nccl() {
   static Nccl instance;
@@ -637,9 +661,10 @@ static int attn_decode(const void* q, const void* kcache, const void* vcache, vo
   int device = 0;
   MLD_CUDA_CHECK(cudaGetDevice(&device));
   MLD_REQUIRE(device < 64, "device ordinal too large");
-  return launch_attn_decode(static_cast<const __half*>(q), static_cast<const __half*>(kcache),
-                            static_cast<const __half*>(vcache), static_cast<__half*>(out), heads, n_tokens,
-                            static_cast<cudaStream_t>(stream));
+  const AttnShape s = attn_shape(heads, n_tokens, sm_count(device), attn_resident_heads<8>(kMaxAttnParts));
+  return (s.warps == 8 ? launch_attn_decode_t<8> : launch_attn_decode_t<4>)(
+      static_cast<const __half*>(q), static_cast<const __half*>(kcache), static_cast<const __half*>(vcache),
+      static_cast<__half*>(out), heads, n_tokens, s.parts, static_cast<cudaStream_t>(stream));
 }
 
 int mld_attn_decode(const void* q, const void* kcache, const void* vcache, void* out, int32_t heads, int32_t head_dim,

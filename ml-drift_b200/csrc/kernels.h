@@ -109,6 +109,13 @@ struct StripArgs {
   int trace_skip_math;        // tuning builds only: consume the stages without computing
 };
 
+// How decode attention splits its heads: CTAs of `warps` warps, `parts` of them to a head.  heads_by_16: how many heads the device
+// holds at once in clusters of 16 CTAs of eight warps.
+struct AttnShape {
+  int warps, parts;
+};
+AttnShape attn_shape(int heads, int n_tokens, int sms, int heads_by_16);
+
 struct StripGeometry {
   int gran, units, strips, ksplit, grid, w;
   int rows_per_split;

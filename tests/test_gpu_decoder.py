@@ -474,6 +474,14 @@ def test_attention_decode_resident_parts(mld, heads, n_tokens):
     test_attention_decode_parts(mld, heads, n_tokens)
 
 
+# either side of 64 and 128 tokens, of one CTA to a head (148 heads), of all CTAs resident (296), and odd numbers of parts
+@pytest.mark.parametrize("heads,n_tokens", [
+    (8, 64), (8, 65), (8, 128), (8, 129), (56, 2000), (75, 400), (70, 700), (96, 1500), (112, 500), (140, 600), (148, 700),
+    (149, 700), (151, 2000), (172, 513), (173, 513), (296, 100), (296, 513), (297, 100), (297, 513), (600, 130)])
+def test_attention_decode_splits_of_the_heads(mld, heads, n_tokens):
+    test_attention_decode_parts(mld, heads, n_tokens)
+
+
 def test_attention_decode_on_two_streams(mld):
     g = torch.Generator(device="cuda").manual_seed(3)
     cases = []
