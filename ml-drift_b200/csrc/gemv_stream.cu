@@ -1018,12 +1018,17 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
     } else if (C <= 16 * most) {
       // Strips of two whole boxes.  As many as SMs or more, or K cut so that a CTA has up to eight stages (it also turns that
       // much of the vector into digits) where clusters of that size are all resident at once and every SM has work: 4096 x
-      // 11008 10.0 / 9.0 (2 x 86 CTAs; 3 x 86 9.2), 4096 x 14336 10.0 / 9.5, 14336 x 4096 12.9 / 9.9, 8192 x 8192 11.0 / 10.2
-      // (4 x 64), 4096 x 22016 14.8 / 13.1, 1536 x 21568 8.9 / 6.7, INT8 4096 x 11008 13.9 / 12.8.  On the other side of the
+      // 11008 10.0 / 9.0 (2 x 86 CTAs; 3 x 86 9.2), 4096 x 14336 10.0 / 9.5, 14336 x 4096 12.9 / 10.3,
+      // 4096 x 22016 14.8 / 13.1, 1536 x 21568 8.9 / 6.7, INT8 4096 x 11008 13.9 / 12.8.  On the other side of the
       // line: clusters of three (4736 x 8320 7.6 / 8.7), fewer than sixteen stages to cut (INT8 2432 x 6048 6.0 / 6.4) and
       // idle SMs (2048 x 16384 6.2 / 7.6).
       // (Only where strips reach into their second box: the form for more than two parts has two.)
-      const int full = div_up(C, 16);
+      // More than two parts only where the rule above fills its boxes badly for the number of stages that there are to share out:
+      // smaller parts and the longer meeting cost more than empty chunks in short strips (per cent of the boxes filled:
+      // 4608 x 8192 86 7.9 / 8.9, INT8 4608 x 3072 65 6.6 / 7.2, INT8 6144 x 4096 86 8.2 / 9.3, 8704 x 4584 97 8.2 / 8.8; on the other side
+      // 6144 x 5120 54 8.9 / 7.9, 10240 x 5120 54 13.1 / 9.8, 14336 x 4096 86 12.9 / 10.3, 16384 x 4608 97 14.4 / 13.0).
+      const int full = div_up(C, 16), filled = 100 * C / (strips * w * 8);
+      const int line = n_st >= 60 ? 100 : n_st >= 40 ? 90 : 2 * n_st + 10;
       if (full >= sms) {
         S = 1;
       } else if (n_st >= 16 && C > 8) {
@@ -1032,7 +1037,7 @@ StripGeometry strip_geometry(int bits, int N, int K, int m_total, int group_slic
           S = s;
           if (div_up(n_st, s) <= 8) break;
         }
-        if (full * S < sms) S = 0;
+        if (full * S < sms || (S > 2 && filled > line)) S = 0;
       }
     }
     if (S > 0) {

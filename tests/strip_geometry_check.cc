@@ -6,6 +6,16 @@
 
 int main() {
   using namespace mld;
+  // one token on 148 SMs: K cut into more than two parts only where it pays
+  const int parts[][4] = {{4, 8192, 4608, 2}, {8, 3072, 4608, 2}, {8, 4096, 6144, 2}, {4, 4584, 8704, 2},  // bits, N, K, parts
+                          {4, 5120, 6144, 4}, {4, 5120, 10240, 5}, {4, 4096, 14336, 7}, {4, 4608, 16384, 7}};
+  for (const auto& c : parts) {
+    const StripGeometry g = strip_geometry(c[0], c[1], c[2], 1, 8, MLD_SCALE_BLOCK, 148, true, 0, false, true);
+    if (g.ksplit != c[3]) {
+      printf("bits %d N %d K %d: %d parts\n", c[0], c[1], c[2], g.ksplit);
+      return 1;
+    }
+  }
   long n = 0;
   for (int sms : {1, 2, 3, 4, 6, 8, 9, 16, 74, 147, 148})
     for (int bits : {4, 8})
