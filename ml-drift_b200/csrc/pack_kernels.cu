@@ -10,7 +10,6 @@ namespace mld {
 
 namespace {
 
-constexpr int kPackBlocks = 256;                 // blocks that pack_rows_kernel's grid has at least, where the rows allow
 constexpr int kTileSlices = 32;                  // 32 x 32 blocks of 4x4 per CTA
 constexpr int kTileCh = kTileSlices * 4;         // 128 channels each way
 constexpr int kRowPitch = kTileSlices * 16 + 4;  // bytes per src-slice row of the staged tile (+4: bank spread)
@@ -201,22 +200,24 @@ __device__ __forceinline__ void st_global_32b(uint8_t* p, const uint32_t (&a)[4]
 // A lane's run is stored 32 bytes at a time where every run starts on a 32-byte boundary (WIDE: whole groups of four
 // output slices and of 16 outputs): one whole sector per store instead of four quarter-filled requests.  14336 x 4096 to
 // INT4: 47.2 us, 38.3 with these stores, and 16 less with the exchange of words free of branches.
-// 2^across_shift of the block's eight warps lie side by side along the input channels and gridDim.y such blocks take turns
-// along them, the other warps take further rows.  The sums of a row's weights stay in registers until a block is through;
-// where one block covers all of a row it writes them, and neither atomics nor a fill ahead of the kernel are needed.
+// 2^across_shift of the block's eight warps lie side by side along the input channels and `beside` blocks, whose numbers follow
+// each other, take turns along them; the other warps take further rows.  The sums of a row's weights stay in registers until a
+// block is through; where one block covers all of a row it writes them, and neither atomics nor a fill ahead of the kernel are
+// needed.
 template <int BITS, bool WIDE>
-__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_shift) {
+__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_shift, int beside) {
   pdl_wait();
   __shared__ int32_t sums[8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hw = blockIdx.z;
   const int across = 1 << across_shift, part = warp & (across - 1);
+  const int row_block = blockIdx.x / beside, turn = blockIdx.x - row_block * beside;
   const int r = lane >> 3, c = lane & 7;                 // row of the step's four, 16-byte chunk of the 128 inputs
-  const int o0 = (blockIdx.x * (8 >> across_shift) + (warp >> across_shift)) * 16;  // first of the warp's 16 output rows
+  const int o0 = (row_block * (8 >> across_shift) + (warp >> across_shift)) * 16;  // first of the warp's 16 output rows
   const int8_t* src = reinterpret_cast<const int8_t*>(a.src);
   const uint32_t padw = (a.pad & 0xFFu) * 0x01010101u;
   int32_t rowsum[4] = {0, 0, 0, 0};
-  for (int base = (blockIdx.y * across + part) * 128; base < a.I && o0 < a.dst_slices * 4; base += gridDim.y * across * 128) {
+  for (int base = (turn * across + part) * 128; base < a.I && o0 < a.dst_slices * 4; base += beside * across * 128) {
     const int i0 = base + c * 16;                          // first input channel of this lane's chunk
     uint32_t blk[4][4];                                    // [step = output slice][word k = input channel of the block]
     uint4 v4[4];
@@ -299,13 +300,16 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_s
     v += __shfl_xor_sync(0xffffffffu, v, 4);
     if (c == 0) sums[warp][st * 4 + r] = v;
   }
-  __syncthreads();
+  if (across > 1)
+    __syncthreads();
+  else
+    __syncwarp();  // (the rows are this warp's alone)
   if (part == 0 && lane < 16) {
     const int o = o0 + lane;
     int32_t v = 0;
     for (int w = 0; w < across; ++w) v += sums[warp + w][lane];
     if (o < a.O && o < a.sum_len) {
-      if (gridDim.y == 1 && gridDim.z == 1)
+      if (beside == 1 && gridDim.z == 1)
         a.sum_i[o] = v;
       else if (v != 0)
         atomicAdd(a.sum_i + o, v);
@@ -585,22 +589,32 @@ int pack_weights_impl(const mld_pack_desc* d, const void* src, void* dst, int32_
                         (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
   if (!rows_fit) MLD_CUDA_CHECK(clear_sums());
   if (rows_fit) {
-    // Warps side by side along a row as far as it has 128 channels for them; blocks beside them only where there are too few
-    // rows to keep the SMs busy (512 rows of 11008: 32 blocks of eight warps otherwise).
-    const int chunks = div_up(a.I, 128);
-    int across_shift = 0;
-    while (across_shift < 3 && (2 << across_shift) <= chunks) ++across_shift;
-    const int rows = 16 * (8 >> across_shift), blocks = div_up(a.dst_slices * 4, rows) * a.HW;
-    const int most = div_up(chunks, 1 << across_shift);
-    int beside = div_up(kPackBlocks, blocks);
-    if (beside > most) beside = most;
-    // (the rows along x, where a grid may have 2^31 blocks: a block has no more than 16 of them)
-    dim3 rgrid(div_up(a.dst_slices * 4, rows), beside, a.HW);
+    // Without sums a warp takes one group of 128 channels: 4096 x 14336 to INT4 18.6 us, 25.0 with blocks that go through whole
+    // rows.  With sums whole rows save the fill (and its wait) ahead of the kernel, which pays where rows are short or many:
+    // 1024 x 4096 to INT4 6.7 us, 8.5 with the fill, 14336 x 4096 21.6 / 22.3, 8192 x 8192 24.8 / 25.6; on the other side 4096 x
+    // 14336 27.3 / 22.7, 2048 x 8192 14.8 / 10.9.  There a warp takes two groups, or one where the blocks would be few (512 x 11008
+    // 9.4 us, 10.4 with two).  Of whole rows eight warps share one, or two where there are thousands of them (151936 x 1024 55.0 /
+    // 46.5 us), or four where that leaves fewer warps without a group in the last turn (14173 x 3120 18.5 / 17.1).
+    const int chunks = div_up(a.I, 128), rows16 = div_up(a.dst_slices * 4, 16) * a.HW;
+    int across_shift = 0, beside = chunks;
+    if (n_sums > 0) {
+      const int idle8 = align_n(chunks, 8) - chunks, idle4 = align_n(chunks, 4) - chunks;
+      const bool many = rows16 >= 1300, uneven = 5 * idle8 > chunks;
+      if (many ? chunks <= 10 || !uneven : chunks <= 40 || rows16 >= 400) {
+        across_shift = many && chunks <= 10 ? 1 : rows16 >= 700 && uneven && idle4 < idle8 ? 2 : 3;
+        while (across_shift > 0 && (1 << across_shift) > chunks) --across_shift;
+        beside = 1;
+      } else if (div_up(rows16, 8) * div_up(chunks, 2) >= 256) {
+        beside = div_up(chunks, 2);
+      }
+    }
+    // (one dimension for both, of up to 2^31 blocks)
+    const dim3 rgrid(div_up(a.dst_slices * 4, 16 * (8 >> across_shift)) * beside, 1, a.HW);
     if (beside > 1 || a.HW > 1) MLD_CUDA_CHECK(clear_sums());
     const bool wide = a.dst_slices % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
     const auto kern = d->bits == 8 ? (wide ? pack_rows_kernel<8, true> : pack_rows_kernel<8, false>)
                                    : (wide ? pack_rows_kernel<4, true> : pack_rows_kernel<4, false>);
-    MLD_CUDA_CHECK(launch_overlapped(kern, rgrid, dim3(256), 0, stream, a, across_shift));
+    MLD_CUDA_CHECK(launch_overlapped(kern, rgrid, dim3(256), 0, stream, a, across_shift, beside));
   } else if (d->source == MLD_SRC_UINT4_PACKED && a.I % 32 == 0 && a.O % 4 == 0 && !a.swap_dims &&
              a.group == a.dst_slices && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
              (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {

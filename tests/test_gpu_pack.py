@@ -213,6 +213,28 @@ def test_pack_rows_sums(mld, oracle, shape, bits):
         assert np.array_equal(sums.cpu().numpy(), oracle.weights_sum_i(q))
 
 
+# with sums: blocks of whole rows shared by eight, four and two warps, rows shared by blocks that take one and two groups of channels;
+# without: a group to a warp.  The layout in plain torch: [I/4][O/4][4 inputs][4 outputs]
+@pytest.mark.parametrize("O,I", [(272, 5120), (11300, 3088), (20820, 640), (20832, 1296), (20832, 2080), (400, 5136), (3000, 5264),
+                                 (6416, 5136), (16, 16), (20800, 16)])
+@pytest.mark.parametrize("bits", [8, 4])
+def test_pack_rows_splits(mld, bits, O, I):
+    lo, hi = (-128, 128) if bits == 8 else (-8, 8)
+    q = torch.randint(lo, hi, (O, I), device="cuda", dtype=torch.int32, generator=torch.Generator("cuda").manual_seed(O + I)).to(torch.int8)
+    O4 = (O + 3) // 4 * 4
+    u = torch.zeros((O4, I), dtype=torch.uint8, device="cuda") + (128 if bits == 8 else 8)
+    u[:O] = (q.to(torch.int16) - lo).to(torch.uint8)
+    want = u.reshape(O4 // 4, 4, I // 4, 4).permute(2, 0, 3, 1).reshape(-1)
+    if bits == 4:
+        want = want[0::2] | want[1::2] << 4
+    for want_sum in (False, True):
+        got, sums = mld.pack_weights(q, (O, 1, 1, I), bits, want_sum=want_sum)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+        if want_sum:
+            assert torch.equal(sums, q.sum(1, dtype=torch.int32))
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 def test_pack_rows_of_a_tall_matrix(mld, bits):
     # more than 65535 blocks of rows (16 to a block from 1024 inputs on); the layout in plain torch: [I/4][O/4][4 inputs][4 outputs]
