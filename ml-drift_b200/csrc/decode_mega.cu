@@ -338,7 +338,7 @@ struct Runs {
 // items (head-major) are split evenly and a CTA may touch several heads.
 struct AttnSplit {
   int nt, I, G, heads, P;
-  __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
+  __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_, int stages) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
     P = G >= heads ? G / heads : 0;
     if (P > kMaxParts) P = kMaxParts;
     // No more parts than give each of a part's warps a tile, while the merging part can read the others in one round: warps
@@ -347,7 +347,7 @@ struct AttnSplit {
     // 8 heads 169.4 / 154.1, 20 heads 221.9 / 202.8; 19 tiles 16 heads 192.7 / 182.0, 24 heads 232.4 / 221.1; 29 tiles 12 heads
     // 185.9 / 174.9; 47 tiles 16 heads 194.8 / 187.6; 16 tiles 32 heads 271.3 / 270.0; with 6 of 8 parts for 63 tiles,
     // 8 heads 168.1 / 172.2.
-    const int needed = (nt + kCW - 1) / kCW;
+    const int each = stages / 2 < kCW ? stages / 2 : kCW, needed = (nt + each - 1) / each;
     if (needed < P && needed <= kOneRound + 1) P = needed;
   }
   __device__ __forceinline__ void range(int cta, int& i0, int& i1) const {
@@ -456,7 +456,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
 #pragma unroll 1
     for (int kind = 0; kind < kOpsPerLayer; ++kind) {
       if (kind == kAttn) {
-        const AttnSplit split(a.heads, nt, G);
+        const AttnSplit split(a.heads, nt, G, a.stages);
         int ai0, ai1;
         split.range(cta, ai0, ai1);
         const Runs runs(ai0, ai1, nt);
@@ -1177,7 +1177,7 @@ __device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
   const int g = lane >> 2, t = lane & 3;
   const int nt = a.pos / kTile + 1;
   const int width = a.heads * kHeadDim;
-  const AttnSplit split(a.heads, nt, G);
+  const AttnSplit split(a.heads, nt, G, a.stages);
   int i0, i1;
   split.range(cta, i0, i1);
   const Runs runs(i0, i1, nt);
