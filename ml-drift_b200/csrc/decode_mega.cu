@@ -341,12 +341,15 @@ struct AttnSplit {
   __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_, int stages) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
     P = G >= heads ? G / heads : 0;
     if (P > kMaxParts) P = kMaxParts;
-    // No more parts than give each of a part's warps a tile, while the merging part can read the others in one round: warps
-    // take up to kCW tiles side by side, and merging costs two trips through L2 (publishing and reading the partials), a
-    // round more a third.  us a step of 8 layers with all 8 (24 heads: 6, 32 heads: 4) parts / as many as needed: 13 tiles
-    // 8 heads 169.4 / 154.1, 20 heads 221.9 / 202.8; 19 tiles 16 heads 192.7 / 182.0, 24 heads 232.4 / 221.1; 29 tiles 12 heads
-    // 185.9 / 174.9; 47 tiles 16 heads 194.8 / 187.6; 16 tiles 32 heads 271.3 / 270.0; with 6 of 8 parts for 63 tiles,
-    // 8 heads 168.1 / 172.2.
+    // No more parts than give each of a part's warps a tile and all of a part's tiles their two stages of the ring, while the
+    // merging part can read the others in one round: warps take up to kCW tiles side by side, and merging costs two trips
+    // through L2 (publishing and reading the partials), a round more a third.  us a step of 8 layers with all 8 (20 heads: 7,
+    // 24 heads: 6) parts / as many as needed: 13 tiles 8 heads 169.4 / 154.1, 20 heads 221.9 / 202.8; 19 tiles 16 heads 192.7 /
+    // 182.0, 24 heads 232.4 / 221.1; 29 tiles 12 heads 185.9 / 174.9; 47 tiles 16 heads 194.8 / 187.6; with 6 of 8 parts for 63
+    // tiles, 8 heads 168.1 / 172.2, with 5 170.6 / 181.0.  Parts of eleven tiles, 22 stages of 21, wait for a stage: 22 tiles in 2 / 3
+    // parts 4 heads 171.3 / 159.2, 6 heads 167.9 / 148.6, 12 heads 184.9 / 174.6.
+    // (Eight parts cost 4 to 6 heads 5 % more than with a flag to a partial; reading seven records in one round, a lane to a
+    // maximum, mends that and costs 24 and 32 heads 1.5 to 3 %.)
     const int each = stages / 2 < kCW ? stages / 2 : kCW, needed = (nt + each - 1) / each;
     if (needed < P && needed <= kOneRound + 1) P = needed;
   }

@@ -110,9 +110,15 @@ def test_decode_step_matches_oracle(mld, oracle, mode, L, heads, ffn, T, pos, bl
     dec.close()
 
 
-# Attention tiles of 32 tokens, the new token's among them: one part up to 11, two up to 22, ... five up to 55, then eight.
+# Attention tiles of 32 tokens, the new token's among them: either side of whole multiples of eleven, a tile to a warp.
 @pytest.mark.parametrize("pos", [351, 352, 703, 704, 1055, 1056, 1407, 1408, 1759, 1760, 2047])
 def test_parts_of_a_head(mld, oracle, pos):
+    test_decode_step_matches_oracle(mld, oracle, "mega", 1, 2, 256, 2048, pos, 32)
+
+
+# ... and of ten, half the ring's stages: one part up to 10, two up to 20, ... five up to 50, then eight
+@pytest.mark.parametrize("pos", [319, 320, 639, 640, 959, 960, 1279, 1280, 1599, 1600])
+def test_parts_of_a_head_by_the_ring(mld, oracle, pos):
     test_decode_step_matches_oracle(mld, oracle, "mega", 1, 2, 256, 2048, pos, 32)
 
 
