@@ -4,6 +4,8 @@
 // (common/task/weights_conversion.cc); these kernels are HBM-bound, so they
 // read rows coalesced, transpose in registers (or, for ragged shapes, through
 // shared memory) and write whole 4x4 blocks with vector stores.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace mld {
@@ -200,20 +202,20 @@ __device__ __forceinline__ void st_global_32b(uint8_t* p, const uint32_t (&a)[4]
 // A lane's run is stored 32 bytes at a time where every run starts on a 32-byte boundary (WIDE: whole groups of four
 // output slices and of 16 outputs): one whole sector per store instead of four quarter-filled requests.  14336 x 4096 to
 // INT4: 47.2 us, 38.3 with these stores, and 16 less with the exchange of words free of branches.
-// 2^across_shift of the block's eight warps lie side by side along the input channels and `beside` blocks, whose numbers follow
-// each other, take turns along them; the other warps take further rows.  The sums of a row's weights stay in registers until a
-// block is through; where one block covers all of a row it writes them, and neither atomics nor a fill ahead of the kernel are
-// needed.
-template <int BITS, bool WIDE>
-__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_shift, int beside) {
+// The sums of a row's weights stay in registers until a warp is through.  WHOLE: a block covers whole rows, 2^split of its eight
+// warps side by side along the input channels, the others on further rows; it writes the sums, and neither atomics nor a fill
+// ahead of the kernel are needed.  Otherwise every warp has rows of its own, and `split` blocks, whose numbers follow each other,
+// take turns along the input channels.  (Two forms: with both as numbers of one, whole rows take 0.7 us of 22 longer.)
+template <int BITS, bool WIDE, bool WHOLE>
+__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int split) {
   pdl_wait();
   __shared__ int32_t sums[8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hw = blockIdx.z;
-  const int across = 1 << across_shift, part = warp & (across - 1);
-  const int row_block = blockIdx.x / beside, turn = blockIdx.x - row_block * beside;
+  const int across = WHOLE ? 1 << split : 1, part = WHOLE ? warp & (across - 1) : 0;
+  const int beside = WHOLE ? 1 : split, row_block = blockIdx.x / beside, turn = blockIdx.x - row_block * beside;
   const int r = lane >> 3, c = lane & 7;                 // row of the step's four, 16-byte chunk of the 128 inputs
-  const int o0 = (row_block * (8 >> across_shift) + (warp >> across_shift)) * 16;  // first of the warp's 16 output rows
+  const int o0 = (WHOLE ? row_block * (8 >> split) + (warp >> split) : row_block * 8 + warp) * 16;  // first of the warp's 16 output rows
   const int8_t* src = reinterpret_cast<const int8_t*>(a.src);
   const uint32_t padw = (a.pad & 0xFFu) * 0x01010101u;
   int32_t rowsum[4] = {0, 0, 0, 0};
@@ -300,7 +302,7 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_s
     v += __shfl_xor_sync(0xffffffffu, v, 4);
     if (c == 0) sums[warp][st * 4 + r] = v;
   }
-  if (across > 1)
+  if constexpr (WHOLE)
     __syncthreads();
   else
     __syncwarp();  // (the rows are this warp's alone)
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs a, int across_s
     int32_t v = 0;
     for (int w = 0; w < across; ++w) v += sums[warp + w][lane];
     if (o < a.O && o < a.sum_len) {
-      if (beside == 1 && gridDim.z == 1)
+      if (WHOLE && gridDim.z == 1)
         a.sum_i[o] = v;
       else if (v != 0)
         atomicAdd(a.sum_i + o, v);
@@ -596,25 +598,30 @@ int pack_weights_impl(const mld_pack_desc* d, const void* src, void* dst, int32_
     // 9.4 us, 10.4 with two).  Of whole rows eight warps share one, or two where there are thousands of them (151936 x 1024 55.0 /
     // 46.5 us), or four where that leaves fewer warps without a group in the last turn (14173 x 3120 18.5 / 17.1).
     const int chunks = div_up(a.I, 128), rows16 = div_up(a.dst_slices * 4, 16) * a.HW;
-    int across_shift = 0, beside = chunks;
+    bool whole = false;
+    int split = chunks;
     if (n_sums > 0) {
       const int idle8 = align_n(chunks, 8) - chunks, idle4 = align_n(chunks, 4) - chunks;
       const bool many = rows16 >= 1300, uneven = 5 * idle8 > chunks;
-      if (many ? chunks <= 10 || !uneven : chunks <= 40 || rows16 >= 400) {
-        across_shift = many && chunks <= 10 ? 1 : rows16 >= 700 && uneven && idle4 < idle8 ? 2 : 3;
-        while (across_shift > 0 && (1 << across_shift) > chunks) --across_shift;
-        beside = 1;
+      whole = many ? chunks <= 10 || !uneven : chunks <= 40 || rows16 >= 400;
+      if (whole) {
+        split = many && chunks <= 10 ? 1 : rows16 >= 700 && uneven && idle4 < idle8 ? 2 : 3;
+        while (split > 0 && (1 << split) > chunks) --split;
       } else if (div_up(rows16, 8) * div_up(chunks, 2) >= 256) {
-        beside = div_up(chunks, 2);
+        split = div_up(chunks, 2);
       }
     }
-    // (one dimension for both, of up to 2^31 blocks)
-    const dim3 rgrid(div_up(a.dst_slices * 4, 16 * (8 >> across_shift)) * beside, 1, a.HW);
-    if (beside > 1 || a.HW > 1) MLD_CUDA_CHECK(clear_sums());
+    // (one dimension for rows and turns, of up to 2^31 blocks)
+    const dim3 rgrid(whole ? div_up(a.dst_slices * 4, 16 * (8 >> split)) : div_up(a.dst_slices * 4, 128) * split, 1, a.HW);
+    if (!whole || a.HW > 1) MLD_CUDA_CHECK(clear_sums());
     const bool wide = a.dst_slices % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
-    const auto kern = d->bits == 8 ? (wide ? pack_rows_kernel<8, true> : pack_rows_kernel<8, false>)
-                                   : (wide ? pack_rows_kernel<4, true> : pack_rows_kernel<4, false>);
-    MLD_CUDA_CHECK(launch_overlapped(kern, rgrid, dim3(256), 0, stream, a, across_shift, beside));
+    const auto form = [&](auto bits, auto w) {
+      return whole ? pack_rows_kernel<bits(), w(), true> : pack_rows_kernel<bits(), w(), false>;
+    };
+    using std::integral_constant;
+    const auto kern = d->bits == 8 ? (wide ? form(integral_constant<int, 8>(), std::true_type()) : form(integral_constant<int, 8>(), std::false_type()))
+                                   : (wide ? form(integral_constant<int, 4>(), std::true_type()) : form(integral_constant<int, 4>(), std::false_type()));
+    MLD_CUDA_CHECK(launch_overlapped(kern, rgrid, dim3(256), 0, stream, a, split));
   } else if (d->source == MLD_SRC_UINT4_PACKED && a.I % 32 == 0 && a.O % 4 == 0 && !a.swap_dims &&
              a.group == a.dst_slices && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
              (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
