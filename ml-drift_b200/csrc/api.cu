@@ -254,13 +254,14 @@ int mld_fc_is_gemv_recommended(int32_t precision, int32_t tokens) {
 // constants means from 200 tokens up.  The same rule with this library's measured costs: a pass costs more the more inputs a
 // channel has, dequantising inside the GEMM a little for every tile of 256 tokens.  us in a graph, inside / converted:
 //   float, K = 8192: 8192 -> 8192 INT4 1024 tokens 117 / 158, 2048 253 / 257, 4096 410 / 440
-//   float, K = 4096: 4096 -> 4096 INT4 1024 tokens 34.7 / 35.2, 2048 60.7 / 65.8, 3072 96 / 89; INT8 63 / 71, 92.5 / 91;
-//     -> 6144 INT4 2048 tokens 89.5 / 90.7, 3072 151 / 133; -> 14336 1024 tokens 97 / 118, 2048 159 / 168 (twenty calls in a row,
-//     under the power cap, 212 / 200), 3072 308 / 284
-//   float, K = 3072: -> 8192 INT4 1024 tokens 47.5 / 56.3, 2048 94 / 90; -> 3072 INT8 28.5 / 32.5, 42.5 / 42.3
-//   float below: 2048 -> 2048 INT4 520 tokens 35.3 / 33.7, 1024 23.9 / 23.2; -> 8192 39.1 / 38.5; 1024 -> 4096 21.8 / 20.2
-//   int8 activations: 8192 -> 28672 2048 tokens 371 / 402, 8192 -> 3584 2048 88 / 96, 4096 152 / 154; 4096 -> 14336 1024
-//     tokens 77 / 87, 2048 129 / 124; 4096 -> 4096 520 tokens 34.3 / 32.2, 1024 36.7 / 36.4
+//   float, K = 4096: 4096 -> 4096 INT4 1024 tokens 36.5 / 37.1, 2048 62 / 67, 3072 90 / 91; INT8 63 / 71, 92.5 / 91;
+//     -> 6144 INT4 2048 tokens 89.5 / 90.7, 3072 151 / 133; -> 14336 1024 tokens 97 / 119, 2048 159 / 168 in a burst, under the
+//     power cap 185 / 199 and as far as 238 / 229, 3072 308 / 284
+//   float, K = 3072: -> 8192 INT4 1024 tokens 49 / 56, 2048 90 / 92; -> 3072 INT8 28.5 / 32.5, 42.5 / 42.3
+//   float below: 2048 -> 2048 INT4 520 tokens 22.4 / 22.0, 1024 23.5 / 23.1; -> 8192 33.9 / 34.8, 40.1 / 39.0; 1024 -> 4096
+//     20.7 / 18.6, 21.2 / 19.8
+//   int8 activations: 8192 -> 28672 2048 tokens 371 / 402, 8192 -> 3584 2048 89 / 95, 4096 152 / 154; 4096 -> 14336 1024
+//     tokens 77 / 87, 2048 129 / 126; 4096 -> 4096 520 tokens 49 to 52 / 46 to 48, 1024 38 to 42 / 38 to 39
 static bool convert_pays(const mld_fc_desc& d, int tokens) {
   int most = 512;
   if (d.prefill_act_quant != 0) {
@@ -703,11 +704,13 @@ int mld::fc_run_internal(mld_fc_plan* plan, const void* src, const void* weights
   const bool streams = plan->stream_ok && aligned && layout_ok && (!d.has_zero_point || zp != nullptr);
   // The streaming kernel beyond the decode rule's tokens.  Up to 16, with exact operands (the GEMM multiplies dequantised
   // weights: inputs that meet zero weights must cost nothing here either), it takes less time than the GEMM where its boxes
-  // are filled or the inputs are few.  us in a graph, streaming / GEMM, 9 and 16 tokens (30 matrices measured for each of
-  // INT4 block 32, INT4 and INT8 per channel): INT4 block 32, 4096 -> 4096 13.6 / 17.5, 14.9 / 17.6; 4096 -> 14336
-  // 29.4 / 33.8, 30.9 / 34.0; 2048 -> 11008 17.5 / 19.7, 18.6 / 19.6; INT8 2048 -> 2048 7.8 / 12.3, 7.9 / 12.3; and on the
-  // other side of the line, with boxes filled to 58 and 65 per cent, 8192 -> 11008 52.5 / 46.2, 53.7 / 46.6; 4096 -> 11008
-  // 29.0 / 28.6, 30.2 / 28.7; 8192 -> 12288 53.6 / 51.4, 54.5 / 51.4.  At 24 tokens it loses (4096 -> 11008: 47 / 29).
+  // are filled or the inputs are few.  us in a graph, streaming / GEMM, 9 and 16 tokens: INT4 block 32, 1024 -> 4096 7.9 / 11.1,
+  // 9.3 / 11.0; 2048 -> 2048 9.7 / 11.6, 10.5 / 11.6; 4096 -> 4096 13.5 / 15.0, 15.1 / 15.4; INT8 2048 -> 2048 7.8 / 12.0, 8.2 /
+  // 12.0; and on the other side of the line, with boxes filled to 58 and 65 per cent, 8192 -> 11008 49.9 / 32.1, 53.8 / 32.0;
+  // 4096 -> 11008 28.1 / 21.6, 30.8 / 21.6; 8192 -> 12288 50.1 / 34.5, 53.9 / 34.5.  The line was drawn with a slower GEMM; by
+  // these figures it lies too far out: with filled boxes and many outputs or inputs the GEMM is the faster one now, 4096 -> 14336
+  // 28.9 / 25.0, 30.5 / 25.1; 8192 -> 8192 31.9 / 27.4, 34.5 / 27.5; 11008 -> 4096 25.9 / 22.6, 27.3 / 22.6; 2048 -> 11008 17.3 /
+  // 16.3, 18.5 / 16.2; INT8 4096 -> 14336 29.8 / 23.2, 30.4 / 23.3.
   // With zero points the alternative is the general kernel (2048 -> 4096, 12 tokens: 48 against 10.4 us), so there it takes
   // as many tokens as two launches hold.
   const bool few = d.force_path == 0 && d.prefill_act_quant == 0 && d.prefill_route == MLD_PREFILL_ROUTE_AUTO &&
