@@ -94,6 +94,7 @@ struct MegaArgs {
   const MegaLayer* layers;
   int n_layers, d_model, heads, ffn, pos;
   int stages;          // ring depth
+  int attn_parts;      // CTAs that share a head (see AttnSplit)
   int xs_bytes;        // shared-memory bytes of the input-vector / attention scratch area
   int us_floats;       // entries of the per-32-input sums of the input vector
   float rms_eps, min_ts, max_ts, q_scale;
@@ -333,26 +334,12 @@ struct Runs {
   }
 };
 
-// A CTA's attention items.  With at least as many CTAs as heads, P = grid / heads CTAs share a head
+// A CTA's attention items.  With at least as many CTAs as heads, P CTAs share a head (see attn_parts)
 // (CTA c: head c / P, tiles [part nt / P, (part + 1) nt / P)) and every CTA has one run; otherwise the
 // items (head-major) are split evenly and a CTA may touch several heads.
 struct AttnSplit {
   int nt, I, G, heads, P;
-  __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_, int stages) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_) {
-    P = G >= heads ? G / heads : 0;
-    if (P > kMaxParts) P = kMaxParts;
-    // No more parts than give each of a part's warps a tile and all of a part's tiles their two stages of the ring, while the
-    // merging part can read the others in one round: warps take up to kCW tiles side by side, and merging costs two trips
-    // through L2 (publishing and reading the partials), a round more a third.  us a step of 8 layers with all 8 (20 heads: 7,
-    // 24 heads: 6) parts / as many as needed: 13 tiles 8 heads 169.4 / 154.1, 20 heads 221.9 / 202.8; 19 tiles 16 heads 192.7 /
-    // 182.0, 24 heads 232.4 / 221.1; 29 tiles 12 heads 185.9 / 174.9; 47 tiles 16 heads 194.8 / 187.6; with 6 of 8 parts for 63
-    // tiles, 8 heads 168.1 / 172.2, with 5 170.6 / 181.0.  Parts of eleven tiles, 22 stages of 21, wait for a stage: 22 tiles in 2 / 3
-    // parts 4 heads 171.3 / 159.2, 6 heads 167.9 / 148.6, 12 heads 184.9 / 174.6.
-    // (Eight parts cost 4 to 6 heads 5 % more than with a flag to a partial; reading seven records in one round, a lane to a
-    // maximum, mends that and costs 24 and 32 heads 1.5 to 3 %.)
-    const int each = stages / 2 < kCW ? stages / 2 : kCW, needed = (nt + each - 1) / each;
-    if (needed < P && needed <= kOneRound + 1) P = needed;
-  }
+  __device__ __forceinline__ AttnSplit(int heads_, int nt_, int G_, int parts) : nt(nt_), I(heads_ * nt_), G(G_), heads(heads_), P(parts) {}
   __device__ __forceinline__ void range(int cta, int& i0, int& i1) const {
     if (P > 0) {
       const int head = cta / P, part = cta - head * P;
@@ -459,7 +446,7 @@ __device__ void producer_loop(const MegaArgs& a, uint8_t* ring, uint64_t* full, 
 #pragma unroll 1
     for (int kind = 0; kind < kOpsPerLayer; ++kind) {
       if (kind == kAttn) {
-        const AttnSplit split(a.heads, nt, G, a.stages);
+        const AttnSplit split(a.heads, nt, G, a.attn_parts);
         int ai0, ai1;
         split.range(cta, ai0, ai1);
         const Runs runs(ai0, ai1, nt);
@@ -1180,7 +1167,7 @@ __device__ __forceinline__ void run_attention(Ctx& c, const MegaLayer* ly) {
   const int g = lane >> 2, t = lane & 3;
   const int nt = a.pos / kTile + 1;
   const int width = a.heads * kHeadDim;
-  const AttnSplit split(a.heads, nt, G, a.stages);
+  const AttnSplit split(a.heads, nt, G, a.attn_parts);
   int i0, i1;
   split.range(cta, i0, i1);
   const Runs runs(i0, i1, nt);
@@ -2208,6 +2195,22 @@ int mega_device_status(MegaDecoder* m, int* code) {
   return MLD_OK;
 }
 
+// How many CTAs share a head (0: fewer CTAs than heads), worked out on the host, once a step.
+// No more parts than give each of a part's warps a tile and all of a part's tiles their two stages of the ring, while the
+// merging part can read the others in one round: warps take up to kCW tiles side by side, and merging costs two trips
+// through L2 (publishing and reading the partials), a round more a third.  us a step of 8 layers with all 8 (20 heads: 7,
+// 24 heads: 6) parts / as many as needed: 13 tiles 8 heads 169.4 / 154.1, 20 heads 221.9 / 202.8; 19 tiles 16 heads 192.7 /
+// 182.0, 24 heads 232.4 / 221.1; 29 tiles 12 heads 185.9 / 174.9; 47 tiles 16 heads 194.8 / 187.6; with 6 of 8 parts for 63
+// tiles, 8 heads 168.1 / 172.2, with 5 170.6 / 181.0.  Parts of eleven tiles, 22 stages of 21, wait for a stage: 22 tiles in 2 / 3
+// parts 4 heads 171.3 / 159.2, 6 heads 167.9 / 148.6, 12 heads 184.9 / 174.6.
+// (Eight parts cost 4 to 6 heads 5 % more than with a flag to a partial; reading seven records in one round, a lane to a
+// maximum, mends that and costs 24 and 32 heads 1.5 to 3 %.)
+static int attn_parts(int heads, int nt, int grid, int stages) {
+  const int most = grid < heads ? 0 : grid / heads < kMaxParts ? grid / heads : kMaxParts;
+  const int each = stages / 2 < kCW ? stages / 2 : kCW, needed = (nt + each - 1) / each;
+  return needed < most && needed <= kOneRound + 1 ? needed : most;
+}
+
 int mega_step(MegaDecoder* m, const void* x_in, void* x_out, int pos, cudaStream_t stream) {
   for (char s : m->layer_set) MLD_REQUIRE(s != 0, "layer weights not set");
   MegaArgs a;
@@ -2235,6 +2238,7 @@ int mega_step(MegaDecoder* m, const void* x_in, void* x_out, int pos, cudaStream
   a.off_xbar = m->off_xbar;
   a.pos = pos;
   a.stages = m->stages;
+  a.attn_parts = attn_parts(m->heads_local, pos / kTile + 1, m->grid, m->stages);
   a.xs_bytes = m->xs_bytes;
   a.us_floats = m->us_floats;
   a.rms_eps = c.rms_eps;
